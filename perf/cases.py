@@ -118,8 +118,8 @@ def draw(rng):
 def _axis_board(seed, w, h, layers, n_nets, pads):
     """A board on non-uniform lines: per-axis gap prices (length x 16), unit
     enter weights, ~10% obstacles; with `pads` also a courtyard mask along the
-    rim, a static via mask, own pads around both endpoints, and one layer
-    transition without vias on boards of more than three layers."""
+    rim, a static via mask, own pads around both endpoints, and no vias into the
+    last layer of a board of more than three (a plane layer without pins)."""
     rng = np.random.default_rng(seed)
     dims = mrcuda.Dims(w, h, layers)
     cost = np.ones((layers, h, w), dtype=np.uint32)
@@ -134,11 +134,12 @@ def _axis_board(seed, w, h, layers, n_nets, pads):
             rim[s] |= mrcuda.BOARD_TRACE_NODE | mrcuda.BOARD_VIA_NODE
         board = rim.reshape(-1)
         via = (rng.random(w * h * layers) < 0.02).astype(np.uint8)
+    closed = pads and layers > 3
     nets = []
     for i in range(n_nets):
         ends, own = [], []
         for _ in range(2):
-            x, y, l = int(rng.integers(4, w - 4)), int(rng.integers(4, h - 4)), int(rng.integers(0, layers))
+            x, y, l = int(rng.integers(4, w - 4)), int(rng.integers(4, h - 4)), int(rng.integers(0, layers - closed))
             ends.append(dims.idx3(x, y, l))
             if pads:  # a 3 x 3 pad; its cells are obstacles to every other net
                 cost[l, y - 1:y + 2, x - 1:x + 2] = mrcuda.OBSTACLE
@@ -149,8 +150,8 @@ def _axis_board(seed, w, h, layers, n_nets, pads):
         nets.append(mrcuda.NetEndpoints(f"a{i}", ends[0], ends[1], own, own[:1] if pads else []))
     grid = mrcuda.Grid(dims, cost.reshape(-1), board, via)
     vias = [80] * (layers - 1)
-    if pads and layers > 3:
-        vias[1] = None
+    if closed:
+        vias[-1] = None
     x = (16 * rng.integers(1, 9, w - 1)).astype(np.uint32)
     y = (16 * rng.integers(1, 9, h - 1)).astype(np.uint32)
     return W.Workload("axis", grid, nets, mrcuda.net_windows(dims, nets), x, y, vias)
