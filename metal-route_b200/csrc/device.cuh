@@ -38,6 +38,8 @@ constexpr uint8_t kStaticVia = 1u << 6;   // Grid::via_forbidden (exemptible by 
 // (board via node, or static via mask without the net's exemption).
 constexpr uint8_t kViaBlocked = 1u << 6;
 
+struct BoardGoal;
+
 struct DevBoard {
     uint32_t w, h, layers;
     uint32_t via_mask;          // bit k: the k <-> k+1 transition is allowed
@@ -54,6 +56,41 @@ struct DevBoard {
     // cell inside each field's range DevField::over_off .. + n_over
     const uint32_t *over_cells;
     const uint4 *over_price;
+    // nullable: lower bounds of the step prices: their head (zeroed before
+    // planes_kernel) and the prefix sums HX[w], HY[h], HV[layers] (goal_kernel)
+    BoardGoal *goal;
+    uint32_t *goal_sums;
+    const uint4 *bound;         // nullable: directed prices no price of this batch is below (default: directed)
+};
+
+// Lower bounds a goal-directed launch prices the rest of a path with.  The
+// remaining price from cell c to the net's target t is at least
+// e * (|HX[xc] - HX[xt]| + |HY[yc] - HY[yt]| + |HV[lc] - HV[lt]|): every path
+// crosses each column gap, row gap and layer transition between the two, each
+// at no less than its cheapest base price times e, the smallest enter weight
+// (at most 1 for a net that enters its own pads).
+struct BoardGoal {
+    uint32_t inv_min_dir;       // ~(smallest directed price), accumulated by planes_kernel from zero
+    uint32_t inv_min_cost;      // ~(smallest enter weight)
+    u64 sum_dir, n_dir;         // of the directed prices from -x: their mean sets the first threshold
+    u64 sum_cost, n_cost;
+    uint32_t min_cost;          // written by goal_kernel: the smallest enter weight,
+    uint32_t min_step;          // the smallest planar base price,
+    uint32_t min_via;           // the smallest via base price
+    float spread;               // and the share of the bound that the first threshold adds
+};
+
+// Search state of one field of a goal-directed launch.  A label at cell c with
+// f = dist + bound(c) above `ub` cannot lie on a cheapest path and is not
+// propagated.  Until the target has a label, improvements with f above `thr`
+// wait (RelaxArgs::tpark) and are released when the field runs dry.
+struct FieldGoal {
+    uint32_t ub;                // dist of the target so far (kMax: not reached)
+    uint32_t thr;
+    uint32_t f0;                // bound from source to target
+    uint32_t phases;            // releases so far
+    uint32_t active;            // tiles of this field queued or held
+    uint32_t pad_[3];
 };
 
 // One field = one net solved inside one window.

@@ -703,8 +703,21 @@ struct mrc_batch {
     uint32_t total_tiles = 0, max_tiles = 0, tile_h = 32, threads = kRelaxThreads, grid = 1;
     size_t smem = 0;
     DBuf d_tover;                  // per tile: holds price overrides of its field (has_over batches)
-    DBuf d_boards, d_fields, d_pads, d_lab, d_tstamp, d_tvisit, d_lists, d_costs, d_lens, d_offsets, d_cells, d_ctl,
-        d_out;
+    DBuf d_boards, d_fields, d_pads, d_lists, d_costs, d_lens, d_offsets, d_cells, d_out;
+    // What a launch starts from, in two blocks so that a reset is two memsets:
+    // zeros (control block, tile stamps, then the queue's ticket tags or the
+    // rounds form's visited words) and ones (the label arena, waiting f per tile;
+    // the rounds form needs no reset of its labels)
+    DBuf d_zero, d_ones;
+    size_t zero_bytes = 0, ones_bytes = 0, o_tstamp = 0, o_tail = 0, o_tpark = 0;
+    Ctl *ctl() const { return d_zero.as<Ctl>(); }
+    uint32_t *tstamp() const { return reinterpret_cast<uint32_t *>(d_zero.as<unsigned char>() + o_tstamp); }
+    u64 *tags() const { return async_q ? reinterpret_cast<u64 *>(d_zero.as<unsigned char>() + o_tail) : nullptr; }
+    uint32_t *tvisit() const {
+        return async_q ? nullptr : reinterpret_cast<uint32_t *>(d_zero.as<unsigned char>() + o_tail);
+    }
+    u64 *lab() const { return d_ones.as<u64>(); }
+    uint32_t *tpark() const { return reinterpret_cast<uint32_t *>(d_ones.as<unsigned char>() + o_tpark); }
     uint32_t launches = 0;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -722,6 +735,11 @@ struct mrc_batch {
     DBuf d_planes, d_pchunks;    // step-price planes of every board, chunk table of their kernel
     DBuf d_tmaps;                // one TMA tensor map per board over its planes (CTA queue form)
     uint64_t n_pchunks = 0;
+    // goal-directed relax (the CTA queue form with price planes, when only paths
+    // and costs are asked for): lower bounds per board, state per field, waiting f per tile
+    bool goal = false;
+    DBuf d_goal, d_fgoal;
+    uint32_t list_cap = 1;       // slots of the tile lists
     // the planes hold prices of the batch's boards, which never change: computed by
     // the first launch after a layout and kept for the launches that follow
     bool planes_valid = false;
@@ -829,13 +847,14 @@ mrc_status batch_layout(mrc_batch *bt, uint32_t tile_h, uint32_t threads) {
     if (toff > 0x7FFFFFFFull) return fail(MRC_ERR_LIMIT, "batch has more than 2^31 tiles");
     bt->total_tiles = (uint32_t)std::max<uint64_t>(toff, 1);
     bt->max_tiles = max_tiles;
+    bt->goal = cta_pl && !(bt->flags & MRC_FLAG_KEEP_FIELDS) && toff >= (uint64_t)kGoalTilesPerSm * ctx->sms;
     int per_sm = 1;
     if (bt->warp) {
         MRC_CUDA(warp_relax_occupancy(&per_sm), "relax occupancy");
     } else {
-        MRC_CUDA(relax_configure(tile_h, threads, bt->smem, bt->async_q, cta_pl, bt->has_over),
+        MRC_CUDA(relax_configure(tile_h, threads, bt->smem, bt->async_q, cta_pl, bt->has_over, bt->goal),
                  "configure relax kernel");
-        MRC_CUDA(relax_occupancy(tile_h, threads, bt->smem, &per_sm, bt->async_q, cta_pl, bt->has_over),
+        MRC_CUDA(relax_occupancy(tile_h, threads, bt->smem, &per_sm, bt->async_q, cta_pl, bt->has_over, bt->goal),
                  "relax occupancy");
     }
     if (per_sm < 1) return fail(MRC_ERR_LIMIT, "relax kernel does not fit on one SM");
@@ -862,6 +881,18 @@ mrc_status batch_layout(mrc_batch *bt, uint32_t tile_h, uint32_t threads) {
         for (size_t k = 0; k < bt->devs.size(); ++k)
             bt->devs[k].planes = reinterpret_cast<uint32_t *>(bt->d_planes.as<unsigned char>() + poff[k]);
         bt->n_pchunks = chunks.back();
+        uint64_t gwords = 0;
+        for (DevBoard &d : bt->devs) {
+            if (bt->goal) gwords += goal_words(d.w, d.h, d.layers);
+        }
+        if (bt->goal) {
+            MRC_TRY(bt->d_goal.get(ctx, gwords * 4, "price bounds"));
+            gwords = 0;
+            for (DevBoard &d : bt->devs) {
+                d.goal_sums = bt->d_goal.as<uint32_t>() + gwords;
+                gwords += goal_words(d.w, d.h, d.layers);
+            }
+        }
         MRC_TRY(upload(ctx, bt->d_pchunks, chunks.data(), chunks.size() * 8, "plane chunk table"));
         if (cta_pl) {
             std::vector<CUtensorMap> maps(bt->devs.size());
@@ -882,13 +913,37 @@ mrc_status batch_layout(mrc_batch *bt, uint32_t tile_h, uint32_t threads) {
         bt->d_tmaps.reset();
         bt->n_pchunks = 0;
     }
-    MRC_TRY(upload(ctx, bt->d_boards, bt->devs.data(), bt->devs.size() * sizeof(DevBoard), "upload board table"));
+    {  // the board table, and behind it the zeroed heads of the price bounds
+        const size_t nb = bt->devs.size(), o_heads = (nb * sizeof(DevBoard) + 255) & ~(size_t)255;
+        std::vector<unsigned char> table(o_heads + (bt->goal ? nb * sizeof(BoardGoal) : 0), 0);
+        MRC_TRY(bt->d_boards.get(ctx, std::max<size_t>(table.size(), 4), "board table"));
+        BoardGoal *heads = reinterpret_cast<BoardGoal *>(bt->d_boards.as<unsigned char>() + o_heads);
+        for (size_t k = 0; k < nb; ++k) bt->devs[k].goal = bt->goal ? heads + k : nullptr;
+        if (nb) std::memcpy(table.data(), bt->devs.data(), nb * sizeof(DevBoard));
+        MRC_CUDA(cudaMemcpyAsync(bt->d_boards.p, table.data(), table.size(), cudaMemcpyHostToDevice, ctx->stream),
+                 "upload board table");
+    }
     MRC_TRY(upload(ctx, bt->d_fields, bt->fields.data(), bt->fields.size() * sizeof(DevField), "upload fields"));
-    MRC_TRY(bt->d_tstamp.get(ctx, (size_t)bt->total_tiles * 4, "tile stamps"));
-    MRC_TRY(bt->d_tvisit.get(ctx, (size_t)bt->total_tiles * 4, "tile flags"));
     if (bt->has_over) MRC_TRY(bt->d_tover.get(ctx, (size_t)bt->total_tiles, "override tile flags"));
     else bt->d_tover.reset();
-    MRC_TRY(bt->d_lists.get(ctx, (size_t)bt->total_tiles * 3 * 8, "tile lists"));
+    // a ring of at least kMinRing slots: a slot comes round again only after that
+    // many more pushes, however few tiles the batch has
+    bt->list_cap = std::max(bt->total_tiles, kMinRing);
+    MRC_TRY(bt->d_lists.get(ctx, (size_t)bt->list_cap * (bt->async_q ? 1 : 3) * 8, "tile lists"));
+    auto up256 = [](size_t v) { return (v + 255) & ~(size_t)255; };
+    bt->o_tstamp = up256(sizeof(Ctl));
+    bt->o_tail = up256(bt->o_tstamp + (size_t)bt->total_tiles * 4);
+    bt->zero_bytes = bt->o_tail + (bt->async_q ? (size_t)bt->list_cap * 8 : (size_t)bt->total_tiles * 4);
+    MRC_TRY(bt->d_zero.get(ctx, bt->zero_bytes, "tile state"));
+    bt->o_tpark = up256(std::max<uint64_t>(bt->total_cells, 1) * 8);
+    bt->ones_bytes = bt->o_tpark + (bt->goal ? (size_t)bt->total_tiles * 4 : 0);
+    MRC_TRY(bt->d_ones.get(ctx, bt->ones_bytes, "labels"));
+    if (bt->goal) {
+        MRC_TRY(bt->d_fgoal.get(ctx, std::max<size_t>(bt->fields.size(), 1) * sizeof(FieldGoal), "field goals"));
+    } else {
+        bt->d_goal.reset();
+        bt->d_fgoal.reset();
+    }
     return MRC_OK;
 }
 
@@ -970,12 +1025,10 @@ mrc_status batch_build(mrc_context *ctx, std::vector<const mrc_board *> boards, 
     for (const mrc_board *b : bt->boards) bt->devs.push_back(b->dev);
     MRC_TRY(batch_layout(bt, tile_h, threads));
     MRC_TRY(upload(ctx, bt->d_pads, pads.data(), pads.size() * 4, "upload pads"));
-    MRC_TRY(bt->d_lab.get(ctx, std::max<uint64_t>(off, 1) * 8, "labels"));
     MRC_TRY(bt->d_costs.get(ctx, std::max<size_t>(n, 1) * 4, "costs"));
     MRC_TRY(bt->d_lens.get(ctx, std::max<size_t>(n, 1) * 4, "lengths"));
     MRC_TRY(bt->d_offsets.get(ctx, ((size_t)n + 1) * 8, "offsets"));
     MRC_TRY(bt->d_cells.get(ctx, std::max<uint64_t>(off, 1) * 4, "path cells"));
-    MRC_TRY(bt->d_ctl.get(ctx, sizeof(Ctl), "control block"));
     if (flags & MRC_FLAG_KEEP_FIELDS) MRC_TRY(bt->d_out.get(ctx, std::max<uint64_t>(off, 1) * 4, "fields"));
     if (flags & MRC_FLAG_TIME_KERNELS) {
         MRC_CUDA(cudaEventCreate(&bt->ev0), "create event");
@@ -990,8 +1043,8 @@ PathArgs path_args(const mrc_batch *bt) {
     pa.fields = bt->d_fields.as<DevField>();
     pa.n_fields = (uint32_t)bt->fields.size();
     pa.pads = bt->d_pads.as<uint32_t>();
-    pa.lab = bt->d_lab.as<u64>();
-    pa.tvisit = bt->d_tvisit.as<uint32_t>();
+    pa.lab = bt->lab();
+    pa.tvisit = bt->tvisit();
     pa.tover = bt->has_over ? bt->d_tover.as<uint8_t>() : nullptr;
     pa.tile_h = bt->tile_h;
     pa.arena_filled = bt->async_q ? 1u : 0u;
@@ -1002,8 +1055,22 @@ PathArgs path_args(const mrc_batch *bt) {
     pa.lens = bt->d_lens.as<uint32_t>();
     pa.offsets = bt->d_offsets.as<unsigned long long>();
     pa.cells = bt->d_cells.as<uint32_t>();
-    pa.status = &bt->d_ctl.as<Ctl>()->status;
+    pa.status = &bt->ctl()->status;
     return pa;
+}
+
+// Step-price planes of the batch's boards and, for a goal-directed batch, the
+// lower bounds made from the minima that kernel accumulates.
+mrc_status planes_enqueue(mrc_batch *bt, cudaStream_t st, uint32_t *launches) {
+    MRC_CUDA(planes_launch(bt->d_boards.as<DevBoard>(), bt->d_pchunks.as<uint64_t>(), (uint32_t)bt->devs.size(),
+                           bt->n_pchunks, (uint32_t)bt->ctx->sms, st),
+             "launch step-price planes");
+    *launches += 1;
+    if (bt->goal) {
+        MRC_CUDA(goal_launch(bt->d_boards.as<DevBoard>(), (uint32_t)bt->devs.size(), st), "launch price bounds");
+        *launches += 1;
+    }
+    return MRC_OK;
 }
 
 // The launch sequence of one batch: reset, relax, paths (+ fields).
@@ -1012,18 +1079,16 @@ PathArgs path_args(const mrc_batch *bt) {
 mrc_status batch_enqueue(mrc_batch *bt, cudaStream_t st, bool capturing) {
     const uint32_t n = (uint32_t)bt->fields.size();
     uint32_t launches = 0;
-    MRC_CUDA(cudaMemsetAsync(bt->d_ctl.p, 0, sizeof(Ctl), st), "reset control block");
-    MRC_CUDA(cudaMemsetAsync(bt->d_tstamp.p, 0, (size_t)bt->total_tiles * 4, st), "reset tile stamps");
-    MRC_CUDA(cudaMemsetAsync(bt->d_tvisit.p, 0, (size_t)bt->total_tiles * 4, st), "reset tile flags");
+    MRC_CUDA(cudaMemsetAsync(bt->d_zero.p, 0, bt->zero_bytes, st), "reset tile state");
     RelaxArgs ra{};
     ra.boards = bt->d_boards.as<DevBoard>();
     ra.max_layers = bt->max_layers;
     ra.fields = bt->d_fields.as<DevField>();
     ra.n_fields = n;
     ra.pads = bt->d_pads.as<uint32_t>();
-    ra.lab = bt->d_lab.as<u64>();
-    ra.tstamp = bt->d_tstamp.as<uint32_t>();
-    ra.tvisit = bt->d_tvisit.as<uint32_t>();
+    ra.lab = bt->lab();
+    ra.tstamp = bt->tstamp();
+    ra.tvisit = bt->tvisit();
     ra.tover = nullptr;
     if (bt->has_over && n) {
         MRC_CUDA(cudaMemsetAsync(bt->d_tover.p, 0, (size_t)bt->total_tiles, st), "reset override tile flags");
@@ -1034,25 +1099,23 @@ mrc_status batch_enqueue(mrc_batch *bt, cudaStream_t st, bool capturing) {
         ra.tover = bt->d_tover.as<uint8_t>();
     }
     ra.lists = bt->d_lists.as<u64>();
-    ra.list_cap = bt->total_tiles;
-    ra.ctl = bt->d_ctl.as<Ctl>();
+    ra.tags = bt->tags();
+    ra.list_cap = bt->list_cap;
+    if (bt->goal) {
+        ra.goal = bt->d_fgoal.as<FieldGoal>();
+        ra.tpark = bt->tpark();
+    }
+    ra.ctl = bt->ctl();
     ra.tile_h = bt->tile_h;
     ra.round_limit = 64u * bt->max_tiles + 4096u;
     ra.activation_limit = 1024ull * bt->total_tiles + 65536ull;  // runaway guard, far above any measured need
-    if (n && bt->async_q) {
-        MRC_CUDA(cudaMemsetAsync(bt->d_lab.p, 0xFF, bt->total_cells * 8, st), "fill label arena");
-        MRC_CUDA(cudaMemsetAsync(bt->d_lists.as<u64>() + bt->total_tiles, 0, (size_t)bt->total_tiles * 8, st),
-                 "reset queue tags");
-    }
+    if (n && bt->async_q) MRC_CUDA(cudaMemsetAsync(bt->d_ones.p, 0xFF, bt->ones_bytes, st), "fill label arena");
     if (n) {
         const unsigned rec = capturing ? cudaEventRecordExternal : cudaEventRecordDefault;
         if (bt->ev0) MRC_CUDA(cudaEventRecordWithFlags(bt->ev0, st, rec), "record event");
         const bool cta_pl = bt->async_q && !bt->warp && bt->cta_planes;
         if ((bt->warp || cta_pl) && !bt->planes_valid) {
-            MRC_CUDA(planes_launch(bt->d_boards.as<DevBoard>(), bt->d_pchunks.as<uint64_t>(),
-                                   (uint32_t)bt->devs.size(), bt->n_pchunks, (uint32_t)bt->ctx->sms, st),
-                     "launch step-price planes");
-            launches += 1;
+            MRC_TRY(planes_enqueue(bt, st, &launches));
             // a captured graph recomputes them on every replay (it is captured with
             // valid planes, see mrc_batch_capture_graph, so this is the fallback)
             if (!capturing) bt->planes_valid = true;
@@ -1061,7 +1124,7 @@ mrc_status batch_enqueue(mrc_batch *bt, cudaStream_t st, bool capturing) {
             MRC_CUDA(warp_relax_launch(ra, bt->grid, st), "launch relax kernel");
             launches += 2;  // seeds, relax
         } else {
-            MRC_CUDA(relax_launch(ra, bt->grid, bt->threads, bt->smem, st, bt->async_q, cta_pl, bt->has_over),
+            MRC_CUDA(relax_launch(ra, bt->grid, bt->threads, bt->smem, st, bt->async_q, cta_pl, bt->has_over, bt->goal),
                      "launch relax kernel");
             launches += bt->async_q ? 2 : 1;  // (+ the seed kernel)
         }
@@ -1101,7 +1164,7 @@ mrc_status batch_collect(mrc_batch *bt, bool keep_fields, std::vector<uint32_t> 
     cudaStream_t st = bt->stream;
     const uint32_t n = (uint32_t)bt->fields.size();
     uint32_t status = 0;
-    MRC_CUDA(cudaMemcpyAsync(&status, &bt->d_ctl.as<Ctl>()->status, 4, cudaMemcpyDeviceToHost, st), "read status");
+    MRC_CUDA(cudaMemcpyAsync(&status, &bt->ctl()->status, 4, cudaMemcpyDeviceToHost, st), "read status");
     std::vector<uint64_t> off(n + 1);
     costs->assign(n, kMax);
     if (n) MRC_CUDA(cudaMemcpyAsync(costs->data(), bt->d_costs.p, (size_t)n * 4, cudaMemcpyDeviceToHost, st), "read costs");
@@ -1556,9 +1619,8 @@ mrc_status mrc_batch_capture_graph(mrc_context *ctx, mrc_batch *batch) {
     // every replay of this layout
     const bool cta_pl = batch->async_q && !batch->warp && batch->cta_planes;
     if ((batch->warp || cta_pl) && !batch->planes_valid && !batch->fields.empty()) {
-        MRC_CUDA(planes_launch(batch->d_boards.as<DevBoard>(), batch->d_pchunks.as<uint64_t>(),
-                               (uint32_t)batch->devs.size(), batch->n_pchunks, (uint32_t)ctx->sms, ctx->stream),
-                 "launch step-price planes");
+        uint32_t launches = 0;
+        MRC_TRY(planes_enqueue(batch, ctx->stream, &launches));
         MRC_CUDA(cudaStreamSynchronize(ctx->stream), "step-price planes");
         batch->planes_valid = true;
     }
@@ -1721,7 +1783,7 @@ mrc_status mrc_batch_stats(const mrc_batch *batch, uint64_t out[4]) {
     if (!batch || !out) return fail(MRC_ERR_INVALID_ARGUMENT, "NULL argument");
     Ctl c;
     std::memset(&c, 0, sizeof(c));
-    if (batch->d_ctl.p) MRC_CUDA(cudaMemcpy(&c, batch->d_ctl.p, sizeof(Ctl), cudaMemcpyDeviceToHost), "read counters");
+    if (batch->d_zero.p) MRC_CUDA(cudaMemcpy(&c, batch->ctl(), sizeof(Ctl), cudaMemcpyDeviceToHost), "read counters");
     out[0] = c.activations;
     out[1] = c.sweeps;
     out[2] = batch->warp ? c.rows : c.rounds;
@@ -2090,12 +2152,14 @@ mrc_status mrc_negotiation_route(mrc_context *ctx, mrc_negotiation *ng, mrc_roun
             }
             ng->snap->dev.over_cells = ng->d_over_cells.as<uint32_t>();
             ng->snap->dev.over_price = ng->d_over_price.as<uint4>();
+            ng->snap->dev.bound = ng->base->dev.directed;  // a net's own prices may lie below the snapshot's
         }
         mrc_result *raw = nullptr;
         const mrc_status rs =
             solve(ctx, {ng->snap.get()}, std::move(nets), std::move(wins), MRC_FLAG_RETRY_FULL, &raw, nullptr);
         ng->snap->dev.over_cells = nullptr;
         ng->snap->dev.over_price = nullptr;
+        ng->snap->dev.bound = nullptr;
         MRC_TRY(rs);
         std::unique_ptr<mrc_result> res(raw);
         if (ng->clear) {  // the routed nets' old copper and footprints leave before the new ones enter

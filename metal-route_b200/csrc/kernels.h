@@ -13,6 +13,14 @@ namespace mrc {
 constexpr int kRelaxThreads = 256;  // default CTA width of the relax kernel
 constexpr uint64_t kTilesPerCta = 8;  // tiles per CTA at which a queue launch can use one more CTA
 constexpr uint32_t kCountBatch = 64;    // activations a queue CTA counts locally before adding them to the launch's
+constexpr uint32_t kMinRing = 4096;     // fewest slots of the tile queue
+// Tiles per SM from which a batch that asks for paths only is solved goal-directed.
+// Smaller ones wait on one field's chain of tiles, where the limits cost more
+// than the tiles they save (40 two-pin nets on 201x160: 0.99 x, 48 nets with
+// pads on 233x187x4: 0.93 x); larger ones are bound by the tiles themselves
+// (640 uneven instances: 1.54 x, 160 long nets on 1280x1153x6: 1.55 x).
+constexpr uint32_t kGoalTilesPerSm = 64;
+constexpr uint32_t kGoalPhases = 4;     // releases of waiting tiles by threshold before all of them go
 constexpr uint32_t kContinueLimit = 4;  // activations of one held tile before it goes back to the queue
 
 // Status bits reported through Ctl::status / PathArgs::status.
@@ -30,11 +38,14 @@ struct RelaxArgs {
     const uint32_t *pads;       // sorted pad lists, indexed by DevField offsets
     u64 *lab;                   // label arena (dist << 32 | hops)
     uint32_t *tstamp;           // per tile: last round it was queued for, + 1 (zeroed)
-    uint32_t *tvisit;           // per tile: labels valid (zeroed)
+    uint32_t *tvisit;           // rounds form: per tile, labels valid (zeroed)
     const uint8_t *tover;       // nullable: per tile, 1 = its field has directed-price overrides inside it
-    u64 *lists;                 // 3 rotating lists of (field << 32 | tile)
-    uint32_t list_cap;          // total tiles of the batch
+    u64 *lists;                 // 3 rotating lists of (field << 32 | tile); queue form: the ring of items
+    u64 *tags;                  // queue form: ticket tags of the ring (zeroed)
+    uint32_t list_cap;          // entries of one list (at least the batch's tiles)
     Ctl *ctl;                   // zeroed before launch
+    FieldGoal *goal;            // goal-directed launches: per field (written by the seed kernel)
+    uint32_t *tpark;            // goal-directed: per tile, the smallest f waiting to enter it (0xFF filled)
     uint32_t tile_h;            // 32, 16 or 8
     uint32_t round_limit;       // guard on the number of rounds
     unsigned long long activation_limit;  // guard on tile activations (asynchronous form)
@@ -226,6 +237,12 @@ __host__ __device__ inline size_t walk_smem_bytes(uint32_t layers, uint32_t tile
 // tensor map over the planes has 16-byte strides.
 __host__ __device__ inline uint32_t planes_pitch(uint32_t w) { return (w + 3u) & ~3u; }
 uint64_t planes_chunks(uint64_t cells);
+// Words of one board's prefix sums (DevBoard::goal_sums); goal_launch makes them
+// of the minima that planes_launch accumulated into the zeroed heads.
+inline uint64_t goal_words(uint32_t w, uint32_t h, uint32_t layers) {
+    return ((uint64_t)w + h + layers + 31) & ~(uint64_t)31;
+}
+cudaError_t goal_launch(const DevBoard *boards, uint32_t n_boards, cudaStream_t st);
 cudaError_t planes_launch(const DevBoard *boards, const uint64_t *chunk_start, uint32_t n_boards, uint64_t n_chunks,
                           uint32_t sms, cudaStream_t st);
 
@@ -235,16 +252,18 @@ size_t relax_smem_bytes(uint32_t layers, uint32_t tile_h, bool directed, bool pl
 // The relax kernel is instantiated for threads in {128, 256} per CTA.
 // `async` selects the queue-driven form (relax_async_kernel) over the
 // bulk-synchronous rounds (relax_rounds_kernel); the async form needs the label
-// arena filled with 0xFF and the queue tags (lists[cap, 2 cap)) zeroed.
+// arena filled with 0xFF and the queue tags zeroed.
 // over: the fields carry directed-price overrides (DevField::n_over); those
 // kernels exist for kOverTileH-row tiles and kOverThreads threads only.
 constexpr uint32_t kOverTileH = 8, kOverThreads = 256;
+// goal: the goal-directed form of the queue kernel with price planes (paths and
+// costs only, RelaxArgs::goal).
 cudaError_t relax_configure(uint32_t tile_h, uint32_t threads, size_t smem, bool async = false, bool planes = false,
-                            bool over = false);
+                            bool over = false, bool goal = false);
 cudaError_t relax_occupancy(uint32_t tile_h, uint32_t threads, size_t smem, int *blocks_per_sm, bool async = false,
-                            bool planes = false, bool over = false);
+                            bool planes = false, bool over = false, bool goal = false);
 cudaError_t relax_launch(const RelaxArgs &a, uint32_t grid, uint32_t threads, size_t smem, cudaStream_t st,
-                         bool async = false, bool planes = false, bool over = false);
+                         bool async = false, bool planes = false, bool over = false, bool goal = false);
 // tover[f.tile_off + t] = 1 for every tile t of every field that holds one of
 // the field's directed-price overrides (tover zeroed before).
 cudaError_t mark_over_tiles_launch(const DevField *fields, uint32_t n_fields, const DevBoard *boards, uint32_t tile_h,

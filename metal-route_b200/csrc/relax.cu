@@ -91,7 +91,9 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // at -x, +x, -y, +y, the layer below and the layer above.
 enum { kFromNegX = 0, kFromPosX = 1, kFromNegY = 2, kFromPosY = 3, kFromBelow = 4, kFromAbove = 5 };
 
-template <int TH, bool FB>  // FB: fell marks as bytes (the price-plane kernels)
+// FB: fell marks as bytes (the price-plane kernels).  GD: goal-directed, labels
+// whose bound f = dist + remaining price exceeds `ub` are not kept.
+template <int TH, bool FB, bool GD>
 struct Tile {
     u64 *lab;        // [L][TH+2][34] labels with a one-cell halo ring
     uint32_t *st;    // [6][L][TH][sp] step prices into interior cells (column x at sp-offset xo + x)
@@ -103,6 +105,18 @@ struct Tile {
     uint8_t *fl;     // [L][TH+2][kFlPitch] board flag bytes of the tile and its halo (computed prices only)
     uint32_t L;
     uint32_t sp, xo; // price row pitch and column offset: 32, 0 computed; kPlaneTmaBoxW, tx0 & 3 from the planes
+    const uint32_t *hx, *hy, *hl;  // GD: remaining price along each axis, by staged column, staged row and layer
+    uint32_t ub;                   // GD: no cheapest path has a larger f
+    // f of a label with this dist at staged (l, sy, sx): at most kCap, and equal to
+    // the dist's own saturation rule (a sum that reaches kMax is unreachable)
+    __device__ __forceinline__ uint32_t bound(uint32_t dist, uint32_t l, uint32_t sy, uint32_t sx) const {
+        return min(dsum(dsum(dist, hx[sx]), dsum(hy[sy], hl[l])), kCap);
+    }
+    // is a label worth keeping (interior cell)
+    __device__ __forceinline__ bool within(u64 lab_v, uint32_t l, uint32_t y, uint32_t x) const {
+        if constexpr (GD) return bound((uint32_t)(lab_v >> 32), l, y + 1, x + 1) <= ub;
+        else return true;
+    }
     __device__ __forceinline__ uint32_t li(uint32_t l, uint32_t sy, uint32_t sx) const {
         return (l * (TH + 2) + sy) * kLabPitch + sx;
     }
@@ -137,6 +151,7 @@ struct Tile {
 // f(t) = min(A, t (+) (D, H)) with a Kogge-Stone scan (H, the hop count, is the
 // group's cell count), and every cell takes min(local, incoming (+) prefix).
 // `halo(line, &before, &after)` gives the label indices outside both ends;
+// `keep(line, pos, label)` says whether a lower label is worth storing and
 // `touch(line, pos)` marks the crossing lines of a cell whose label fell.
 // Both directions of a line run in one pass: the forward scan, then, on its
 // results still in registers, the backward scan (mirror image: shuffles down,
@@ -144,9 +159,9 @@ struct Tile {
 // backward scan, so one load and one store of each label serve both.  `cell(line, pos, &lab,
 // &step_fwd, &step_bwd)`: step_fwd prices the move into the cell from its
 // predecessor in traversal order, step_bwd the move from its successor.
-template <int K, int S, class CellFn, class HaloFn, class TouchFn>
+template <int K, int S, class CellFn, class HaloFn, class KeepFn, class TouchFn>
 __device__ __forceinline__ bool seg_pass(u64 *lab, const uint32_t *st, uint8_t *dirty, uint32_t nlines, CellFn cell,
-                                          HaloFn halo, TouchFn touch) {
+                                          HaloFn halo, KeepFn keep, TouchFn touch) {
     bool changed = false;
     const uint32_t lanes_total = nlines * S;
     for (uint32_t base = 0; base < lanes_total; base += blockDim.x) {
@@ -235,7 +250,7 @@ __device__ __forceinline__ bool seg_pass(u64 *lab, const uint32_t *st, uint8_t *
         }
 #pragma unroll
         for (int i = 0; i < K; ++i) {
-            if (u[i] < v[i]) {
+            if (u[i] < v[i] && keep(line, seg * K + i, u[i])) {
                 lab[li[i]] = u[i];
                 touch(line, seg * K + i);
                 changed = true;
@@ -290,8 +305,8 @@ __device__ __forceinline__ bool via_blocked(const DevField &f, const uint32_t *p
     return (cell_tile_flags(f, pads, gcell, gf) & kViaBlocked) != 0;
 }
 
-template <int TH, bool FB>
-__device__ __forceinline__ bool stack_pass(const Tile<TH, FB> &t);
+template <int TH, bool FB, bool GD>
+__device__ __forceinline__ bool stack_pass(const Tile<TH, FB, GD> &t);
 
 // With 8-row tiles and 4 cells per lane, the row lanes of a layer (8 rows x 8
 // lanes) and its column lanes (32 columns x 2 lanes) fall on the same pair of
@@ -303,8 +318,8 @@ __device__ __forceinline__ void pair_barrier() {
 }
 
 // The row and the column pass of a sweep on their own (the reversed sweep's).
-template <int TH, bool FB>
-__device__ __forceinline__ bool row_pass(const Tile<TH, FB> &t) {
+template <int TH, bool FB, bool GD>
+__device__ __forceinline__ bool row_pass(const Tile<TH, FB, GD> &t) {
     constexpr int KC = kLaneCells, SR = 32 / KC;  // cells per lane, lanes per row
     return seg_pass<KC, SR>(
         t.lab, t.st, t.rowd, t.L * TH,
@@ -318,11 +333,12 @@ __device__ __forceinline__ bool row_pass(const Tile<TH, FB> &t) {
             *hf = t.li(line / TH, line % TH + 1, 0);
             *hb = t.li(line / TH, line % TH + 1, 33);
         },
+        [&](uint32_t line, uint32_t pos, u64 v) { return t.within(v, line / TH, line % TH, pos); },
         [&](uint32_t line, uint32_t pos) { t.touched_by_row(line / TH, line % TH, pos); });
 }
 
-template <int TH, bool FB>
-__device__ __forceinline__ bool col_pass(const Tile<TH, FB> &t) {
+template <int TH, bool FB, bool GD>
+__device__ __forceinline__ bool col_pass(const Tile<TH, FB, GD> &t) {
     constexpr int KC = kLaneCells, SC = TH / KC;  // cells per lane, lanes per column
     return seg_pass<KC, SC>(
         t.lab, t.st, t.cold, t.L * 32,
@@ -336,6 +352,7 @@ __device__ __forceinline__ bool col_pass(const Tile<TH, FB> &t) {
             *hf = t.li(line / 32, 0, line % 32 + 1);
             *hb = t.li(line / 32, TH + 1, line % 32 + 1);
         },
+        [&](uint32_t line, uint32_t pos, u64 v) { return t.within(v, line / 32, pos, line % 32); },
         [&](uint32_t line, uint32_t pos) { t.touched_by_col(line / 32, pos, line % 32); });
 }
 
@@ -352,8 +369,8 @@ __device__ __forceinline__ void plane_barrier() {
 // One sweep of a staged tile: rows (8 lanes x 4 cells), columns (TH/4 lanes x
 // 4 cells), layer stacks (one thread each), each forward then backward, only
 // over lines whose dirty flag is set.
-template <int TH, bool FB>
-__device__ __forceinline__ bool relax_tile(const Tile<TH, FB> &t) {
+template <int TH, bool FB, bool GD>
+__device__ __forceinline__ bool relax_tile(const Tile<TH, FB, GD> &t) {
     constexpr int KC = kLaneCells;          // cells per lane in a line pass
     constexpr int SR = 32 / KC, SC = TH / KC;  // lanes per row / per column
     const uint32_t L = t.L;
@@ -370,6 +387,7 @@ __device__ __forceinline__ bool relax_tile(const Tile<TH, FB> &t) {
             *hf = t.li(line / TH, line % TH + 1, 0);
             *hb = t.li(line / TH, line % TH + 1, 33);
         },
+        [&](uint32_t line, uint32_t pos, u64 v) { return t.within(v, line / TH, line % TH, pos); },
         [&](uint32_t line, uint32_t pos) { t.touched_by_row(line / TH, line % TH, pos); });
     // rows -> columns: only the warps of the same layers exchange data
     if constexpr (TH == 8 && kLaneCells == 4) {
@@ -389,35 +407,36 @@ __device__ __forceinline__ bool relax_tile(const Tile<TH, FB> &t) {
             *hf = t.li(line / 32, 0, line % 32 + 1);
             *hb = t.li(line / 32, TH + 1, line % 32 + 1);
         },
+        [&](uint32_t line, uint32_t pos, u64 v) { return t.within(v, line / 32, pos, line % 32); },
         [&](uint32_t line, uint32_t pos) { t.touched_by_col(line / 32, pos, line % 32); });
     if (L > 1) {
         __syncthreads();
-        ch |= stack_pass<TH, FB>(t);
+        ch |= stack_pass(t);
     }
     return ch;
 }
 
 // Columns first, then rows and stacks: the queue form's order (fewer sweeps per
 // activation than rows first on its 32 x 8 tiles).
-template <int TH, bool FB>
-__device__ __forceinline__ bool relax_tile_cols_first(const Tile<TH, FB> &t) {
+template <int TH, bool FB, bool GD>
+__device__ __forceinline__ bool relax_tile_cols_first(const Tile<TH, FB, GD> &t) {
     bool ch = col_pass(t);
     plane_barrier<TH>();
     ch |= row_pass(t);
     if (t.L > 1) {
         __syncthreads();
-        ch |= stack_pass<TH, FB>(t);
+        ch |= stack_pass(t);
     }
     return ch;
 }
 
 // The same passes in the opposite order (stacks, columns, rows); the rounds
 // form alternates the two orders between sweeps.
-template <int TH, bool FB>
-__device__ __forceinline__ bool relax_tile_rev(const Tile<TH, FB> &t) {
+template <int TH, bool FB, bool GD>
+__device__ __forceinline__ bool relax_tile_rev(const Tile<TH, FB, GD> &t) {
     bool ch = false;
     if (t.L > 1) {
-        ch = stack_pass<TH, FB>(t);
+        ch = stack_pass(t);
         __syncthreads();
     }
     ch |= col_pass(t);
@@ -432,8 +451,8 @@ __device__ __forceinline__ bool relax_tile_rev(const Tile<TH, FB> &t) {
 // shared memory.
 constexpr uint32_t kStackRegs = 4;
 
-template <int TH, bool FB>
-__device__ __forceinline__ bool stack_pass(const Tile<TH, FB> &t) {
+template <int TH, bool FB, bool GD>
+__device__ __forceinline__ bool stack_pass(const Tile<TH, FB, GD> &t) {
     const uint32_t L = t.L;
     bool ch = false;
     for (uint32_t r = threadIdx.x; r < TH * 32; r += blockDim.x) {
@@ -451,7 +470,7 @@ __device__ __forceinline__ bool stack_pass(const Tile<TH, FB> &t) {
             for (uint32_t l = 0; l < kStackRegs; ++l) {
                 if (l < L) {
                     const u64 w = ext2(prev, l ? t.st[t.si(kFromBelow, l, y, x)] : kMax, 1);
-                    if (w < v[l]) {
+                    if (w < v[l] && t.within(w, l, y, x)) {
                         v[l] = w;
                         fell |= 1u << l;
                     }
@@ -463,7 +482,7 @@ __device__ __forceinline__ bool stack_pass(const Tile<TH, FB> &t) {
             for (int l = (int)kStackRegs - 1; l >= 0; --l) {
                 if ((uint32_t)l < L) {
                     const u64 w = ext2(prev, (uint32_t)l + 1 < L ? t.st[t.si(kFromAbove, (uint32_t)l, y, x)] : kMax, 1);
-                    if (w < v[l]) {
+                    if (w < v[l] && t.within(w, (uint32_t)l, y, x)) {
                         v[l] = w;
                         fell |= 1u << l;
                     }
@@ -485,7 +504,7 @@ __device__ __forceinline__ bool stack_pass(const Tile<TH, FB> &t) {
             const uint32_t c = t.li(l, y + 1, x + 1);
             const u64 cur = t.lab[c];
             const u64 w = umin64(cur, ext2(prev, l ? t.st[t.si(kFromBelow, l, y, x)] : kMax, 1));
-            if (w < cur) {
+            if (w < cur && t.within(w, l, y, x)) {
                 t.lab[c] = w;
                 t.touched_by_stack(l, y, x);
                 ch = true;
@@ -498,7 +517,7 @@ __device__ __forceinline__ bool stack_pass(const Tile<TH, FB> &t) {
             const u64 cur = t.lab[c];
             const u64 w =
                 umin64(cur, ext2(prev, (uint32_t)l + 1 < L ? t.st[t.si(kFromAbove, (uint32_t)l, y, x)] : kMax, 1));
-            if (w < cur) {
+            if (w < cur && t.within(w, (uint32_t)l, y, x)) {
                 t.lab[c] = w;
                 t.touched_by_stack((uint32_t)l, y, x);
                 ch = true;
@@ -569,13 +588,17 @@ static __device__ __noinline__ void stage_overrides(const DevBoard &b, const Dev
 // OV: the batch carries per-net directed-price overrides (negotiation with a
 // clearance; always 8-row tiles, 256 threads); without it none of the override
 // lookups is compiled in.
-template <int TH, bool ASYNC, bool PL, bool OV>
-__device__ __forceinline__ void process_item(const RelaxArgs &a, uint32_t fi, uint32_t t, uint32_t round,
+// GD (with PL): goal-directed (FieldGoal); returns true when this item was the
+// last one of its field in flight, which the caller then releases or ends.
+template <int TH, bool ASYNC, bool PL, bool OV, bool GD>
+__device__ __forceinline__ bool process_item(const RelaxArgs &a, uint32_t fi, uint32_t t, uint32_t round,
                                              unsigned char *smem_raw, uint64_t *mbar, uint32_t &tma_phase,
                                              unsigned long long *s_cnt) {
     const uint32_t SW = kTW + 2, SH = TH + 2;
-    Tile<TH, PL> tile;
+    Tile<TH, PL, GD> tile;
     __shared__ uint32_t s_push[4];
+    __shared__ uint32_t s_park[4];                    // GD: smallest f that enters each neighbour above the threshold
+    __shared__ uint32_t s_hx[kTW + 2], s_hy[TH + 2], s_hl[32], s_lim[2];
     __shared__ uint32_t s_vis[5];  // self, left, right, top, bottom
     __shared__ uint32_t s_pads[kPadCache], s_vpads[kVPadCache];
     Ctl *ctl = a.ctl;
@@ -613,11 +636,14 @@ __device__ __forceinline__ void process_item(const RelaxArgs &a, uint32_t fi, ui
     const uint32_t tw = min(kTW, f.ww - txi * kTW), th = min(TH, f.wh - tyi * TH);
     const int wx0 = (int)f.x0, wy0 = (int)f.y0, wx1 = (int)(f.x0 + f.ww), wy1 = (int)(f.y0 + f.wh);
     const u64 *lab = a.lab + f.lab_off;
+    uint32_t *live = GD ? &a.goal[fi].active : &ctl->count[1];  // the count this item and its pushes are in
+    bool last = false;
     if constexpr (ASYNC) {
         // hold the tile before reading any label: a neighbour that improves our
         // halo after this point marks it dirty, and we queue it again when done
         if (tid == 0) {
             atomicExch(a.tstamp + f.tile_off + t, kTileHeld);
+            if constexpr (GD) a.tpark[f.tile_off + t] = kMax;  // what waited is in the labels read from here on
             __threadfence();
         }
     } else if (tid < 5) {
@@ -630,6 +656,35 @@ __device__ __forceinline__ void process_item(const RelaxArgs &a, uint32_t fi, ui
         s_vis[tid] = u == kNone ? 0u : __ldcg(a.tvisit + f.tile_off + u);
     }
     if (tid < 4) s_push[tid] = 0;
+    // GD: the field's limits and the remaining price along each axis
+    const uint32_t dst_r = f.dst % (b.w * b.h), dst_x = dst_r % b.w, dst_y = dst_r / b.w, dst_l = f.dst / (b.w * b.h);
+    const bool dst_here = dst_x >= (uint32_t)tx0 && dst_x < (uint32_t)tx0 + kTW && dst_y >= (uint32_t)ty0 &&
+                          dst_y < (uint32_t)ty0 + TH && dst_x < f.x0 + f.ww && dst_y < f.y0 + f.wh;
+    const uint32_t dst_li = dst_here ? tile.li(dst_l, dst_y - ty0 + 1, dst_x - tx0 + 1) : 0u;
+    if constexpr (GD) {
+        if (tid < 4) s_park[tid] = kMax;
+        if (tid == 32) {
+            const uint2 lim = __ldcg(reinterpret_cast<const uint2 *>(a.goal + fi));
+            s_lim[0] = lim.x;  // an older (larger) bound of the target is still a bound
+            s_lim[1] = lim.y;  // the threshold only moves while no item of the field is in flight
+        }
+        const BoardGoal *bg = b.goal;
+        const uint32_t *hx = b.goal_sums, *hy = hx + b.w, *hv = hy + b.h;
+        uint32_t e = __ldg(&bg->min_cost);
+        if (f.n_pads) e = min(e, 1u);  // its own pads are entered at weight 1
+        auto rest = [&](const uint32_t *p, int at, int n, uint32_t to) {
+            const uint32_t u = __ldg(p + min(max(at, 0), n - 1)), v = __ldg(p + to);
+            return capmul(u > v ? u - v : v - u, e);
+        };
+        for (uint32_t i = tid; i < SW + SH + L; i += blockDim.x) {
+            if (i < SW) s_hx[i] = rest(hx, tx0 + (int)i - 1, (int)b.w, dst_x);
+            else if (i < SW + SH) s_hy[i - SW] = rest(hy, ty0 + (int)(i - SW) - 1, (int)b.h, dst_y);
+            else s_hl[i - SW - SH] = rest(hv, (int)(i - SW - SH), (int)L, dst_l);
+        }
+        tile.hx = s_hx;
+        tile.hy = s_hy;
+        tile.hl = s_hl;
+    }
     if (f.n_pads <= kPadCache)
         for (uint32_t i = tid; i < f.n_pads; i += blockDim.x) s_pads[i] = __ldg(a.pads + f.pad_off + i);
     if (f.n_vpads <= kVPadCache)
@@ -649,6 +704,7 @@ __device__ __forceinline__ void process_item(const RelaxArgs &a, uint32_t fi, ui
     for (uint32_t i = tid; i < L * TH + L * kTW + TH * kTW; i += blockDim.x) tile.rowd[i] = 0;
     for (uint32_t i = tid; i < fell_words; i += blockDim.x) tile.fellw[i] = 0;
     __syncthreads();
+    if constexpr (GD) tile.ub = s_lim[0];
 
     // ---- step prices into every interior cell: phase 1 -----------------
     // Per interior cell its cost (parked in the below-plane) and its four
@@ -729,7 +785,7 @@ __device__ __forceinline__ void process_item(const RelaxArgs &a, uint32_t fi, ui
             const uint32_t sx = i % SW, r = i / SW, sy = r % SH, l = r / SH;
             tile.lab[tile.li(l, sy, sx)] = lv[k];
             if (!PL) tile.fl[(l * SH + sy) * kFlPitch + sx] = fv[k];
-            if (lv[k] != kInf) {
+            if (lv[k] != kInf && (!GD || tile.bound((uint32_t)(lv[k] >> 32), l, sy, sx) <= tile.ub)) {
                 const bool row_in = sy >= 1 && sy <= TH, col_in = sx >= 1 && sx <= kTW;
                 if (row_in) tile.rowd[l * TH + sy - 1] = 1;
                 if (col_in) tile.cold[l * kTW + sx - 1] = 1;
@@ -870,6 +926,9 @@ __device__ __forceinline__ void process_item(const RelaxArgs &a, uint32_t fi, ui
             // sweeps on the one-activation tiles it runs); the queue form runs
             // columns first, where alternation costs sweeps
             bool ch;
+            if constexpr (GD) {  // the target's own tile tightens its bound from sweep to sweep
+                if (dst_here) tile.ub = min(tile.ub, (uint32_t)(tile.lab[dst_li] >> 32));
+            }
             if constexpr (!ASYNC) ch = (sweep & 1) ? relax_tile_rev(tile) : relax_tile(tile);
             else ch = relax_tile_cols_first(tile);
             ++sweep;
@@ -878,6 +937,16 @@ __device__ __forceinline__ void process_item(const RelaxArgs &a, uint32_t fi, ui
             if (sweep > sweep_limit) {
                 if (tid == 0) atomicOr(&ctl->status, kStatusRoundLimit);
                 break;
+            }
+        }
+
+        if constexpr (GD) {
+            if (dst_here) {
+                tile.ub = min(tile.ub, (uint32_t)(tile.lab[dst_li] >> 32));
+                if (tid == 0 && tile.ub < s_lim[0]) {  // held by this CTA alone: no other writer
+                    s_lim[0] = tile.ub;
+                    *(volatile uint32_t *)&a.goal[fi].ub = tile.ub;
+                }
             }
         }
 
@@ -953,7 +1022,18 @@ __device__ __forceinline__ void process_item(const RelaxArgs &a, uint32_t fi, ui
                 uint32_t step = __ldg(b.planes + (uint64_t)pin * wp * b.h * L + ((uint64_t)l * b.h + gy_n) * wp + gx_n);
                 if (step == kMax || nb_over)
                     step = exact_in_price(b, f, a.pads, pin, (l * b.h + gy_n) * b.w + gx_n, l, gy_n, gx_n);
-                if (ext2(lb, step, 1) < tile.lab[tile.li(l, nsy, nsx)]) s_push[side] = 1;
+                const u64 cand = ext2(lb, step, 1);
+                if (cand < tile.lab[tile.li(l, nsy, nsx)]) {
+                    if constexpr (GD) {
+                        const uint32_t fv = tile.bound((uint32_t)(cand >> 32), l, nsy, nsx);
+                        if (fv > tile.ub) continue;
+                        if (fv > s_lim[1]) {
+                            atomicMin(&s_park[side], fv);
+                            continue;
+                        }
+                    }
+                    s_push[side] = 1;
+                }
                 continue;
             }
             const uint32_t gn = (l * b.h + (uint32_t)(ty0 + (int)nsy - 1)) * b.w + (uint32_t)(tx0 + (int)nsx - 1);
@@ -983,11 +1063,9 @@ __device__ __forceinline__ void process_item(const RelaxArgs &a, uint32_t fi, ui
             __threadfence();  // labels before the visited flag and the queue entries
             if (tid == 4) {
                 if constexpr (ASYNC) {
-                    // nothing reads the visited words during a queue launch: a plain
-                    // store; the work counters are per CTA (s_cnt), added to the
-                    // launch's every kCountBatch activations and when the CTA exits,
-                    // so this thread makes no round trip to L2 here
-                    a.tvisit[f.tile_off + t] = 1u;
+                    // the work counters are per CTA (s_cnt), added to the launch's
+                    // every kCountBatch activations and when the CTA exits, so this
+                    // thread makes no round trip to L2 here
                     s_cnt[1] += sweep;
                     if (++s_cnt[0] == kCountBatch) {
                         if (atomicAdd(&ctl->activations, (unsigned long long)kCountBatch) + kCountBatch >
@@ -1004,7 +1082,7 @@ __device__ __forceinline__ void process_item(const RelaxArgs &a, uint32_t fi, ui
             } else if (s_push[tid]) {
                 const uint32_t u = tid == 0 ? t - 1 : tid == 1 ? t + 1 : tid == 2 ? t - ntx : t + ntx;
                 if constexpr (ASYNC) {
-                    async_push(a, fi, f.tile_off, u);
+                    async_push(a, fi, f.tile_off, u, live);
                 } else {
                     const uint32_t want = round + 2;  // stamp s = queued for round s-1
                     if (atomicMax(a.tstamp + f.tile_off + u, want) < want) {
@@ -1017,6 +1095,10 @@ __device__ __forceinline__ void process_item(const RelaxArgs &a, uint32_t fi, ui
                         }
                     }
                 }
+            } else if (GD && s_park[tid] != kMax) {
+                const uint32_t u = tid == 0 ? t - 1 : tid == 1 ? t + 1 : tid == 2 ? t - ntx : t + ntx;
+                atomicMin(a.tpark + f.tile_off + u, s_park[tid]);
+                __threadfence();  // before this item leaves the field's count
             }
         }
         __syncthreads();
@@ -1036,15 +1118,22 @@ __device__ __forceinline__ void process_item(const RelaxArgs &a, uint32_t fi, ui
                         s_more = 1;
                     } else {
                         atomicExch(stw, kTileQueued);
-                        async_enqueue(a, fi, t);
+                        async_enqueue(a, fi, t, live);
                     }
                 }
-                if (!s_more) async_done(ctl);  // this item leaves the in-flight count
+                if (!s_more) {  // this item leaves the in-flight count
+                    const uint32_t left = atomicSub(live, 1u) - 1u;
+                    if (GD && left == 0) s_more = 2;
+                }
             }
             __syncthreads();
-            if (!s_more) break;
+            if (s_more != 1) {
+                last = s_more == 2;
+                break;
+            }
             __threadfence();  // the neighbours' labels were written before they marked this tile
             if (tid < 4) s_push[tid] = 0;
+            if (GD && tid < 4) s_park[tid] = kMax;
             for (uint32_t i = tid; i < fell_words; i += blockDim.x) tile.fellw[i] = 0;
             // the halo ring again: an improved cell marks the line that ends at it
             const uint32_t nr = 2 * L * TH + 2 * L * kTW;
@@ -1071,6 +1160,7 @@ __device__ __forceinline__ void process_item(const RelaxArgs &a, uint32_t fi, ui
                 u64 &cur = tile.lab[tile.li(l, sy, sx)];
                 if (v < cur) {
                     cur = v;
+                    if (GD && tile.bound((uint32_t)(v >> 32), l, sy, sx) > tile.ub) continue;
                     if (row) tile.rowd[l * TH + sy - 1] = 1;
                     else tile.cold[l * kTW + sx - 1] = 1;
                 }
@@ -1079,6 +1169,70 @@ __device__ __forceinline__ void process_item(const RelaxArgs &a, uint32_t fi, ui
         }
     }
     __syncthreads();  // (queue form: the tile was released, or queued again, inside the loop)
+    return last;
+}
+
+// A goal-directed field with nothing in flight: queue the waiting tiles that can
+// still matter, or end the field.  The calling CTA is the field's only worker.
+// Without a target label the threshold grows (twice the distance above the
+// bound, at least to the smallest f that waits; everything after kGoalPhases
+// releases); with one, every f up to the target's dist goes.
+__device__ void field_release(const RelaxArgs &a, uint32_t fi, uint32_t tile_h) {
+    __shared__ uint32_t s_min;
+    const DevField f = a.fields[fi];
+    FieldGoal *fg = a.goal + fi;
+    const uint32_t ntiles = ((f.ww + kTW - 1) / kTW) * ((f.wh + tile_h - 1) / tile_h);
+    uint32_t *park = a.tpark + f.tile_off;
+    for (;;) {
+        __threadfence();
+        if (threadIdx.x == 0) s_min = kMax;
+        __syncthreads();
+        const uint32_t ub = *(volatile const uint32_t *)&fg->ub;
+        uint32_t m = kMax;
+        for (uint32_t i = threadIdx.x; i < ntiles; i += 4 * blockDim.x) {
+            uint32_t v[4];
+#pragma unroll
+            for (uint32_t k = 0; k < 4; ++k) v[k] = i + k * blockDim.x < ntiles ? __ldcg(park + i + k * blockDim.x) : kMax;
+#pragma unroll
+            for (uint32_t k = 0; k < 4; ++k) m = min(m, v[k]);
+        }
+        m = __reduce_min_sync(0xFFFFFFFFu, m);
+        if ((threadIdx.x & 31) == 0 && m != kMax) atomicMin(&s_min, m);
+        __syncthreads();
+        m = s_min;
+        if (m == kMax || m > ub) {  // nothing waits that could matter: the field is final
+            if (threadIdx.x == 0) atomicSub(&a.ctl->count[1], 1u);
+            return;
+        }
+        uint32_t thr = kMax;
+        const uint32_t f0 = __ldcg(&fg->f0), phases = __ldcg(&fg->phases);
+        if (ub == kMax && phases + 1 < kGoalPhases) {
+            const uint32_t was = *(volatile const uint32_t *)&fg->thr, slack = was - f0;
+            thr = max(dsum(was, slack), dsum(m, slack / 2));
+        }
+        if (threadIdx.x == 0) atomicAdd(&fg->active, 1u);  // this CTA, until every release is queued
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            *(volatile uint32_t *)&fg->thr = thr;
+            fg->phases = phases + 1;
+            __threadfence();
+        }
+        __syncthreads();
+        const uint32_t lim = min(thr, ub);
+        for (uint32_t i = threadIdx.x; i < ntiles; i += blockDim.x) {
+            const uint32_t v = __ldcg(park + i);
+            if (v == kMax || v > lim) continue;
+            async_push(a, fi, f.tile_off, i, &fg->active);
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            __threadfence();
+            s_min = atomicSub(&fg->active, 1u) - 1u;
+        }
+        __syncthreads();
+        if (s_min != 0) return;  // the field's other workers carry it on
+        __syncthreads();
+    }
 }
 
 template <int TH, int NT, bool OV>
@@ -1128,7 +1282,7 @@ __global__ void __launch_bounds__(NT) relax_rounds_kernel(RelaxArgs a) {
             const u64 item = s_item;
             if (item == kInf) break;
             uint32_t no_phase = 0;
-            process_item<TH, false, false, OV>(a, (uint32_t)(item >> 32), (uint32_t)item, round, smem_raw, nullptr,
+            process_item<TH, false, false, OV, false>(a, (uint32_t)(item >> 32), (uint32_t)item, round, smem_raw, nullptr,
                                                no_phase, nullptr);
         }
         grid_barrier(ctl, gridDim.x);
@@ -1141,7 +1295,7 @@ __global__ void __launch_bounds__(NT) relax_rounds_kernel(RelaxArgs a) {
 // valid from the start), and a tile is held by one CTA at a time: improvements
 // that reach a held tile mark it dirty and its holder queues it once more.
 // 64 registers a thread: four 256-thread CTAs per SM
-template <int TH, int NT, bool PL, bool OV>
+template <int TH, int NT, bool PL, bool OV, bool GD>
 __global__ void __launch_bounds__(NT, 65536 / (NT * 64)) relax_async_kernel(RelaxArgs a) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ u64 s_item;
@@ -1161,8 +1315,12 @@ __global__ void __launch_bounds__(NT, 65536 / (NT * 64)) relax_async_kernel(Rela
         __syncthreads();
         const u64 item = s_item;
         if (item == kInf) break;
-        process_item<TH, true, PL, OV>(a, (uint32_t)(item >> 32), (uint32_t)item, 0, smem_raw, &s_mbar, tma_phase,
-                                       s_cnt);
+        const bool last = process_item<TH, true, PL, OV, GD>(a, (uint32_t)(item >> 32), (uint32_t)item, 0, smem_raw,
+                                                             &s_mbar, tma_phase, s_cnt);
+        if (GD && last) {
+            field_release(a, (uint32_t)(item >> 32), TH);
+            __syncthreads();
+        }
     }
     if (threadIdx.x == 0) {
         if (s_cnt[0]) atomicAdd(&a.ctl->activations, s_cnt[0]);
@@ -1186,7 +1344,30 @@ __global__ void async_seed_kernel(RelaxArgs a) {
             const uint32_t ntx = (f.ww + kTW - 1) / kTW;
             const uint32_t t = ((sy - f.y0) / TH) * ntx + (sx - f.x0) / kTW;
             __threadfence();
-            async_push(a, fi, f.tile_off, t);
+            uint32_t *live = &a.ctl->count[1];
+            if (a.goal) {  // goal-directed: the launch counts fields, the field its items
+                const BoardGoal *bg = b.goal;
+                const uint32_t *hx = b.goal_sums, *hy = hx + b.w, *hv = hy + b.h;
+                const uint32_t dl = f.dst / plane, dr = f.dst % plane, dx = dr % b.w, dy = dr / b.w;
+                const uint32_t e = f.n_pads ? min(bg->min_cost, 1u) : bg->min_cost;
+                auto rest = [&](const uint32_t *p, uint32_t u, uint32_t v) {
+                    return capmul(p[u] > p[v] ? p[u] - p[v] : p[v] - p[u], e);
+                };
+                const uint32_t f0 = min(dsum(dsum(rest(hx, sx, dx), rest(hy, sy, dy)), rest(hv, sl, dl)), kCap);
+                // first threshold: room for two vias, a detour of two cells, and the
+                // board's spread of prices; with a zero bound nothing waits
+                const u64 room = (u64)((double)bg->spread * f0) + 2ull * capmul(bg->min_via, e) +
+                                 4ull * capmul(bg->min_step, e);
+                FieldGoal g{};
+                g.ub = kMax;
+                g.f0 = f0;
+                g.thr = (f0 == 0 || f0 + room >= kCap) ? kMax : (uint32_t)(f0 + room);
+                a.goal[fi] = g;
+                __threadfence();
+                atomicAdd(live, 1u);
+                live = &a.goal[fi].active;
+            }
+            async_push(a, fi, f.tile_off, t, live);
         }
     }
 }
@@ -1623,29 +1804,35 @@ size_t relax_smem_bytes(uint32_t layers, uint32_t tile_h, bool directed, bool pl
 
 namespace {
 template <int TH>
-const void *relax_fn_th(bool wide, bool async, bool planes) {
+const void *relax_fn_th(bool wide, bool async, bool planes, bool goal) {
+    if (async && planes && goal)
+        return wide ? (const void *)relax_async_kernel<TH, 256, true, false, true>
+                    : (const void *)relax_async_kernel<TH, 128, true, false, true>;
     if (async && planes)
-        return wide ? (const void *)relax_async_kernel<TH, 256, true, false>
-                    : (const void *)relax_async_kernel<TH, 128, true, false>;
+        return wide ? (const void *)relax_async_kernel<TH, 256, true, false, false>
+                    : (const void *)relax_async_kernel<TH, 128, true, false, false>;
     if (async)
-        return wide ? (const void *)relax_async_kernel<TH, 256, false, false>
-                    : (const void *)relax_async_kernel<TH, 128, false, false>;
+        return wide ? (const void *)relax_async_kernel<TH, 256, false, false, false>
+                    : (const void *)relax_async_kernel<TH, 128, false, false, false>;
     return wide ? (const void *)relax_rounds_kernel<TH, 256, false> : (const void *)relax_rounds_kernel<TH, 128, false>;
 }
 
-const void *relax_fn(uint32_t tile_h, uint32_t threads, bool async, bool planes, bool over) {
+const void *relax_fn(uint32_t tile_h, uint32_t threads, bool async, bool planes, bool over, bool goal) {
+    if (goal && !(async && planes)) return nullptr;  // the bounds are computed with the price planes
     if (over) {  // the override variants exist for the 8 x 256 configuration only
         if (tile_h != kOverTileH || threads != kOverThreads) return nullptr;
-        if (async && planes) return (const void *)relax_async_kernel<kOverTileH, kOverThreads, true, true>;
-        if (async) return (const void *)relax_async_kernel<kOverTileH, kOverThreads, false, true>;
+        if (async && planes)
+            return goal ? (const void *)relax_async_kernel<kOverTileH, kOverThreads, true, true, true>
+                        : (const void *)relax_async_kernel<kOverTileH, kOverThreads, true, true, false>;
+        if (async) return (const void *)relax_async_kernel<kOverTileH, kOverThreads, false, true, false>;
         return (const void *)relax_rounds_kernel<kOverTileH, kOverThreads, true>;
     }
     const bool wide = threads >= 256;
     switch (tile_h) {
-        case 8: return relax_fn_th<8>(wide, async, planes);
-        case 16: return relax_fn_th<16>(wide, async, planes);
-        case 32: return relax_fn_th<32>(wide, async, planes);
-        default: return relax_fn_th<64>(wide, async, planes);
+        case 8: return relax_fn_th<8>(wide, async, planes, goal);
+        case 16: return relax_fn_th<16>(wide, async, planes, goal);
+        case 32: return relax_fn_th<32>(wide, async, planes, goal);
+        default: return relax_fn_th<64>(wide, async, planes, goal);
     }
 }
 
@@ -1659,22 +1846,22 @@ const void *seed_fn(uint32_t tile_h) {
 }
 }  // namespace
 
-cudaError_t relax_configure(uint32_t tile_h, uint32_t threads, size_t smem, bool async, bool planes, bool over) {
-    const void *fn = relax_fn(tile_h, threads, async, planes, over);
+cudaError_t relax_configure(uint32_t tile_h, uint32_t threads, size_t smem, bool async, bool planes, bool over, bool goal) {
+    const void *fn = relax_fn(tile_h, threads, async, planes, over, goal);
     if (!fn) return cudaErrorInvalidValue;
     return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
 }
 
 cudaError_t relax_occupancy(uint32_t tile_h, uint32_t threads, size_t smem, int *blocks_per_sm, bool async,
-                            bool planes, bool over) {
-    const void *fn = relax_fn(tile_h, threads, async, planes, over);
+                            bool planes, bool over, bool goal) {
+    const void *fn = relax_fn(tile_h, threads, async, planes, over, goal);
     if (!fn) return cudaErrorInvalidValue;
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, fn, (int)threads, smem);
 }
 
 cudaError_t relax_launch(const RelaxArgs &a, uint32_t grid, uint32_t threads, size_t smem, cudaStream_t st,
-                         bool async, bool planes, bool over) {
-    const void *fn = relax_fn(a.tile_h, threads, async, planes, over);
+                         bool async, bool planes, bool over, bool goal) {
+    const void *fn = relax_fn(a.tile_h, threads, async, planes, over, goal);
     if (!fn) return cudaErrorInvalidValue;
     RelaxArgs copy = a;
     void *args[] = {&copy};

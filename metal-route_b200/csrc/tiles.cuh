@@ -33,7 +33,7 @@ __device__ __forceinline__ u64 umin64(u64 a, u64 b) { return a < b ? a : b; }
 
 // Work queue of the asynchronous form.  count[0] = tickets handed to pushers
 // (tail), head[0] = tickets handed to poppers, count[1] = items queued or in
-// flight.  lists[0, cap) holds the items, lists[cap, 2 cap) their ticket tags
+// flight.  lists[0, cap) holds the items, tags[0, cap) their ticket tags
 // (ticket + 1, zeroed before launch).  A tile is queued at most once at a time
 // (its tstamp word is the queued flag), so cap = total tiles never overflows.
 constexpr uint32_t kQueueSpinLimit = 1u << 24;  // polls of one wait (~16 s with the backoff below)
@@ -45,22 +45,25 @@ constexpr uint32_t kQueueSpinLimit = 1u << 24;  // polls of one wait (~16 s with
 // workers at once).
 constexpr uint32_t kTileIdle = 0, kTileQueued = 1, kTileHeld = 2, kTileHeldDirty = 3;
 
-__device__ __forceinline__ void async_enqueue(const RelaxArgs &a, uint32_t fi, uint32_t u) {
+// `live`: the count of items queued or in flight, the launch's (count[1]) or, in
+// a goal-directed launch, the field's (count[1] then counts unfinished fields).
+__device__ __forceinline__ void async_enqueue(const RelaxArgs &a, uint32_t fi, uint32_t u, uint32_t *live) {
     Ctl *c = a.ctl;
-    atomicAdd(&c->count[1], 1u);  // in flight before it is visible
+    atomicAdd(live, 1u);  // in flight before it is visible
     const uint32_t h = atomicAdd(&c->count[0], 1u);
     const size_t slot = h % a.list_cap;
     a.lists[slot] = ((u64)fi << 32) | u;
     __threadfence();
-    atomicExch(a.lists + a.list_cap + slot, (u64)h + 1u);
+    atomicExch(a.tags + slot, (u64)h + 1u);
 }
 
-__device__ __forceinline__ void async_push(const RelaxArgs &a, uint32_t fi, uint32_t tile_off, uint32_t u) {
+__device__ __forceinline__ void async_push(const RelaxArgs &a, uint32_t fi, uint32_t tile_off, uint32_t u,
+                                           uint32_t *live) {
     uint32_t *st = a.tstamp + tile_off + u;
     for (int tries = 0; tries < 1024; ++tries) {
         const uint32_t old = atomicCAS(st, kTileIdle, kTileQueued);
         if (old == kTileIdle) {
-            async_enqueue(a, fi, u);
+            async_enqueue(a, fi, u, live);
             return;
         }
         if (old == kTileQueued || old == kTileHeldDirty) return;  // it will read our labels
@@ -76,12 +79,9 @@ __device__ __forceinline__ void async_release(const RelaxArgs &a, uint32_t fi, u
     uint32_t *st = a.tstamp + tile_off + t;
     if (atomicCAS(st, kTileHeld, kTileIdle) == kTileHeldDirty) {
         atomicExch(st, kTileQueued);
-        async_enqueue(a, fi, t);
+        async_enqueue(a, fi, t, &a.ctl->count[1]);
     }
 }
-
-// An item is done: it leaves the in-flight count (after its own pushes were counted).
-__device__ __forceinline__ void async_done(Ctl *c) { atomicSub(&c->count[1], 1u); }
 
 // Next item for the calling worker (one thread), or kInf when no work is left.  The
 // wait is bounded: kQueueSpinLimit polls, then kStatusBarrier and an exit.
@@ -89,7 +89,7 @@ __device__ __forceinline__ u64 async_pop(const RelaxArgs &a) {
     Ctl *c = a.ctl;
     const uint32_t h = atomicAdd(&c->head[0], 1u);
     const size_t slot = h % a.list_cap;
-    const volatile u64 *tag = a.lists + a.list_cap + slot;
+    const volatile u64 *tag = a.tags + slot;
     // Each waiter polls its own slot tag; the shared in-flight count and status
     // words (which every worker updates) are read only every 16th poll, and the
     // sleep between polls doubles up to 1 us, so thousands of idle waiters do
