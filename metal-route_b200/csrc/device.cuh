@@ -78,6 +78,8 @@ struct BoardGoal {
     uint32_t min_step;          // the smallest planar base price,
     uint32_t min_via;           // the smallest via base price
     float spread;               // and the share of the bound that the first threshold adds
+    uint32_t wide;              // packed planes: a finite price did not fit (planes_kernel)
+    uint32_t pad_;
 };
 
 // Search state of one field of a goal-directed launch.  A label at cell c with
@@ -105,8 +107,11 @@ struct DevField {
     uint32_t board;             // index of this field's board in the batch's board array
     uint32_t n_over;            // directed-price overrides of this field (DevBoard::over_cells)
     uint32_t over_off;
-    uint32_t pad_;
+    uint32_t xa;                // columns by which the tile grid starts before the window
 };
+
+// Tiles (32 columns) across a field's window.
+__device__ __forceinline__ uint32_t field_ntx(const DevField &f) { return (f.ww + f.xa + 31u) / 32u; }
 
 // Control block of one batch launch (device memory, zeroed before launch).
 // The words that workers update atomically on every item (the list counts,

@@ -723,14 +723,13 @@ struct mrc_batch {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     cudaGraphExec_t graph = nullptr;  // captured launch sequence (mrc_batch_capture_graph)
     // Set before batch_build by callers that run several batches at once: a
-    // fixed tile configuration, a shared-memory floor (every concurrent batch
-    // has the same per-CTA footprint) and a divisor of the co-resident grid.
+    // fixed tile configuration and a divisor of the grid.
     uint32_t force_tile_h = 0, force_threads = 0, grid_num = 1, grid_div = 1;
     bool grid_by_work = false;  // the grid may grow past grid_num/grid_div up to what the tiles can use
     bool async_q = false;  // relax schedule: asynchronous work queue instead of rounds
     bool warp = false;     // the warp-per-tile schedule (implies the queue and a +inf-filled arena)
-    bool cta_planes = true;  // the CTA queue form stages step prices from the price planes by TMA
-    size_t smem_floor = 0;
+    bool cta_planes = true;  // schedule 1: the layer kernel (where it applies: `layer`), else the CTA queue form
+    bool layer = false;      // this layout runs the layer kernel (packed price planes by TMA)
     std::vector<DevBoard> devs;  // the board table (step-price plane pointers patched in by batch_layout)
     DBuf d_planes, d_pchunks;    // step-price planes of every board, chunk table of their kernel
     DBuf d_tmaps;                // one TMA tensor map per board over its planes (CTA queue form)
@@ -759,7 +758,7 @@ mrc_status choose_tile(mrc_context *ctx, uint32_t layers, bool directed, uint32_
     const size_t hard = std::min<size_t>(ctx->smem_optin ? ctx->smem_optin : (227u << 10), 227u << 10) - 1024;
     for (size_t budget : {(size_t)(75u << 10), (size_t)(110u << 10), hard}) {
         for (uint32_t th : {8u, 16u, 32u, 64u}) {
-            const size_t s = std::max(relax_smem_bytes(layers, th, directed, true), relax_smem_bytes(layers, th, directed, false));
+            const size_t s = relax_smem_bytes(layers, th, directed);
             if (s <= budget) {
                 *tile_h = th;
                 *smem = s;
@@ -830,16 +829,20 @@ mrc_status batch_layout(mrc_batch *bt, uint32_t tile_h, uint32_t threads) {
         threads = kOverThreads;
     }
     if (bt->warp) bt->async_q = true;
-    const bool cta_pl = bt->async_q && !bt->warp && bt->cta_planes;
+    // schedule 1 with another tile height than the layer kernel's, or with more
+    // layers than it takes, runs the CTA queue form with prices formed per tile
+    bt->layer = bt->async_q && !bt->warp && bt->cta_planes && tile_h == kLayerTileH && bt->max_layers <= kLayerMax;
     bt->tile_h = bt->warp ? kWarpTileH : tile_h;
     bt->threads = bt->warp ? warp_relax_threads() : threads;
     bt->smem =
-        bt->warp ? 0 : std::max(relax_smem_bytes(bt->max_layers, tile_h, bt->directed_any, cta_pl), bt->smem_floor);
+        bt->warp ? 0 : bt->layer ? layer_smem_bytes(bt->max_layers)
+                                 : relax_smem_bytes(bt->max_layers, tile_h, bt->directed_any);
     uint64_t toff = 0;
     uint32_t max_tiles = 1;
     for (DevField &f : bt->fields) {
+        f.xa = bt->layer ? f.x0 & 3u : 0u;  // a tile's first column is a multiple of 4 (16 bytes, the TMA rule)
         const uint32_t tw = bt->warp ? warp_tile_w(bt->boards[f.board]->view.layers) : 32u;
-        const uint64_t tiles = (uint64_t)((f.ww + tw - 1) / tw) * ((f.wh + bt->tile_h - 1) / bt->tile_h);
+        const uint64_t tiles = (uint64_t)((f.ww + f.xa + tw - 1) / tw) * ((f.wh + bt->tile_h - 1) / bt->tile_h);
         f.tile_off = (uint32_t)std::min<uint64_t>(toff, 0xFFFFFFFFull);
         toff += tiles;
         max_tiles = (uint32_t)std::max<uint64_t>(max_tiles, tiles);
@@ -847,15 +850,15 @@ mrc_status batch_layout(mrc_batch *bt, uint32_t tile_h, uint32_t threads) {
     if (toff > 0x7FFFFFFFull) return fail(MRC_ERR_LIMIT, "batch has more than 2^31 tiles");
     bt->total_tiles = (uint32_t)std::max<uint64_t>(toff, 1);
     bt->max_tiles = max_tiles;
-    bt->goal = cta_pl && !(bt->flags & MRC_FLAG_KEEP_FIELDS) && toff >= (uint64_t)kGoalTilesPerSm * ctx->sms;
+    bt->goal = bt->layer && !(bt->flags & MRC_FLAG_KEEP_FIELDS) && toff >= (uint64_t)kGoalTilesPerSm * ctx->sms;
     int per_sm = 1;
     if (bt->warp) {
         MRC_CUDA(warp_relax_occupancy(&per_sm), "relax occupancy");
+    } else if (bt->layer) {
+        MRC_CUDA(layer_configure(bt->max_layers, bt->smem, bt->has_over, bt->goal, &per_sm), "configure relax kernel");
     } else {
-        MRC_CUDA(relax_configure(tile_h, threads, bt->smem, bt->async_q, cta_pl, bt->has_over, bt->goal),
-                 "configure relax kernel");
-        MRC_CUDA(relax_occupancy(tile_h, threads, bt->smem, &per_sm, bt->async_q, cta_pl, bt->has_over, bt->goal),
-                 "relax occupancy");
+        MRC_CUDA(relax_configure(tile_h, threads, bt->smem, bt->async_q, bt->has_over), "configure relax kernel");
+        MRC_CUDA(relax_occupancy(tile_h, threads, bt->smem, &per_sm, bt->async_q, bt->has_over), "relax occupancy");
     }
     if (per_sm < 1) return fail(MRC_ERR_LIMIT, "relax kernel does not fit on one SM");
     // cooperative launch: every CTA must be co-resident
@@ -867,7 +870,7 @@ mrc_status batch_layout(mrc_batch *bt, uint32_t tile_h, uint32_t threads) {
     bt->grid = (uint32_t)std::max<uint64_t>(1u, grid);
     // board table, with the step-price planes of every board (warp schedule,
     // CTA queue form) and their tensor maps (CTA queue form)
-    if (bt->warp || cta_pl) {
+    if (bt->warp || bt->layer) {
         std::vector<uint64_t> poff(bt->devs.size()), chunks(bt->devs.size() + 1, 0);
         uint64_t total = 0;
         for (size_t k = 0; k < bt->devs.size(); ++k) {
@@ -894,7 +897,7 @@ mrc_status batch_layout(mrc_batch *bt, uint32_t tile_h, uint32_t threads) {
             }
         }
         MRC_TRY(upload(ctx, bt->d_pchunks, chunks.data(), chunks.size() * 8, "plane chunk table"));
-        if (cta_pl) {
+        if (bt->layer) {
             std::vector<CUtensorMap> maps(bt->devs.size());
             for (size_t k = 0; k < bt->devs.size(); ++k) MRC_TRY(encode_planes_map(bt->devs[k], tile_h, &maps[k]));
             // pool blocks are 256-byte aligned: every 128-byte map is 64-byte aligned
@@ -915,10 +918,10 @@ mrc_status batch_layout(mrc_batch *bt, uint32_t tile_h, uint32_t threads) {
     }
     {  // the board table, and behind it the zeroed heads of the price bounds
         const size_t nb = bt->devs.size(), o_heads = (nb * sizeof(DevBoard) + 255) & ~(size_t)255;
-        std::vector<unsigned char> table(o_heads + (bt->goal ? nb * sizeof(BoardGoal) : 0), 0);
+        std::vector<unsigned char> table(o_heads + (bt->layer ? nb * sizeof(BoardGoal) : 0), 0);
         MRC_TRY(bt->d_boards.get(ctx, std::max<size_t>(table.size(), 4), "board table"));
         BoardGoal *heads = reinterpret_cast<BoardGoal *>(bt->d_boards.as<unsigned char>() + o_heads);
-        for (size_t k = 0; k < nb; ++k) bt->devs[k].goal = bt->goal ? heads + k : nullptr;
+        for (size_t k = 0; k < nb; ++k) bt->devs[k].goal = bt->layer ? heads + k : nullptr;
         if (nb) std::memcpy(table.data(), bt->devs.data(), nb * sizeof(DevBoard));
         MRC_CUDA(cudaMemcpyAsync(bt->d_boards.p, table.data(), table.size(), cudaMemcpyHostToDevice, ctx->stream),
                  "upload board table");
@@ -1016,7 +1019,7 @@ mrc_status batch_build(mrc_context *ctx, std::vector<const mrc_board *> boards, 
         f.board = nc.board;
         f.n_over = nc.n_over;
         f.over_off = nc.over_off;
-        f.pad_ = 0;
+        f.xa = 0;
         if (pads.size() > 0xFFFFFFF0u) return fail(MRC_ERR_LIMIT, "pad lists exceed 2^32 entries");
     }
     bt->total_cells = off;
@@ -1048,9 +1051,9 @@ PathArgs path_args(const mrc_batch *bt) {
     pa.tover = bt->has_over ? bt->d_tover.as<uint8_t>() : nullptr;
     pa.tile_h = bt->tile_h;
     pa.arena_filled = bt->async_q ? 1u : 0u;
-    const bool cta_pl = bt->async_q && !bt->warp && bt->cta_planes;
+    pa.hop_bits = layer_hop_bits(bt->max_layers);
     const size_t ws = walk_smem_bytes(bt->max_layers, bt->tile_h);
-    pa.walk_smem = (cta_pl && !bt->has_over && ws <= kWalkSmemLimit) ? (uint32_t)ws : 0u;
+    pa.walk_smem = (bt->layer && !bt->has_over && ws <= kWalkSmemLimit) ? (uint32_t)ws : 0u;
     pa.costs = bt->d_costs.as<uint32_t>();
     pa.lens = bt->d_lens.as<uint32_t>();
     pa.offsets = bt->d_offsets.as<unsigned long long>();
@@ -1063,7 +1066,7 @@ PathArgs path_args(const mrc_batch *bt) {
 // lower bounds made from the minima that kernel accumulates.
 mrc_status planes_enqueue(mrc_batch *bt, cudaStream_t st, uint32_t *launches) {
     MRC_CUDA(planes_launch(bt->d_boards.as<DevBoard>(), bt->d_pchunks.as<uint64_t>(), (uint32_t)bt->devs.size(),
-                           bt->n_pchunks, (uint32_t)bt->ctx->sms, st),
+                           bt->n_pchunks, (uint32_t)bt->ctx->sms, bt->layer ? layer_hop_bits(bt->max_layers) : 0, st),
              "launch step-price planes");
     *launches += 1;
     if (bt->goal) {
@@ -1113,8 +1116,7 @@ mrc_status batch_enqueue(mrc_batch *bt, cudaStream_t st, bool capturing) {
     if (n) {
         const unsigned rec = capturing ? cudaEventRecordExternal : cudaEventRecordDefault;
         if (bt->ev0) MRC_CUDA(cudaEventRecordWithFlags(bt->ev0, st, rec), "record event");
-        const bool cta_pl = bt->async_q && !bt->warp && bt->cta_planes;
-        if ((bt->warp || cta_pl) && !bt->planes_valid) {
+        if ((bt->warp || bt->layer) && !bt->planes_valid) {
             MRC_TRY(planes_enqueue(bt, st, &launches));
             // a captured graph recomputes them on every replay (it is captured with
             // valid planes, see mrc_batch_capture_graph, so this is the fallback)
@@ -1124,7 +1126,8 @@ mrc_status batch_enqueue(mrc_batch *bt, cudaStream_t st, bool capturing) {
             MRC_CUDA(warp_relax_launch(ra, bt->grid, st), "launch relax kernel");
             launches += 2;  // seeds, relax
         } else {
-            MRC_CUDA(relax_launch(ra, bt->grid, bt->threads, bt->smem, st, bt->async_q, cta_pl, bt->has_over, bt->goal),
+            MRC_CUDA(bt->layer ? layer_launch(ra, bt->grid, bt->smem, st, bt->has_over, bt->goal)
+                               : relax_launch(ra, bt->grid, bt->threads, bt->smem, st, bt->async_q, bt->has_over),
                      "launch relax kernel");
             launches += bt->async_q ? 2 : 1;  // (+ the seed kernel)
         }
@@ -1617,8 +1620,7 @@ mrc_status mrc_batch_capture_graph(mrc_context *ctx, mrc_batch *batch) {
     }
     // the boards' price planes first, outside the graph: they stay valid for
     // every replay of this layout
-    const bool cta_pl = batch->async_q && !batch->warp && batch->cta_planes;
-    if ((batch->warp || cta_pl) && !batch->planes_valid && !batch->fields.empty()) {
+    if ((batch->warp || batch->layer) && !batch->planes_valid && !batch->fields.empty()) {
         uint32_t launches = 0;
         MRC_TRY(planes_enqueue(batch, ctx->stream, &launches));
         MRC_CUDA(cudaStreamSynchronize(ctx->stream), "step-price planes");
@@ -1679,13 +1681,12 @@ mrc_status mrc_batch_autotune(mrc_context *ctx, mrc_batch *batch, uint32_t *tile
     // candidates: (tile height, CTA width, schedule); the warp schedule has one shape
     std::vector<std::array<uint32_t, 3>> cands;
     if (layers <= kWarpMaxLayers) cands.push_back({kWarpTileH, warp_relax_threads(), 2u});
+    if (layers <= kLayerMax) cands.push_back({kLayerTileH, (uint32_t)kRelaxThreads, 1u});  // so has the layer kernel
     for (uint32_t th : {8u, 16u, 32u, 64u}) {
-        if (relax_smem_bytes(layers, th, batch->directed_any, true) > hard ||
-            relax_smem_bytes(layers, th, batch->directed_any, false) > hard)
-            continue;
+        if (relax_smem_bytes(layers, th, batch->directed_any) > hard) continue;
         for (uint32_t nt : {128u, 256u}) {
             if (4u * layers * th < nt / 2) continue;  // most lanes would idle in the line passes
-            for (uint32_t sched : {0u, 1u, 3u}) cands.push_back({th, nt, sched});
+            for (uint32_t sched : {0u, 3u}) cands.push_back({th, nt, sched});
         }
     }
     for (const auto &cand : cands) {
@@ -1737,8 +1738,7 @@ mrc_status mrc_batch_set_config(mrc_context *ctx, mrc_batch *batch, uint32_t til
     Lock lock(ctx, 0);
     MRC_TRY(set_device(ctx));
     const size_t hard = std::min<size_t>(ctx->smem_optin ? ctx->smem_optin : (227u << 10), 227u << 10) - 1024;
-    if (relax_smem_bytes(batch->max_layers, tile_h, batch->directed_any, true) > hard ||
-        relax_smem_bytes(batch->max_layers, tile_h, batch->directed_any, false) > hard)
+    if (relax_smem_bytes(batch->max_layers, tile_h, batch->directed_any) > hard)
         return fail(MRC_ERR_LIMIT, "tile does not fit in shared memory");
     return batch_layout(batch, tile_h, threads);
 }
@@ -2432,7 +2432,7 @@ struct mrc_server {
     std::vector<cudaStream_t> streams;
     std::vector<cudaEvent_t> staged;
     std::vector<bool> slot_busy;
-    size_t budget = 0, inflight_bytes = 0, peak_bytes = 0, smem_floor = 0;
+    size_t budget = 0, inflight_bytes = 0, peak_bytes = 0;
     uint32_t tile_h = 8, threads = kRelaxThreads;
     uint64_t next_ticket = 1, next_batch = 1;
     uint64_t submitted = 0, completed = 0, failed = 0, launches = 0, largest = 0;
@@ -2527,7 +2527,6 @@ mrc_status server_launch(mrc_server *s, ServerBatch *b) {
     b->bt->grid_num = (uint32_t)b->slots.size();
     b->bt->grid_div = s->p.slots;
     b->bt->grid_by_work = true;
-    b->bt->smem_floor = s->smem_floor;
     MRC_TRY(batch_build(ctx, std::move(boards), std::move(nets), std::move(wins), b->flags, b->bt.get()));
     cudaStream_t st = s->streams[b->slots[0]];
     MRC_CUDA(cudaEventRecord(s->staged[b->slots[0]], ctx->stream), "record staging");
@@ -2759,10 +2758,9 @@ mrc_status mrc_server_create(mrc_context *ctx, const mrc_server_params *params, 
         s->budget = allowed > 0 ? (size_t)allowed : 0;
         s->tile_h = 8;
         s->threads = kRelaxThreads;
-        s->smem_floor = relax_smem_bytes(s->p.max_layers, s->tile_h, true, true);
         int per_sm = 0;
-        MRC_CUDA(relax_configure(s->tile_h, s->threads, s->smem_floor, true, true), "configure relax kernel");
-        MRC_CUDA(relax_occupancy(s->tile_h, s->threads, s->smem_floor, &per_sm, true, true), "relax occupancy");
+        MRC_CUDA(layer_configure(s->p.max_layers, layer_smem_bytes(s->p.max_layers), false, true, &per_sm),
+                 "configure relax kernel");
         if ((uint32_t)per_sm * (uint32_t)ctx->sms < s->p.slots) return fail(MRC_ERR_LIMIT, "too many slots");
         s->streams.resize(s->p.slots);
         s->staged.resize(s->p.slots);
@@ -3199,7 +3197,7 @@ extern "C" mrc_status mrc_route_isolated_batch_noalloc(const mrc_isolated_reques
         const uint64_t t = (uint64_t)((f.ww + 31) / 32) * ((f.wh + tile_h - 1) / tile_h);
         f.tile_off = (uint32_t)std::min<uint64_t>(tiles, 0xFFFFFFFFull);
         f.board = 0;
-        f.pad_ = 0;
+        f.xa = 0;
         tiles += t;
         max_tiles = (uint32_t)std::max<uint64_t>(max_tiles, t);
     }

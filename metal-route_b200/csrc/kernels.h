@@ -60,8 +60,9 @@ struct PathArgs {
     const uint32_t *tvisit;
     const uint8_t *tover;            // nullable: as RelaxArgs::tover
     uint32_t tile_h;
+    uint32_t hop_bits;               // of the packed price planes (tile-staged walk)
     uint32_t arena_filled;           // 1: the label arena was +inf-filled (queue schedule), tvisit not needed
-    uint32_t walk_smem;              // > 0: the tile-staged walk (price planes + TMA maps, no overrides), its smem
+    uint32_t walk_smem;              // > 0: the tile-staged walk (packed planes + TMA maps, no overrides), its smem
     uint32_t *costs;                 // [n] by output slot
     uint32_t *lens;                  // [n] by output slot
     unsigned long long *offsets;     // [n+1] by output slot
@@ -236,6 +237,10 @@ __host__ __device__ inline size_t walk_smem_bytes(uint32_t layers, uint32_t tile
 // Rows of a price plane are padded to a multiple of 4 cells (16 bytes), so a
 // tensor map over the planes has 16-byte strides.
 __host__ __device__ inline uint32_t planes_pitch(uint32_t w) { return (w + 3u) & ~3u; }
+// hop_bits: 0 = plain prices (the warp schedule), else packed for the layer
+// kernel: (price << hop_bits) | 1, kPackedInf for no step; a board with a finite
+// price that does not fit is marked (BoardGoal::wide).
+constexpr uint32_t kPackedInf = 1u << 30;
 uint64_t planes_chunks(uint64_t cells);
 // Words of one board's prefix sums (DevBoard::goal_sums); goal_launch makes them
 // of the minima that planes_launch accumulated into the zeroed heads.
@@ -244,11 +249,11 @@ inline uint64_t goal_words(uint32_t w, uint32_t h, uint32_t layers) {
 }
 cudaError_t goal_launch(const DevBoard *boards, uint32_t n_boards, cudaStream_t st);
 cudaError_t planes_launch(const DevBoard *boards, const uint64_t *chunk_start, uint32_t n_boards, uint64_t n_chunks,
-                          uint32_t sms, cudaStream_t st);
+                          uint32_t sms, uint32_t hop_bits, cudaStream_t st);
 
-// Shared memory of one tile of 32 x tile_h cells over `layers` (tile_h in {8, 16, 32, 64}); `planes`: the
-// queue form that stages the step prices from the boards' price planes by TMA (DevBoard::planes, ::tmap).
-size_t relax_smem_bytes(uint32_t layers, uint32_t tile_h, bool directed, bool planes = false);
+// Shared memory of one tile of 32 x tile_h cells over `layers` (tile_h in {8, 16, 32, 64}) with 64-bit labels
+// and prices formed per tile.
+size_t relax_smem_bytes(uint32_t layers, uint32_t tile_h, bool directed);
 // The relax kernel is instantiated for threads in {128, 256} per CTA.
 // `async` selects the queue-driven form (relax_async_kernel) over the
 // bulk-synchronous rounds (relax_rounds_kernel); the async form needs the label
@@ -256,14 +261,25 @@ size_t relax_smem_bytes(uint32_t layers, uint32_t tile_h, bool directed, bool pl
 // over: the fields carry directed-price overrides (DevField::n_over); those
 // kernels exist for kOverTileH-row tiles and kOverThreads threads only.
 constexpr uint32_t kOverTileH = 8, kOverThreads = 256;
-// goal: the goal-directed form of the queue kernel with price planes (paths and
-// costs only, RelaxArgs::goal).
-cudaError_t relax_configure(uint32_t tile_h, uint32_t threads, size_t smem, bool async = false, bool planes = false,
-                            bool over = false, bool goal = false);
+cudaError_t relax_configure(uint32_t tile_h, uint32_t threads, size_t smem, bool async = false, bool over = false);
 cudaError_t relax_occupancy(uint32_t tile_h, uint32_t threads, size_t smem, int *blocks_per_sm, bool async = false,
-                            bool planes = false, bool over = false, bool goal = false);
+                            bool over = false);
 cudaError_t relax_launch(const RelaxArgs &a, uint32_t grid, uint32_t threads, size_t smem, cudaStream_t st,
-                         bool async = false, bool planes = false, bool over = false, bool goal = false);
+                         bool async = false, bool over = false);
+// source labels and source tiles of a queue form (relax_launch includes it)
+cudaError_t seed_launch(const RelaxArgs &a, cudaStream_t st);
+
+// The layer kernel (layer_relax.cu): the queue form on 32 x 8 tiles with a warp
+// per layer, labels packed into 32 bits, prices from the boards' packed price
+// planes by TMA; boards of up to kLayerMax layers.  goal: paths and costs only
+// (RelaxArgs::goal).
+constexpr uint32_t kLayerMax = 16;
+constexpr uint32_t kLayerTileH = 8;
+// bits of a packed word that hold hops (the rest, below bit 30, the dist)
+__host__ __device__ inline uint32_t layer_hop_bits(uint32_t max_layers) { return max_layers <= 8 ? 12 : 13; }
+size_t layer_smem_bytes(uint32_t max_layers);
+cudaError_t layer_configure(uint32_t max_layers, size_t smem, bool over, bool goal, int *blocks_per_sm);
+cudaError_t layer_launch(const RelaxArgs &a, uint32_t grid, size_t smem, cudaStream_t st, bool over, bool goal);
 // tover[f.tile_off + t] = 1 for every tile t of every field that holds one of
 // the field's directed-price overrides (tover zeroed before).
 cudaError_t mark_over_tiles_launch(const DevField *fields, uint32_t n_fields, const DevBoard *boards, uint32_t tile_h,

@@ -1,0 +1,675 @@
+// layer_relax.cu — the queue-driven relax kernel with a warp per layer and 32-bit labels.
+//
+// A CTA holds one 32 x 8 tile over all L layers of a field, warp l its layer l:
+// lane x keeps the eight labels of column x in registers.  Inside an activation a
+// label is one word, (dist - least staged dist) << HB | (hops - least staged
+// hops), and a step price is (price << HB) | 1, so the lexicographic min-plus step
+// of (dist, hops) is one add-and-min instruction (__viaddmin_u32) where 64-bit
+// labels with saturation take about ten.  kBig is +inf: label + price stays below
+// 2^32, and a min with a label at most kBig clamps the sum.  A sweep is:
+//   columns  each lane runs its column down and up in registers (the halo rows in
+//            two more registers), no data exchanged;
+//   rows     through shared memory (one store and two 16-byte loads a lane): four
+//            lanes a row, eight cells each, joined by a two-step scan; the warp
+//            repeats columns and rows until its plane is closed, with no CTA barrier;
+//   stacks   a thread per (y, x) runs the layers up and down; only here the warps
+//            of a tile meet.
+// What changed is found by comparing registers (old and new label of the own
+// column), so there are no dirty-line or fell marks.
+//
+// The packing is exact or not used: a tile whose staged labels spread too far, or
+// whose largest final label comes within one price of kBig (the only way a sum
+// could have been clamped), is relaxed on 64-bit labels instead (wide_item), from
+// the labels in HBM, which this kernel has not touched by then.  So is every tile
+// of a board with a finite price of 2^(29 - HB) or more.
+//
+// Bound by the chain of activations (a queue hop, the label loads, the sweeps, the
+// write-back) on small batches and by instruction issue on large ones.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+
+#include "cta_tile.cuh"
+#include "device.cuh"
+#include "kernels.h"
+#include "tiles.cuh"
+#include "tma.cuh"
+
+namespace mrc {
+namespace {
+
+constexpr int TH = kLayerTileH;
+constexpr uint32_t kBig = kPackedInf;   // +inf
+constexpr uint32_t kNarrow = 1u << 29;  // staged labels, final labels and prices lie below
+// Pitch of a row of labels or prices: 16-byte aligned, and the rows' segments and
+// the columns of a warp fall on distinct banks.
+constexpr uint32_t kPitch = kPlaneTmaBoxW;
+constexpr uint32_t kSpecCap = 512;      // cells of a tile priced for the net itself
+constexpr int kPlaneIters = 4;          // column and row passes of a plane between two meetings
+
+__host__ __device__ inline size_t layer_st_off(uint32_t L) { return ((size_t)L * TH * kPitch * 4 + 127) & ~(size_t)127; }
+
+struct LayerShared {
+    u64 item;
+    uint64_t mbar;  // completion of the price-plane TMA loads
+    unsigned long long cnt[2];  // activations and sweeps not yet added to the launch's
+    uint32_t n_spec, wide, dmin, hmin, hmax, ub, thr, more;
+    uint32_t push[4], park[4];  // left, right, top, bottom
+    uint32_t hy[TH + 2];        // GD: remaining price along y, rows -1 .. TH
+    uint32_t spec[kSpecCap];
+};
+
+// The 64-bit form of one item, from the start (the hold is taken again, which
+// drops a dirty mark, but the labels are read after it).
+template <bool OV, bool GD>
+__device__ __noinline__ bool wide_item(const RelaxArgs &a, uint32_t fi, uint32_t t, unsigned char *smem_raw,
+                                       unsigned long long *cnt) {
+    return process_item<TH, true, OV, GD, true>(a, fi, t, 0, smem_raw, cnt);
+}
+
+// The exact price, on the records in global memory (so that the caller's copies
+// stay in registers).
+__device__ __noinline__ uint32_t exact_price(const DevBoard *b, const DevField *f, const uint32_t *pads, uint32_t dir,
+                                             uint32_t l, uint32_t y, uint32_t x) {
+    return exact_in_price(*b, *f, pads, (int)dir, (l * b->h + y) * b->w + x, l, y, x);
+}
+
+template <int HB>
+__device__ __forceinline__ uint32_t pack_price(uint32_t p, uint32_t *wide) {
+    if (p < (kNarrow >> HB)) return (p << HB) | 1u;
+    if (p != kMax) *wide = 1;
+    return kBig;
+}
+
+// Relaxes one held-to-be item; thread 0 returns whether it was the field's last
+// one in flight (GD).
+template <int LM, bool OV, bool GD>
+__device__ __forceinline__ bool layer_item(const RelaxArgs &a, uint32_t fi, uint32_t t, unsigned char *smem_raw,
+                                           LayerShared &sh, uint32_t &phase) {
+    constexpr int HB = LM <= 8 ? 12 : 13;
+    constexpr uint32_t kHopMask = (1u << HB) - 1u;
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, wl = tid >> 5;
+    const uint32_t r = lane >> 2, seg = lane & 3u;  // row layout: row and segment of 8 cells
+    const DevField f = a.fields[fi];
+    const DevBoard b = a.boards[f.board];
+    const uint32_t L = b.layers;
+    const uint32_t ntx = field_ntx(f), nty = (f.wh + TH - 1) / TH;
+    const uint32_t tyi = t / ntx, txi = t - tyi * ntx;
+    const int tx0 = (int)(f.x0 - f.xa + txi * kTW), ty0 = (int)(f.y0 + tyi * TH);
+    const uint32_t tw = min(kTW, f.ww + f.xa - txi * kTW), th = min((uint32_t)TH, f.wh - tyi * TH);
+    const uint32_t xlo = txi == 0 ? f.xa : 0u;
+    uint32_t *lab = reinterpret_cast<uint32_t *>(smem_raw);
+    uint32_t *st = reinterpret_cast<uint32_t *>(smem_raw + layer_st_off(L));
+    uint32_t *live = GD ? &a.goal[fi].active : &a.ctl->count[1];
+    uint32_t *state = a.tstamp + f.tile_off + t;
+    const bool mine = wl < L;                            // this warp has a layer
+    const bool col_in = mine && lane >= xlo && lane < tw;  // this lane has a column of the window
+    if (tid == 0) {
+        // every thread is past the previous item: the planes of this tile go
+        // global -> shared while the labels are read
+        fence_proxy_async_smem();
+        mbar_expect_tx(&sh.mbar, 6u * L * TH * kPitch * 4u);
+        tma_load_4d(st, b.tmap, tx0, ty0, 0, 0, &sh.mbar);
+        // hold the tile before reading any label: a neighbour that improves our
+        // halo after this point marks it dirty, and we carry it on
+        atomicExch(state, kTileHeld);
+        if constexpr (GD) a.tpark[f.tile_off + t] = kMax;  // what waited is in the labels read from here on
+        __threadfence();
+        if constexpr (GD) {
+            const uint2 lim = __ldcg(reinterpret_cast<const uint2 *>(a.goal + fi));
+            sh.ub = lim.x;   // an older (larger) bound of the target is still a bound
+            sh.thr = lim.y;  // the threshold only moves while no item of the field is in flight
+        }
+    }
+    const uint32_t board_wide = __ldg(&b.goal->wide);
+    // GD: remaining price along each axis
+    uint32_t hx = 0, hxs = 0, hl = 0;
+    bool dst_here = false, dst_mine = false;
+    uint32_t dst_row = 0;
+    if constexpr (GD) {
+        const uint32_t plane = b.w * b.h, dst_l = f.dst / plane, dr = f.dst - dst_l * plane, dst_y = dr / b.w,
+                       dst_x = dr - dst_y * b.w;
+        const uint32_t *px = b.goal_sums, *py = px + b.w, *pv = py + b.h;
+        uint32_t e = __ldg(&b.goal->min_cost);
+        if (f.n_pads) e = min(e, 1u);  // its own pads are entered at weight 1
+        auto rest = [&](const uint32_t *p, int at, uint32_t n, uint32_t to) {
+            const uint32_t u = __ldg(p + min(max(at, 0), (int)n - 1)), v = __ldg(p + to);
+            return capmul(u > v ? u - v : v - u, e);
+        };
+        hx = rest(px, tx0 + (int)lane, b.w, dst_x);
+        hxs = rest(px, seg == 0 ? tx0 - 1 : tx0 + (int)kTW, b.w, dst_x);
+        hl = rest(pv, (int)wl, L, dst_l);
+        if (wl == 0 && lane < TH + 2) sh.hy[lane] = rest(py, ty0 + (int)lane - 1, b.h, dst_y);
+        dst_here = dst_x >= (uint32_t)tx0 + xlo && dst_x < (uint32_t)tx0 + tw && dst_y >= (uint32_t)ty0 &&
+                   dst_y < (uint32_t)ty0 + th;
+        dst_row = dst_y - (uint32_t)ty0;
+        dst_mine = dst_here && wl == dst_l && lane == dst_x - (uint32_t)tx0;
+    }
+    // f of a label (dist) at a cell with these remaining prices
+    auto bound = [&](uint32_t dist, uint32_t h) { return min(dsum(dist, h), kCap); };
+    __syncthreads();
+
+    const u64 *glab = a.lab + f.lab_off;
+    const int64_t row0 = ((int64_t)wl * f.wh + (ty0 - (int)f.y0)) * (int64_t)f.ww + (tx0 - (int)f.x0);
+    uint32_t pt = kBig, pb = kBig, ps = kBig;  // prices into the neighbour tiles' border cells
+    const bool top = tyi > 0, bottom = tyi + 1 < nty;
+    const bool side = mine && r < th && ((seg == 0 && txi > 0) || (seg == 3 && txi + 1 < ntx));
+    for (uint32_t cont = 0;; ++cont) {
+        // ---- labels of the column, the halo rows and the halo columns ----------
+        u64 v[TH], vt = kInf, vb = kInf, vs = kInf;
+#pragma unroll
+        for (int y = 0; y < TH; ++y) {
+            v[y] = kInf;
+            if (col_in && y < (int)th) v[y] = __ldcg(glab + row0 + (int64_t)y * f.ww + lane);
+        }
+        if (col_in && top) vt = __ldcg(glab + row0 - (int64_t)f.ww + lane);
+        if (col_in && bottom) vb = __ldcg(glab + row0 + (int64_t)TH * f.ww + lane);
+        if (side) vs = __ldcg(glab + row0 + (int64_t)r * f.ww + (seg == 0 ? -1 : (int)kTW));
+        if (cont == 0) {
+            const uint32_t wp = planes_pitch(b.w);
+            const uint64_t NP = (uint64_t)wp * b.h * L;
+            const uint32_t *pl = b.planes + ((uint64_t)wl * b.h + (uint32_t)ty0) * wp + (uint32_t)tx0;
+            if (col_in && top) pt = __ldg(pl + kInPosY * NP + lane - wp);
+            if (col_in && bottom) pb = __ldg(pl + kInNegY * NP + lane + (uint64_t)TH * wp);
+            if (side) ps = __ldg(pl + (seg == 0 ? kInPosX : kInNegX) * NP + (uint64_t)r * wp + (seg == 0 ? -1 : (int)kTW));
+            // cells of this tile whose prices depend on the net: its own pads, its via pads
+            for (uint32_t k = tid; k < f.n_pads + f.n_vpads; k += blockDim.x) {
+                const bool q = k >= f.n_pads;
+                const uint32_t c = __ldg(a.pads + (q ? f.vpad_off + k - f.n_pads : f.pad_off + k));
+                const uint32_t plane = b.w * b.h, l = c / plane, rr = c - l * plane, gy = rr / b.w, gx = rr - gy * b.w;
+                const uint32_t x = gx - (uint32_t)tx0, y = gy - (uint32_t)ty0;
+                if (x < xlo || x >= tw || y >= th) continue;
+                const uint32_t i = atomicAdd(&sh.n_spec, 1u);
+                if (i < kSpecCap) sh.spec[i] = (q ? 1u << 31 : 0u) | (l << 16) | (y << 8) | x;
+                else sh.wide = 1;
+            }
+        }
+        {
+            uint32_t dm = kMax, hm = kMax, hM = 0;
+            auto see = [&](u64 q) {
+                const uint32_t d = (uint32_t)(q >> 32), h = (uint32_t)q;
+                dm = min(dm, d);
+                hm = min(hm, h);
+                if (d != kMax) hM = max(hM, h);
+            };
+#pragma unroll
+            for (int y = 0; y < TH; ++y) see(v[y]);
+            see(vt);
+            see(vb);
+            see(vs);
+            dm = __reduce_min_sync(0xFFFFFFFFu, dm);
+            hm = __reduce_min_sync(0xFFFFFFFFu, hm);
+            hM = __reduce_max_sync(0xFFFFFFFFu, hM);
+            if (lane == 0 && dm != kMax) {
+                atomicMin(&sh.dmin, dm);
+                atomicMin(&sh.hmin, hm);
+                atomicMax(&sh.hmax, hM);
+            }
+        }
+        __syncthreads();
+        const uint32_t dbase = sh.dmin, hbase = sh.hmin;
+        // hops of a path through the tile stay below the dist bits, and no dist of
+        // the tile can saturate
+        bool bad = dbase != kMax && ((int64_t)(sh.hmax - hbase) + 256 * L + 4 > (int64_t)kHopMask ||
+                                     dbase > kMax - (kBig >> HB));
+        uint32_t ub = kMax;
+        uint32_t w[TH], w0[TH], lim[TH], ht, hb, hs;
+        if constexpr (GD) ub = sh.ub;
+        auto pack = [&](u64 q, uint32_t h) {
+            const uint32_t d = (uint32_t)(q >> 32);
+            if (d == kMax) return kBig;
+            if (GD && bound(d, h) > ub) return kBig;  // past the target's bound it does not matter
+            const uint32_t rel = d - dbase;
+            if (rel < (kNarrow >> HB)) return (rel << HB) | (((uint32_t)q - hbase) & kHopMask);
+            bad = true;
+            return kBig;
+        };
+        // GD: labels at or above lim[y] are past the target's bound
+        auto set_limits = [&]() {
+#pragma unroll
+            for (int y = 0; y < TH; ++y) {
+                lim[y] = kBig;
+                if constexpr (GD) {
+                    if (ub != kMax) {
+                        const int64_t room = (int64_t)ub - dbase - hx - hl - sh.hy[y + 1];
+                        lim[y] = room < 0 ? 0u : room < (int64_t)((kBig >> HB) - 1) ? (uint32_t)(room + 1) << HB : kBig;
+                    }
+                }
+            }
+        };
+        set_limits();
+        const uint32_t hxl = dsum(hx, hl);
+#pragma unroll
+        for (int y = 0; y < TH; ++y) w0[y] = w[y] = pack(v[y], GD ? dsum(hxl, sh.hy[y + 1]) : 0);
+        ht = pack(vt, GD ? dsum(hxl, sh.hy[0]) : 0);
+        hb = pack(vb, GD ? dsum(hxl, sh.hy[TH + 1]) : 0);
+        hs = pack(vs, GD ? dsum(dsum(hxs, hl), sh.hy[r + 1]) : 0);
+        if (cont == 0) {
+            // the planes: a bounded wait for the TMA load (a load that never lands
+            // sets the status and the launch ends without results)
+            for (uint32_t spins = 0; !mbar_try_wait(&sh.mbar, phase & 1u); ++spins) {
+                if (spins == kTmaSpinLimit) {
+                    if (tid == 0) atomicOr(&a.ctl->status, kStatusQueueOverflow);
+                } else if (spins > 2 * kTmaSpinLimit) {
+                    break;
+                }
+            }
+            ++phase;
+            if (board_wide) {
+                __syncthreads();  // everybody is past the load and the staged words
+                return wide_item<OV, GD>(a, fi, t, smem_raw, sh.cnt);
+            }
+            if (mine && (tw < kTW || th < TH || xlo)) {  // no step enters a cell past the window
+                for (uint32_t y = 0; y < TH; ++y) {
+                    if (col_in && y < th) continue;
+                    for (uint32_t p = 0; p < 6; ++p) st[((p * L + wl) * TH + y) * kPitch + lane] = kBig;
+                }
+            }
+            const uint32_t ns = min(sh.n_spec, kSpecCap);
+            const bool over = OV && f.n_over && a.tover[f.tile_off + t];
+            for (uint32_t i = tid; i < 6 * ns; i += blockDim.x) {
+                const uint32_t e = sh.spec[i / 6], p0 = i % 6;
+                uint32_t l = (e >> 16) & 0xFFu, p = p0;
+                const uint32_t y = (e >> 8) & 0xFFu, x = e & 0xFFu;
+                if (e >> 31) {  // a via pad: the via steps at its cell and at the cells below and above it
+                    l = l + p0 / 2 - 1u;
+                    if (l >= L) continue;
+                    p = (p0 & 1u) ? kInAbove : kInBelow;
+                }
+                const uint32_t gy = (uint32_t)ty0 + y, gx = (uint32_t)tx0 + x;
+                st[((p * L + l) * TH + y) * kPitch + x] =
+                    pack_price<HB>(exact_price(a.boards + f.board, a.fields + fi, a.pads, p, l, gy, gx), &sh.wide);
+            }
+            if (over) {  // cells where this net's own directed prices differ from the board's
+                const uint32_t *oc = b.over_cells + f.over_off;
+                for (uint32_t j = tid; j < L * th; j += blockDim.x) {
+                    const uint32_t l = j / th, y = j - l * th, gy = (uint32_t)ty0 + y;
+                    const uint32_t lo_c = (l * b.h + gy) * b.w + (uint32_t)tx0 + xlo, hi_c = lo_c - xlo + tw;
+                    for (uint32_t k = over_lower_bound(oc, f.n_over, lo_c); k < f.n_over; ++k) {
+                        const uint32_t c = __ldg(oc + k);
+                        if (c >= hi_c) break;
+                        const uint32_t gx = c - (l * b.h + gy) * b.w;
+                        for (uint32_t p = kInNegX; p <= kInPosY; ++p)
+                            st[((p * L + l) * TH + y) * kPitch + gx - (uint32_t)tx0] =
+                                pack_price<HB>(exact_price(a.boards + f.board, a.fields + fi, a.pads, p, l, gy, gx),
+                                               &sh.wide);
+                    }
+                }
+            }
+            if (ns || over) __syncthreads();
+        }
+
+        // ---- relax to local convergence --------------------------------------
+        uint32_t *colp = lab + (wl * TH) * kPitch + lane;              // this lane's column, row y at + y * kPitch
+        uint4 *rowp = reinterpret_cast<uint4 *>(lab + (wl * TH + r) * kPitch + seg * 8);
+        const uint32_t *stc = st + (wl * TH) * kPitch + lane;          // prices of the column, plane p at + p * L * TH * kPitch
+        const uint32_t *str = st + (wl * TH + r) * kPitch + seg * 8;   // prices of the row segment
+        const uint32_t SP = L * TH * kPitch;
+        bool plane = false;  // this warp's plane is open (warp-uniform)
+        if (mine) {
+            bool any = (ht & hb & hs) != kBig;
+#pragma unroll
+            for (int y = 0; y < TH; ++y) {
+                any |= w[y] < lim[y];
+                colp[y * kPitch] = w[y];
+            }
+            plane = __any_sync(0xFFFFFFFFu, any);
+        }
+        bool stk = plane;    // labels that the stacks have not seen
+        uint32_t sweep = 0;
+        const uint32_t sweep_limit = L * kTW * TH + 4;
+        for (;;) {
+            if (plane) {
+                for (int it = 0;; ++it) {
+                    // columns
+                    bool ch = false;
+                    {
+                        uint32_t u[TH], prev = ht;
+#pragma unroll
+                        for (int y = 0; y < TH; ++y)
+                            prev = u[y] = __viaddmin_u32(prev, stc[kInNegY * SP + y * kPitch], w[y]);
+                        prev = hb;
+#pragma unroll
+                        for (int y = TH - 1; y >= 0; --y) {
+                            prev = u[y] = __viaddmin_u32(prev, stc[kInPosY * SP + y * kPitch], u[y]);
+                            ch |= u[y] < min(w[y], lim[y]);
+                            w[y] = u[y];
+                        }
+                    }
+                    ch = __any_sync(0xFFFFFFFFu, ch);
+                    stk |= ch;
+                    if (it > 0 && !ch) {  // the rows were closed by the last row pass
+                        plane = false;
+                        break;
+                    }
+                    // rows
+                    __syncwarp();
+#pragma unroll
+                    for (int y = 0; y < TH; ++y) colp[y * kPitch] = w[y];
+                    __syncwarp();
+                    {
+                        uint32_t u[8], p[8], P[8];
+                        *reinterpret_cast<uint4 *>(u) = rowp[0];
+                        *reinterpret_cast<uint4 *>(u + 4) = rowp[1];
+                        const uint4 *pf = reinterpret_cast<const uint4 *>(str + kInNegX * SP);
+                        *reinterpret_cast<uint4 *>(p) = pf[0];
+                        *reinterpret_cast<uint4 *>(p + 4) = pf[1];
+                        // forward: the halo column enters the first segment's chain
+                        if (seg == 0) u[0] = __viaddmin_u32(hs, p[0], u[0]);
+                        P[0] = p[0];
+#pragma unroll
+                        for (int i = 1; i < 8; ++i) {
+                            u[i] = __viaddmin_u32(u[i - 1], p[i], u[i]);
+                            P[i] = __viaddmin_u32(P[i - 1], p[i], kBig);
+                        }
+                        uint32_t A = u[7], D = P[7];
+#pragma unroll
+                        for (int o = 1; o < 4; o <<= 1) {
+                            const uint32_t Ap = __shfl_up_sync(0xFFFFFFFFu, A, o, 4);
+                            const uint32_t Dp = __shfl_up_sync(0xFFFFFFFFu, D, o, 4);
+                            if (seg >= (uint32_t)o) {
+                                A = __viaddmin_u32(Ap, D, A);
+                                D = __viaddmin_u32(Dp, D, kBig);
+                            }
+                        }
+                        uint32_t C = __shfl_up_sync(0xFFFFFFFFu, A, 1, 4);
+                        if (seg == 0) C = kBig;
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) u[i] = __viaddmin_u32(C, P[i], u[i]);
+                        // backward over the forward results
+                        const uint4 *pq = reinterpret_cast<const uint4 *>(str + kInPosX * SP);
+                        *reinterpret_cast<uint4 *>(p) = pq[0];
+                        *reinterpret_cast<uint4 *>(p + 4) = pq[1];
+                        if (seg == 3) u[7] = __viaddmin_u32(hs, p[7], u[7]);
+                        P[7] = p[7];
+#pragma unroll
+                        for (int i = 6; i >= 0; --i) {
+                            u[i] = __viaddmin_u32(u[i + 1], p[i], u[i]);
+                            P[i] = __viaddmin_u32(P[i + 1], p[i], kBig);
+                        }
+                        A = u[0];
+                        D = P[0];
+#pragma unroll
+                        for (int o = 1; o < 4; o <<= 1) {
+                            const uint32_t Ap = __shfl_down_sync(0xFFFFFFFFu, A, o, 4);
+                            const uint32_t Dp = __shfl_down_sync(0xFFFFFFFFu, D, o, 4);
+                            if (seg + (uint32_t)o < 4u) {
+                                A = __viaddmin_u32(Ap, D, A);
+                                D = __viaddmin_u32(Dp, D, kBig);
+                            }
+                        }
+                        C = __shfl_down_sync(0xFFFFFFFFu, A, 1, 4);
+                        if (seg == 3) C = kBig;
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) u[i] = __viaddmin_u32(C, P[i], u[i]);
+                        rowp[0] = *reinterpret_cast<uint4 *>(u);
+                        rowp[1] = *reinterpret_cast<uint4 *>(u + 4);
+                    }
+                    __syncwarp();
+                    ch = false;
+#pragma unroll
+                    for (int y = 0; y < TH; ++y) {
+                        const uint32_t n = colp[y * kPitch];
+                        ch |= n < min(w[y], lim[y]);
+                        w[y] = n;
+                    }
+                    plane = __any_sync(0xFFFFFFFFu, ch);
+                    stk |= plane;
+                    if (!plane || it + 1 == kPlaneIters) break;
+                }
+            }
+            ++sweep;
+            if constexpr (GD) {  // the target's own tile tightens its bound from sweep to sweep
+                if (dst_mine && !bad) {
+                    uint32_t q = kBig;
+#pragma unroll
+                    for (int y = 0; y < TH; ++y)
+                        if (y == (int)dst_row) q = w[y];
+                    if (q < kBig && dbase + (q >> HB) < sh.ub) {  // this lane alone writes it
+                        sh.ub = dbase + (q >> HB);
+                        *(volatile uint32_t *)&a.goal[fi].ub = sh.ub;
+                    }
+                }
+            }
+            if (!__syncthreads_or(stk || plane)) break;
+            if (GD && dst_here) {
+                ub = *(volatile uint32_t *)&sh.ub;
+                set_limits();
+            }
+            if (sweep > sweep_limit) {
+                if (tid == 0) atomicOr(&a.ctl->status, kStatusRoundLimit);
+                break;
+            }
+            stk = false;
+            if (L == 1) continue;
+            // the plane's labels are in shared memory, as of the last row pass or the
+            // start; a column pass that ended the loop changed nothing
+            for (uint32_t s = tid; s < TH * kTW; s += blockDim.x) {
+                uint32_t *q = lab + (s >> 5) * kPitch + lane;
+                const uint32_t *pu = st + kInBelow * SP + (s >> 5) * kPitch + lane;
+                const uint32_t *pd = st + kInAbove * SP + (s >> 5) * kPitch + lane;
+                constexpr uint32_t LS = TH * kPitch;  // words from a layer to the next
+                uint32_t c[LM];
+#pragma unroll
+                for (int l = 0; l < LM; ++l)
+                    if (l < (int)L) c[l] = q[l * LS];
+#pragma unroll
+                for (int l = 1; l < LM; ++l)
+                    if (l < (int)L) c[l] = __viaddmin_u32(c[l - 1], pu[l * LS], c[l]);
+#pragma unroll
+                for (int l = LM - 2; l >= 0; --l)
+                    if (l + 1 < (int)L) c[l] = __viaddmin_u32(c[l + 1], pd[l * LS], c[l]);
+#pragma unroll
+                for (int l = 0; l < LM; ++l)
+                    if (l < (int)L) q[l * LS] = c[l];
+            }
+            __syncthreads();
+            if (mine) {
+                bool ch = false;
+#pragma unroll
+                for (int y = 0; y < TH; ++y) {
+                    const uint32_t n = colp[y * kPitch];
+                    ch |= n < min(w[y], lim[y]);
+                    w[y] = n;
+                }
+                plane |= __any_sync(0xFFFFFFFFu, ch);
+            }
+        }
+
+        // ---- is the packing exact for this tile? -------------------------------
+        if (mine) {
+#pragma unroll
+            for (int y = 0; y < TH; ++y) bad |= w[y] >= kNarrow && w[y] < kBig;
+        }
+        if (__syncthreads_or(bad || *(volatile uint32_t *)&sh.wide))
+            return wide_item<OV, GD>(a, fi, t, smem_raw, sh.cnt);
+        if constexpr (GD) {
+            ub = *(volatile uint32_t *)&sh.ub;
+            if (dst_here) set_limits();
+        }
+
+        // ---- write back the labels that fell -----------------------------------
+        if (mine) {
+            u64 *out = a.lab + f.lab_off + row0 + lane;
+#pragma unroll
+            for (int y = 0; y < TH; ++y)
+                if (w[y] < min(w0[y], lim[y]))
+                    out[(int64_t)y * f.ww] = ((u64)(dbase + (w[y] >> HB)) << 32) | (hbase + (w[y] & kHopMask));
+            // ---- neighbours this tile can improve --------------------------------
+            // `price` into the neighbour's cell (at gx, gy) from ours with label `own`,
+            // its staged label `there`; dir: the plane of the move; h: remaining price
+            auto check = [&](uint32_t s, bool ok, uint32_t own, uint32_t price, uint32_t there, uint32_t dir, uint32_t gx,
+                             uint32_t gy, uint32_t nb, uint32_t h) {
+                uint32_t fv = kMax;
+                bool better = false;
+                if (ok && own < kBig) {
+                    bool exact = f.n_pads && price == kBig;
+                    if constexpr (OV) exact |= f.n_over && a.tover[f.tile_off + nb];
+                    if (exact) {  // its own pad there, or its own price
+                        const uint32_t p = exact_price(a.boards + f.board, a.fields + fi, a.pads, dir, wl, gy, gx);
+                        const u64 c64 = ext2(((u64)(dbase + (own >> HB)) << 32) | (hbase + (own & kHopMask)), p, 1);
+                        const u64 t64 = there >= kBig ? kInf : ((u64)(dbase + (there >> HB)) << 32) |
+                                                                   (hbase + (there & kHopMask));
+                        better = c64 < t64;
+                        fv = (uint32_t)(c64 >> 32);
+                    } else {
+                        const uint32_t cand = own + price;
+                        better = cand < there;
+                        fv = dbase + (cand >> HB);
+                    }
+                    if constexpr (GD) {
+                        if (better) {
+                            fv = bound(fv, h);
+                            better = fv <= ub;
+                        }
+                    }
+                }
+                if constexpr (GD) {
+                    const bool now = __any_sync(0xFFFFFFFFu, better && fv <= sh.thr);
+                    const uint32_t m = __reduce_min_sync(0xFFFFFFFFu, better ? fv : kMax);
+                    if (lane == 0) {
+                        if (now) sh.push[s] = 1;
+                        else if (m != kMax) atomicMin(&sh.park[s], m);
+                    }
+                } else {
+                    if (__any_sync(0xFFFFFFFFu, better) && lane == 0) sh.push[s] = 1;
+                }
+            };
+            const uint32_t hxy = GD ? hxl : 0u;
+            if (top) check(2, col_in, w[0], pt, ht, kInPosY, (uint32_t)tx0 + lane, (uint32_t)ty0 - 1, t - ntx,
+                           GD ? dsum(hxy, sh.hy[0]) : 0u);
+            if (bottom) check(3, col_in, w[TH - 1], pb, hb, kInNegY, (uint32_t)tx0 + lane, (uint32_t)ty0 + TH, t + ntx,
+                              GD ? dsum(hxy, sh.hy[TH + 1]) : 0u);
+            const uint32_t edge = side ? lab[(wl * TH + r) * kPitch + (seg == 0 ? 0u : kTW - 1)] : kBig;
+            const uint32_t hsd = GD ? dsum(dsum(hxs, hl), sh.hy[r + 1]) : 0u;
+            if (txi > 0) check(0, side && seg == 0, edge, ps, hs, kInPosX, (uint32_t)tx0 - 1, (uint32_t)ty0 + r, t - 1, hsd);
+            if (txi + 1 < ntx)
+                check(1, side && seg == 3, edge, ps, hs, kInNegX, (uint32_t)tx0 + kTW, (uint32_t)ty0 + r, t + 1, hsd);
+        }
+        __syncthreads();
+        if (tid < 4) {
+            const uint32_t u = tid == 0 ? t - 1 : tid == 1 ? t + 1 : tid == 2 ? t - ntx : t + ntx;
+            __threadfence();  // labels before the queue entries
+            if (sh.push[tid]) {
+                async_push(a, fi, f.tile_off, u, live);
+            } else if (GD && sh.park[tid] != kMax) {
+                atomicMin(a.tpark + f.tile_off + u, sh.park[tid]);
+                __threadfence();  // before this item leaves the field's count
+            }
+            sh.push[tid] = 0;
+            sh.park[tid] = kMax;
+        } else if (tid == 4) {
+            __threadfence();
+            // release the tile with one atomic, or, if a neighbour improved it
+            // meanwhile, hold it again and carry it on, or queue it once more
+            uint32_t more = 0;
+            if (atomicCAS(state, kTileHeld, kTileIdle) != kTileHeld) {  // held and dirty
+                if (cont + 1 < kContinueLimit) {
+                    atomicExch(state, kTileHeld);
+                    __threadfence();
+                    more = 1;
+                } else {
+                    atomicExch(state, kTileQueued);
+                    async_enqueue(a, fi, t, live);
+                }
+            }
+            sh.more = more;
+            sh.dmin = sh.hmin = kMax;
+            sh.hmax = 0;
+            sh.cnt[1] += sweep;
+            if (++sh.cnt[0] == kCountBatch) {
+                if (atomicAdd(&a.ctl->activations, (unsigned long long)kCountBatch) + kCountBatch > a.activation_limit)
+                    atomicOr(&a.ctl->status, kStatusActivationLimit);
+                atomicAdd(&a.ctl->sweeps, sh.cnt[1]);
+                sh.cnt[0] = sh.cnt[1] = 0;
+            }
+        }
+        __syncthreads();
+        if (!sh.more) break;
+    }
+    bool last = false;
+    if (tid == 0) {  // this item leaves the count, after its own pushes
+        const uint32_t left = atomicSub(live, 1u) - 1u;
+        last = GD && left == 0;
+    }
+    return last;
+}
+
+constexpr u64 kReleaseField = kInf - 1;  // marks, in place of an item, a field to release
+
+template <int LM, bool OV, bool GD>
+__global__ void __launch_bounds__(LM * 32, LM == 4 ? 5 : LM == 8 ? 3 : 1) relax_layer_kernel(const __grid_constant__ RelaxArgs a) {
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    __shared__ LayerShared sh;
+    uint32_t phase = 0, fi = 0;
+    bool last = false;
+    if (threadIdx.x == 0) {
+        sh.cnt[0] = sh.cnt[1] = 0;
+        mbar_init(&sh.mbar, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    for (;;) {
+        if (threadIdx.x == 0) {
+            sh.item = GD && last ? kReleaseField : async_pop(a);
+            sh.n_spec = sh.wide = 0;
+            sh.dmin = sh.hmin = kMax;
+            sh.hmax = 0;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                sh.push[k] = 0;
+                sh.park[k] = kMax;
+            }
+        }
+        __syncthreads();
+        const u64 item = sh.item;
+        if (item == kInf) break;
+        if (GD && item == kReleaseField) {
+            field_release(a, fi, TH);
+            last = false;
+        } else {
+            fi = (uint32_t)(item >> 32);
+            last = layer_item<LM, OV, GD>(a, fi, (uint32_t)item, smem_raw, sh, phase);
+        }
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        if (sh.cnt[0]) atomicAdd(&a.ctl->activations, sh.cnt[0]);
+        if (sh.cnt[1]) atomicAdd(&a.ctl->sweeps, sh.cnt[1]);
+    }
+}
+
+template <int LM>
+const void *layer_fn_lm(bool over, bool goal) {
+    if (over) return goal ? (const void *)relax_layer_kernel<LM, true, true> : (const void *)relax_layer_kernel<LM, true, false>;
+    return goal ? (const void *)relax_layer_kernel<LM, false, true> : (const void *)relax_layer_kernel<LM, false, false>;
+}
+
+const void *layer_fn(uint32_t max_layers, bool over, bool goal) {
+    return max_layers <= 4 ? layer_fn_lm<4>(over, goal) : max_layers <= 8 ? layer_fn_lm<8>(over, goal)
+                                                                          : layer_fn_lm<16>(over, goal);
+}
+
+}  // namespace
+
+size_t layer_smem_bytes(uint32_t max_layers) {
+    const size_t narrow = layer_st_off(max_layers) + (size_t)6 * max_layers * TH * kPitch * 4;
+    return std::max(narrow, tile_layout(max_layers, TH).total);  // a wide tile is staged in the same block
+}
+
+cudaError_t layer_configure(uint32_t max_layers, size_t smem, bool over, bool goal, int *blocks_per_sm) {
+    const void *fn = layer_fn(max_layers, over, goal);
+    const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, fn, (int)max_layers * 32, smem);
+}
+
+cudaError_t layer_launch(const RelaxArgs &a, uint32_t grid, size_t smem, cudaStream_t st, bool over, bool goal) {
+    const cudaError_t e = seed_launch(a, st);
+    if (e != cudaSuccess) return e;
+    RelaxArgs copy = a;
+    void *args[] = {&copy};
+    return cudaLaunchKernel(layer_fn(a.max_layers, over, goal), dim3(grid), dim3(a.max_layers * 32), args, smem, st);
+}
+
+}  // namespace mrc

@@ -52,7 +52,7 @@ constexpr uint32_t kMaxRounds = 8;  // relaxation rounds of one activation (see 
 __device__ __forceinline__ bool via_blocked_board(uint8_t fl) { return (fl & (kViaNode | kStaticVia)) != 0; }
 
 __global__ void __launch_bounds__(256) planes_kernel(const DevBoard *boards, const uint64_t *chunk_start,
-                                                     uint32_t n_boards, uint64_t n_chunks) {
+                                                     uint32_t n_boards, uint64_t n_chunks, uint32_t hop_bits) {
     for (uint64_t ch = blockIdx.x; ch < n_chunks; ch += gridDim.x) {
         uint32_t lo = 0, hi = n_boards - 1;  // the last board whose first chunk is <= ch
         while (lo < hi) {
@@ -120,7 +120,18 @@ __global__ void __launch_bounds__(256) planes_kernel(const DevBoard *boards, con
             }
             const uint64_t o = ((uint64_t)l * b.h + y) * wp + x;
 #pragma unroll
-            for (int p = 0; p < 6; ++p) out[(uint64_t)p * NP + o] = s[p];
+            for (int p = 0; p < 6; ++p) {
+                uint32_t v = s[p];
+                if (hop_bits) {  // the layer kernel's words
+                    if (v < (1u << (29 - hop_bits))) {
+                        v = (v << hop_bits) | 1u;
+                    } else {
+                        if (v != kMax) b.goal->wide = 1;
+                        v = kPackedInf;
+                    }
+                }
+                out[(uint64_t)p * NP + o] = v;
+            }
         }
         if (b.goal) {
             BoardGoal *g = b.goal;
@@ -816,10 +827,10 @@ __global__ void warp_seed_kernel(RelaxArgs a) {
 uint64_t planes_chunks(uint64_t cells) { return (cells + kPlaneChunk - 1) / kPlaneChunk; }
 
 cudaError_t planes_launch(const DevBoard *boards, const uint64_t *chunk_start, uint32_t n_boards, uint64_t n_chunks,
-                          uint32_t sms, cudaStream_t st) {
+                          uint32_t sms, uint32_t hop_bits, cudaStream_t st) {
     if (!n_boards || !n_chunks) return cudaSuccess;
     const uint64_t blocks = std::min<uint64_t>(n_chunks, (uint64_t)sms * 8);
-    planes_kernel<<<(uint32_t)blocks, 256, 0, st>>>(boards, chunk_start, n_boards, n_chunks);
+    planes_kernel<<<(uint32_t)blocks, 256, 0, st>>>(boards, chunk_start, n_boards, n_chunks, hop_bits);
     return cudaGetLastError();
 }
 

@@ -18,8 +18,8 @@ INCLUDE = os.path.join(REPO, "include")
 BUILD = os.path.join(ROOT, "_build")
 LIB = os.path.join(PKG, "libmr_cuda.so")
 
-SOURCES = ["relax.cu", "warp_relax.cu", "negotiate.cu", "engine.cu"]
-HEADERS = ["device.cuh", "kernels.h", "tiles.cuh"]
+SOURCES = ["relax.cu", "layer_relax.cu", "warp_relax.cu", "negotiate.cu", "engine.cu"]
+HEADERS = ["cta_tile.cuh", "device.cuh", "kernels.h", "tiles.cuh", "tma.cuh"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC,-O3", "-I" + INCLUDE, "-I" + CSRC]
 

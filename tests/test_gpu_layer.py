@@ -1,0 +1,75 @@
+"""The layer kernel (32-bit tile labels, a warp per layer) against the oracle at
+the sizes where it can go wrong: window widths and heights around its 32 x 8
+tiles, window columns off its 4-column grid, every layer count class, and
+prices and path costs on both sides of what a packed word holds."""
+import numpy as np
+import pytest
+
+import mrcuda
+from mrcuda.types import COST_MAX, Dims, Grid, IsolatedRouteRequest, IsolatedRouteWindow, NetEndpoints
+from test_gpu_parity import _assert_fields
+
+pytestmark = pytest.mark.gpu
+
+
+def _board(rng, layers, price):
+    dims = Dims(72, 21, layers)
+    n = len(dims)
+    cost = np.ones(n, np.uint32)
+    cost[rng.random(n) < 0.15] = COST_MAX
+    d = rng.integers(max(price // 2, 1), price + 1, (n, 4)).astype(np.uint32)
+    d[rng.random((n, 4)) < 0.05] = COST_MAX
+    grid = Grid(dims, cost)
+    free = np.flatnonzero(cost != COST_MAX)
+    nets, wins = [], []
+    for x0 in range(5):  # every offset off the 4-column grid, and the next
+        for ww, wh in ((31, 7), (32, 8), (33, 9), (64, 16), (65, 17), (1, 20), (67 - x0, 1)):
+            x1, y0 = x0 + ww - 1, int(rng.integers(0, 21 - wh + 1))
+            inside = [int(c) for c in free if x0 <= c % 72 <= x1 and y0 <= (c // 72) % 21 < y0 + wh]
+            if not inside:
+                continue
+            src, dst = (int(v) for v in rng.choice(inside, 2))
+            nets.append(NetEndpoints(f"n{len(nets)}", src, dst))
+            wins.append(IsolatedRouteWindow(x0, y0, x1, y0 + wh - 1))
+    return IsolatedRouteRequest(grid, nets, wins, np.ones(71, np.uint32), np.ones(20, np.uint32),
+                                [int(v) for v in rng.integers(1, 2 * price + 1, layers - 1)], d)
+
+
+@pytest.mark.parametrize("layers", [1, 2, 4, 5, 8, 9, 16])
+@pytest.mark.parametrize("price", [1, 30, (1 << 16) - 1, 1 << 16, (1 << 17) - 1, 1 << 17, 1 << 25])
+def test_tile_edges_and_word_limits(oracle, layers, price):
+    req = _board(np.random.default_rng(1000 * layers + price % 997), layers, price)
+    engine = mrcuda.Engine(0)
+    try:
+        exp = oracle.isolated_batch(req, retry_full=False, mode="field")
+        got = engine.route_isolated_batch(req, retry_full=False, keep_fields=True)
+        assert (got.paths, got.search_costs) == exp
+        _assert_fields(oracle, req, got)
+        paths_only = engine.route_isolated_batch(req, retry_full=False)
+        assert (paths_only.paths, paths_only.search_costs) == exp
+    finally:
+        engine.close()
+
+
+def test_a_field_that_leaves_the_packed_range(oracle):
+    """Long hop counts and costs: a serpentine whose labels spread past one word
+    inside a tile (walls every other row, a gap at alternating ends)."""
+    w, h, layers = 64, 40, 2
+    cost = np.ones((layers, h, w), np.uint32)
+    cost[:, 1::2, :] = COST_MAX
+    for k, y in enumerate(range(1, h, 2)):
+        cost[:, y, w - 1 if k % 2 == 0 else 0] = 1
+    grid = Grid(Dims(w, h, layers), cost.reshape(-1))
+    full = IsolatedRouteWindow.full(grid.dims)
+    nets = [NetEndpoints("a", 0, w * h - w), NetEndpoints("b", w * h - w, 5)]
+    engine = mrcuda.Engine(0)
+    try:
+        for step in (1, 900, 60000):
+            req = IsolatedRouteRequest(grid, nets, [full, full], np.full(w - 1, step, np.uint32),
+                                       np.full(h - 1, step, np.uint32), [7])
+            exp = oracle.isolated_batch(req, retry_full=False, mode="field")
+            got = engine.route_isolated_batch(req, retry_full=False, keep_fields=True)
+            assert (got.paths, got.search_costs) == exp, step
+            _assert_fields(oracle, req, got)
+    finally:
+        engine.close()
