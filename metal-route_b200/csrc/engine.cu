@@ -1052,8 +1052,7 @@ PathArgs path_args(const mrc_batch *bt) {
     pa.tile_h = bt->tile_h;
     pa.arena_filled = bt->async_q ? 1u : 0u;
     pa.hop_bits = layer_hop_bits(bt->max_layers);
-    const size_t ws = walk_smem_bytes(bt->max_layers, bt->tile_h);
-    pa.walk_smem = (bt->layer && !bt->has_over && ws <= kWalkSmemLimit) ? (uint32_t)ws : 0u;
+    pa.walk_smem = bt->layer && !bt->has_over ? (uint32_t)walk_smem_bytes(bt->max_layers) : 0u;
     pa.costs = bt->d_costs.as<uint32_t>();
     pa.lens = bt->d_lens.as<uint32_t>();
     pa.offsets = bt->d_offsets.as<unsigned long long>();

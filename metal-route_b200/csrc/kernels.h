@@ -62,7 +62,7 @@ struct PathArgs {
     uint32_t tile_h;
     uint32_t hop_bits;               // of the packed price planes (tile-staged walk)
     uint32_t arena_filled;           // 1: the label arena was +inf-filled (queue schedule), tvisit not needed
-    uint32_t walk_smem;              // > 0: the tile-staged walk (packed planes + TMA maps, no overrides), its smem
+    uint32_t walk_smem;              // > 0: the tile-staged walk (packed planes, no overrides), its smem
     uint32_t *costs;                 // [n] by output slot
     uint32_t *lens;                  // [n] by output slot
     unsigned long long *offsets;     // [n+1] by output slot
@@ -223,16 +223,16 @@ cudaError_t warp_relax_launch(const RelaxArgs &a, uint32_t grid, cudaStream_t st
 // the tile's 32 columns plus the slack of rounding its first column down to a
 // multiple of 4 (16 bytes, the TMA rule for the innermost coordinate).
 constexpr uint32_t kPlaneTmaBoxW = 36;
-// Tile-staged path walk: tiles of 32 x walk_tile_rows cells over all layers,
-// their price planes brought by TMA loads of the relax kernel's box.
-constexpr uint32_t kWalkRows = 16;          // walk tile rows (at least the relax tile height)
-constexpr size_t kWalkSmemLimit = 200u << 10;  // larger tiles take the per-step walk
-__host__ __device__ inline uint32_t walk_tile_rows(uint32_t tile_h) { return tile_h > kWalkRows ? tile_h : kWalkRows; }
-__host__ __device__ inline size_t walk_smem_planes(uint32_t layers, uint32_t tile_h) {
-    return (size_t)(walk_tile_rows(tile_h) / tile_h) * 6 * layers * tile_h * kPlaneTmaBoxW * 4;
-}
-__host__ __device__ inline size_t walk_smem_bytes(uint32_t layers, uint32_t tile_h) {
-    return walk_smem_planes(layers, tile_h) + (size_t)layers * (walk_tile_rows(tile_h) + 2) * 34 * 8;
+// Tile-staged path walk: windows of 32 x walk_rows cells over all layers, a label
+// word and a predecessor offset per cell (ring included).
+__host__ __device__ inline uint32_t walk_rows(uint32_t layers) { return layers == 1 ? 64 : layers == 2 ? 32 : 16; }
+inline size_t walk_smem_bytes(uint32_t max_layers) {
+    size_t most = 0;
+    for (uint32_t l = 1; l <= max_layers; ++l) {
+        const size_t s = (size_t)l * (walk_rows(l) + 2) * 34 * 6;
+        most = s > most ? s : most;
+    }
+    return most;
 }
 // Rows of a price plane are padded to a multiple of 4 cells (16 bytes), so a
 // tensor map over the planes has 16-byte strides.

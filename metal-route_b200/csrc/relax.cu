@@ -31,7 +31,6 @@
 #include "device.cuh"
 #include "kernels.h"
 #include "tiles.cuh"
-#include "tma.cuh"
 
 namespace mrc {
 
@@ -699,16 +698,25 @@ cudaError_t relax_launch(const RelaxArgs &a, uint32_t grid, uint32_t threads, si
     return cudaLaunchKernelExC(&cfg, fn, args);
 }
 
-// Tile-staged walk, for batches whose boards carry price planes and a TMA map
-// (the CTA queue form) and whose nets carry no price overrides.  One CTA per
-// field stages a walk tile of 32 x WH cells over all layers — the labels with a
-// one-cell ring by plain loads, the six price planes by WH / tile_h TMA loads of
-// the relax kernel's box — and warp 0 walks inside it from shared memory,
-// re-staging when the path leaves the tile.  A step then costs shared-memory
-// reads instead of a round trip to L2 or HBM.  The step prices are the planes'
-// except on the stacks of the net's endpoints, and for every step of a net with
-// own or via pads, where walk_step prices exactly; the choice among the
-// candidates is path_walk_kernel's.
+// Tile-staged walk, for batches whose boards carry packed price planes (the layer
+// kernel) and whose nets carry no price overrides.  One CTA per field.  The CTA
+// stages the labels of a window of 32 x walk_rows(L) cells over all layers, with a
+// one-cell ring, relative to the current cell (D, H): word = (D - dist) << HB |
+// (H - hops), so q is a predecessor of c by a step with packed price p exactly
+// when word(q) == word(c) + p.  All threads then look for the canonical (lowest
+// CellIdx) predecessor of every cell of the window, reading a price only where a
+// neighbour's label is lower, and keep it as the offset to that neighbour in
+// shared memory; the walk itself is one thread following offsets, a shared-memory
+// load a step, until it leaves the window.  Cells priced for the net itself (own
+// pads, via pads) are looked up with exact prices, and a step that no word
+// describes (too large a price, a board of wide prices) is taken from HBM.
+//
+// Bound by a window's two round trips to HBM (labels, prices), some 3 us, and the
+// number of windows; a step inside one costs about 50 cycles.  Testing the six
+// neighbours step by step in one warp took about 0.5 us a step, and 6 us where the
+// prices are the net's own.  Longest of 256 paths on 512x512x4: 267 -> 162 us;
+// 640 instances with pads: 820 -> 147 us.  512 threads, so that the rows of a
+// window and the prices of its cells are one round of loads each (256: 211 us).
 //
 // Origin of the walk tile along one axis of extent e for a walk at c heading in
 // direction d (-1, 0, +1): a few cells behind c, so most of the tile lies ahead.
@@ -731,149 +739,253 @@ __device__ __noinline__ uint32_t walk_step_exact(const DevBoard *b, const DevFie
     return walk_step(*b, *f, pads, p, cur, x, y, l, kind, false);
 }
 
-__global__ void __launch_bounds__(256) path_walk_tiled_kernel(PathArgs a) {
-    extern __shared__ __align__(128) unsigned char wsm[];
-    __shared__ __align__(8) uint64_t s_mbar;
-    __shared__ int s_tile[2];   // walk tile origin (board x, y)
-    __shared__ uint32_t s_done;
+constexpr int kWalkThreads = 512;
+constexpr uint32_t kWalkSteps = 512;     // steps recorded per window
+constexpr uint32_t kWalkUnroll = 8;      // steps taken between two looks at whether the walk goes on
+constexpr uint32_t kWalkSpec = 256;      // cells of a window priced for the net itself
+
+__global__ void __launch_bounds__(kWalkThreads, 2) path_walk_tiled_kernel(PathArgs a) {
+    extern __shared__ __align__(16) unsigned char wsm[];
+    __shared__ uint32_t s_path[kWalkSteps + kWalkUnroll];          // cells walked in this window (indices into it)
+    __shared__ uint32_t s_spec[kWalkSpec], s_code[kWalkSpec];
+    __shared__ uint32_t s_nspec, s_n, s_ok, s_next[3];  // s_ok, s_next: after a step from HBM, the cell and its label
     const DevField f = a.fields[blockIdx.x];
     const uint32_t len = a.lens[f.out];
     if (len == 0) return;  // the same for the whole CTA
     const DevBoard b = a.boards[f.board];
-    const uint32_t L = b.layers, TH = a.tile_h, WH = walk_tile_rows(TH), nload = WH / TH;
-    const uint32_t plane = b.w * b.h;
-    uint32_t *pl = reinterpret_cast<uint32_t *>(wsm);
-    u64 *lab = reinterpret_cast<u64 *>(wsm + walk_smem_planes(L, TH));
-    const uint32_t box_words = 6 * L * TH * kPlaneTmaBoxW;
-    const bool exact_all = (f.n_pads | f.n_vpads) != 0 || b.goal->wide;
-    const uint32_t src_xy = f.src % plane, dst_xy = f.dst % plane;
-    const int sx = (int)(src_xy % b.w), sy = (int)(src_xy / b.w);  // the walk heads for the source
-    const int dstx = (int)(dst_xy % b.w), dsty = (int)(dst_xy / b.w);
+    const uint32_t L = b.layers, WH = walk_rows(L), W = kTW, PW = W + 2, PL = (WH + 2) * PW;  // ring included
+    const uint32_t HB = a.hop_bits, hop_mask = (1u << HB) - 1u, dist_lim = 1u << (29 - HB);
+    const uint32_t plane = b.w * b.h, tid = threadIdx.x, lane = tid & 31;
+    uint32_t *word = reinterpret_cast<uint32_t *>(wsm);
+    int16_t *delta = reinterpret_cast<int16_t *>(word + L * PL);
     const int wx0 = (int)f.x0, wy0 = (int)f.y0, wx1 = (int)(f.x0 + f.ww), wy1 = (int)(f.y0 + f.wh);
-    const uint32_t lane = threadIdx.x & 31;
+    const u64 *lab = a.lab + f.lab_off;
+    const uint32_t wp = planes_pitch(b.w);
+    const uint64_t NP = (uint64_t)wp * b.h * L;
+    const bool wide = b.goal->wide != 0;
     uint32_t *out = a.cells + a.offsets[f.out];
-    // walk state (warp 0)
-    uint32_t cur = f.dst, pos = len - 1;
-    int cx = (int)((f.dst % plane) % b.w), cy = (int)((f.dst % plane) / b.w), cl = (int)(f.dst / plane);
-    u64 need = a.lab[f.lab_off + ((uint64_t)(uint32_t)cl * f.wh + (uint32_t)(cy - wy0)) * f.ww + (uint32_t)(cx - wx0)];
-    uint32_t phase = 0;
-    // Per-lane constants of a step: the neighbour offset of kind `lane` (lanes 0-5),
-    // the in-price plane of the move from it into the current cell, and the
-    // relax tile height as a shift (tile heights are powers of two).
-    int ox = 0, oy = 0, oz = 0;
-    if (lane < 6) walk_offset((int)lane, ox, oy, oz);
-    const uint32_t pin = lane == 0 ? kInBelow : lane == 1 ? kInNegY : lane == 2 ? kInNegX
-                       : lane == 3 ? kInPosX : lane == 4 ? kInPosY : kInAbove;
-    const uint32_t th_shift = (uint32_t)__ffs((int)TH) - 1u;
-    if (threadIdx.x == 0) {
-        mbar_init(&s_mbar, 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        s_tile[0] = walk_origin(cx, walk_dir(cx, sx), (int)kTW);
-        s_tile[1] = walk_origin(cy, walk_dir(cy, sy), (int)WH);
-        s_done = 0;
+    const uint32_t src_xy = f.src % plane;
+    const int sx = (int)(src_xy % b.w), sy = (int)(src_xy / b.w);  // the walk heads for the source
+    // the current cell and its label (the same in every thread)
+    uint32_t pos = len - 1;
+    int cx, cy, cl;
+    {
+        const uint32_t r = f.dst % plane;
+        cx = (int)(r % b.w);
+        cy = (int)(r / b.w);
+        cl = (int)(f.dst / plane);
     }
-    for (;;) {
-        __syncthreads();
-        const int tx0 = s_tile[0], ty0 = s_tile[1];
-        const uint32_t xo = (uint32_t)tx0 & 3u;
-        if (threadIdx.x == 0) {
-            fence_proxy_async_smem();
-            mbar_expect_tx(&s_mbar, nload * box_words * 4u);
-            for (uint32_t j = 0; j < nload; ++j)
-                tma_load_4d(pl + j * box_words, b.tmap, tx0 & ~3, ty0 + (int)(j * TH), 0, 0, &s_mbar);
-        }
-        // labels of the tile and its ring (+inf outside the window), kStageBatch
-        // loads in flight per thread before any is stored
-        const uint32_t nl = L * (WH + 2) * 34;
-        constexpr uint32_t kStageBatch = 8;
-        for (uint32_t i0 = threadIdx.x; i0 < nl; i0 += kStageBatch * blockDim.x) {
-            u64 v[kStageBatch];
+    u64 need = __ldcg(lab + ((uint64_t)(uint32_t)cl * f.wh + (uint32_t)(cy - wy0)) * f.ww + (uint32_t)(cx - wx0));
+    if (tid == 0) {
+        out[pos] = f.dst;
+        s_nspec = s_n = 0;
+    }
+    int dx = walk_dir(cx, sx), dy = walk_dir(cy, sy);
+    while (pos) {
+        const int tx0 = walk_origin(cx, dx, (int)W), ty0 = walk_origin(cy, dy, (int)WH);
+        const uint32_t D = (uint32_t)(need >> 32), H = (uint32_t)need;
+        __syncthreads();  // every thread is past the previous window
+        if (!wide) {
+            // ---- labels of the window and its ring: a warp per row, several rows in flight
+            // word of the cell in column xx, row yy (ring included) of layer l, from its label
+            auto put = [&](uint32_t i, u64 v, int gx, int gy, int l) {
+                // cells of the path have no larger dist than (D, H), and fewer hops by
+                // at least their distance in cells
+                const uint32_t d = (uint32_t)(v >> 32), h = (uint32_t)v;
+                const uint32_t away = (uint32_t)(abs(gx - cx) + abs(gy - cy) + abs(l - cl));
+                const bool in = d <= D && h <= H && D - d < dist_lim && H - h <= hop_mask && H - h >= away;
+                word[i] = in ? ((D - d) << HB) | (H - h) : kMax;
+                delta[i] = 0;
+            };
+            auto label = [&](int gx, int gy, uint32_t l) -> u64 {
+                if (gx < wx0 || gx >= wx1 || gy < wy0 || gy >= wy1) return kInf;
+                return __ldcg(lab + ((uint64_t)l * f.wh + (uint32_t)(gy - wy0)) * f.ww + (uint32_t)(gx - wx0));
+            };
+            const uint32_t rows = L * (WH + 2), wid = tid >> 5, nw = blockDim.x >> 5;
+            // the last two columns, their loads issued with the rows'
+            const uint32_t eq = tid >> 1, ex = W + (tid & 1u), el = eq / (WH + 2);
+            const int egx = tx0 + (int)ex - 1, egy = ty0 + (int)(eq - el * (WH + 2)) - 1;
+            const u64 ev = eq < rows ? label(egx, egy, el) : kInf;
+            constexpr uint32_t kRows = 8;
+            for (uint32_t r0 = wid; r0 < rows; r0 += kRows * nw) {
+                u64 v[kRows];
 #pragma unroll
-            for (uint32_t k = 0; k < kStageBatch; ++k) {
-                const uint32_t i = i0 + k * blockDim.x;
-                const uint32_t sx = i % 34, r = i / 34, sy = r % (WH + 2), l = r / (WH + 2);
-                const int gx = tx0 + (int)sx - 1, gy = ty0 + (int)sy - 1;
-                v[k] = kInf;
-                if (i < nl && gx >= wx0 && gx < wx1 && gy >= wy0 && gy < wy1)
-                    v[k] = __ldcg(a.lab + f.lab_off + ((uint64_t)l * f.wh + (uint32_t)(gy - wy0)) * f.ww +
-                                  (uint32_t)(gx - wx0));
-            }
-#pragma unroll
-            for (uint32_t k = 0; k < kStageBatch; ++k)
-                if (i0 + k * blockDim.x < nl) lab[i0 + k * blockDim.x] = v[k];
-        }
-        // bounded wait for the planes (a load that never lands breaks the path)
-        for (uint32_t spins = 0; !mbar_try_wait(&s_mbar, phase & 1u); ++spins) {
-            if (spins > kTmaSpinLimit) {
-                if (threadIdx.x == 0) {
-                    atomicOr(a.status, kStatusPathBroken);
-                    s_done = 1;
+                for (uint32_t k = 0; k < kRows; ++k) {
+                    const uint32_t q = r0 + k * nw, l = q / (WH + 2), yy = q - l * (WH + 2);
+                    v[k] = q < rows ? label(tx0 + (int)lane - 1, ty0 + (int)yy - 1, l) : kInf;
                 }
-                break;
+#pragma unroll
+                for (uint32_t k = 0; k < kRows; ++k) {
+                    const uint32_t q = r0 + k * nw, l = q / (WH + 2), yy = q - l * (WH + 2);
+                    if (q < rows) put(q * PW + lane, v[k], tx0 + (int)lane - 1, ty0 + (int)yy - 1, (int)l);
+                }
             }
-        }
-        ++phase;
-        __syncthreads();
-        if (s_done) return;
-        if (threadIdx.x < 32) {
-            for (;;) {
-                if (lane == 0) out[pos] = cur;
-                if (pos == 0) {
-                    if (lane == 0) {
-                        if (cur != f.src) atomicOr(a.status, kStatusPathBroken);
-                        s_done = 1;
+            if (eq < rows) put(eq * PW + ex, ev, egx, egy, (int)el);
+            for (uint32_t e = tid + blockDim.x; e < 2 * rows; e += blockDim.x) {  // (more than 14 layers)
+                const uint32_t q = e >> 1, xx = W + (e & 1u), l = q / (WH + 2), yy = q - l * (WH + 2);
+                const int gx = tx0 + (int)xx - 1, gy = ty0 + (int)yy - 1;
+                put(q * PW + xx, label(gx, gy, l), gx, gy, (int)l);
+            }
+            // cells priced for the net itself: own pads; a via pad's cell and the cells below and above it
+            for (uint32_t k = tid; k < f.n_pads + 3 * f.n_vpads; k += blockDim.x) {
+                const uint32_t m = k - f.n_pads;
+                const uint32_t c = __ldg(a.pads + (k < f.n_pads ? f.pad_off + k : f.vpad_off + m / 3));
+                const uint32_t l = c / plane + (k < f.n_pads ? 0u : m % 3 - 1u), r = c % plane, gy = r / b.w, gx = r - gy * b.w;
+                const uint32_t xx = gx - (uint32_t)tx0, yy = gy - (uint32_t)ty0;
+                if (l >= L || xx >= W || yy >= WH) continue;
+                const uint32_t i = atomicAdd(&s_nspec, 1u);
+                if (i < kWalkSpec) {
+                    s_spec[i] = l * PL + (yy + 1) * PW + xx + 1;
+                    s_code[i] = 6;
+                }
+            }
+            __syncthreads();
+            // ---- the predecessor of every cell: neighbours in ascending CellIdx ----
+            const int off[6] = {-(int)PL, -(int)PW, -1, 1, (int)PW, (int)PL};
+            constexpr uint32_t in_plane[6] = {kInBelow, kInNegY, kInNegX, kInPosX, kInPosY, kInAbove};
+            constexpr uint32_t kCells = 4;  // cells of one thread whose prices are in flight together
+            for (uint32_t r0 = wid; r0 < L * WH; r0 += kCells * nw) {
+                uint32_t p[kCells][6];
+#pragma unroll
+                for (uint32_t k = 0; k < kCells; ++k) {
+                    const uint32_t q = r0 + k * nw, l = q / WH, yy = q % WH;
+                    const uint32_t at = l * PL + (yy + 1) * PW + lane + 1;
+                    const bool have = q < L * WH && word[at] != kMax;
+                    const uint32_t wc = have ? word[at] : 0u;
+                    const uint32_t *pr = b.planes + ((uint64_t)l * b.h + (uint32_t)(ty0 + (int)yy)) * wp + (uint32_t)(tx0 + (int)lane);
+#pragma unroll
+                    for (int n = 0; n < 6; ++n) {
+                        p[k][n] = kPackedInf;
+                        if (!have || (n == 0 && l == 0) || (n == 5 && l + 1 == L)) continue;
+                        const uint32_t wq = word[(int)at + off[n]];
+                        if (wq != kMax && wq > wc) p[k][n] = __ldg(pr + in_plane[n] * NP);
                     }
-                    break;
                 }
+#pragma unroll
+                for (uint32_t k = 0; k < kCells; ++k) {
+                    const uint32_t q = r0 + k * nw, l = q / WH, yy = q % WH;
+                    const uint32_t at = l * PL + (yy + 1) * PW + lane + 1;
+                    if (q >= L * WH) continue;
+                    const uint32_t wc = word[at];
+                    int dl = 0;
+#pragma unroll
+                    for (int n = 5; n >= 0; --n)  // a price was read only where the neighbour has a word
+                        if (p[k][n] < kPackedInf && word[(int)at + off[n]] == wc + p[k][n]) dl = off[n];
+                    if (dl) delta[at] = (int16_t)dl;
+                }
+            }
+            if (s_nspec) {  // the same for the whole CTA
+                __syncthreads();
+                const uint32_t ns = min(s_nspec, kWalkSpec);
+                for (uint32_t i = tid; i < 6 * ns; i += blockDim.x) {
+                    const uint32_t e = i / 6, at = s_spec[e];
+                    const int kind = (int)(i % 6);
+                    const uint32_t l = at / PL, q = at - l * PL, yy = q / PW, xx = q - yy * PW;
+                    const uint32_t wc = word[at];
+                    if (wc == kMax || (kind == 0 && l == 0) || (kind == 5 && l + 1 == L)) continue;
+                    int px = tx0 + (int)xx - 1, py = ty0 + (int)yy - 1, pz = (int)l;
+                    const uint32_t gx = (uint32_t)px, gy = (uint32_t)py;
+                    const int off = kind == 0 ? -(int)PL : kind == 1 ? -(int)PW : kind == 2 ? -1 : kind == 3 ? 1
+                                  : kind == 4 ? (int)PW : (int)PL;
+                    const uint32_t wq = word[(int)at + off];
+                    if (wq == kMax) continue;
+                    walk_offset(kind, px, py, pz);
+                    const uint32_t st = walk_step_exact(a.boards + f.board, a.fields + blockIdx.x, a.pads,
+                                                        ((uint32_t)pz * b.h + (uint32_t)py) * b.w + (uint32_t)px,
+                                                        (l * b.h + gy) * b.w + gx, gx, gy, l, kind);
+                    if (st < dist_lim && wq == wc + ((st << HB) | 1u)) atomicMin(&s_code[e], (uint32_t)kind);
+                }
+                __syncthreads();
+                for (uint32_t e = tid; e < ns; e += blockDim.x) {
+                    const uint32_t c = s_code[e];
+                    delta[s_spec[e]] = (int16_t)(c == 0 ? -(int)PL : c == 1 ? -(int)PW : c == 2 ? -1 : c == 3 ? 1
+                                               : c == 4 ? (int)PW : c == 5 ? (int)PL : 0);
+                }
+                // more such cells than the list holds: none of the window's steps is taken from it
+                if (s_nspec > kWalkSpec) {
+                    __syncthreads();
+                    if (tid == 0) delta[(uint32_t)cl * PL + (uint32_t)(cy - ty0 + 1) * PW + (uint32_t)(cx - tx0 + 1)] = 0;
+                }
+            }
+            __syncthreads();
+            // ---- the walk ---------------------------------------------------------
+            if (tid == 0) {
+                uint32_t at = (uint32_t)cl * PL + (uint32_t)(cy - ty0 + 1) * PW + (uint32_t)(cx - tx0 + 1), n = 0;
+                const uint32_t most = min(pos, kWalkSteps);
+                // an offset is 0 on the ring and where no predecessor was found: the walk
+                // then stays where it is, so several steps go by before it is looked at
+                for (;;) {
+                    uint32_t moved = 0;
+#pragma unroll
+                    for (uint32_t k = 0; k < kWalkUnroll; ++k) {
+                        const int d = delta[at];
+                        at = (uint32_t)((int)at + d);
+                        s_path[n + k] = at;
+                        moved += d != 0;
+                    }
+                    n += moved;
+                    if (moved < kWalkUnroll || n >= most) break;
+                }
+                s_n = min(n, most);
+                s_nspec = 0;  // for the next window
+            }
+            __syncthreads();
+        }
+        const uint32_t n = s_n;
+        if (n) {
+            for (uint32_t k = tid; k < n; k += blockDim.x) {
+                const uint32_t at = s_path[k], l = at / PL, q = at - l * PL, yy = q / PW, xx = q - yy * PW;
+                out[pos - 1 - k] = (l * b.h + (uint32_t)(ty0 + (int)yy - 1)) * b.w + (uint32_t)(tx0 + (int)xx - 1);
+            }
+            const uint32_t at = s_path[n - 1], l = at / PL, q = at - l * PL, yy = q / PW, xx = q - yy * PW, w = word[at];
+            cx = tx0 + (int)xx - 1;
+            cy = ty0 + (int)yy - 1;
+            cl = (int)l;
+            need = ((u64)(D - (w >> HB)) << 32) | (H - (w & hop_mask));
+            pos -= n;
+        } else {
+            // one step from HBM with exact prices
+            if (tid < 32) {
                 bool ok = false;
                 uint32_t p = 0;
                 u64 lp = kInf;
-                const int px = cx + ox, py = cy + oy, pz = cl + oz;
+                int px = cx, py = cy, pz = cl;
+                const uint32_t cur = ((uint32_t)cl * b.h + (uint32_t)cy) * b.w + (uint32_t)cx;
+                if (lane < 6) walk_offset((int)lane, px, py, pz);
                 if (lane < 6 && walk_inside(f, b, px, py, pz)) {
                     p = ((uint32_t)pz * b.h + (uint32_t)py) * b.w + (uint32_t)px;
-                    lp = lab[((uint32_t)pz * (WH + 2) + (uint32_t)(py - ty0 + 1)) * 34 + (uint32_t)(px - tx0 + 1)];
-                    uint32_t st;
-                    if (exact_all || (cx == sx && cy == sy) || (cx == dstx && cy == dsty)) {
-                        st = walk_step_exact(a.boards + f.board, a.fields + blockIdx.x, a.pads, p, cur, (uint32_t)cx,
-                                             (uint32_t)cy, (uint32_t)cl, (int)lane);
-                    } else {
-                        // in-price plane `pin` at cur, from the TMA box of cur's relax-tile rows
-                        const uint32_t yy = (uint32_t)(cy - ty0), j = yy >> th_shift;
-                        st = pl[j * box_words + ((pin * L + (uint32_t)cl) * TH + (yy & (TH - 1u))) * kPlaneTmaBoxW +
-                                (uint32_t)(cx - tx0) + xo];
-                        st = st >= kPackedInf ? kMax : st >> a.hop_bits;
-                    }
+                    lp = __ldcg(lab + ((uint64_t)(uint32_t)pz * f.wh + (uint32_t)(py - wy0)) * f.ww + (uint32_t)(px - wx0));
+                    const uint32_t st = walk_step_exact(a.boards + f.board, a.fields + blockIdx.x, a.pads, p, cur,
+                                                        (uint32_t)cx, (uint32_t)cy, (uint32_t)cl, (int)lane);
                     ok = lp != kInf && extend(lp, st) == need;
                 }
                 const uint32_t m = __ballot_sync(0xFFFFFFFFu, ok);
-                if (m == 0) {
-                    if (lane == 0) {
-                        atomicOr(a.status, kStatusPathBroken);
-                        s_done = 1;
-                    }
-                    break;
-                }
-                const uint32_t win = __ffs(m) - 1;
-                cur = __shfl_sync(0xFFFFFFFFu, p, win);
-                need = __shfl_sync(0xFFFFFFFFu, lp, win);
-                cx = __shfl_sync(0xFFFFFFFFu, px, win);
-                cy = __shfl_sync(0xFFFFFFFFu, py, win);
-                cl = __shfl_sync(0xFFFFFFFFu, pz, win);
-                --pos;
-                if (cx < tx0 || cx >= tx0 + (int)kTW || cy < ty0 || cy >= ty0 + (int)WH) {
-                    if (lane == 0) {  // the path left the tile: stage one ahead of cur
-                        const int dx = cx < tx0 ? -1 : cx >= tx0 + (int)kTW ? 1 : walk_dir(cx, sx);
-                        const int dy = cy < ty0 ? -1 : cy >= ty0 + (int)WH ? 1 : walk_dir(cy, sy);
-                        s_tile[0] = walk_origin(cx, dx, (int)kTW);
-                        s_tile[1] = walk_origin(cy, dy, (int)WH);
-                    }
-                    break;
+                const uint32_t win = m ? __ffs(m) - 1 : 0;
+                p = __shfl_sync(0xFFFFFFFFu, p, win);
+                lp = __shfl_sync(0xFFFFFFFFu, lp, win);
+                if (lane == 0) {
+                    s_ok = m;
+                    s_next[0] = p;
+                    s_next[1] = (uint32_t)(lp >> 32);
+                    s_next[2] = (uint32_t)lp;
+                    if (m) out[pos - 1] = p;
+                    else atomicOr(a.status, kStatusPathBroken);
                 }
             }
+            __syncthreads();
+            if (s_ok == 0) return;
+            const uint32_t p = s_next[0], r = p % plane;
+            cx = (int)(r % b.w);
+            cy = (int)(r / b.w);
+            cl = (int)(p / plane);
+            need = ((u64)s_next[1] << 32) | s_next[2];
+            --pos;
         }
-        __syncthreads();
-        if (s_done) return;
+        // the side the path left the window by, else towards the source
+        dx = cx < tx0 ? -1 : cx >= tx0 + (int)W ? 1 : walk_dir(cx, sx);
+        dy = cy < ty0 ? -1 : cy >= ty0 + (int)WH ? 1 : walk_dir(cy, sy);
     }
+    if (tid == 0 && ((uint32_t)cl * b.h + (uint32_t)cy) * b.w + (uint32_t)cx != f.src) atomicOr(a.status, kStatusPathBroken);
 }
 
 namespace {
@@ -912,7 +1024,7 @@ cudaError_t path_launch(const PathArgs &a, cudaStream_t st) {
         e = cudaFuncSetAttribute(path_walk_tiled_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)a.walk_smem);
         if (e != cudaSuccess) return e;
-        path_walk_tiled_kernel<<<a.n_fields, 256, a.walk_smem, st>>>(a);
+        path_walk_tiled_kernel<<<a.n_fields, kWalkThreads, a.walk_smem, st>>>(a);
     } else if (a.n_fields) {
         const uint32_t warps_per_block = 8;
         path_walk_kernel<<<(a.n_fields + warps_per_block - 1) / warps_per_block, 32 * warps_per_block, 0, st>>>(a);
