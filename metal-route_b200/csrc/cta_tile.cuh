@@ -487,8 +487,8 @@ static __device__ __noinline__ void stage_overrides(const DevBoard &b, const Dev
 
 // OV: the batch carries per-net directed-price overrides (negotiation with a
 // clearance; always 8-row tiles); without it none of the override lookups is
-// compiled in.  GD: goal-directed (FieldGoal); returns true when this item was
-// the last one of its field in flight, which the caller then releases or ends.
+// compiled in.  GD: goal-directed (FieldGoal).  Returns true when this item was
+// the last one in flight, of the launch or (GD) of its field.
 // WHOLE: see plane_barrier.
 template <int TH, bool ASYNC, bool OV, bool GD, bool WHOLE = false>
 __device__ __forceinline__ bool process_item(const RelaxArgs &a, uint32_t fi, uint32_t t, uint32_t round,
@@ -939,7 +939,7 @@ __device__ __forceinline__ bool process_item(const RelaxArgs &a, uint32_t fi, ui
                 }
                 if (!s_more) {  // this item leaves the in-flight count
                     const uint32_t left = atomicSub(live, 1u) - 1u;
-                    if (GD && left == 0) s_more = 2;
+                    if (left == 0) s_more = 2;
                 }
             }
             __syncthreads();
@@ -987,69 +987,6 @@ __device__ __forceinline__ bool process_item(const RelaxArgs &a, uint32_t fi, ui
     }
     __syncthreads();  // (queue form: the tile was released, or queued again, inside the loop)
     return last;
-}
-
-// A goal-directed field with nothing in flight: queue the waiting tiles that can
-// still matter, or end the field.  The calling CTA is the field's only worker.
-// Without a target label the threshold grows (twice the distance above the
-// bound, at least to the smallest f that waits; everything after kGoalPhases
-// releases); with one, every f up to the target's dist goes.
-static __device__ __noinline__ void field_release(const RelaxArgs &a, uint32_t fi, uint32_t tile_h) {
-    __shared__ uint32_t s_min;
-    const DevField f = a.fields[fi];
-    FieldGoal *fg = a.goal + fi;
-    const uint32_t ntiles = field_ntx(f) * ((f.wh + tile_h - 1) / tile_h);
-    uint32_t *park = a.tpark + f.tile_off;
-    for (;;) {
-        __threadfence();
-        if (threadIdx.x == 0) s_min = kMax;
-        __syncthreads();
-        const uint32_t ub = *(volatile const uint32_t *)&fg->ub;
-        uint32_t m = kMax;
-        for (uint32_t i = threadIdx.x; i < ntiles; i += 4 * blockDim.x) {
-            uint32_t v[4];
-#pragma unroll
-            for (uint32_t k = 0; k < 4; ++k) v[k] = i + k * blockDim.x < ntiles ? __ldcg(park + i + k * blockDim.x) : kMax;
-#pragma unroll
-            for (uint32_t k = 0; k < 4; ++k) m = min(m, v[k]);
-        }
-        m = __reduce_min_sync(0xFFFFFFFFu, m);
-        if ((threadIdx.x & 31) == 0 && m != kMax) atomicMin(&s_min, m);
-        __syncthreads();
-        m = s_min;
-        if (m == kMax || m > ub) {  // nothing waits that could matter: the field is final
-            if (threadIdx.x == 0) atomicSub(&a.ctl->count[1], 1u);
-            return;
-        }
-        uint32_t thr = kMax;
-        const uint32_t f0 = __ldcg(&fg->f0), phases = __ldcg(&fg->phases);
-        if (ub == kMax && phases + 1 < kGoalPhases) {
-            const uint32_t was = *(volatile const uint32_t *)&fg->thr, slack = was - f0;
-            thr = max(dsum(was, slack), dsum(m, slack / 2));
-        }
-        if (threadIdx.x == 0) atomicAdd(&fg->active, 1u);  // this CTA, until every release is queued
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            *(volatile uint32_t *)&fg->thr = thr;
-            fg->phases = phases + 1;
-            __threadfence();
-        }
-        __syncthreads();
-        const uint32_t lim = min(thr, ub);
-        for (uint32_t i = threadIdx.x; i < ntiles; i += blockDim.x) {
-            const uint32_t v = __ldcg(park + i);
-            if (v == kMax || v > lim) continue;
-            async_push(a, fi, f.tile_off, i, &fg->active);
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            __threadfence();
-            s_min = atomicSub(&fg->active, 1u) - 1u;
-        }
-        __syncthreads();
-        if (s_min != 0) return;  // the field's other workers carry it on
-        __syncthreads();
-    }
 }
 
 }  // namespace mrc

@@ -848,6 +848,8 @@ mrc_status batch_layout(mrc_batch *bt, uint32_t tile_h, uint32_t threads) {
         max_tiles = (uint32_t)std::max<uint64_t>(max_tiles, tiles);
     }
     if (toff > 0x7FFFFFFFull) return fail(MRC_ERR_LIMIT, "batch has more than 2^31 tiles");
+    if (bt->async_q && (bt->fields.size() >= (1u << 28) || max_tiles >= (1u << 28)))
+        return fail(MRC_ERR_LIMIT, "a queue item holds 2^28 fields and 2^28 tiles of a field");
     bt->total_tiles = (uint32_t)std::max<uint64_t>(toff, 1);
     bt->max_tiles = max_tiles;
     bt->goal = bt->layer && !(bt->flags & MRC_FLAG_KEEP_FIELDS) && toff >= (uint64_t)kGoalTilesPerSm * ctx->sms;
@@ -867,6 +869,8 @@ mrc_status batch_layout(mrc_batch *bt, uint32_t tile_h, uint32_t threads) {
     // a launch with work for the whole device takes it (its CTAs start as the
     // CTAs of launches already in flight exit: the queue form needs no co-residency)
     if (bt->grid_by_work && bt->async_q) grid = std::max(grid, std::min<uint64_t>(full, toff / kTilesPerCta));
+    // the layer kernel: no more CTAs than tiles (each would only poll)
+    if (bt->layer) grid = std::min<uint64_t>(grid, toff);
     bt->grid = (uint32_t)std::max<uint64_t>(1u, grid);
     // board table, with the step-price planes of every board (warp schedule,
     // CTA queue form) and their tensor maps (CTA queue form)
@@ -929,10 +933,16 @@ mrc_status batch_layout(mrc_batch *bt, uint32_t tile_h, uint32_t threads) {
     MRC_TRY(upload(ctx, bt->d_fields, bt->fields.data(), bt->fields.size() * sizeof(DevField), "upload fields"));
     if (bt->has_over) MRC_TRY(bt->d_tover.get(ctx, (size_t)bt->total_tiles, "override tile flags"));
     else bt->d_tover.reset();
-    // a ring of at least kMinRing slots: a slot comes round again only after that
-    // many more pushes, however few tiles the batch has
-    bt->list_cap = std::max(bt->total_tiles, kMinRing);
-    MRC_TRY(bt->d_lists.get(ctx, (size_t)bt->list_cap * (bt->async_q ? 1 : 3) * 8, "tile lists"));
+    // queue forms: a ring of at least kMinRing slots, a power of two; a slot comes
+    // round again only after that many more pushes, however few tiles the batch has
+    bt->list_cap = bt->total_tiles;
+    if (bt->async_q) {
+        bt->list_cap = kMinRing;
+        while (bt->list_cap < bt->total_tiles) bt->list_cap *= 2;
+        bt->d_lists.reset();
+    } else {
+        MRC_TRY(bt->d_lists.get(ctx, (size_t)bt->list_cap * 3 * 8, "tile lists"));
+    }
     auto up256 = [](size_t v) { return (v + 255) & ~(size_t)255; };
     bt->o_tstamp = up256(sizeof(Ctl));
     bt->o_tail = up256(bt->o_tstamp + (size_t)bt->total_tiles * 4);

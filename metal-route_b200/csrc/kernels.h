@@ -13,7 +13,7 @@ namespace mrc {
 constexpr int kRelaxThreads = 256;  // default CTA width of the relax kernel
 constexpr uint64_t kTilesPerCta = 8;  // tiles per CTA at which a queue launch can use one more CTA
 constexpr uint32_t kCountBatch = 64;    // activations a queue CTA counts locally before adding them to the launch's
-constexpr uint32_t kMinRing = 4096;     // fewest slots of the tile queue
+constexpr uint32_t kMinRing = 8192;     // fewest slots of the tile queue: more than CTAs of any launch
 // Tiles per SM from which a batch that asks for paths only is solved goal-directed.
 // Smaller ones wait on one field's chain of tiles, where the limits cost more
 // than the tiles they save (40 two-pin nets on 201x160: 0.99 x, 48 nets with
@@ -40,9 +40,9 @@ struct RelaxArgs {
     uint32_t *tstamp;           // per tile: last round it was queued for, + 1 (zeroed)
     uint32_t *tvisit;           // rounds form: per tile, labels valid (zeroed)
     const uint8_t *tover;       // nullable: per tile, 1 = its field has directed-price overrides inside it
-    u64 *lists;                 // 3 rotating lists of (field << 32 | tile); queue form: the ring of items
-    u64 *tags;                  // queue form: ticket tags of the ring (zeroed)
-    uint32_t list_cap;          // entries of one list (at least the batch's tiles)
+    u64 *lists;                 // rounds form: 3 rotating lists of (field << 32 | tile)
+    u64 *tags;                  // queue form: the ring of items (zeroed)
+    uint32_t list_cap;          // entries of one list, or of the ring (a power of two); at least the batch's tiles
     Ctl *ctl;                   // zeroed before launch
     FieldGoal *goal;            // goal-directed launches: per field (written by the seed kernel)
     uint32_t *tpark;            // goal-directed: per tile, the smallest f waiting to enter it (0xFF filled)

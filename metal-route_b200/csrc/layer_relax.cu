@@ -81,8 +81,8 @@ __device__ __forceinline__ uint32_t pack_price(uint32_t p, uint32_t *wide) {
     return kBig;
 }
 
-// Relaxes one held-to-be item; thread 0 returns whether it was the field's last
-// one in flight (GD).
+// Relaxes one held-to-be item; thread 0 returns whether it was the last one in
+// flight, of the launch or (GD) of its field.
 template <int LM, bool OV, bool GD>
 __device__ __forceinline__ bool layer_item(const RelaxArgs &a, uint32_t fi, uint32_t t, unsigned char *smem_raw,
                                            LayerShared &sh, uint32_t &phase) {
@@ -105,21 +105,21 @@ __device__ __forceinline__ bool layer_item(const RelaxArgs &a, uint32_t fi, uint
     const bool mine = wl < L;                            // this warp has a layer
     const bool col_in = mine && lane >= xlo && lane < tw;  // this lane has a column of the window
     if (tid == 0) {
+        // hold the tile before reading any label: a neighbour that improves our
+        // halo after this point marks it dirty, and we carry it on
+        atomicExch(state, kTileHeld);
         // every thread is past the previous item: the planes of this tile go
         // global -> shared while the labels are read
         fence_proxy_async_smem();
         mbar_expect_tx(&sh.mbar, 6u * L * TH * kPitch * 4u);
         tma_load_4d(st, b.tmap, tx0, ty0, 0, 0, &sh.mbar);
-        // hold the tile before reading any label: a neighbour that improves our
-        // halo after this point marks it dirty, and we carry it on
-        atomicExch(state, kTileHeld);
-        if constexpr (GD) a.tpark[f.tile_off + t] = kMax;  // what waited is in the labels read from here on
-        __threadfence();
         if constexpr (GD) {
+            a.tpark[f.tile_off + t] = kMax;  // what waited is in the labels read from here on
             const uint2 lim = __ldcg(reinterpret_cast<const uint2 *>(a.goal + fi));
             sh.ub = lim.x;   // an older (larger) bound of the target is still a bound
             sh.thr = lim.y;  // the threshold only moves while no item of the field is in flight
         }
+        __threadfence();
     }
     const uint32_t board_wide = __ldg(&b.goal->wide);
     // GD: remaining price along each axis
@@ -154,6 +154,7 @@ __device__ __forceinline__ bool layer_item(const RelaxArgs &a, uint32_t fi, uint
     uint32_t pt = kBig, pb = kBig, ps = kBig;  // prices into the neighbour tiles' border cells
     const bool top = tyi > 0, bottom = tyi + 1 < nty;
     const bool side = mine && r < th && ((seg == 0 && txi > 0) || (seg == 3 && txi + 1 < ntx));
+    bool last = false;
     for (uint32_t cont = 0;; ++cont) {
         // ---- labels of the column, the halo rows and the halo columns ----------
         u64 v[TH], vt = kInf, vb = kInf, vs = kInf;
@@ -547,55 +548,151 @@ __device__ __forceinline__ bool layer_item(const RelaxArgs &a, uint32_t fi, uint
                 check(1, side && seg == 3, edge, ps, hs, kInNegX, (uint32_t)tx0 + kTW, (uint32_t)ty0 + r, t + 1, hsd);
         }
         __syncthreads();
-        if (tid < 4) {
-            const uint32_t u = tid == 0 ? t - 1 : tid == 1 ? t + 1 : tid == 2 ? t - ntx : t + ntx;
-            __threadfence();  // labels before the queue entries
-            if (sh.push[tid]) {
-                async_push(a, fi, f.tile_off, u, live);
-            } else if (GD && sh.park[tid] != kMax) {
-                atomicMin(a.tpark + f.tile_off + u, sh.park[tid]);
-                __threadfence();  // before this item leaves the field's count
-            }
-            sh.push[tid] = 0;
-            sh.park[tid] = kMax;
-        } else if (tid == 4) {
-            __threadfence();
-            // release the tile with one atomic, or, if a neighbour improved it
-            // meanwhile, hold it again and carry it on, or queue it once more
+        if (tid < 32) {
+            // Lanes 0-3: the neighbours this tile improves; lane 4: the tile itself,
+            // released, or, if a neighbour improved it meanwhile, held again and
+            // carried on, or queued once more.  The lanes go through each round trip
+            // together: the states, then the count of items in flight (this item out,
+            // the pushed ones in) beside the tickets, then the slots.
+            const uint32_t u = lane == 0 ? t - 1 : lane == 1 ? t + 1 : lane == 2 ? t - ntx : lane == 3 ? t + ntx : t;
+            const bool push = lane < 4 && sh.push[lane & 3u], park = GD && lane < 4 && !push && sh.park[lane & 3u] != kMax;
+            uint32_t *us = a.tstamp + f.tile_off + u;
+            bool queued = false;  // this lane has an item to publish
             uint32_t more = 0;
-            if (atomicCAS(state, kTileHeld, kTileIdle) != kTileHeld) {  // held and dirty
-                if (cont + 1 < kContinueLimit) {
-                    atomicExch(state, kTileHeld);
-                    __threadfence();
-                    more = 1;
-                } else {
-                    atomicExch(state, kTileQueued);
-                    async_enqueue(a, fi, t, live);
+            __threadfence();      // the labels before the states
+            if (push || lane == 4) {
+                uint32_t old = atomicCAS(us, push ? kTileIdle : kTileHeld, push ? kTileQueued : kTileIdle);
+                if (push) {
+                    for (int tries = 0; old == kTileHeld; ++tries) {  // held: mark it dirty, or find it released
+                        if (atomicCAS(us, kTileHeld, kTileHeldDirty) == kTileHeld) break;
+                        old = atomicCAS(us, kTileIdle, kTileQueued);
+                        if (tries == 1024) {
+                            atomicOr(&a.ctl->status, kStatusQueueOverflow);
+                            break;
+                        }
+                    }
+                    queued = old == kTileIdle;  // else its holder, or the next one, reads our labels
+                } else if (old != kTileHeld) {  // held and dirty
+                    more = cont + 1 < kContinueLimit;
+                    queued = !more;
+                    atomicExch(us, more ? kTileHeld : kTileQueued);
                 }
             }
-            sh.more = more;
-            sh.dmin = sh.hmin = kMax;
-            sh.hmax = 0;
-            sh.cnt[1] += sweep;
-            if (++sh.cnt[0] == kCountBatch) {
-                if (atomicAdd(&a.ctl->activations, (unsigned long long)kCountBatch) + kCountBatch > a.activation_limit)
-                    atomicOr(&a.ctl->status, kStatusActivationLimit);
-                atomicAdd(&a.ctl->sweeps, sh.cnt[1]);
-                sh.cnt[0] = sh.cnt[1] = 0;
+            if (park) atomicMin(a.tpark + f.tile_off + u, sh.park[lane & 3u]);
+            if (__any_sync(0xFFFFFFFFu, park || more)) __threadfence();  // before the count; before the labels are read again
+            more = __shfl_sync(0xFFFFFFFFu, more, 4);
+            const uint32_t mask = __ballot_sync(0xFFFFFFFFu, queued), n = __popc(mask);
+            uint32_t got = 0;
+            if ((lane == 0 && (n || !more)) || (lane == 1 && n))
+                got = atomicAdd(lane == 0 ? live : &a.ctl->count[0], lane == 0 ? n + more - 1u : n);
+            const uint32_t in_flight = __shfl_sync(0xFFFFFFFFu, got, 0), h0 = __shfl_sync(0xFFFFFFFFu, got, 1);
+            if (queued) queue_store(a, h0 + __popc(mask & ((1u << lane) - 1u)), queue_item(fi, u));
+            last = !more && in_flight + n == 1u;
+            if (lane == 0) {
+                sh.more = more;
+                sh.dmin = sh.hmin = kMax;
+                sh.hmax = 0;
+                sh.cnt[1] += sweep;
+                if (++sh.cnt[0] == kCountBatch) {
+                    if (atomicAdd(&a.ctl->activations, (unsigned long long)kCountBatch) + kCountBatch > a.activation_limit)
+                        atomicOr(&a.ctl->status, kStatusActivationLimit);
+                    atomicAdd(&a.ctl->sweeps, sh.cnt[1]);
+                    sh.cnt[0] = sh.cnt[1] = 0;
+                }
+            }
+            __syncwarp();
+            if (lane < 4) {
+                sh.push[lane] = 0;
+                sh.park[lane] = kMax;
             }
         }
         __syncthreads();
         if (!sh.more) break;
     }
-    bool last = false;
-    if (tid == 0) {  // this item leaves the count, after its own pushes
-        const uint32_t left = atomicSub(live, 1u) - 1u;
-        last = GD && left == 0;
-    }
     return last;
 }
 
-constexpr u64 kReleaseField = kInf - 1;  // marks, in place of an item, a field to release
+// The launch is over: an end word for every ticket that a CTA of the launch holds
+// or will take.
+__device__ __forceinline__ void end_launch(const RelaxArgs &a) {
+    const uint32_t tail = *(volatile const uint32_t *)&a.ctl->count[0];
+    for (uint32_t k = threadIdx.x; k < gridDim.x; k += blockDim.x) queue_store(a, tail + k, kSlotItem);
+}
+
+// A goal-directed field with nothing in flight: queue the waiting tiles that can
+// still matter, or end the field.  The calling CTA is the field's only worker.
+// Without a target label the threshold grows (twice the distance above the
+// bound, at least to the smallest f that waits; everything after kGoalPhases
+// releases); with one, every f up to the target's dist goes.
+// Returns whether it was the launch's last field.
+__device__ __noinline__ bool field_release(const RelaxArgs &a, uint32_t fi) {
+    __shared__ uint32_t s_min;
+    const DevField f = a.fields[fi];
+    FieldGoal *fg = a.goal + fi;
+    const uint32_t ntiles = field_ntx(f) * ((f.wh + TH - 1) / TH);
+    uint32_t *park = a.tpark + f.tile_off;
+    for (;;) {
+        __threadfence();
+        if (threadIdx.x == 0) s_min = kMax;
+        __syncthreads();
+        const uint32_t ub = *(volatile const uint32_t *)&fg->ub;
+        uint32_t m = kMax;
+        for (uint32_t i = threadIdx.x; i < ntiles; i += 4 * blockDim.x) {
+            uint32_t v[4];
+#pragma unroll
+            for (uint32_t k = 0; k < 4; ++k) v[k] = i + k * blockDim.x < ntiles ? __ldcg(park + i + k * blockDim.x) : kMax;
+#pragma unroll
+            for (uint32_t k = 0; k < 4; ++k) m = min(m, v[k]);
+        }
+        m = __reduce_min_sync(0xFFFFFFFFu, m);
+        if ((threadIdx.x & 31) == 0 && m != kMax) atomicMin(&s_min, m);
+        __syncthreads();
+        m = s_min;
+        if (m == kMax || m > ub) {  // nothing waits that could matter: the field is final
+            __syncthreads();
+            if (threadIdx.x == 0) s_min = atomicSub(&a.ctl->count[1], 1u);
+            __syncthreads();
+            return s_min == 1u;
+        }
+        uint32_t thr = kMax;
+        const uint32_t f0 = __ldcg(&fg->f0), phases = __ldcg(&fg->phases);
+        if (ub == kMax && phases + 1 < kGoalPhases) {
+            const uint32_t was = *(volatile const uint32_t *)&fg->thr, slack = was - f0;
+            thr = max(dsum(was, slack), dsum(m, slack / 2));
+        }
+        if (threadIdx.x == 0) atomicAdd(&fg->active, 1u);  // this CTA, until every release is queued
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            *(volatile uint32_t *)&fg->thr = thr;
+            fg->phases = phases + 1;
+            __threadfence();
+        }
+        __syncthreads();
+        const uint32_t lim = min(thr, ub);
+        const uint32_t lane = threadIdx.x & 31u;
+        for (uint32_t i0 = threadIdx.x - lane; i0 < ntiles; i0 += blockDim.x) {
+            const uint32_t i = i0 + lane, v = i < ntiles ? __ldcg(park + i) : kMax;
+            const bool go = v != kMax && v <= lim && atomicCAS(a.tstamp + f.tile_off + i, kTileIdle, kTileQueued) == kTileIdle;
+            const uint32_t mask = __ballot_sync(0xFFFFFFFFu, go), n = __popc(mask);
+            if (!n) continue;
+            uint32_t got = 0;
+            if (lane < 2) got = atomicAdd(lane == 0 ? &fg->active : &a.ctl->count[0], n);
+            const uint32_t live = __shfl_sync(0xFFFFFFFFu, got, 0), h0 = __shfl_sync(0xFFFFFFFFu, got, 1);
+            // (live is used so that its round trip ends before the items are visible)
+            if (go && live != kMax) queue_store(a, h0 + __popc(mask & ((1u << lane) - 1u)), queue_item(fi, i));
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            __threadfence();
+            s_min = atomicSub(&fg->active, 1u) - 1u;
+        }
+        __syncthreads();
+        if (s_min != 0) return false;  // the field's other workers carry it on
+        __syncthreads();
+    }
+}
+
+constexpr u64 kReleaseField = kInf - 1;  // in place of an item: this CTA finished the last one in flight
 
 template <int LM, bool OV, bool GD>
 __global__ void __launch_bounds__(LM * 32, LM == 4 ? 5 : LM == 8 ? 3 : 1) relax_layer_kernel(const __grid_constant__ RelaxArgs a) {
@@ -611,7 +708,7 @@ __global__ void __launch_bounds__(LM * 32, LM == 4 ? 5 : LM == 8 ? 3 : 1) relax_
     __syncthreads();
     for (;;) {
         if (threadIdx.x == 0) {
-            sh.item = GD && last ? kReleaseField : async_pop(a);
+            sh.item = last ? kReleaseField : async_pop<64>(a);
             sh.n_spec = sh.wide = 0;
             sh.dmin = sh.hmin = kMax;
             sh.hmax = 0;
@@ -624,8 +721,11 @@ __global__ void __launch_bounds__(LM * 32, LM == 4 ? 5 : LM == 8 ? 3 : 1) relax_
         __syncthreads();
         const u64 item = sh.item;
         if (item == kInf) break;
-        if (GD && item == kReleaseField) {
-            field_release(a, fi, TH);
+        if (item == kReleaseField) {  // nothing in flight: of the field (GD), of the launch
+            if (!GD || field_release(a, fi)) {
+                end_launch(a);
+                break;
+            }
             last = false;
         } else {
             fi = (uint32_t)(item >> 32);

@@ -31,12 +31,24 @@ __device__ __forceinline__ uint32_t dsum(uint32_t a, uint32_t b) {
 
 __device__ __forceinline__ u64 umin64(u64 a, u64 b) { return a < b ? a : b; }
 
-// Work queue of the asynchronous form.  count[0] = tickets handed to pushers
-// (tail), head[0] = tickets handed to poppers, count[1] = items queued or in
-// flight.  lists[0, cap) holds the items, tags[0, cap) their ticket tags
-// (ticket + 1, zeroed before launch).  A tile is queued at most once at a time
-// (its tstamp word is the queued flag), so cap = total tiles never overflows.
-constexpr uint32_t kQueueSpinLimit = 1u << 24;  // polls of one wait (~16 s with the backoff below)
+// Work queue of the queue forms.  count[0] = tickets handed to pushers (tail),
+// head[0] = tickets handed to poppers, count[1] = items queued or in flight (or,
+// goal-directed, unfinished fields).  tags[0, list_cap), list_cap a power of two, is
+// the ring: one 64-bit word per slot, lap << 56 | field << 28 | tile, so an item is
+// published and taken with one store and one load (zeroed before launch; laps count
+// 1..255).  A tile is queued at most once at a time (its tstamp word is the queued
+// flag), so list_cap >= total tiles never overflows.
+constexpr uint32_t kQueueSpinLimit = 1u << 25;  // polls of one wait (seconds with the backoff below)
+constexpr u64 kSlotItem = (1ull << 56) - 1;     // the item bits of a slot word; all ones: the launch is over
+
+__device__ __forceinline__ u64 queue_lap(const RelaxArgs &a, uint32_t h) {
+    return (u64)((h >> (31 - __clz((int)a.list_cap))) % 255u + 1u) << 56;
+}
+// Publishes item (fi, u) under ticket h; what the item relies on was ordered before.
+__device__ __forceinline__ void queue_store(const RelaxArgs &a, uint32_t h, u64 item) {
+    __stcg(a.tags + (h & (a.list_cap - 1u)), queue_lap(a, h) | item);
+}
+__device__ __forceinline__ u64 queue_item(uint32_t fi, uint32_t u) { return ((u64)fi << 28) | u; }
 
 // Tile states in the tstamp word: 0 idle, 1 queued, 2 held by a worker,
 // 3 held and improved again meanwhile (the holder continues it in place, or
@@ -48,13 +60,10 @@ constexpr uint32_t kTileIdle = 0, kTileQueued = 1, kTileHeld = 2, kTileHeldDirty
 // `live`: the count of items queued or in flight, the launch's (count[1]) or, in
 // a goal-directed launch, the field's (count[1] then counts unfinished fields).
 __device__ __forceinline__ void async_enqueue(const RelaxArgs &a, uint32_t fi, uint32_t u, uint32_t *live) {
-    Ctl *c = a.ctl;
     atomicAdd(live, 1u);  // in flight before it is visible
-    const uint32_t h = atomicAdd(&c->count[0], 1u);
-    const size_t slot = h % a.list_cap;
-    a.lists[slot] = ((u64)fi << 32) | u;
+    const uint32_t h = atomicAdd(&a.ctl->count[0], 1u);
     __threadfence();
-    atomicExch(a.tags + slot, (u64)h + 1u);
+    queue_store(a, h, queue_item(fi, u));
 }
 
 __device__ __forceinline__ void async_push(const RelaxArgs &a, uint32_t fi, uint32_t tile_off, uint32_t u,
@@ -83,23 +92,26 @@ __device__ __forceinline__ void async_release(const RelaxArgs &a, uint32_t fi, u
     }
 }
 
-// Next item for the calling worker (one thread), or kInf when no work is left.  The
-// wait is bounded: kQueueSpinLimit polls, then kStatusBarrier and an exit.
+// Next item for the calling worker (one thread) as field << 32 | tile, or kInf when
+// no work is left.  The wait is bounded: kQueueSpinLimit polls, then
+// kStatusBarrier and an exit.  Each waiter polls its own slot; the shared words
+// (the in-flight count, the status) are read every kCheck-th poll, and the sleep
+// between polls doubles up to 128 ns: a longer one delays every hop of a lone
+// field, whose next item goes to the CTA that has waited longest.
+template <uint32_t kCheck = 16>
 __device__ __forceinline__ u64 async_pop(const RelaxArgs &a) {
     Ctl *c = a.ctl;
     const uint32_t h = atomicAdd(&c->head[0], 1u);
-    const size_t slot = h % a.list_cap;
-    const volatile u64 *tag = a.tags + slot;
-    // Each waiter polls its own slot tag; the shared in-flight count and status
-    // words (which every worker updates) are read only every 16th poll, and the
-    // sleep between polls doubles up to 1 us, so thousands of idle waiters do
-    // not flood one L2 line while the busy workers update it.
+    const volatile u64 *slot = a.tags + (h & (a.list_cap - 1u));
+    const u64 lap = queue_lap(a, h);
     for (uint32_t spins = 0;; ++spins) {
-        if (*tag == (u64)h + 1u) {
+        const u64 v = *slot;
+        if ((v & ~kSlotItem) == lap) {
             __threadfence();
-            return __ldcg(a.lists + slot);
+            const u64 item = v & kSlotItem;
+            return item == kSlotItem ? kInf : ((item >> 28) << 32) | (item & 0xFFFFFFFu);
         }
-        if ((spins & 15u) == 15u) {
+        if (spins % kCheck == kCheck - 1u) {
             if (*(volatile const uint32_t *)&c->count[1] == 0u) return kInf;  // nothing queued or running
             if (*(volatile const uint32_t *)&c->status) return kInf;
         }
@@ -107,7 +119,7 @@ __device__ __forceinline__ u64 async_pop(const RelaxArgs &a) {
             atomicOr(&c->status, kStatusBarrier);
             return kInf;
         }
-        __nanosleep(32u << min(spins >> 4, 5u));
+        __nanosleep(spins < 32u ? 20u : spins < 64u ? 64u : 128u);
     }
 }
 
