@@ -54,7 +54,8 @@ struct LayerShared {
     uint64_t mbar;  // completion of the price-plane TMA loads
     unsigned long long cnt[2];  // activations and sweeps not yet added to the launch's
     uint32_t n_spec, wide, dmin, hmin, hmax, ub, thr, more;
-    uint32_t push[4], park[4];  // left, right, top, bottom
+    uint32_t push;              // bits: left, right, top, bottom improved
+    uint32_t park[4];           // GD: the smallest f that waits to enter each
     uint32_t hy[TH + 2];        // GD: remaining price along y, rows -1 .. TH
     uint32_t spec[kSpecCap];
 };
@@ -79,6 +80,60 @@ __device__ __forceinline__ uint32_t pack_price(uint32_t p, uint32_t *wide) {
     if (p < (kNarrow >> HB)) return (p << HB) | 1u;
     if (p != kMax) *wide = 1;
     return kBig;
+}
+
+// The stacks of rows y = y0, y0 + step, ...: the layers upward, then downward.  NL is
+// the layer count at compile time, so that all labels and prices of a stack are
+// loaded before any is used.
+template <int NL>
+__device__ __forceinline__ void stack_rows(uint32_t *lab, const uint32_t *st, uint32_t y0, uint32_t step) {
+    constexpr uint32_t LS = TH * kPitch, SP = NL * LS;  // words from a layer, from a plane, to the next
+#pragma unroll 2
+    for (uint32_t y = y0; y < TH; y += step) {
+        uint32_t *q = lab + y * kPitch;
+        const uint32_t *pu = st + kInBelow * SP + y * kPitch, *pd = st + kInAbove * SP + y * kPitch;
+        uint32_t c[NL], up[NL], down[NL];
+#pragma unroll
+        for (int l = 0; l < NL; ++l) {
+            c[l] = q[l * LS];
+            if (l) up[l] = pu[l * LS];
+            if (l + 1 < NL) down[l] = pd[l * LS];
+        }
+#pragma unroll
+        for (int l = 1; l < NL; ++l) c[l] = __viaddmin_u32(c[l - 1], up[l], c[l]);
+#pragma unroll
+        for (int l = NL - 2; l >= 0; --l) c[l] = __viaddmin_u32(c[l + 1], down[l], c[l]);
+#pragma unroll
+        for (int l = 0; l < NL; ++l) q[l * LS] = c[l];
+    }
+}
+
+template <int LM>
+__device__ __forceinline__ void stack_pass_layers(uint32_t *lab, const uint32_t *st, uint32_t L, uint32_t y0,
+                                                  uint32_t step) {
+    switch (L) {
+        case 2: return stack_rows<2>(lab, st, y0, step);
+        case 3: return stack_rows<3>(lab, st, y0, step);
+        case 4: return stack_rows<4>(lab, st, y0, step);
+    }
+    if constexpr (LM > 4) {
+        switch (L) {
+            case 5: return stack_rows<5>(lab, st, y0, step);
+            case 6: return stack_rows<6>(lab, st, y0, step);
+            case 7: return stack_rows<7>(lab, st, y0, step);
+            case 8: return stack_rows<8>(lab, st, y0, step);
+        }
+    }
+    if constexpr (LM > 8) {  // 9 .. 16 layers, in shared memory
+        const uint32_t LS = TH * kPitch, SP = L * LS;
+        for (uint32_t y = y0; y < TH; y += step) {
+            uint32_t *q = lab + y * kPitch;
+            const uint32_t *pu = st + kInBelow * SP + y * kPitch, *pd = st + kInAbove * SP + y * kPitch;
+            uint32_t c = q[0];
+            for (uint32_t l = 1; l < L; ++l) q[l * LS] = c = __viaddmin_u32(c, pu[l * LS], q[l * LS]);
+            for (uint32_t l = L - 1; l-- > 0;) q[l * LS] = c = __viaddmin_u32(c, pd[l * LS], q[l * LS]);
+        }
+    }
 }
 
 // Relaxes one held-to-be item; thread 0 returns whether it was the last one in
@@ -445,25 +500,7 @@ __device__ __forceinline__ bool layer_item(const RelaxArgs &a, uint32_t fi, uint
             if (L == 1) continue;
             // the plane's labels are in shared memory, as of the last row pass or the
             // start; a column pass that ended the loop changed nothing
-            for (uint32_t s = tid; s < TH * kTW; s += blockDim.x) {
-                uint32_t *q = lab + (s >> 5) * kPitch + lane;
-                const uint32_t *pu = st + kInBelow * SP + (s >> 5) * kPitch + lane;
-                const uint32_t *pd = st + kInAbove * SP + (s >> 5) * kPitch + lane;
-                constexpr uint32_t LS = TH * kPitch;  // words from a layer to the next
-                uint32_t c[LM];
-#pragma unroll
-                for (int l = 0; l < LM; ++l)
-                    if (l < (int)L) c[l] = q[l * LS];
-#pragma unroll
-                for (int l = 1; l < LM; ++l)
-                    if (l < (int)L) c[l] = __viaddmin_u32(c[l - 1], pu[l * LS], c[l]);
-#pragma unroll
-                for (int l = LM - 2; l >= 0; --l)
-                    if (l + 1 < (int)L) c[l] = __viaddmin_u32(c[l + 1], pd[l * LS], c[l]);
-#pragma unroll
-                for (int l = 0; l < LM; ++l)
-                    if (l < (int)L) q[l * LS] = c[l];
-            }
+            stack_pass_layers<LM>(lab + lane, st + lane, L, wl, blockDim.x >> 5);
             __syncthreads();
             if (mine) {
                 bool ch = false;
@@ -497,55 +534,66 @@ __device__ __forceinline__ bool layer_item(const RelaxArgs &a, uint32_t fi, uint
                 if (w[y] < min(w0[y], lim[y]))
                     out[(int64_t)y * f.ww] = ((u64)(dbase + (w[y] >> HB)) << 32) | (hbase + (w[y] & kHopMask));
             // ---- neighbours this tile can improve --------------------------------
-            // `price` into the neighbour's cell (at gx, gy) from ours with label `own`,
-            // its staged label `there`; dir: the plane of the move; h: remaining price
-            auto check = [&](uint32_t s, bool ok, uint32_t own, uint32_t price, uint32_t there, uint32_t dir, uint32_t gx,
-                             uint32_t gy, uint32_t nb, uint32_t h) {
-                uint32_t fv = kMax;
-                bool better = false;
-                if (ok && own < kBig) {
-                    bool exact = f.n_pads && price == kBig;
-                    if constexpr (OV) exact |= f.n_over && a.tover[f.tile_off + nb];
-                    if (exact) {  // its own pad there, or its own price
-                        const uint32_t p = exact_price(a.boards + f.board, a.fields + fi, a.pads, dir, wl, gy, gx);
-                        const u64 c64 = ext2(((u64)(dbase + (own >> HB)) << 32) | (hbase + (own & kHopMask)), p, 1);
-                        const u64 t64 = there >= kBig ? kInf : ((u64)(dbase + (there >> HB)) << 32) |
-                                                                   (hbase + (there & kHopMask));
-                        better = c64 < t64;
-                        fv = (uint32_t)(c64 >> 32);
-                    } else {
-                        const uint32_t cand = own + price;
-                        better = cand < there;
-                        fv = dbase + (cand >> HB);
-                    }
-                    if constexpr (GD) {
-                        if (better) {
-                            fv = bound(fv, h);
-                            better = fv <= ub;
-                        }
-                    }
-                }
-                if constexpr (GD) {
-                    const bool now = __any_sync(0xFFFFFFFFu, better && fv <= sh.thr);
-                    const uint32_t m = __reduce_min_sync(0xFFFFFFFFu, better ? fv : kMax);
-                    if (lane == 0) {
-                        if (now) sh.push[s] = 1;
-                        else if (m != kMax) atomicMin(&sh.park[s], m);
-                    }
-                } else {
-                    if (__any_sync(0xFFFFFFFFu, better) && lane == 0) sh.push[s] = 1;
-                }
-            };
-            const uint32_t hxy = GD ? hxl : 0u;
-            if (top) check(2, col_in, w[0], pt, ht, kInPosY, (uint32_t)tx0 + lane, (uint32_t)ty0 - 1, t - ntx,
-                           GD ? dsum(hxy, sh.hy[0]) : 0u);
-            if (bottom) check(3, col_in, w[TH - 1], pb, hb, kInNegY, (uint32_t)tx0 + lane, (uint32_t)ty0 + TH, t + ntx,
-                              GD ? dsum(hxy, sh.hy[TH + 1]) : 0u);
+            // Each lane has three border cells: the top and the bottom of its column
+            // and, in the row layout, the first or last of its row.  own: our label
+            // there; price: of the move into the neighbour; there: the neighbour's
+            // staged label.
             const uint32_t edge = side ? lab[(wl * TH + r) * kPitch + (seg == 0 ? 0u : kTW - 1)] : kBig;
-            const uint32_t hsd = GD ? dsum(dsum(hxs, hl), sh.hy[r + 1]) : 0u;
-            if (txi > 0) check(0, side && seg == 0, edge, ps, hs, kInPosX, (uint32_t)tx0 - 1, (uint32_t)ty0 + r, t - 1, hsd);
-            if (txi + 1 < ntx)
-                check(1, side && seg == 3, edge, ps, hs, kInNegX, (uint32_t)tx0 + kTW, (uint32_t)ty0 + r, t + 1, hsd);
+            uint32_t own[3] = {w[0], w[TH - 1], edge}, price[3] = {pt, pb, ps}, there[3] = {ht, hb, hs};
+            uint32_t fv[3];    // GD: f of the improved label
+            bool better[3];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const uint32_t cand = own[k] + price[k];
+                better[k] = cand < there[k];  // (no price or label: at least kBig, as `there` at most)
+                fv[k] = dbase + (cand >> HB);
+            }
+            if (f.n_pads || (OV && f.n_over)) {  // its own pads, or its own prices, beyond the border
+#pragma unroll 1
+                for (int k = 0; k < 3; ++k) {
+                    const uint32_t o = k == 0 ? w[0] : k == 1 ? w[TH - 1] : edge, p0 = k == 0 ? pt : k == 1 ? pb : ps;
+                    const bool ok = (k == 0 ? col_in && top : k == 1 ? col_in && bottom : side) && o < kBig;
+                    bool exact = f.n_pads && p0 == kBig;
+                    if constexpr (OV) {
+                        const uint32_t nb = k == 0 ? t - ntx : k == 1 ? t + ntx : seg == 0 ? t - 1 : t + 1;
+                        exact |= ok && f.n_over && a.tover[f.tile_off + nb];
+                    }
+                    if (!ok || !exact) continue;
+                    const uint32_t gx = k < 2 ? (uint32_t)tx0 + lane : seg == 0 ? (uint32_t)tx0 - 1 : (uint32_t)tx0 + kTW;
+                    const uint32_t gy = k == 0 ? (uint32_t)ty0 - 1 : k == 1 ? (uint32_t)ty0 + TH : (uint32_t)ty0 + r;
+                    const uint32_t dir = k == 0 ? kInPosY : k == 1 ? kInNegY : seg == 0 ? kInPosX : kInNegX;
+                    const uint32_t p = exact_price(a.boards + f.board, a.fields + fi, a.pads, dir, wl, gy, gx);
+                    const uint32_t q = k == 0 ? ht : k == 1 ? hb : hs;
+                    const u64 c64 = ext2(((u64)(dbase + (o >> HB)) << 32) | (hbase + (o & kHopMask)), p, 1);
+                    const u64 q64 = q >= kBig ? kInf : ((u64)(dbase + (q >> HB)) << 32) | (hbase + (q & kHopMask));
+                    const bool b64 = c64 < q64;
+                    if (k == 0) { better[0] = b64; fv[0] = (uint32_t)(c64 >> 32); }
+                    else if (k == 1) { better[1] = b64; fv[1] = (uint32_t)(c64 >> 32); }
+                    else { better[2] = b64; fv[2] = (uint32_t)(c64 >> 32); }
+                }
+            }
+            bool wait[3] = {false, false, false};
+            if constexpr (GD) {
+                const uint32_t thr = sh.thr;
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    const uint32_t h = k == 0 ? dsum(hxl, sh.hy[0]) : k == 1 ? dsum(hxl, sh.hy[TH + 1])
+                                                                            : dsum(dsum(hxs, hl), sh.hy[r + 1]);
+                    fv[k] = bound(fv[k], h);
+                    better[k] &= fv[k] <= ub;
+                    wait[k] = better[k] && fv[k] > thr;
+                    better[k] &= !wait[k];
+                }
+            }
+            uint32_t sides = (__any_sync(0xFFFFFFFFu, better[2] && seg == 0) ? 1u : 0u) |
+                             (__any_sync(0xFFFFFFFFu, better[2] && seg == 3) ? 2u : 0u) |
+                             (__any_sync(0xFFFFFFFFu, better[0]) ? 4u : 0u) | (__any_sync(0xFFFFFFFFu, better[1]) ? 8u : 0u);
+            if (lane == 0 && sides) atomicOr(&sh.push, sides);
+            if (GD && __any_sync(0xFFFFFFFFu, wait[0] || wait[1] || wait[2])) {
+                if (wait[0]) atomicMin(&sh.park[2], fv[0]);
+                if (wait[1]) atomicMin(&sh.park[3], fv[1]);
+                if (wait[2]) atomicMin(&sh.park[seg == 0 ? 0 : 1], fv[2]);
+            }
         }
         __syncthreads();
         if (tid < 32) {
@@ -555,7 +603,7 @@ __device__ __forceinline__ bool layer_item(const RelaxArgs &a, uint32_t fi, uint
             // together: the states, then the count of items in flight (this item out,
             // the pushed ones in) beside the tickets, then the slots.
             const uint32_t u = lane == 0 ? t - 1 : lane == 1 ? t + 1 : lane == 2 ? t - ntx : lane == 3 ? t + ntx : t;
-            const bool push = lane < 4 && sh.push[lane & 3u], park = GD && lane < 4 && !push && sh.park[lane & 3u] != kMax;
+            const bool push = lane < 4 && ((sh.push >> lane) & 1u), park = GD && lane < 4 && !push && sh.park[lane & 3u] != kMax;
             uint32_t *us = a.tstamp + f.tile_off + u;
             bool queued = false;  // this lane has an item to publish
             uint32_t more = 0;
@@ -601,10 +649,8 @@ __device__ __forceinline__ bool layer_item(const RelaxArgs &a, uint32_t fi, uint
                 }
             }
             __syncwarp();
-            if (lane < 4) {
-                sh.push[lane] = 0;
-                sh.park[lane] = kMax;
-            }
+            if (lane < 4) sh.park[lane] = kMax;
+            if (lane == 0) sh.push = 0;
         }
         __syncthreads();
         if (!sh.more) break;
@@ -712,11 +758,9 @@ __global__ void __launch_bounds__(LM * 32, LM == 4 ? 5 : LM == 8 ? 3 : 1) relax_
             sh.n_spec = sh.wide = 0;
             sh.dmin = sh.hmin = kMax;
             sh.hmax = 0;
+            sh.push = 0;
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                sh.push[k] = 0;
-                sh.park[k] = kMax;
-            }
+            for (int k = 0; k < 4; ++k) sh.park[k] = kMax;
         }
         __syncthreads();
         const u64 item = sh.item;
