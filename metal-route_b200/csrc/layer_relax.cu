@@ -53,7 +53,7 @@ struct LayerShared {
     u64 item;
     uint64_t mbar;  // completion of the price-plane TMA loads
     unsigned long long cnt[2];  // activations and sweeps not yet added to the launch's
-    uint32_t n_spec, wide, dmin, hmin, hmax, ub, thr, more;
+    uint32_t n_spec, near_pad, wide, dmin, hmin, hmax, ub, thr, more;
     uint32_t push;              // bits: left, right, top, bottom improved
     uint32_t park[4];           // GD: the smallest f that waits to enter each
     uint32_t hy[TH + 2];        // GD: remaining price along y, rows -1 .. TH
@@ -133,6 +133,19 @@ __device__ __forceinline__ void stack_pass_layers(uint32_t *lab, const uint32_t 
             for (uint32_t l = 1; l < L; ++l) q[l * LS] = c = __viaddmin_u32(c, pu[l * LS], q[l * LS]);
             for (uint32_t l = L - 1; l-- > 0;) q[l * LS] = c = __viaddmin_u32(c, pd[l * LS], q[l * LS]);
         }
+    }
+}
+
+// Labels of one layer of the tiles beyond `sides` of the tile at (x, y) of a ww x wh
+// window into L2: one 128-byte line a lane, three lines a row of eight.
+__device__ __noinline__ void prefetch_neighbours(const u64 *lab, uint32_t sides, uint32_t lane, int x, int y,
+                                                 uint32_t ww, uint32_t wh) {
+    for (; sides; sides &= sides - 1u) {
+        const uint32_t k = __ffs(sides) - 1u;  // left, right, top, bottom
+        const int lx = x + (k == 0 ? -(int)kTW : k == 1 ? (int)kTW : 0) + (int)(lane & 3u) * 16;
+        const int ly = y + (k == 2 ? -TH : k == 3 ? TH : 0) + (int)(lane >> 2);
+        if ((lane & 3u) < 3u && lx < (int)ww && ly < (int)wh)
+            prefetch_l2(lab + (uint64_t)(uint32_t)ly * ww + (uint32_t)max(lx, 0));
     }
 }
 
@@ -234,6 +247,7 @@ __device__ __forceinline__ bool layer_item(const RelaxArgs &a, uint32_t fi, uint
                 const uint32_t c = __ldg(a.pads + (q ? f.vpad_off + k - f.n_pads : f.pad_off + k));
                 const uint32_t plane = b.w * b.h, l = c / plane, rr = c - l * plane, gy = rr / b.w, gx = rr - gy * b.w;
                 const uint32_t x = gx - (uint32_t)tx0, y = gy - (uint32_t)ty0;
+                if (x + 1u <= kTW + 1u && y + 1u <= TH + 1u) sh.near_pad = 1;  // in the tile or its ring
                 if (x < xlo || x >= tw || y >= th) continue;
                 const uint32_t i = atomicAdd(&sh.n_spec, 1u);
                 if (i < kSpecCap) sh.spec[i] = (q ? 1u << 31 : 0u) | (l << 16) | (y << 8) | x;
@@ -548,12 +562,12 @@ __device__ __forceinline__ bool layer_item(const RelaxArgs &a, uint32_t fi, uint
                 better[k] = cand < there[k];  // (no price or label: at least kBig, as `there` at most)
                 fv[k] = dbase + (cand >> HB);
             }
-            if (f.n_pads || (OV && f.n_over)) {  // its own pads, or its own prices, beyond the border
+            if (sh.near_pad || (OV && f.n_over)) {  // its own pads, or its own prices, beyond the border
 #pragma unroll 1
                 for (int k = 0; k < 3; ++k) {
                     const uint32_t o = k == 0 ? w[0] : k == 1 ? w[TH - 1] : edge, p0 = k == 0 ? pt : k == 1 ? pb : ps;
                     const bool ok = (k == 0 ? col_in && top : k == 1 ? col_in && bottom : side) && o < kBig;
-                    bool exact = f.n_pads && p0 == kBig;
+                    bool exact = p0 == kBig;
                     if constexpr (OV) {
                         const uint32_t nb = k == 0 ? t - ntx : k == 1 ? t + ntx : seg == 0 ? t - 1 : t + 1;
                         exact |= ok && f.n_over && a.tover[f.tile_off + nb];
@@ -651,6 +665,15 @@ __device__ __forceinline__ bool layer_item(const RelaxArgs &a, uint32_t fi, uint
             __syncwarp();
             if (lane < 4) sh.park[lane] = kMax;
             if (lane == 0) sh.push = 0;
+        } else if constexpr (LM > 4) {
+            // Meanwhile the other warps send for the labels of the tiles being queued,
+            // so that they are in L2 when a CTA takes them (layer 0 with layer 1).  Only
+            // with more than four layers, where it takes 10 % off (1280x1153x6 1.78 ->
+            // 1.60 ms, 640 uneven instances 707 -> 657 us); on four layers the tile's
+            // registers are short and it costs 2 % (512x512x4 1.44 -> 1.48 ms).
+            const uint32_t sides = *(volatile uint32_t *)&sh.push;
+            for (uint32_t l = wl == 1 ? 0u : wl; l <= wl && l < L; ++l)
+                prefetch_neighbours(glab + (int64_t)l * f.wh * f.ww, sides, lane, tx0 - (int)f.x0, ty0 - (int)f.y0, f.ww, f.wh);
         }
         __syncthreads();
         if (!sh.more) break;
@@ -755,7 +778,7 @@ __global__ void __launch_bounds__(LM * 32, LM == 4 ? 5 : LM == 8 ? 3 : 1) relax_
     for (;;) {
         if (threadIdx.x == 0) {
             sh.item = last ? kReleaseField : async_pop<64>(a);
-            sh.n_spec = sh.wide = 0;
+            sh.n_spec = sh.near_pad = sh.wide = 0;
             sh.dmin = sh.hmin = kMax;
             sh.hmax = 0;
             sh.push = 0;

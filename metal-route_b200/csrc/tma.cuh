@@ -36,4 +36,6 @@ __device__ __forceinline__ void tma_load_4d(void *dst, const void *tmap, int c0,
         : "memory");
 }
 
+__device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 }  // namespace mrc

@@ -4,6 +4,7 @@ import numpy as np
 import pytest
 
 import mrcuda
+from mrcuda import workloads as W
 from mrcuda.types import IsolatedRouteRequest
 from test_gpu_parity import _random_case
 
@@ -48,5 +49,20 @@ def test_goal_directed_batches_equal_the_oracle(oracle, directed, zero):
                 paths, costs = oracle.isolated_batch(r, retry_full=retry, mode="field")
                 assert out.paths == paths * times, (k, retry)
                 assert out.search_costs == costs * times, (k, retry)
+    finally:
+        engine.close()
+
+
+@pytest.mark.parametrize("seed", [2, 7])
+def test_congestion_board_paths_only(oracle, seed):
+    """Prices whose bound is loose (a path costs 1.4 x it), so that improvements
+    wait for the target and are released in several steps."""
+    req = W.congestion_board(seed=seed).request()
+    exp = oracle.isolated_batch(req, mode="astar")
+    engine = mrcuda.Engine(0)
+    try:
+        for _ in range(3):
+            got = engine.route_isolated_batch(req)
+            assert (got.paths, got.search_costs) == exp
     finally:
         engine.close()
