@@ -555,14 +555,11 @@ __device__ __forceinline__ bool process_item(const RelaxArgs &a, uint32_t fi, ui
             s_lim[0] = lim.x;  // an older (larger) bound of the target is still a bound
             s_lim[1] = lim.y;  // the threshold only moves while no item of the field is in flight
         }
-        const BoardGoal *bg = b.goal;
-        const uint32_t *hx = b.goal_sums, *hy = hx + b.w, *hv = hy + b.h;
-        uint32_t e = __ldg(&bg->min_cost);
-        if (f.n_pads) e = min(e, 1u);  // its own pads are entered at weight 1
-        auto rest = [&](const uint32_t *p, int at, int n, uint32_t to) {
-            const uint32_t u = __ldg(p + min(max(at, 0), n - 1)), v = __ldg(p + to);
-            return capmul(u > v ? u - v : v - u, e);
+        const uint32_t e = goal_weight(*b.goal, f), each = ~b.goal->inv_min_dir;
+        auto rest = [&](const uint32_t *sums, int at, int n, uint32_t to) {
+            return goal_rest(sums, each, e, (uint32_t)min(max(at, 0), n - 1), to);
         };
+        const uint32_t *hx = b.directed ? nullptr : b.x_sum, *hy = b.directed ? nullptr : b.y_sum, *hv = b.via_sum;
         for (uint32_t i = tid; i < SW + SH + L; i += blockDim.x) {
             if (i < SW) s_hx[i] = rest(hx, tx0 + (int)i - 1, (int)b.w, dst_x);
             else if (i < SW + SH) s_hy[i - SW] = rest(hy, ty0 + (int)(i - SW) - 1, (int)b.h, dst_y);

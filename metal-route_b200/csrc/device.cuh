@@ -56,28 +56,21 @@ struct DevBoard {
     // cell inside each field's range DevField::over_off .. + n_over
     const uint32_t *over_cells;
     const uint4 *over_price;
-    // nullable: lower bounds of the step prices: their head (zeroed before
-    // planes_kernel) and the prefix sums HX[w], HY[h], HV[layers] (goal_kernel)
-    BoardGoal *goal;
-    uint32_t *goal_sums;
+    BoardGoal *goal;            // nullable: extremes of the prices (zeroed before planes_kernel)
+    // prefix sums of the gap and via prices (saturating at kCap), the smallest gap
+    // and the smallest allowed via
+    const uint32_t *x_sum, *y_sum, *via_sum;  // w, h, layers
+    uint32_t min_gap, min_via;
     const uint4 *bound;         // nullable: directed prices no price of this batch is below (default: directed)
 };
 
-// Lower bounds a goal-directed launch prices the rest of a path with.  The
-// remaining price from cell c to the net's target t is at least
-// e * (|HX[xc] - HX[xt]| + |HY[yc] - HY[yt]| + |HV[lc] - HV[lt]|): every path
-// crosses each column gap, row gap and layer transition between the two, each
-// at no less than its cheapest base price times e, the smallest enter weight
-// (at most 1 for a net that enters its own pads).
+// Extremes of a board's prices, accumulated by planes_kernel from zero: what a
+// goal-directed launch bounds the rest of a path with (goal_rest).
 struct BoardGoal {
-    uint32_t inv_min_dir;       // ~(smallest directed price), accumulated by planes_kernel from zero
+    uint32_t inv_min_dir;       // ~(smallest directed price)
     uint32_t inv_min_cost;      // ~(smallest enter weight)
     u64 sum_dir, n_dir;         // of the directed prices from -x: their mean sets the first threshold
     u64 sum_cost, n_cost;
-    uint32_t min_cost;          // written by goal_kernel: the smallest enter weight,
-    uint32_t min_step;          // the smallest planar base price,
-    uint32_t min_via;           // the smallest via base price
-    float spread;               // and the share of the bound that the first threshold adds
     uint32_t wide;              // packed planes: a finite price did not fit (planes_kernel)
     uint32_t pad_;
 };
@@ -144,6 +137,28 @@ __device__ __forceinline__ u64 extend(u64 prev, uint32_t step) {
     uint32_t nd = d + step;
     bool bad = (d == kMax) | (step == kMax) | (nd < d) | (nd == kMax);
     return bad ? kInf : (((u64)nd << 32) | (uint32_t)((uint32_t)prev + 1u));
+}
+
+// Least price of a path's moves along one axis (or between the layers) from `at`
+// to `to`: it crosses every gap between the two, each at no less than its
+// cheapest base price (`sums`: prefix sums of the gaps; null: `each` per gap of a
+// directed board) times e, the smallest enter weight.
+__device__ __forceinline__ uint32_t goal_rest(const uint32_t *sums, uint32_t each, uint32_t e, uint32_t at,
+                                              uint32_t to) {
+    uint32_t d;
+    if (sums) {
+        const uint32_t u = __ldg(sums + at), v = __ldg(sums + to);
+        d = u > v ? u - v : v - u;
+    } else {
+        d = capmul(at > to ? at - to : to - at, each);
+    }
+    return capmul(d, e);
+}
+
+// e of a net: at most 1 when it enters its own pads.
+__device__ __forceinline__ uint32_t goal_weight(const BoardGoal &g, const DevField &f) {
+    const uint32_t e = ~g.inv_min_cost;
+    return f.n_pads ? (e < 1u ? e : 1u) : e;
 }
 
 __device__ __forceinline__ bool sorted_has(const uint32_t *a, uint32_t n, uint32_t key) {

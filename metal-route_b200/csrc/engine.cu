@@ -357,11 +357,64 @@ struct mrc_board {
     std::vector<uint8_t> board;    // host copy of the board mask (may be empty)
     std::vector<uint8_t> viaf;     // host copy of the static via mask (may be empty)
     bool directed = false;
-    DBuf d_cost, d_flags, d_x, d_y, d_via, d_dir;
+    DBuf d_cost, d_flags, d_edges, d_dir;
     DevBoard dev{};
 };
 
 namespace {
+
+// The edge prices of a board as one block of words: x, y and via prices, then the
+// prefix sums of each (what a path pays at least between two lines or layers).
+struct EdgeWords {
+    size_t y, via, x_sum, y_sum, via_sum, total;  // x at 0
+    EdgeWords(uint32_t w, uint32_t h, uint32_t layers) {
+        y = w ? w - 1 : 0;
+        via = y + (h ? h - 1 : 0);
+        x_sum = via + std::max(layers - 1, 1u);
+        y_sum = x_sum + w;
+        via_sum = y_sum + h;
+        total = via_sum + layers;
+    }
+};
+
+void fill_edges(const mrc_edges &e, uint32_t w, uint32_t h, uint32_t layers, uint32_t *out, DevBoard *dev) {
+    const EdgeWords o(w, h, layers);
+    auto sums = [](const uint32_t *gap, uint32_t n, uint32_t *to) {
+        uint64_t at = 0;
+        for (uint32_t i = 0; i < n; ++i) {
+            if (i) at = std::min<uint64_t>(at + gap[i - 1], kCap);
+            to[i] = (uint32_t)at;
+        }
+    };
+    if (e.n_x_edge_costs) std::memcpy(out, e.x_edge_costs, (size_t)e.n_x_edge_costs * 4);
+    if (e.n_y_edge_costs) std::memcpy(out + o.y, e.y_edge_costs, (size_t)e.n_y_edge_costs * 4);
+    out[o.via] = 0;
+    dev->via_mask = 0;
+    dev->min_gap = dev->min_via = kMax;
+    for (uint32_t k = 0; k < e.n_via_edge_costs; ++k) {
+        out[o.via + k] = e.via_edge_costs[k];
+        if (!e.via_allowed[k]) continue;
+        dev->via_mask |= 1u << k;
+        dev->min_via = std::min(dev->min_via, e.via_edge_costs[k]);
+    }
+    for (uint32_t i = 0; i < e.n_x_edge_costs; ++i) dev->min_gap = std::min(dev->min_gap, e.x_edge_costs[i]);
+    for (uint32_t i = 0; i < e.n_y_edge_costs; ++i) dev->min_gap = std::min(dev->min_gap, e.y_edge_costs[i]);
+    if (dev->min_gap == kMax) dev->min_gap = 0;
+    if (dev->min_via == kMax) dev->min_via = 0;
+    sums(out, w, out + o.x_sum);
+    sums(out + o.y, h, out + o.y_sum);
+    sums(out + o.via, layers, out + o.via_sum);
+}
+
+void view_edges(const uint32_t *base, uint32_t w, uint32_t h, uint32_t layers, DevBoard *dev) {
+    const EdgeWords o(w, h, layers);
+    dev->x_edge = base;
+    dev->y_edge = base + o.y;
+    dev->via_edge = base + o.via;
+    dev->x_sum = base + o.x_sum;
+    dev->y_sum = base + o.y_sum;
+    dev->via_sum = base + o.via_sum;
+}
 
 // The device-readable address of page-locked, mapped host memory; null for
 // pageable memory.
@@ -430,25 +483,16 @@ mrc_status board_build(mrc_context *ctx, const mrc_grid *grid, const mrc_edges *
             MRC_CUDA(cudaStreamSynchronize(ctx->stream), "combine masks");
         }
     }
-    std::vector<uint32_t> vias(std::max<uint32_t>(ev, 1), 0);
-    uint32_t via_mask = 0;
-    for (uint32_t k = 0; k < ev; ++k) {
-        vias[k] = edges->via_edge_costs[k];
-        if (edges->via_allowed[k]) via_mask |= 1u << k;
-    }
-    MRC_TRY(upload(ctx, b->d_x, edges->x_edge_costs, (size_t)ex * 4, "upload x edges"));
-    MRC_TRY(upload(ctx, b->d_y, edges->y_edge_costs, (size_t)ey * 4, "upload y edges"));
-    MRC_TRY(upload(ctx, b->d_via, vias.data(), vias.size() * 4, "upload via edges"));
+    std::vector<uint32_t> words(EdgeWords(g.w, g.h, g.layers).total, 0);
+    fill_edges(*edges, g.w, g.h, g.layers, words.data(), &b->dev);
+    MRC_TRY(upload(ctx, b->d_edges, words.data(), words.size() * 4, "upload edge prices"));
     if (b->directed) MRC_TRY(upload(ctx, b->d_dir, edges->directed_in_costs, n * 16, "upload directed prices"));
     b->dev.w = g.w;
     b->dev.h = g.h;
     b->dev.layers = g.layers;
-    b->dev.via_mask = via_mask;
     b->dev.cost = b->d_cost.as<uint32_t>();
     b->dev.flags = has_flags ? b->d_flags.as<uint8_t>() : nullptr;
-    b->dev.x_edge = b->d_x.as<uint32_t>();
-    b->dev.y_edge = b->d_y.as<uint32_t>();
-    b->dev.via_edge = b->d_via.as<uint32_t>();
+    view_edges(b->d_edges.as<uint32_t>(), g.w, g.h, g.layers, &b->dev);
     b->dev.directed = b->directed ? b->d_dir.as<uint4>() : nullptr;
     return MRC_OK;
 }
@@ -467,7 +511,7 @@ struct BoardPack {
 };
 
 struct PackOff {
-    size_t cost, flags, x, y, via, dir;
+    size_t cost, flags, edges, dir;
 };
 
 void pack_views(BoardPack *pk, const std::vector<PackOff> &offs) {
@@ -480,9 +524,7 @@ void pack_views(BoardPack *pk, const std::vector<PackOff> &offs) {
         b.dev.layers = b.view.layers;
         b.dev.cost = reinterpret_cast<const uint32_t *>(base + o.cost);
         b.dev.flags = o.flags != SIZE_MAX ? base + o.flags : nullptr;
-        b.dev.x_edge = reinterpret_cast<const uint32_t *>(base + o.x);
-        b.dev.y_edge = reinterpret_cast<const uint32_t *>(base + o.y);
-        b.dev.via_edge = reinterpret_cast<const uint32_t *>(base + o.via);
+        view_edges(reinterpret_cast<const uint32_t *>(base + o.edges), b.dev.w, b.dev.h, b.dev.layers, &b.dev);
         b.dev.directed = o.dir != SIZE_MAX ? reinterpret_cast<const uint4 *>(base + o.dir) : nullptr;
     }
 }
@@ -496,13 +538,13 @@ mrc_status board_pack_direct(mrc_context *ctx, const mrc_isolated_request *inst,
                              const std::vector<std::array<const void *, 4>> &src) {
     MRC_TRY(pk->data.get(ctx, std::max<size_t>(total, 256), "instance boards"));
     auto up16 = [](size_t v) { return (v + 15) & ~(size_t)15; };
-    // stage layout: per instance the device bytes from o.x to the end of the via
-    // prices (same padding as on the device), then the spans, then chunk starts
+    // stage layout: per instance its edge prices, then the spans, then chunk starts
     std::vector<size_t> small(n);
     size_t sb = 0;
     for (uint32_t k = 0; k < n; ++k) {
         small[k] = sb;
-        sb += up16(offs[k].via + (size_t)std::max(inst[k].edges.n_via_edge_costs, 1u) * 4 - offs[k].x);
+        const GridView &g = pk->boards[k]->view;
+        sb += up16(EdgeWords(g.w, g.h, g.layers).total * 4);
     }
     const size_t max_spans = (size_t)4 * n;
     const size_t o_spans = sb, o_chunks = up16(o_spans + max_spans * sizeof(HostSpan));
@@ -526,22 +568,12 @@ mrc_status board_pack_direct(mrc_context *ctx, const mrc_isolated_request *inst,
         const GridView &g = pk->boards[k]->view;
         const mrc_edges &e = inst[k].edges;
         const PackOff &o = offs[k];
-        unsigned char *sm = host + small[k];
-        if (e.n_x_edge_costs) std::memcpy(sm, e.x_edge_costs, (size_t)e.n_x_edge_costs * 4);
-        if (e.n_y_edge_costs) std::memcpy(sm + (o.y - o.x), e.y_edge_costs, (size_t)e.n_y_edge_costs * 4);
-        uint32_t *via = reinterpret_cast<uint32_t *>(sm + (o.via - o.x));
-        uint32_t mask = 0;
-        via[0] = 0;
-        for (uint32_t i = 0; i < e.n_via_edge_costs; ++i) {
-            via[i] = e.via_edge_costs[i];
-            if (e.via_allowed[i]) mask |= 1u << i;
-        }
-        pk->boards[k]->dev.via_mask = mask;
+        fill_edges(e, g.w, g.h, g.layers, reinterpret_cast<uint32_t *>(host + small[k]), &pk->boards[k]->dev);
         ctx->in_place_bytes += (size_t)g.n * 4 + (o.flags != SIZE_MAX ? g.n : 0) + (o.dir != SIZE_MAX ? (size_t)g.n * 16 : 0);
         add(src[k][0], nullptr, o.cost, (size_t)g.n * 4, 0);
         if (o.flags != SIZE_MAX) add(src[k][1], src[k][2], o.flags, g.n, g.via_forbidden ? 1 : 0);
         if (o.dir != SIZE_MAX) add(src[k][3], nullptr, o.dir, (size_t)g.n * 16, 0);
-        add(host_dev + small[k], nullptr, o.x, o.via + (size_t)std::max(e.n_via_edge_costs, 1u) * 4 - o.x, 0);
+        add(host_dev + small[k], nullptr, o.edges, EdgeWords(g.w, g.h, g.layers).total * 4, 0);
     }
     // the gather list itself goes over in one copy (the kernel searches it per chunk)
     const size_t list_bytes = up16((size_t)ns * sizeof(HostSpan)) + (size_t)ns * 8;
@@ -585,9 +617,7 @@ mrc_status board_pack_build(mrc_context *ctx, const mrc_isolated_request *inst, 
         Off &o = offs[k];
         o.cost = take(g.n * 4);
         o.flags = (g.board || g.via_forbidden) ? take(g.n) : SIZE_MAX;
-        o.x = take((size_t)ex * 4);
-        o.y = take((size_t)ey * 4);
-        o.via = take((size_t)std::max(ev, 1u) * 4);
+        o.edges = take(EdgeWords(g.w, g.h, g.layers).total * 4);
         o.dir = b->directed ? take(g.n * 16) : SIZE_MAX;
         pk->boards.push_back(std::move(b));
     }
@@ -621,16 +651,8 @@ mrc_status board_pack_build(mrc_context *ctx, const mrc_isolated_request *inst, 
                     fl[i] = (uint8_t)((g.board ? g.board[i] : 0) | (g.via_forbidden[i] ? kStaticVia : 0));
             }
         }
-        if (e.n_x_edge_costs) std::memcpy(host + o.x, e.x_edge_costs, (size_t)e.n_x_edge_costs * 4);
-        if (e.n_y_edge_costs) std::memcpy(host + o.y, e.y_edge_costs, (size_t)e.n_y_edge_costs * 4);
-        uint32_t *via = reinterpret_cast<uint32_t *>(host + o.via);
-        uint32_t mask = 0;
-        for (uint32_t i = 0; i < e.n_via_edge_costs; ++i) {
-            via[i] = e.via_edge_costs[i];
-            if (e.via_allowed[i]) mask |= 1u << i;
-        }
+        fill_edges(e, g.w, g.h, g.layers, reinterpret_cast<uint32_t *>(host + o.edges), &pk->boards[k]->dev);
         if (o.dir != SIZE_MAX) std::memcpy(host + o.dir, e.directed_in_costs, g.n * 16);
-        pk->boards[k]->dev.via_mask = mask;
     };
     // Worker threads fill instances in index order; this thread ships every
     // completed prefix of >= 32 MB to the device while the rest is still filled.
@@ -734,10 +756,10 @@ struct mrc_batch {
     DBuf d_planes, d_pchunks;    // step-price planes of every board, chunk table of their kernel
     DBuf d_tmaps;                // one TMA tensor map per board over its planes (CTA queue form)
     uint64_t n_pchunks = 0;
-    // goal-directed relax (the CTA queue form with price planes, when only paths
-    // and costs are asked for): lower bounds per board, state per field, waiting f per tile
+    // goal-directed relax (the layer kernel, when only paths and costs are asked
+    // for): state per field; extremes of the prices per board and waiting f per tile elsewhere
     bool goal = false;
-    DBuf d_goal, d_fgoal;
+    DBuf d_fgoal;
     uint32_t list_cap = 1;       // slots of the tile lists
     // the planes hold prices of the batch's boards, which never change: computed by
     // the first launch after a layout and kept for the launches that follow
@@ -852,7 +874,7 @@ mrc_status batch_layout(mrc_batch *bt, uint32_t tile_h, uint32_t threads) {
         return fail(MRC_ERR_LIMIT, "a queue item holds 2^28 fields and 2^28 tiles of a field");
     bt->total_tiles = (uint32_t)std::max<uint64_t>(toff, 1);
     bt->max_tiles = max_tiles;
-    bt->goal = bt->layer && !(bt->flags & MRC_FLAG_KEEP_FIELDS) && toff >= (uint64_t)kGoalTilesPerSm * ctx->sms;
+    bt->goal = bt->layer && !(bt->flags & MRC_FLAG_KEEP_FIELDS);
     int per_sm = 1;
     if (bt->warp) {
         MRC_CUDA(warp_relax_occupancy(&per_sm), "relax occupancy");
@@ -888,18 +910,6 @@ mrc_status batch_layout(mrc_batch *bt, uint32_t tile_h, uint32_t threads) {
         for (size_t k = 0; k < bt->devs.size(); ++k)
             bt->devs[k].planes = reinterpret_cast<uint32_t *>(bt->d_planes.as<unsigned char>() + poff[k]);
         bt->n_pchunks = chunks.back();
-        uint64_t gwords = 0;
-        for (DevBoard &d : bt->devs) {
-            if (bt->goal) gwords += goal_words(d.w, d.h, d.layers);
-        }
-        if (bt->goal) {
-            MRC_TRY(bt->d_goal.get(ctx, gwords * 4, "price bounds"));
-            gwords = 0;
-            for (DevBoard &d : bt->devs) {
-                d.goal_sums = bt->d_goal.as<uint32_t>() + gwords;
-                gwords += goal_words(d.w, d.h, d.layers);
-            }
-        }
         MRC_TRY(upload(ctx, bt->d_pchunks, chunks.data(), chunks.size() * 8, "plane chunk table"));
         if (bt->layer) {
             std::vector<CUtensorMap> maps(bt->devs.size());
@@ -954,7 +964,6 @@ mrc_status batch_layout(mrc_batch *bt, uint32_t tile_h, uint32_t threads) {
     if (bt->goal) {
         MRC_TRY(bt->d_fgoal.get(ctx, std::max<size_t>(bt->fields.size(), 1) * sizeof(FieldGoal), "field goals"));
     } else {
-        bt->d_goal.reset();
         bt->d_fgoal.reset();
     }
     return MRC_OK;
@@ -1071,17 +1080,12 @@ PathArgs path_args(const mrc_batch *bt) {
     return pa;
 }
 
-// Step-price planes of the batch's boards and, for a goal-directed batch, the
-// lower bounds made from the minima that kernel accumulates.
+// Step-price planes of the batch's boards (and the extremes of the prices).
 mrc_status planes_enqueue(mrc_batch *bt, cudaStream_t st, uint32_t *launches) {
     MRC_CUDA(planes_launch(bt->d_boards.as<DevBoard>(), bt->d_pchunks.as<uint64_t>(), (uint32_t)bt->devs.size(),
                            bt->n_pchunks, (uint32_t)bt->ctx->sms, bt->layer ? layer_hop_bits(bt->max_layers) : 0, st),
              "launch step-price planes");
     *launches += 1;
-    if (bt->goal) {
-        MRC_CUDA(goal_launch(bt->d_boards.as<DevBoard>(), (uint32_t)bt->devs.size(), st), "launch price bounds");
-        *launches += 1;
-    }
     return MRC_OK;
 }
 
@@ -2458,7 +2462,7 @@ size_t request_footprint(const ServerRequest &r, uint32_t tile_h) {
                      (uint64_t)r.grid.w * r.grid.h * (r.grid.layers ? r.grid.layers : 1u)};
     size_t b = 0;
     if (!r.resident) {
-        b += al(g.n * 4) + al((size_t)g.w * 4) + al((size_t)g.h * 4) + al(128);
+        b += al(g.n * 4) + al(EdgeWords(g.w, g.h, g.layers).total * 4);
         if (r.grid.board_constraint || r.grid.via_forbidden) b += al(g.n);
         if (r.req.edges.directed_in_costs) b += al(g.n * 16);
     }

@@ -14,12 +14,6 @@ constexpr int kRelaxThreads = 256;  // default CTA width of the relax kernel
 constexpr uint64_t kTilesPerCta = 8;  // tiles per CTA at which a queue launch can use one more CTA
 constexpr uint32_t kCountBatch = 64;    // activations a queue CTA counts locally before adding them to the launch's
 constexpr uint32_t kMinRing = 8192;     // fewest slots of the tile queue: more than CTAs of any launch
-// Tiles per SM from which a batch that asks for paths only is solved goal-directed.
-// Smaller ones wait on one field's chain of tiles, where the limits cost more
-// than the tiles they save (40 two-pin nets on 201x160: 0.99 x, 48 nets with
-// pads on 233x187x4: 0.93 x); larger ones are bound by the tiles themselves
-// (640 uneven instances: 1.54 x, 160 long nets on 1280x1153x6: 1.55 x).
-constexpr uint32_t kGoalTilesPerSm = 64;
 constexpr uint32_t kGoalPhases = 4;     // releases of waiting tiles by threshold before all of them go
 constexpr uint32_t kContinueLimit = 4;  // activations of one held tile before it goes back to the queue
 
@@ -242,12 +236,6 @@ __host__ __device__ inline uint32_t planes_pitch(uint32_t w) { return (w + 3u) &
 // price that does not fit is marked (BoardGoal::wide).
 constexpr uint32_t kPackedInf = 1u << 30;
 uint64_t planes_chunks(uint64_t cells);
-// Words of one board's prefix sums (DevBoard::goal_sums); goal_launch makes them
-// of the minima that planes_launch accumulated into the zeroed heads.
-inline uint64_t goal_words(uint32_t w, uint32_t h, uint32_t layers) {
-    return ((uint64_t)w + h + layers + 31) & ~(uint64_t)31;
-}
-cudaError_t goal_launch(const DevBoard *boards, uint32_t n_boards, cudaStream_t st);
 cudaError_t planes_launch(const DevBoard *boards, const uint64_t *chunk_start, uint32_t n_boards, uint64_t n_chunks,
                           uint32_t sms, uint32_t hop_bits, cudaStream_t st);
 

@@ -197,13 +197,11 @@ __device__ __forceinline__ bool layer_item(const RelaxArgs &a, uint32_t fi, uint
     if constexpr (GD) {
         const uint32_t plane = b.w * b.h, dst_l = f.dst / plane, dr = f.dst - dst_l * plane, dst_y = dr / b.w,
                        dst_x = dr - dst_y * b.w;
-        const uint32_t *px = b.goal_sums, *py = px + b.w, *pv = py + b.h;
-        uint32_t e = __ldg(&b.goal->min_cost);
-        if (f.n_pads) e = min(e, 1u);  // its own pads are entered at weight 1
-        auto rest = [&](const uint32_t *p, int at, uint32_t n, uint32_t to) {
-            const uint32_t u = __ldg(p + min(max(at, 0), (int)n - 1)), v = __ldg(p + to);
-            return capmul(u > v ? u - v : v - u, e);
+        const uint32_t e = goal_weight(*b.goal, f), each = ~b.goal->inv_min_dir;
+        auto rest = [&](const uint32_t *sums, int at, uint32_t n, uint32_t to) {
+            return goal_rest(sums, each, e, (uint32_t)min(max(at, 0), (int)n - 1), to);
         };
+        const uint32_t *px = b.directed ? nullptr : b.x_sum, *py = b.directed ? nullptr : b.y_sum, *pv = b.via_sum;
         hx = rest(px, tx0 + (int)lane, b.w, dst_x);
         hxs = rest(px, seg == 0 ? tx0 - 1 : tx0 + (int)kTW, b.w, dst_x);
         hl = rest(pv, (int)wl, L, dst_l);

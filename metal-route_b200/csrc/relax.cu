@@ -162,18 +162,25 @@ __global__ void async_seed_kernel(RelaxArgs a) {
             __threadfence();
             uint32_t *live = &a.ctl->count[1];
             if (a.goal) {  // goal-directed: the launch counts fields, the field its items
-                const BoardGoal *bg = b.goal;
-                const uint32_t *hx = b.goal_sums, *hy = hx + b.w, *hv = hy + b.h;
+                const BoardGoal bg = *b.goal;
                 const uint32_t dl = f.dst / plane, dr = f.dst % plane, dx = dr % b.w, dy = dr / b.w;
-                const uint32_t e = f.n_pads ? min(bg->min_cost, 1u) : bg->min_cost;
-                auto rest = [&](const uint32_t *p, uint32_t u, uint32_t v) {
-                    return capmul(p[u] > p[v] ? p[u] - p[v] : p[v] - p[u], e);
-                };
-                const uint32_t f0 = min(dsum(dsum(rest(hx, sx, dx), rest(hy, sy, dy)), rest(hv, sl, dl)), kCap);
-                // first threshold: room for two vias, a detour of two cells, and the
-                // board's spread of prices; with a zero bound nothing waits
-                const u64 room = (u64)((double)bg->spread * f0) + 2ull * capmul(bg->min_via, e) +
-                                 4ull * capmul(bg->min_step, e);
+                const uint32_t e = goal_weight(bg, f), each = ~bg.inv_min_dir;
+                const uint32_t f0 = min(dsum(dsum(goal_rest(b.directed ? nullptr : b.x_sum, each, e, sx, dx),
+                                                  goal_rest(b.directed ? nullptr : b.y_sum, each, e, sy, dy)),
+                                             goal_rest(b.via_sum, 0, e, sl, dl)), kCap);
+                // First threshold: room for two vias, a detour of two cells, and a share
+                // of the bound.  A path through random prices avoids the dear ones: its
+                // mean step lies about a third of the way from the cheapest to the mean
+                // price (congestion board: path cost 1.38 x the bound where mean /
+                // cheapest is 2.3; negotiation board 1.01 x at 1.1).  Relax time of the
+                // congestion board with a share of 0, 0.17, 0.35 and 0.6 of that
+                // distance: 4.9, 4.9, 4.5, 4.9 ms.  With a zero bound nothing waits.
+                float spread = 1.0f;  // mean over cheapest price
+                if (bg.n_cost && ~bg.inv_min_cost) spread *= (float)bg.sum_cost / (float)bg.n_cost / (float)~bg.inv_min_cost;
+                if (b.directed && bg.n_dir && each) spread *= (float)bg.sum_dir / (float)bg.n_dir / (float)each;
+                spread = fminf(fmaxf(0.35f * (spread - 1.0f), 0.0f), 2.0f);
+                const u64 room = (u64)((double)spread * f0) + 2ull * capmul(b.min_via, e) +
+                                 4ull * capmul(b.directed ? each : b.min_gap, e);
                 FieldGoal g{};
                 g.ub = kMax;
                 g.f0 = f0;

@@ -159,70 +159,6 @@ __global__ void __launch_bounds__(256) planes_kernel(const DevBoard *boards, con
     }
 }
 
-// Prefix sums of the cheapest base prices, one CTA per board.  A directed board
-// has one cheapest price for all gaps; axis prices keep their gap lengths.
-// The first threshold of a search adds `spread` of the bound: a path through
-// random prices avoids the dear ones, its mean step lies about a third of the
-// way from the cheapest to the mean price (congestion board: path cost 1.38 x
-// the bound where mean / cheapest is 2.3; negotiation board 1.01 x at 1.1).
-__device__ __forceinline__ void prefix_sums(uint32_t *out, uint32_t n, const uint32_t *gap, uint32_t each) {
-    __shared__ u64 part[256];
-    const uint32_t per = (n + 255) / 256, lo = min(n, threadIdx.x * per), hi = min(n, lo + per);
-    u64 s = 0;  // gap i - 1 lies between i - 1 and i
-    for (uint32_t i = max(lo, 1u); i < hi; ++i) s += gap ? __ldg(gap + i - 1) : each;
-    part[threadIdx.x] = s;
-    __syncthreads();
-    for (uint32_t o = 1; o < 256; o <<= 1) {
-        const u64 v = threadIdx.x >= o ? part[threadIdx.x - o] : 0;
-        __syncthreads();
-        part[threadIdx.x] += v;
-        __syncthreads();
-    }
-    u64 at = part[threadIdx.x] - s;
-    for (uint32_t i = lo; i < hi; ++i) {
-        if (i) at += gap ? __ldg(gap + i - 1) : each;
-        out[i] = at < kCap ? (uint32_t)at : kCap;
-    }
-    __syncthreads();
-}
-
-__device__ __forceinline__ uint32_t block_min_gap(const uint32_t *gap, uint32_t n) {
-    __shared__ uint32_t m;
-    if (threadIdx.x == 0) m = kMax;
-    __syncthreads();
-    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) atomicMin(&m, __ldg(gap + i));
-    __syncthreads();
-    const uint32_t r = m;
-    __syncthreads();
-    return r;
-}
-
-__global__ void __launch_bounds__(256) goal_kernel(const DevBoard *boards) {
-    const DevBoard b = boards[blockIdx.x];
-    BoardGoal *g = b.goal;
-    uint32_t *hx = b.goal_sums, *hy = hx + b.w, *hv = hy + b.h;
-    // no enterable cell, no directed price: every bound zero
-    const uint32_t min_cost = g->n_cost ? ~g->inv_min_cost : 0u;
-    const uint32_t min_dir = g->inv_min_dir ? ~g->inv_min_dir : 0u;
-    prefix_sums(hx, b.w, b.directed ? nullptr : b.x_edge, min_dir);
-    prefix_sums(hy, b.h, b.directed ? nullptr : b.y_edge, min_dir);
-    prefix_sums(hv, b.layers, b.via_edge, 0);
-    const uint32_t step = b.directed ? min_dir : min(b.w > 1 ? block_min_gap(b.x_edge, b.w - 1) : kMax,
-                                                     b.h > 1 ? block_min_gap(b.y_edge, b.h - 1) : kMax);
-    if (threadIdx.x == 0) {
-        uint32_t via = kMax;
-        for (uint32_t k = 0; k + 1 < b.layers; ++k)
-            if ((b.via_mask >> k) & 1u) via = min(via, __ldg(b.via_edge + k));
-        g->min_cost = min_cost;
-        g->min_step = step == kMax ? 0u : step;
-        g->min_via = via == kMax ? 0u : via;
-        float r = 1.0f;  // mean over cheapest price
-        if (min_cost && g->n_cost) r *= (float)g->sum_cost / (float)g->n_cost / (float)min_cost;
-        if (b.directed && min_dir && g->n_dir) r *= (float)g->sum_dir / (float)g->n_dir / (float)min_dir;
-        g->spread = fminf(fmaxf(0.35f * (r - 1.0f), 0.0f), 2.0f);
-    }
-}
-
 // ---- one tile held by one warp ---------------------------------------------
 
 // Per-warp shared memory.  The tile's labels live here rather than in
@@ -831,12 +767,6 @@ cudaError_t planes_launch(const DevBoard *boards, const uint64_t *chunk_start, u
     if (!n_boards || !n_chunks) return cudaSuccess;
     const uint64_t blocks = std::min<uint64_t>(n_chunks, (uint64_t)sms * 8);
     planes_kernel<<<(uint32_t)blocks, 256, 0, st>>>(boards, chunk_start, n_boards, n_chunks, hop_bits);
-    return cudaGetLastError();
-}
-
-cudaError_t goal_launch(const DevBoard *boards, uint32_t n_boards, cudaStream_t st) {
-    if (!n_boards) return cudaSuccess;
-    goal_kernel<<<n_boards, 256, 0, st>>>(boards);
     return cudaGetLastError();
 }
 
