@@ -901,10 +901,9 @@ mrc_status batch_layout(mrc_batch *bt, uint32_t tile_h, uint32_t threads) {
         uint64_t total = 0;
         for (size_t k = 0; k < bt->devs.size(); ++k) {
             const DevBoard &d = bt->devs[k];
-            const uint64_t cells = (uint64_t)d.w * d.h * d.layers;
             poff[k] = total;
             total += ((uint64_t)planes_pitch(d.w) * d.h * d.layers * 6 * 4 + 255) & ~(uint64_t)255;
-            chunks[k + 1] = chunks[k] + planes_chunks(cells);
+            chunks[k + 1] = chunks[k] + planes_chunks(d.w, d.h, d.layers);
         }
         MRC_TRY(bt->d_planes.get(ctx, std::max<uint64_t>(total, 256), "step-price planes"));
         for (size_t k = 0; k < bt->devs.size(); ++k)

@@ -235,7 +235,7 @@ __host__ __device__ inline uint32_t planes_pitch(uint32_t w) { return (w + 3u) &
 // kernel: (price << hop_bits) | 1, kPackedInf for no step; a board with a finite
 // price that does not fit is marked (BoardGoal::wide).
 constexpr uint32_t kPackedInf = 1u << 30;
-uint64_t planes_chunks(uint64_t cells);
+uint64_t planes_chunks(uint32_t w, uint32_t h, uint32_t layers);
 cudaError_t planes_launch(const DevBoard *boards, const uint64_t *chunk_start, uint32_t n_boards, uint64_t n_chunks,
                           uint32_t sms, uint32_t hop_bits, cudaStream_t st);
 

@@ -44,106 +44,195 @@ constexpr int K = kWarpLaneCells;  // cells per lane per row
 constexpr int TH = kWarpTileH;     // rows per tile
 constexpr int NW = 4;              // warps per CTA
 constexpr uint32_t kFull = 0xFFFFFFFFu;
-constexpr uint64_t kPlaneChunk = 8192;
+constexpr uint32_t kPlaneQuads = 256;  // quads of a chunk, one a thread
 constexpr uint32_t kMaxRounds = 8;  // relaxation rounds of one activation (see warp_item)
 
 // ---- step-price planes ------------------------------------------------------
 
-__device__ __forceinline__ bool via_blocked_board(uint8_t fl) { return (fl & (kViaNode | kStaticVia)) != 0; }
+__device__ __forceinline__ bool via_blocked_board(uint32_t fl) { return (fl & (kViaNode | kStaticVia)) != 0; }
 
-__global__ void __launch_bounds__(256) planes_kernel(const DevBoard *boards, const uint64_t *chunk_start,
+// The flag bytes of four cells of one row, the first at an index that is a
+// multiple of 4 in its row; cells past `n` read as 0.
+__device__ __forceinline__ uint32_t flags4(const uint8_t *p, bool aligned, uint32_t n) {
+    if (aligned) return __ldg(reinterpret_cast<const uint32_t *>(p));
+    uint32_t v = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < 4; ++k)
+        if (k < n) v |= (uint32_t)__ldg(p + k) << (8 * k);
+    return v;
+}
+
+// A thread prices four cells of a row (one 16-byte store per plane), a chunk is
+// kPlaneQuads such quads and a block takes a contiguous run of chunks, so that the
+// extremes of a board go to memory once per block and board.  With one cell per
+// thread and 8192-cell chunks a small board left the chip idle (201x160: 37 us in
+// four blocks, now 6 us; 389x301x3 with directed prices 54 -> 11 us).  On a set of
+// 256 uneven boards (363 MB of planes, 303 -> 244 us) three blocks an SM of 80
+// registers measured best (two of 126: 271 us).
+__global__ void __launch_bounds__(256, 3) planes_kernel(const DevBoard *boards, const uint64_t *chunk_start,
                                                      uint32_t n_boards, uint64_t n_chunks, uint32_t hop_bits) {
-    for (uint64_t ch = blockIdx.x; ch < n_chunks; ch += gridDim.x) {
-        uint32_t lo = 0, hi = n_boards - 1;  // the last board whose first chunk is <= ch
-        while (lo < hi) {
-            const uint32_t mid = (lo + hi + 1) >> 1;
-            if (chunk_start[mid] <= ch) lo = mid;
-            else hi = mid - 1;
-        }
+    __shared__ uint32_t s_u[8][4];
+    __shared__ u64 s_s[8][2];
+    const uint64_t ch0 = n_chunks * blockIdx.x / gridDim.x, ch1 = n_chunks * (blockIdx.x + 1) / gridDim.x;
+    uint32_t lo = 0, hi = n_boards - 1;  // the last board whose first chunk is <= ch0
+    while (lo < hi) {
+        const uint32_t mid = (lo + hi + 1) >> 1;
+        if (chunk_start[mid] <= ch0) lo = mid;
+        else hi = mid - 1;
+    }
+    for (uint64_t ch = ch0; ch < ch1;) {
+        while (chunk_start[lo + 1] <= ch) ++lo;  // (a board without cells has no chunk)
         const DevBoard b = boards[lo];
-        const uint32_t plane = b.w * b.h;
-        const uint64_t N = (uint64_t)plane * b.layers;
-        const uint32_t wp = planes_pitch(b.w);
-        const uint64_t NP = (uint64_t)wp * b.h * b.layers;  // cells of one plane, rows padded
-        const uint64_t c0 = (ch - chunk_start[lo]) * kPlaneChunk, c1 = min(c0 + kPlaneChunk, N);
+        const uint64_t first = chunk_start[lo], end = min(ch1, chunk_start[lo + 1]);
+        const uint32_t plane = b.w * b.h, wp = planes_pitch(b.w), qrow = wp / 4;
+        const uint32_t quads = qrow * b.h * b.layers;
+        const uint64_t NP = (uint64_t)quads * 4;
+        const uint4 *bound = b.bound ? b.bound : b.directed;
+        const bool al = (b.w & 3u) == 0;  // rows (and so quads) start on 16 bytes
         uint32_t *out = b.planes;
         // for the lower bounds: extremes and sums of this thread's cells
-        const uint4 *bound = b.bound ? b.bound : b.directed;
         uint32_t inv_dir = 0, inv_cost = 0, n_dir = 0, n_cost = 0;
         u64 sum_dir = 0, sum_cost = 0;
-        for (uint64_t i = c0 + threadIdx.x; i < c1; i += blockDim.x) {
-            const uint32_t c = (uint32_t)i;
-            const uint32_t l = c / plane, r = c - l * plane, y = r / b.w, x = r - y * b.w;
-            const uint8_t fc = b.flags ? __ldg(b.flags + c) : 0;
-            const uint32_t cost = __ldg(b.cost + c);
-            const uint32_t ec = (fc & kTraceNode) ? kMax : cost;  // obstacles stay kMax here
-            if (b.goal) {
-                if (ec != kMax) {
-                    inv_cost = max(inv_cost, ~cost);
-                    sum_cost += cost;
-                    ++n_cost;
+        for (; ch < end; ++ch) {
+            const uint32_t qi = (uint32_t)(ch - first) * kPlaneQuads + threadIdx.x;  // below 2^32 / 4 + rows
+            if (qi >= quads) continue;
+            const uint32_t row = qi / qrow, x0 = (qi - row * qrow) * 4;
+            const uint32_t l = row / b.h, y = row - l * b.h, c0 = row * b.w + x0, n = min(4u, b.w - x0);
+            // every load of the quad and its neighbours
+            uint32_t cost[4];
+            uint4 d[4], bd[4];
+            if (al) {
+                const uint4 v = __ldg(reinterpret_cast<const uint4 *>(b.cost + c0));
+                cost[0] = v.x; cost[1] = v.y; cost[2] = v.z; cost[3] = v.w;
+            } else {
+#pragma unroll
+                for (uint32_t k = 0; k < 4; ++k) cost[k] = k < n ? __ldg(b.cost + c0 + k) : kMax;
+            }
+#pragma unroll
+            for (uint32_t k = 0; k < 4; ++k) {
+                d[k] = make_uint4(kMax, kMax, kMax, kMax);
+                if (b.directed && k < n) d[k] = __ldg(b.directed + c0 + k);
+                bd[k] = d[k];
+                if (bound != b.directed && k < n) bd[k] = __ldg(bound + c0 + k);
+            }
+            const bool up = y > 0, dn = y + 1 < b.h, below = l > 0 && ((b.via_mask >> (l - 1)) & 1u),
+                       above = l + 1 < b.layers && ((b.via_mask >> l) & 1u);
+            uint32_t f = 0, fu = 0, fd = 0, fb = 0, fa = 0, fl = 0, fr = 0;
+            if (b.flags) {
+                const uint8_t *p = b.flags + c0;
+                f = flags4(p, al, n);
+                if (up) fu = flags4(p - b.w, al, n);
+                if (dn) fd = flags4(p + b.w, al, n);
+                if (below) fb = flags4(p - plane, al, n);
+                if (above) fa = flags4(p + plane, al, n);
+                if (x0 > 0) fl = __ldg(p - 1);
+                if (x0 + 4 < b.w) fr = __ldg(p + 4);
+            }
+            const uint32_t vb = below ? __ldg(b.via_edge + l - 1) : 0, va = above ? __ldg(b.via_edge + l) : 0;
+            uint32_t gx[5] = {0, 0, 0, 0, 0}, gu = 0, gd = 0;  // axis prices of the gaps left of x0 .. x0 + 4
+            if (!b.directed) {
+#pragma unroll
+                for (uint32_t k = 0; k < 5; ++k) {
+                    const uint32_t x = x0 + k;
+                    if (x > 0 && x < b.w) gx[k] = __ldg(b.x_edge + x - 1);
                 }
-                if (bound && !(fc & kTraceNode)) {  // obstacles too: a net enters its own pads
-                    const uint4 d = __ldg(bound + c);
-                    inv_dir = max(max(d.x == kMax ? 0u : ~d.x, d.y == kMax ? 0u : ~d.y),
-                                  max(max(d.z == kMax ? 0u : ~d.z, d.w == kMax ? 0u : ~d.w), inv_dir));
-                    if (d.y != kMax && ec != kMax) {
-                        sum_dir += d.y;
-                        ++n_dir;
+                if (up) gu = __ldg(b.y_edge + y - 1);
+                if (dn) gd = __ldg(b.y_edge + y);
+            }
+            uint32_t s[6][4];
+            // prices and weights of 16 bits multiply in one word (the usual case)
+            uint32_t any = gx[0] | gx[1] | gx[2] | gx[3] | gx[4] | gu | gd | vb | va;
+            for (uint32_t k = 0; k < 4; ++k) {
+                if (b.directed) any |= (d[k].x == kMax ? 0 : d[k].x) | (d[k].y == kMax ? 0 : d[k].y) |
+                                       (d[k].z == kMax ? 0 : d[k].z) | (d[k].w == kMax ? 0 : d[k].w);
+                any |= cost[k] == kMax ? 0 : cost[k];
+            }
+            const bool small = any < 65536u;
+            auto price = [&](uint32_t base, uint32_t w) { return small ? base * w : capmul(base, w); };
+#pragma unroll
+            for (uint32_t k = 0; k < 4; ++k) {
+                const uint32_t x = x0 + k, fc = (f >> (8 * k)) & 0xFFu;
+                const uint32_t ec = (k >= n || (fc & kTraceNode)) ? kMax : cost[k];  // obstacles stay kMax here
+#pragma unroll
+                for (int p = 0; p < 6; ++p) s[p][k] = kMax;
+                if (b.goal && k < n) {
+                    if (ec != kMax) {
+                        inv_cost = max(inv_cost, ~ec);
+                        sum_cost += ec;
+                        ++n_cost;
+                    }
+                    if (bound && !(fc & kTraceNode)) {  // obstacles too: a net enters its own pads
+                        const uint4 q = bd[k];
+                        inv_dir = max(max(q.x == kMax ? 0u : ~q.x, q.y == kMax ? 0u : ~q.y),
+                                      max(max(q.z == kMax ? 0u : ~q.z, q.w == kMax ? 0u : ~q.w), inv_dir));
+                        if (q.y != kMax && ec != kMax) {
+                            sum_dir += q.y;
+                            ++n_dir;
+                        }
                     }
                 }
-            }
-            uint32_t s[6] = {kMax, kMax, kMax, kMax, kMax, kMax};
-            if (ec != kMax) {
-                uint4 d = make_uint4(0, 0, 0, 0);
-                if (b.directed) d = __ldg(b.directed + c);
-                auto planar = [&](uint32_t base, uint32_t p, uint8_t out_bit, uint8_t in_bit) -> uint32_t {
-                    const uint8_t fp = b.flags ? __ldg(b.flags + p) : 0;
+                if (ec == kMax) continue;
+                // price of a planar move from a neighbour with flag byte fp
+                auto planar = [&](uint32_t base, uint32_t fp, uint8_t out_bit, uint8_t in_bit) -> uint32_t {
                     if ((fp & out_bit) | (fc & in_bit)) return kMax;
                     if (b.directed && base == kMax) return kMax;
-                    return capmul(base, ec);
+                    return price(base, ec);
                 };
-                if (x > 0) s[kInNegX] = planar(b.directed ? d.y : __ldg(b.x_edge + x - 1), c - 1, kEdgePosX, kEdgeNegX);
-                if (x + 1 < b.w) s[kInPosX] = planar(b.directed ? d.z : __ldg(b.x_edge + x), c + 1, kEdgeNegX, kEdgePosX);
-                if (y > 0) s[kInNegY] = planar(b.directed ? d.x : __ldg(b.y_edge + y - 1), c - b.w, kEdgePosY, kEdgeNegY);
-                if (y + 1 < b.h) s[kInPosY] = planar(b.directed ? d.w : __ldg(b.y_edge + y), c + b.w, kEdgeNegY, kEdgePosY);
-                if (b.layers > 1 && !via_blocked_board(fc)) {
-                    if (l > 0 && ((b.via_mask >> (l - 1)) & 1u)) {
-                        const uint8_t fq = b.flags ? __ldg(b.flags + c - plane) : 0;
-                        if (!via_blocked_board(fq)) s[kInBelow] = capmul(__ldg(b.via_edge + l - 1), ec);
-                    }
-                    if (l + 1 < b.layers && ((b.via_mask >> l) & 1u)) {
-                        const uint8_t fq = b.flags ? __ldg(b.flags + c + plane) : 0;
-                        if (!via_blocked_board(fq)) s[kInAbove] = capmul(__ldg(b.via_edge + l), ec);
-                    }
+                const uint32_t flx = k ? (f >> (8 * k - 8)) & 0xFFu : fl, frx = k < 3 ? (f >> (8 * k + 8)) & 0xFFu : fr;
+                if (x > 0) s[kInNegX][k] = planar(b.directed ? d[k].y : gx[k], flx, kEdgePosX, kEdgeNegX);
+                if (x + 1 < b.w) s[kInPosX][k] = planar(b.directed ? d[k].z : gx[k + 1], frx, kEdgeNegX, kEdgePosX);
+                if (up) s[kInNegY][k] = planar(b.directed ? d[k].x : gu, (fu >> (8 * k)) & 0xFFu, kEdgePosY, kEdgeNegY);
+                if (dn) s[kInPosY][k] = planar(b.directed ? d[k].w : gd, (fd >> (8 * k)) & 0xFFu, kEdgeNegY, kEdgePosY);
+                if (!via_blocked_board(fc)) {
+                    if (below && !via_blocked_board((fb >> (8 * k)) & 0xFFu)) s[kInBelow][k] = price(vb, ec);
+                    if (above && !via_blocked_board((fa >> (8 * k)) & 0xFFu)) s[kInAbove][k] = price(va, ec);
                 }
             }
-            const uint64_t o = ((uint64_t)l * b.h + y) * wp + x;
+            const uint64_t o = (uint64_t)row * wp + x0;
 #pragma unroll
             for (int p = 0; p < 6; ++p) {
-                uint32_t v = s[p];
                 if (hop_bits) {  // the layer kernel's words
-                    if (v < (1u << (29 - hop_bits))) {
-                        v = (v << hop_bits) | 1u;
-                    } else {
-                        if (v != kMax) b.goal->wide = 1;
-                        v = kPackedInf;
+#pragma unroll
+                    for (uint32_t k = 0; k < 4; ++k) {
+                        uint32_t v = s[p][k];
+                        if (v < (1u << (29 - hop_bits))) {
+                            v = (v << hop_bits) | 1u;
+                        } else {
+                            if (v != kMax) b.goal->wide = 1;
+                            v = kPackedInf;
+                        }
+                        s[p][k] = v;
                     }
                 }
-                out[(uint64_t)p * NP + o] = v;
+                *reinterpret_cast<uint4 *>(out + (uint64_t)p * NP + o) = make_uint4(s[p][0], s[p][1], s[p][2], s[p][3]);
             }
         }
-        if (b.goal) {
-            BoardGoal *g = b.goal;
+        if (b.goal) {  // the same for the whole block
+            const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
             inv_cost = __reduce_max_sync(0xFFFFFFFFu, inv_cost);
             inv_dir = __reduce_max_sync(0xFFFFFFFFu, inv_dir);
             n_cost = __reduce_add_sync(0xFFFFFFFFu, n_cost);
             n_dir = __reduce_add_sync(0xFFFFFFFFu, n_dir);
-            for (int o = 16; o; o >>= 1) {
-                sum_cost += __shfl_xor_sync(0xFFFFFFFFu, sum_cost, o);
-                sum_dir += __shfl_xor_sync(0xFFFFFFFFu, sum_dir, o);
+            for (int q = 16; q; q >>= 1) {
+                sum_cost += __shfl_xor_sync(0xFFFFFFFFu, sum_cost, q);
+                sum_dir += __shfl_xor_sync(0xFFFFFFFFu, sum_dir, q);
             }
-            if ((threadIdx.x & 31) == 0) {
+            __syncthreads();  // (the previous board's are read)
+            if (lane == 0) {
+                s_u[wid][0] = inv_cost; s_u[wid][1] = inv_dir; s_u[wid][2] = n_cost; s_u[wid][3] = n_dir;
+                s_s[wid][0] = sum_cost; s_s[wid][1] = sum_dir;
+            }
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                for (int w = 1; w < 8; ++w) {
+                    inv_cost = max(inv_cost, s_u[w][0]);
+                    inv_dir = max(inv_dir, s_u[w][1]);
+                    n_cost += s_u[w][2];
+                    n_dir += s_u[w][3];
+                    sum_cost += s_s[w][0];
+                    sum_dir += s_s[w][1];
+                }
+                BoardGoal *g = b.goal;
                 if (n_cost) {
                     atomicMax(&g->inv_min_cost, inv_cost);
                     atomicAdd(&g->sum_cost, sum_cost);
@@ -760,7 +849,9 @@ __global__ void warp_seed_kernel(RelaxArgs a) {
 
 }  // namespace
 
-uint64_t planes_chunks(uint64_t cells) { return (cells + kPlaneChunk - 1) / kPlaneChunk; }
+uint64_t planes_chunks(uint32_t w, uint32_t h, uint32_t layers) {
+    return ((uint64_t)(planes_pitch(w) / 4) * h * layers + kPlaneQuads - 1) / kPlaneQuads;
+}
 
 cudaError_t planes_launch(const DevBoard *boards, const uint64_t *chunk_start, uint32_t n_boards, uint64_t n_chunks,
                           uint32_t sms, uint32_t hop_bits, cudaStream_t st) {
