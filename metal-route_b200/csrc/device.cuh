@@ -101,6 +101,7 @@ struct DevField {
     uint32_t n_over;            // directed-price overrides of this field (DevBoard::over_cells)
     uint32_t over_off;
     uint32_t xa;                // columns by which the tile grid starts before the window
+    uint64_t out_off;           // first cell of this field among the emitted fields (output slot order)
 };
 
 // Tiles (32 columns) across a field's window.

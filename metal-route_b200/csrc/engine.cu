@@ -190,6 +190,119 @@ struct HostStage {
     }
 };
 
+// Page-locked, device-mapped host blocks, kept for reuse across calls (locking
+// pages costs far more than filling them) while any context lives: at most
+// kKept bytes of blocks of at most kBlock bytes each; the rest is freed at
+// once, and all of it with the last context.  One per process, as a block may
+// outlive the context that it came from; safe from any thread.
+class HostPool {
+   public:
+    static constexpr size_t kBlock = 64u << 20, kKept = 256u << 20, kLent = 512u << 20;
+    static HostPool &get() {
+        static HostPool *pool = new HostPool();  // not destroyed: blocks may be freed while the process exits
+        return *pool;
+    }
+    // `result`: a block for results, refused (null) when too large to keep or
+    // when kLent bytes are already out, so that results a caller hoards are pageable
+    void *alloc(size_t bytes, bool result) {
+        const size_t want = Pool::size_class(bytes);
+        {
+            std::lock_guard<std::mutex> lk(mu_);
+            if (result && (want > kBlock || lent_ + want > kLent)) return nullptr;
+            auto it = free_.lower_bound(want);
+            if (it != free_.end() && it->first <= 2 * want + (1u << 20)) {
+                void *p = it->second;
+                lend(p, it->first);
+                kept_ -= it->first;
+                free_.erase(it);
+                return p;
+            }
+        }
+        void *p = nullptr;
+        if (cudaHostAlloc(&p, want, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+            (void)cudaGetLastError();
+            return nullptr;
+        }
+        std::lock_guard<std::mutex> lk(mu_);
+        lend(p, want);
+        return p;
+    }
+    void release(void *p) {
+        if (!p) return;
+        {
+            std::lock_guard<std::mutex> lk(mu_);
+            auto it = used_.find(p);
+            if (it == used_.end()) return;
+            const size_t bytes = it->second;
+            used_.erase(it);
+            lent_ -= bytes;
+            if (users_ && bytes <= kBlock && kept_ + bytes <= kKept) {
+                free_.emplace(bytes, p);
+                kept_ += bytes;
+                return;
+            }
+        }
+        cudaFreeHost(p);
+    }
+    void attach() {
+        std::lock_guard<std::mutex> lk(mu_);
+        ++users_;
+    }
+    void detach() {
+        std::multimap<size_t, void *> gone;
+        {
+            std::lock_guard<std::mutex> lk(mu_);
+            if (--users_) return;
+            gone.swap(free_);
+            kept_ = 0;
+        }
+        for (auto &kv : gone) cudaFreeHost(kv.second);
+    }
+
+   private:
+    void lend(void *p, size_t bytes) {
+        used_[p] = bytes;
+        lent_ += bytes;
+    }
+    std::mutex mu_;
+    std::multimap<size_t, void *> free_;
+    std::unordered_map<void *, size_t> used_;
+    size_t kept_ = 0, lent_ = 0;
+    uint32_t users_ = 0;
+};
+
+// The fields of a result: a page-locked block, so that they come over at link
+// rate straight into it, or ordinary memory when the pool refuses.
+class FieldBlock {
+   public:
+    FieldBlock() = default;
+    FieldBlock(const FieldBlock &) = delete;
+    FieldBlock &operator=(const FieldBlock &) = delete;
+    ~FieldBlock() { reset(); }
+    void reset() {
+        if (pooled_) HostPool::get().release(p_);
+        else std::free(p_);
+        p_ = nullptr;
+    }
+    bool alloc(uint64_t n) {
+        reset();
+        const size_t bytes = std::max<uint64_t>(n, 1) * 4;
+        p_ = static_cast<uint32_t *>(HostPool::get().alloc(bytes, true));
+        pooled_ = p_ != nullptr;
+        if (!p_) p_ = static_cast<uint32_t *>(std::malloc(bytes));
+        return p_ != nullptr;
+    }
+    uint32_t *data() const { return p_; }
+    void swap(FieldBlock &o) {
+        std::swap(p_, o.p_);
+        std::swap(pooled_, o.pooled_);
+    }
+
+   private:
+    uint32_t *p_ = nullptr;
+    bool pooled_ = false;
+};
+
 }  // namespace
 
 struct mrc_context {
@@ -198,6 +311,7 @@ struct mrc_context {
     std::mutex mu;
     Pool pool;
     HostStage stage;
+    HostStage down;  // results on their way to the caller
     int sms = 148;
     size_t smem_optin = 0;
     // autotuned relax configuration per (layers, directed): tile height, CTA
@@ -704,7 +818,7 @@ struct mrc_result {
     std::vector<uint32_t> costs;
     bool has_fields = false;
     std::vector<uint64_t> field_offsets;
-    std::vector<uint32_t> fields;
+    FieldBlock fields;
     std::vector<mrc_window> field_windows;
 };
 
@@ -725,7 +839,7 @@ struct mrc_batch {
     uint32_t total_tiles = 0, max_tiles = 0, tile_h = 32, threads = kRelaxThreads, grid = 1;
     size_t smem = 0;
     DBuf d_tover;                  // per tile: holds price overrides of its field (has_over batches)
-    DBuf d_boards, d_fields, d_pads, d_lists, d_costs, d_lens, d_offsets, d_cells, d_out;
+    DBuf d_boards, d_fields, d_pads, d_lists, d_lens, d_heads, d_cells, d_out;
     // What a launch starts from, in two blocks so that a reset is two memsets:
     // zeros (control block, tile stamps, then the queue's ticket tags or the
     // rounds form's visited words) and ones (the label arena, waiting f per tile;
@@ -1041,14 +1155,22 @@ mrc_status batch_build(mrc_context *ctx, std::vector<const mrc_board *> boards, 
         if (pads.size() > 0xFFFFFFF0u) return fail(MRC_ERR_LIMIT, "pad lists exceed 2^32 entries");
     }
     bt->total_cells = off;
+    if (flags & MRC_FLAG_KEEP_FIELDS) {  // fields are emitted in request order
+        std::vector<uint64_t> at(n);
+        uint64_t o = 0;
+        for (uint32_t i = 0; i < n; ++i) {
+            at[i] = o;
+            o += cells_of(i);
+        }
+        for (DevField &f : bt->fields) f.out_off = at[f.out];
+    }
     bt->devs.clear();
     bt->devs.reserve(bt->boards.size());
     for (const mrc_board *b : bt->boards) bt->devs.push_back(b->dev);
     MRC_TRY(batch_layout(bt, tile_h, threads));
     MRC_TRY(upload(ctx, bt->d_pads, pads.data(), pads.size() * 4, "upload pads"));
-    MRC_TRY(bt->d_costs.get(ctx, std::max<size_t>(n, 1) * 4, "costs"));
     MRC_TRY(bt->d_lens.get(ctx, std::max<size_t>(n, 1) * 4, "lengths"));
-    MRC_TRY(bt->d_offsets.get(ctx, ((size_t)n + 1) * 8, "offsets"));
+    MRC_TRY(bt->d_heads.get(ctx, ((size_t)n + 1) * 8 + (size_t)n * 4, "offsets and costs"));  // one download
     MRC_TRY(bt->d_cells.get(ctx, std::max<uint64_t>(off, 1) * 4, "path cells"));
     if (flags & MRC_FLAG_KEEP_FIELDS) MRC_TRY(bt->d_out.get(ctx, std::max<uint64_t>(off, 1) * 4, "fields"));
     if (flags & MRC_FLAG_TIME_KERNELS) {
@@ -1071,9 +1193,9 @@ PathArgs path_args(const mrc_batch *bt) {
     pa.arena_filled = bt->async_q ? 1u : 0u;
     pa.hop_bits = layer_hop_bits(bt->max_layers);
     pa.walk_smem = bt->layer && !bt->has_over ? (uint32_t)walk_smem_bytes(bt->max_layers) : 0u;
-    pa.costs = bt->d_costs.as<uint32_t>();
+    pa.offsets = bt->d_heads.as<unsigned long long>();
+    pa.costs = reinterpret_cast<uint32_t *>(pa.offsets + bt->fields.size() + 1);
     pa.lens = bt->d_lens.as<uint32_t>();
-    pa.offsets = bt->d_offsets.as<unsigned long long>();
     pa.cells = bt->d_cells.as<uint32_t>();
     pa.status = &bt->ctl()->status;
     return pa;
@@ -1173,32 +1295,46 @@ mrc_status status_error(uint32_t status) {
     return fail(MRC_ERR_BACKEND_UNAVAILABLE, "tile queue overflow");
 }
 
-// Copy one batch's outputs (indexed like bt->nets).
-mrc_status batch_collect(mrc_batch *bt, bool keep_fields, std::vector<uint32_t> *costs,
-                         std::vector<std::vector<uint32_t>> *paths, std::vector<std::vector<uint32_t>> *fields) {
+// Outputs of one batch, indexed like bt->nets: paths and fields in CSR form.
+struct BatchOut {
+    std::vector<uint32_t> costs, cells;
+    std::vector<uint64_t> offsets;
+    FieldBlock fields;
+};
+
+// Copy one batch's outputs to the host: status, offsets and costs and as many path
+// cells as such a batch usually has in one go through the page-locked block,
+// fields straight into theirs, and one wait for all of it.
+mrc_status batch_collect(mrc_batch *bt, bool keep_fields, BatchOut *out) {
+    mrc_context *ctx = bt->ctx;
     cudaStream_t st = bt->stream;
     const uint32_t n = (uint32_t)bt->fields.size();
-    uint32_t status = 0;
-    MRC_CUDA(cudaMemcpyAsync(&status, &bt->ctl()->status, 4, cudaMemcpyDeviceToHost, st), "read status");
-    std::vector<uint64_t> off(n + 1);
-    costs->assign(n, kMax);
-    if (n) MRC_CUDA(cudaMemcpyAsync(costs->data(), bt->d_costs.p, (size_t)n * 4, cudaMemcpyDeviceToHost, st), "read costs");
-    MRC_CUDA(cudaMemcpyAsync(off.data(), bt->d_offsets.p, ((size_t)n + 1) * 8, cudaMemcpyDeviceToHost, st), "read offsets");
+    constexpr size_t kCellsPerNet = 256;  // path cells copied before their number is known
+    const uint64_t early = std::min<uint64_t>(bt->total_cells, (uint64_t)n * kCellsPerNet);
+    const size_t heads = ((size_t)n + 1) * 8 + (size_t)n * 4, o_cells = (16 + heads + 15) & ~(size_t)15;
+    MRC_CUDA(ctx->down.reserve(o_cells + early * 4), "pinned download buffer");
+    unsigned char *host = static_cast<unsigned char *>(ctx->down.p);
+    MRC_CUDA(cudaMemcpyAsync(host, &bt->ctl()->status, 4, cudaMemcpyDeviceToHost, st), "read status");
+    MRC_CUDA(cudaMemcpyAsync(host + 16, bt->d_heads.p, heads, cudaMemcpyDeviceToHost, st), "read offsets and costs");
+    if (early) MRC_CUDA(cudaMemcpyAsync(host + o_cells, bt->d_cells.p, early * 4, cudaMemcpyDeviceToHost, st), "read paths");
+    const bool fields = keep_fields && bt->total_cells && bt->d_out.p;
+    if (keep_fields && !out->fields.alloc(bt->total_cells)) return fail(MRC_ERR_OUT_OF_MEMORY, "host memory for the fields");
+    if (fields)
+        MRC_CUDA(cudaMemcpyAsync(out->fields.data(), bt->d_out.p, bt->total_cells * 4, cudaMemcpyDeviceToHost, st), "read fields");
     MRC_CUDA(cudaStreamSynchronize(st), "batch execution");
+    uint32_t status = 0;
+    std::memcpy(&status, host, 4);
     if (status) return status_error(status);
-    std::vector<uint32_t> cells(off[n]);
-    if (off[n]) MRC_CUDA(cudaMemcpy(cells.data(), bt->d_cells.p, off[n] * 4, cudaMemcpyDeviceToHost), "read paths");
-    paths->assign(n, {});
-    for (uint32_t i = 0; i < n; ++i) (*paths)[i].assign(cells.begin() + off[i], cells.begin() + off[i + 1]);
-    if (keep_fields) {
-        fields->assign(n, {});
-        std::vector<uint32_t> all(bt->total_cells);
-        if (bt->total_cells && bt->d_out.p)
-            MRC_CUDA(cudaMemcpy(all.data(), bt->d_out.p, bt->total_cells * 4, cudaMemcpyDeviceToHost), "read fields");
-        for (const DevField &f : bt->fields) {
-            const uint64_t c = (uint64_t)f.ww * f.wh * bt->boards[f.board]->view.layers;
-            (*fields)[f.out].assign(all.begin() + f.lab_off, all.begin() + f.lab_off + c);
-        }
+    const uint64_t *off = reinterpret_cast<const uint64_t *>(host + 16);
+    const uint32_t *costs = reinterpret_cast<const uint32_t *>(off + n + 1), *cells = reinterpret_cast<const uint32_t *>(host + o_cells);
+    out->offsets.assign(off, off + n + 1);
+    out->costs.assign(costs, costs + n);
+    const uint64_t total = off[n], have = std::min(total, early);
+    out->cells.assign(cells, cells + have);
+    if (have < total) {
+        out->cells.resize(total);
+        MRC_CUDA(cudaMemcpy(out->cells.data() + have, bt->d_cells.as<uint32_t>() + have, (total - have) * 4,
+                            cudaMemcpyDeviceToHost), "read paths");
     }
     return MRC_OK;
 }
@@ -1227,65 +1363,82 @@ mrc_status solve(mrc_context *ctx, std::vector<const mrc_board *> boards, std::v
 // Results of a launched batch (waits for it), with the full-board retry.
 mrc_status finish_batch(mrc_context *ctx, mrc_batch *bt, uint32_t flags, mrc_result **out) {
     const bool keep = (flags & MRC_FLAG_KEEP_FIELDS) != 0;
-    std::vector<uint32_t> costs;
-    std::vector<std::vector<uint32_t>> paths, fields;
-    MRC_TRY(batch_collect(bt, keep, &costs, &paths, &fields));
+    BatchOut got;
+    MRC_TRY(batch_collect(bt, keep, &got));
     std::unique_ptr<mrc_result> r(new mrc_result());
     const uint32_t n = (uint32_t)bt->nets.size();
     r->n = n;
     r->field_windows = bt->windows;
+    std::vector<uint32_t> idx;  // nets solved again on their whole board
     if (flags & MRC_FLAG_RETRY_FULL) {
-        std::vector<uint32_t> idx;
         for (uint32_t i = 0; i < n; ++i) {
             const GridView &g = bt->boards[bt->nets[i].board]->view;
-            if (costs[i] == kMax && !is_full(bt->windows[i], g.w, g.h)) idx.push_back(i);
-        }
-        if (!idx.empty()) {
-            std::vector<NetCopy> rn;
-            std::vector<mrc_window> rw;
-            for (uint32_t i : idx) {
-                rn.push_back(bt->nets[i]);
-                const GridView &g = bt->boards[bt->nets[i].board]->view;
-                rw.push_back(full_window(g.w, g.h));
-            }
-            mrc_batch retry;
-            MRC_TRY(batch_build(ctx, bt->boards, std::move(rn), std::move(rw), flags & ~MRC_FLAG_TIME_KERNELS, &retry));
-            // on the engine stream, behind the retry batch's own uploads
-            MRC_TRY(batch_launch(&retry, ctx->stream));
-            std::vector<uint32_t> c2;
-            std::vector<std::vector<uint32_t>> p2, f2;
-            MRC_TRY(batch_collect(&retry, keep, &c2, &p2, &f2));
-            for (size_t k = 0; k < idx.size(); ++k) {
-                costs[idx[k]] = c2[k];
-                paths[idx[k]] = std::move(p2[k]);
-                if (keep) fields[idx[k]] = std::move(f2[k]);
-                r->field_windows[idx[k]] = retry.windows[k];
-            }
-            r->retried = (uint32_t)idx.size();
+            if (got.costs[i] == kMax && !is_full(bt->windows[i], g.w, g.h)) idx.push_back(i);
         }
     }
-    r->costs = std::move(costs);
-    r->offsets.resize(n + 1);
-    uint64_t o = 0;
-    for (uint32_t i = 0; i < n; ++i) {
-        r->offsets[i] = o;
-        o += paths[i].size();
-    }
-    r->offsets[n] = o;
-    r->cells.reserve(o);
-    for (auto &p : paths) r->cells.insert(r->cells.end(), p.begin(), p.end());
-    if (keep) {
-        r->has_fields = true;
-        r->field_offsets.resize(n + 1);
-        uint64_t fo = 0;
+    auto cells_of = [&](uint32_t i) {
+        const mrc_window &w = r->field_windows[i];
+        return (uint64_t)(w.x1 - w.x0 + 1) * (w.y1 - w.y0 + 1) * bt->boards[bt->nets[i].board]->view.layers;
+    };
+    auto lay_fields = [&](std::vector<uint64_t> *at) {
+        at->resize(n + 1);
+        uint64_t o = 0;
         for (uint32_t i = 0; i < n; ++i) {
-            r->field_offsets[i] = fo;
-            fo += fields[i].size();
+            (*at)[i] = o;
+            o += cells_of(i);
         }
-        r->field_offsets[n] = fo;
-        r->fields.reserve(fo);
-        for (auto &f : fields) r->fields.insert(r->fields.end(), f.begin(), f.end());
+        (*at)[n] = o;
+    };
+    r->has_fields = keep;
+    if (keep) lay_fields(&r->field_offsets);
+    if (idx.empty()) {
+        r->costs = std::move(got.costs);
+        r->offsets = std::move(got.offsets);
+        r->cells = std::move(got.cells);
+        r->fields.swap(got.fields);
+        *out = r.release();
+        return MRC_OK;
     }
+    std::vector<NetCopy> rn;
+    std::vector<mrc_window> rw;
+    for (uint32_t i : idx) {
+        rn.push_back(bt->nets[i]);
+        const GridView &g = bt->boards[bt->nets[i].board]->view;
+        rw.push_back(full_window(g.w, g.h));
+    }
+    mrc_batch retry;
+    MRC_TRY(batch_build(ctx, bt->boards, std::move(rn), std::move(rw), flags & ~MRC_FLAG_TIME_KERNELS, &retry));
+    // on the engine stream, behind the retry batch's own uploads
+    MRC_TRY(batch_launch(&retry, ctx->stream));
+    BatchOut again;
+    MRC_TRY(batch_collect(&retry, keep, &again));
+    r->retried = (uint32_t)idx.size();
+    const std::vector<uint64_t> first = r->field_offsets;  // of the window fields
+    for (size_t k = 0; k < idx.size(); ++k) r->field_windows[idx[k]] = retry.windows[k];
+    if (keep) {
+        lay_fields(&r->field_offsets);
+        if (!r->fields.alloc(r->field_offsets[n])) return fail(MRC_ERR_OUT_OF_MEMORY, "host memory for the fields");
+    }
+    r->offsets.resize(n + 1);
+    r->costs = std::move(got.costs);
+    r->cells.reserve(got.cells.size() + again.cells.size());
+    uint64_t fo = 0;  // fields of the retry so far
+    for (uint32_t i = 0, k = 0; i < n; ++i) {
+        const bool re = k < idx.size() && idx[k] == i;
+        const BatchOut &src = re ? again : got;
+        const uint32_t j = re ? k : i;
+        r->offsets[i] = r->cells.size();
+        r->cells.insert(r->cells.end(), src.cells.begin() + src.offsets[j], src.cells.begin() + src.offsets[j + 1]);
+        if (re) r->costs[i] = again.costs[k];
+        if (keep) {
+            const uint64_t c = cells_of(i);
+            std::memcpy(r->fields.data() + r->field_offsets[i], re ? again.fields.data() + fo : got.fields.data() + first[i],
+                        c * 4);
+            if (re) fo += c;
+        }
+        k += re;
+    }
+    r->offsets[n] = r->cells.size();
     *out = r.release();
     return MRC_OK;
 }
@@ -1348,6 +1501,7 @@ mrc_status mrc_context_create(int device, mrc_context **out) {
     ctx->sms = prop.multiProcessorCount;
     ctx->smem_optin = prop.sharedMemPerBlockOptin;
     MRC_CUDA(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking), "create stream");
+    HostPool::get().attach();
     *out = ctx.release();
     return MRC_OK;
 }
@@ -1364,24 +1518,20 @@ void mrc_context_destroy(mrc_context *ctx) {
         ctx->pool.trim();
     }
     delete ctx;
+    HostPool::get().detach();
 }
 
 mrc_status mrc_host_alloc(mrc_context *ctx, size_t bytes, void **out) {
     if (!ctx || !out) return fail(MRC_ERR_INVALID_ARGUMENT, "NULL argument");
     *out = nullptr;
     MRC_TRY(set_device(ctx));
-    void *p = nullptr;
-    if (cudaHostAlloc(&p, std::max<size_t>(bytes, 16), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
-        (void)cudaGetLastError();
-        return fail(MRC_ERR_OUT_OF_MEMORY, "page-locked host allocation of " + std::to_string(bytes) + " bytes failed");
-    }
+    void *p = HostPool::get().alloc(std::max<size_t>(bytes, 16), false);
+    if (!p) return fail(MRC_ERR_OUT_OF_MEMORY, "page-locked host allocation of " + std::to_string(bytes) + " bytes failed");
     *out = p;
     return MRC_OK;
 }
 
-void mrc_host_free(void *p) {
-    if (p) cudaFreeHost(p);
-}
+void mrc_host_free(void *p) { HostPool::get().release(p); }
 
 mrc_status mrc_upload_stats(mrc_context *ctx, uint64_t *staged_bytes, uint64_t *in_place_bytes) {
     if (!ctx || !staged_bytes || !in_place_bytes) return fail(MRC_ERR_INVALID_ARGUMENT, "NULL argument");
@@ -1492,11 +1642,20 @@ mrc_status mrc_distance_fields(mrc_context *ctx, const mrc_grid *grid, const uin
     mrc_board board;
     MRC_TRY(board_build(ctx, grid, &e, false, &board));
     std::vector<mrc_window> wins(nc.size(), full_window(g.w, g.h));
-    mrc_result *r = nullptr;
-    MRC_TRY(solve(ctx, {&board}, std::move(nc), std::move(wins), MRC_FLAG_KEEP_FIELDS, &r, nullptr));
-    std::unique_ptr<mrc_result> hold(r);
-    for (size_t k = 0; k < slot.size(); ++k)
-        std::memcpy(fields + (size_t)slot[k] * g.n, r->fields.data() + r->field_offsets[k], (size_t)g.n * 4);
+    // straight into the caller's rows: one copy while no source is refused
+    mrc_batch bt;
+    MRC_TRY(batch_build(ctx, {&board}, std::move(nc), std::move(wins), MRC_FLAG_KEEP_FIELDS, &bt));
+    MRC_TRY(batch_launch(&bt, ctx->stream));
+    uint32_t status = 0;
+    MRC_CUDA(cudaMemcpyAsync(&status, &bt.ctl()->status, 4, cudaMemcpyDeviceToHost, ctx->stream), "read status");
+    for (size_t k = 0, e; k < slot.size(); k = e) {
+        for (e = k + 1; e < slot.size() && slot[e] == slot[e - 1] + 1;) ++e;
+        MRC_CUDA(cudaMemcpyAsync(fields + (size_t)slot[k] * g.n, bt.d_out.as<uint32_t>() + k * g.n, (e - k) * g.n * 4,
+                                 cudaMemcpyDeviceToHost, ctx->stream),
+                 "read fields");
+    }
+    MRC_CUDA(cudaStreamSynchronize(ctx->stream), "distance fields");
+    if (status) return status_error(status);
     return MRC_OK;
 }
 
@@ -2583,7 +2742,11 @@ void server_reap(mrc_server *s, ServerBatch *b) {
                 const uint64_t f0 = res->field_offsets[first], f1 = res->field_offsets[first + n];
                 o->field_offsets.resize(n + 1);
                 for (uint32_t i = 0; i <= n; ++i) o->field_offsets[i] = res->field_offsets[first + i] - f0;
-                o->fields.assign(res->fields.begin() + f0, res->fields.begin() + f1);
+                if (o->fields.alloc(f1 - f0)) std::memcpy(o->fields.data(), res->fields.data() + f0, (f1 - f0) * 4);
+                else {
+                    r->status = MRC_ERR_OUT_OF_MEMORY;
+                    r->error = "host memory for the fields";
+                }
             }
             r->result = std::move(o);
         }
@@ -3060,6 +3223,7 @@ extern "C" mrc_status mrc_route_isolated_plain(mrc_context *ctx, const mrc_isola
     r->field_windows = wins;
     r->has_fields = keep;
     r->field_offsets.assign(n + 1, 0);
+    std::vector<uint32_t> all;  // fields of every net
     for (uint32_t i = 0; i < n; ++i) {
         std::vector<uint32_t> path, field;
         uint32_t cost = kMax;
@@ -3074,8 +3238,12 @@ extern "C" mrc_status mrc_route_isolated_plain(mrc_context *ctx, const mrc_isola
         r->cells.insert(r->cells.end(), path.begin(), path.end());
         if (keep) {
             r->field_offsets[i + 1] = r->field_offsets[i] + field.size();
-            r->fields.insert(r->fields.end(), field.begin(), field.end());
+            all.insert(all.end(), field.begin(), field.end());
         }
+    }
+    if (keep) {
+        if (!r->fields.alloc(all.size())) return fail(MRC_ERR_OUT_OF_MEMORY, "host memory for the fields");
+        if (!all.empty()) std::memcpy(r->fields.data(), all.data(), all.size() * 4);
     }
     *out = r.release();
     return MRC_OK;

@@ -455,7 +455,8 @@ __global__ void __launch_bounds__(256) path_walk_kernel(PathArgs a) {
 }
 
 // Complete u32 distance field of every field (MRC_FLAG_KEEP_FIELDS).
-// `fields_by_offset` lists the fields in ascending lab_off order.
+// The fields come in ascending lab_off order and are emitted in output slot order,
+// so that they are downloaded as one block.
 __global__ void emit_fields_kernel(PathArgs a, uint32_t *out, uint64_t total) {
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
          i += (uint64_t)gridDim.x * blockDim.x) {
@@ -470,7 +471,7 @@ __global__ void emit_fields_kernel(PathArgs a, uint32_t *out, uint64_t total) {
         const uint32_t li = (uint32_t)(i - f.lab_off);
         const uint32_t rr = li / f.ww, lx = li - rr * f.ww;
         const uint32_t l = rr / f.wh, ly = rr - l * f.wh;
-        out[i] = (uint32_t)(field_label(a, f, lx, ly, l) >> 32);
+        out[f.out_off + li] = (uint32_t)(field_label(a, f, lx, ly, l) >> 32);
     }
 }
 

@@ -453,7 +453,20 @@ class IsolatedBatchResult:
                                    offsets=off - np.uint64(a), cells=self.cells[a:b], costs=self.costs[start:stop])
 
 
+class _ResultHold:
+    """Frees a C result when the arrays that view its memory go away."""
+
+    def __init__(self, lib, res):
+        self.lib, self.res = lib, res
+
+    def __del__(self):
+        if self.res:
+            self.lib.mrc_result_free(self.res)
+            self.res = None
+
+
 def _take_result(L, res, n: int, fields: bool, layers: int = 1) -> IsolatedBatchResult:
+    hold = _ResultHold(L, res)  # freed on return, unless the fields' array keeps it
     try:
         cnt = L.mrc_result_count(res)
         assert cnt == n, (cnt, n)
@@ -471,12 +484,17 @@ def _take_result(L, res, n: int, fields: bool, layers: int = 1) -> IsolatedBatch
         if fields:
             fo = np.ctypeslib.as_array(L.mrc_result_field_offsets(res), shape=(n + 1,)).copy()
             ft = int(fo[-1])
-            fa = (np.ctypeslib.as_array(L.mrc_result_fields(res), shape=(ft,)).copy() if ft
-                  else np.zeros(0, np.uint32))
-            out.fields = [fa[fo[i]:fo[i + 1]] for i in range(n)]
+            if ft:  # the fields stay where the library downloaded them
+                buf = (C.c_uint32 * ft).from_address(C.addressof(L.mrc_result_fields(res).contents))
+                buf._hold = hold
+                fa = np.frombuffer(buf, dtype=np.uint32)
+            else:
+                fa = np.zeros(0, np.uint32)
+            fl = fo.tolist()
+            out.fields = [fa[fl[i]:fl[i + 1]] for i in range(n)]
         return out
     finally:
-        L.mrc_result_free(res)
+        del hold
 
 
 class Board:
@@ -844,6 +862,26 @@ class _HostBlock:
             self.ptr = 0
 
 
+class _ResultBlock(_HostBlock):
+    """A page-locked block lent to a result array; at most LIMIT bytes are lent at
+    once, so that results a caller hoards stay in ordinary memory."""
+
+    LIMIT = 256 << 20
+    lent = 0
+    lock = threading.Lock()
+
+    def __init__(self, lib, ptr: int, nbytes: int):
+        super().__init__(lib, ptr)
+        self.nbytes = nbytes
+        with _ResultBlock.lock:
+            _ResultBlock.lent += nbytes
+
+    def __del__(self):
+        super().__del__()
+        with _ResultBlock.lock:
+            _ResultBlock.lent -= self.nbytes
+
+
 class Engine:
     """One CUDA context of the engine (one per process per device)."""
 
@@ -900,6 +938,21 @@ class Engine:
         buf = (C.c_char * max(nbytes, 1)).from_address(p.value)
         buf._block = _HostBlock(self.lib, p.value)
         return np.frombuffer(buf, dtype=dtype, count=nbytes // dtype.itemsize).reshape(shape)
+
+    def _result_empty(self, shape, dtype) -> np.ndarray:
+        """An uninitialised array for a result the library fills: page-locked (so
+        that it comes over at full link rate) up to 64 MiB, while not too many are
+        held, else ordinary memory."""
+        dtype = np.dtype(dtype)
+        nbytes = int(np.prod(shape, dtype=np.int64)) * dtype.itemsize
+        if not 0 < nbytes <= 64 << 20 or _ResultBlock.lent + nbytes > _ResultBlock.LIMIT:
+            return np.empty(shape, dtype)
+        p = C.c_void_p()
+        if self.lib.mrc_host_alloc(self.ctx, nbytes, C.byref(p)) != MRC_OK:
+            return np.empty(shape, dtype)
+        buf = (C.c_char * nbytes).from_address(p.value)
+        buf._block = _ResultBlock(self.lib, p.value, nbytes)
+        return np.frombuffer(buf, dtype=dtype).reshape(shape)
 
     def upload_stats(self) -> dict:
         """Board bytes moved to HBM so far: staged, and read in place from
@@ -978,7 +1031,7 @@ class Engine:
     def distance_fields(self, grid: Grid, sources: Sequence[int]) -> np.ndarray:
         m = _Marshal()
         src = _u32(sources)
-        out = np.zeros((len(sources), len(grid.dims)), dtype=np.uint32)
+        out = self._result_empty((len(sources), len(grid.dims)), np.uint32)  # every row is written
         if len(sources):
             self._check(self.lib.mrc_distance_fields(self.ctx, C.byref(m.grid(grid)), m.arr(src), len(sources),
                                                      m.arr(out)))
