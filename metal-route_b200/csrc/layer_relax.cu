@@ -45,7 +45,7 @@ constexpr uint32_t kNarrow = 1u << 29;  // staged labels, final labels and price
 // the columns of a warp fall on distinct banks.
 constexpr uint32_t kPitch = kPlaneTmaBoxW;
 constexpr uint32_t kSpecCap = 512;      // cells of a tile priced for the net itself
-constexpr int kPlaneIters = 4;          // column and row passes of a plane between two meetings
+constexpr int kPlaneIters = 2;          // column and row passes of a plane between two meetings
 
 __host__ __device__ inline size_t layer_st_off(uint32_t L) { return ((size_t)L * TH * kPitch * 4 + 127) & ~(size_t)127; }
 
@@ -88,7 +88,7 @@ __device__ __forceinline__ uint32_t pack_price(uint32_t p, uint32_t *wide) {
 template <int NL>
 __device__ __forceinline__ void stack_rows(uint32_t *lab, const uint32_t *st, uint32_t y0, uint32_t step) {
     constexpr uint32_t LS = TH * kPitch, SP = NL * LS;  // words from a layer, from a plane, to the next
-#pragma unroll 2
+#pragma unroll 1
     for (uint32_t y = y0; y < TH; y += step) {
         uint32_t *q = lab + y * kPitch;
         const uint32_t *pu = st + kInBelow * SP + y * kPitch, *pd = st + kInAbove * SP + y * kPitch;
@@ -172,6 +172,7 @@ __device__ __forceinline__ bool layer_item(const RelaxArgs &a, uint32_t fi, uint
     uint32_t *state = a.tstamp + f.tile_off + t;
     const bool mine = wl < L;                            // this warp has a layer
     const bool col_in = mine && lane >= xlo && lane < tw;  // this lane has a column of the window
+    uint2 lim0;
     if (tid == 0) {
         // hold the tile before reading any label: a neighbour that improves our
         // halo after this point marks it dirty, and we carry it on
@@ -183,15 +184,12 @@ __device__ __forceinline__ bool layer_item(const RelaxArgs &a, uint32_t fi, uint
         tma_load_4d(st, b.tmap, tx0, ty0, 0, 0, &sh.mbar);
         if constexpr (GD) {
             a.tpark[f.tile_off + t] = kMax;  // what waited is in the labels read from here on
-            const uint2 lim = __ldcg(reinterpret_cast<const uint2 *>(a.goal + fi));
-            sh.ub = lim.x;   // an older (larger) bound of the target is still a bound
-            sh.thr = lim.y;  // the threshold only moves while no item of the field is in flight
+            lim0 = __ldcg(reinterpret_cast<const uint2 *>(a.goal + fi));
         }
-        __threadfence();
     }
     const uint32_t board_wide = __ldg(&b.goal->wide);
     // GD: remaining price along each axis
-    uint32_t hx = 0, hxs = 0, hl = 0;
+    uint32_t hxl = 0, hxls = 0;  // of this lane's column, and of its halo column, on this layer
     bool dst_here = false, dst_mine = false;
     uint32_t dst_row = 0;
     if constexpr (GD) {
@@ -202,17 +200,22 @@ __device__ __forceinline__ bool layer_item(const RelaxArgs &a, uint32_t fi, uint
             return goal_rest(sums, each, e, (uint32_t)min(max(at, 0), (int)n - 1), to);
         };
         const uint32_t *px = b.directed ? nullptr : b.x_sum, *py = b.directed ? nullptr : b.y_sum, *pv = b.via_sum;
-        hx = rest(px, tx0 + (int)lane, b.w, dst_x);
-        hxs = rest(px, seg == 0 ? tx0 - 1 : tx0 + (int)kTW, b.w, dst_x);
-        hl = rest(pv, (int)wl, L, dst_l);
+        const uint32_t hl = rest(pv, (int)wl, L, dst_l);
+        hxl = dsum(rest(px, tx0 + (int)lane, b.w, dst_x), hl);
+        hxls = dsum(rest(px, seg == 0 ? tx0 - 1 : tx0 + (int)kTW, b.w, dst_x), hl);
         if (wl == 0 && lane < TH + 2) sh.hy[lane] = rest(py, ty0 + (int)lane - 1, b.h, dst_y);
         dst_here = dst_x >= (uint32_t)tx0 + xlo && dst_x < (uint32_t)tx0 + tw && dst_y >= (uint32_t)ty0 &&
                    dst_y < (uint32_t)ty0 + th;
         dst_row = dst_y - (uint32_t)ty0;
         dst_mine = dst_here && wl == dst_l && lane == dst_x - (uint32_t)tx0;
     }
-    // f of a label (dist) at a cell with these remaining prices
-    auto bound = [&](uint32_t dist, uint32_t h) { return min(dsum(dist, h), kCap); };
+    if (tid == 0) {
+        __threadfence();  // the hold before the labels
+        if constexpr (GD) {
+            sh.ub = lim0.x;   // an older (larger) bound of the target is still a bound
+            sh.thr = lim0.y;  // the threshold only moves while no item of the field is in flight
+        }
+    }
     __syncthreads();
 
     const u64 *glab = a.lab + f.lab_off;
@@ -283,35 +286,29 @@ __device__ __forceinline__ bool layer_item(const RelaxArgs &a, uint32_t fi, uint
         uint32_t ub = kMax;
         uint32_t w[TH], w0[TH], lim[TH], ht, hb, hs;
         if constexpr (GD) ub = sh.ub;
-        auto pack = [&](u64 q, uint32_t h) {
-            const uint32_t d = (uint32_t)(q >> 32);
-            if (d == kMax) return kBig;
-            if (GD && bound(d, h) > ub) return kBig;  // past the target's bound it does not matter
-            const uint32_t rel = d - dbase;
-            if (rel < (kNarrow >> HB)) return (rel << HB) | (((uint32_t)q - hbase) & kHopMask);
-            bad = true;
-            return kBig;
+        // GD: the word from which on a label at a cell with remaining price h is past
+        // the bound `top`: (top - dbase - h + 1) << HB between 0 and kBig
+        auto limit = [&](uint32_t top, uint32_t h) -> uint32_t {
+            if (!GD || top == kMax) return kBig;
+            const uint32_t room = top >= dbase ? top - dbase + 1u : 0u;
+            return min(max(room, h) - h, kBig >> HB) << HB;
         };
-        // GD: labels at or above lim[y] are past the target's bound
+        auto pack = [&](u64 q, uint32_t past) {
+            const uint32_t d = (uint32_t)(q >> 32);
+            const uint32_t v = (min(d - dbase, kBig >> HB) << HB) | (((uint32_t)q - hbase) & kHopMask);
+            if (d != kMax && v >= kNarrow && (v < past || past == kBig)) bad = true;  // it matters and does not fit
+            return d == kMax || v >= min(past, kNarrow) ? kBig : v;
+        };
         auto set_limits = [&]() {
 #pragma unroll
-            for (int y = 0; y < TH; ++y) {
-                lim[y] = kBig;
-                if constexpr (GD) {
-                    if (ub != kMax) {
-                        const int64_t room = (int64_t)ub - dbase - hx - hl - sh.hy[y + 1];
-                        lim[y] = room < 0 ? 0u : room < (int64_t)((kBig >> HB) - 1) ? (uint32_t)(room + 1) << HB : kBig;
-                    }
-                }
-            }
+            for (int y = 0; y < TH; ++y) lim[y] = GD ? limit(ub, dsum(hxl, sh.hy[y + 1])) : kBig;
         };
         set_limits();
-        const uint32_t hxl = dsum(hx, hl);
 #pragma unroll
-        for (int y = 0; y < TH; ++y) w0[y] = w[y] = pack(v[y], GD ? dsum(hxl, sh.hy[y + 1]) : 0);
-        ht = pack(vt, GD ? dsum(hxl, sh.hy[0]) : 0);
-        hb = pack(vb, GD ? dsum(hxl, sh.hy[TH + 1]) : 0);
-        hs = pack(vs, GD ? dsum(dsum(hxs, hl), sh.hy[r + 1]) : 0);
+        for (int y = 0; y < TH; ++y) w0[y] = w[y] = pack(v[y], lim[y]);
+        ht = pack(vt, GD ? limit(ub, dsum(hxl, sh.hy[0])) : kBig);
+        hb = pack(vb, GD ? limit(ub, dsum(hxl, sh.hy[TH + 1])) : kBig);
+        hs = pack(vs, GD ? limit(ub, dsum(hxls, sh.hy[r + 1])) : kBig);
         if (cont == 0) {
             // the planes: a bounded wait for the TMA load (a load that never lands
             // sets the status and the launch ends without results)
@@ -533,10 +530,7 @@ __device__ __forceinline__ bool layer_item(const RelaxArgs &a, uint32_t fi, uint
         }
         if (__syncthreads_or(bad || *(volatile uint32_t *)&sh.wide))
             return wide_item<OV, GD>(a, fi, t, smem_raw, sh.cnt);
-        if constexpr (GD) {
-            ub = *(volatile uint32_t *)&sh.ub;
-            if (dst_here) set_limits();
-        }
+        if constexpr (GD) ub = *(volatile uint32_t *)&sh.ub;
 
         // ---- write back the labels that fell -----------------------------------
         if (mine) {
@@ -552,13 +546,19 @@ __device__ __forceinline__ bool layer_item(const RelaxArgs &a, uint32_t fi, uint
             // staged label.
             const uint32_t edge = side ? lab[(wl * TH + r) * kPitch + (seg == 0 ? 0u : kTW - 1)] : kBig;
             uint32_t own[3] = {w[0], w[TH - 1], edge}, price[3] = {pt, pb, ps}, there[3] = {ht, hb, hs};
-            uint32_t fv[3];    // GD: f of the improved label
-            bool better[3];
+            bool better[3], wait[3] = {false, false, false};  // improved; GD: improved, past the threshold
+            uint32_t ex[3] = {kMax, kMax, kMax};               // dist of an exactly priced improvement
+            const uint32_t thr = GD ? sh.thr : kMax;
+            const uint32_t h[3] = {GD ? dsum(hxl, sh.hy[0]) : 0u, GD ? dsum(hxl, sh.hy[TH + 1]) : 0u,
+                                   GD ? dsum(hxls, sh.hy[r + 1]) : 0u};
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
-                const uint32_t cand = own[k] + price[k];
-                better[k] = cand < there[k];  // (no price or label: at least kBig, as `there` at most)
-                fv[k] = dbase + (cand >> HB);
+                const uint32_t cand = own[k] + price[k];  // (no price or label: at least kBig, as `there` at most)
+                better[k] = cand < there[k];
+                if constexpr (GD) {
+                    better[k] &= cand < limit(ub, h[k]);
+                    wait[k] = better[k] && cand >= limit(thr, h[k]);
+                }
             }
             if (sh.near_pad || (OV && f.n_over)) {  // its own pads, or its own prices, beyond the border
 #pragma unroll 1
@@ -579,32 +579,26 @@ __device__ __forceinline__ bool layer_item(const RelaxArgs &a, uint32_t fi, uint
                     const u64 c64 = ext2(((u64)(dbase + (o >> HB)) << 32) | (hbase + (o & kHopMask)), p, 1);
                     const u64 q64 = q >= kBig ? kInf : ((u64)(dbase + (q >> HB)) << 32) | (hbase + (q & kHopMask));
                     const bool b64 = c64 < q64;
-                    if (k == 0) { better[0] = b64; fv[0] = (uint32_t)(c64 >> 32); }
-                    else if (k == 1) { better[1] = b64; fv[1] = (uint32_t)(c64 >> 32); }
-                    else { better[2] = b64; fv[2] = (uint32_t)(c64 >> 32); }
+                    const uint32_t d = (uint32_t)(c64 >> 32), fx = min(dsum(d, k == 0 ? h[0] : k == 1 ? h[1] : h[2]), kCap);
+                    const bool ok64 = b64 && (!GD || fx <= ub), late = GD && ok64 && fx > thr;
+                    if (k == 0) { better[0] = ok64; wait[0] = late; ex[0] = d; }
+                    else if (k == 1) { better[1] = ok64; wait[1] = late; ex[1] = d; }
+                    else { better[2] = ok64; wait[2] = late; ex[2] = d; }
                 }
             }
-            bool wait[3] = {false, false, false};
-            if constexpr (GD) {
-                const uint32_t thr = sh.thr;
 #pragma unroll
-                for (int k = 0; k < 3; ++k) {
-                    const uint32_t h = k == 0 ? dsum(hxl, sh.hy[0]) : k == 1 ? dsum(hxl, sh.hy[TH + 1])
-                                                                            : dsum(dsum(hxs, hl), sh.hy[r + 1]);
-                    fv[k] = bound(fv[k], h);
-                    better[k] &= fv[k] <= ub;
-                    wait[k] = better[k] && fv[k] > thr;
-                    better[k] &= !wait[k];
-                }
-            }
+            for (int k = 0; k < 3; ++k) better[k] &= !wait[k];
             uint32_t sides = (__any_sync(0xFFFFFFFFu, better[2] && seg == 0) ? 1u : 0u) |
                              (__any_sync(0xFFFFFFFFu, better[2] && seg == 3) ? 2u : 0u) |
                              (__any_sync(0xFFFFFFFFu, better[0]) ? 4u : 0u) | (__any_sync(0xFFFFFFFFu, better[1]) ? 8u : 0u);
             if (lane == 0 && sides) atomicOr(&sh.push, sides);
             if (GD && __any_sync(0xFFFFFFFFu, wait[0] || wait[1] || wait[2])) {
-                if (wait[0]) atomicMin(&sh.park[2], fv[0]);
-                if (wait[1]) atomicMin(&sh.park[3], fv[1]);
-                if (wait[2]) atomicMin(&sh.park[seg == 0 ? 0 : 1], fv[2]);
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    if (!wait[k]) continue;
+                    const uint32_t d = ex[k] != kMax ? ex[k] : dbase + ((own[k] + price[k]) >> HB);
+                    atomicMin(&sh.park[k < 2 ? k + 2 : seg == 0 ? 0 : 1], min(dsum(d, h[k]), kCap));
+                }
             }
         }
         __syncthreads();
