@@ -717,7 +717,10 @@ cudaError_t relax_launch(const RelaxArgs &a, uint32_t grid, uint32_t threads, si
 // shared memory; the walk itself is one thread following offsets, a shared-memory
 // load a step, until it leaves the window.  Cells priced for the net itself (own
 // pads, via pads) are looked up with exact prices, and a step that no word
-// describes (too large a price, a board of wide prices) is taken from HBM.
+// describes (too large a price, a board of wide prices) is taken from HBM.  A cell
+// that a neighbour further back than a word holds could precede gets no offset: of
+// two predecessors the one of lower CellIdx may be the one that has no word, and
+// the next window, which starts at the cell, has words for both.
 //
 // Bound by a window's two round trips to HBM (labels, prices), some 3 us, and the
 // number of windows; a step inside one costs about 50 cycles.  Testing the six
@@ -751,6 +754,7 @@ constexpr int kWalkThreads = 512;
 constexpr uint32_t kWalkSteps = 512;     // steps recorded per window
 constexpr uint32_t kWalkUnroll = 8;      // steps taken between two looks at whether the walk goes on
 constexpr uint32_t kWalkSpec = 256;      // cells of a window priced for the net itself
+constexpr uint32_t kWalkFar = kMax - 1;  // word of a cell that may be on the path, further back than a word holds
 
 __global__ void __launch_bounds__(kWalkThreads, 2) path_walk_tiled_kernel(PathArgs a) {
     extern __shared__ __align__(16) unsigned char wsm[];
@@ -794,6 +798,7 @@ __global__ void __launch_bounds__(kWalkThreads, 2) path_walk_tiled_kernel(PathAr
         const uint32_t D = (uint32_t)(need >> 32), H = (uint32_t)need;
         __syncthreads();  // every thread is past the previous window
         if (!wide) {
+            bool far = false;  // a word kWalkFar was set
             // ---- labels of the window and its ring: a warp per row, several rows in flight
             // word of the cell in column xx, row yy (ring included) of layer l, from its label
             auto put = [&](uint32_t i, u64 v, int gx, int gy, int l) {
@@ -801,8 +806,9 @@ __global__ void __launch_bounds__(kWalkThreads, 2) path_walk_tiled_kernel(PathAr
                 // at least their distance in cells
                 const uint32_t d = (uint32_t)(v >> 32), h = (uint32_t)v;
                 const uint32_t away = (uint32_t)(abs(gx - cx) + abs(gy - cy) + abs(l - cl));
-                const bool in = d <= D && h <= H && D - d < dist_lim && H - h <= hop_mask && H - h >= away;
-                word[i] = in ? ((D - d) << HB) | (H - h) : kMax;
+                const bool can = d <= D && h <= H && H - h >= away, in = D - d < dist_lim && H - h <= hop_mask;
+                word[i] = !can ? kMax : in ? ((D - d) << HB) | (H - h) : kWalkFar;
+                far |= can && !in;
                 delta[i] = 0;
             };
             auto label = [&](int gx, int gy, uint32_t l) -> u64 {
@@ -844,10 +850,10 @@ __global__ void __launch_bounds__(kWalkThreads, 2) path_walk_tiled_kernel(PathAr
                 const uint32_t i = atomicAdd(&s_nspec, 1u);
                 if (i < kWalkSpec) {
                     s_spec[i] = l * PL + (yy + 1) * PW + xx + 1;
-                    s_code[i] = 6;
+                    s_code[i] = 7;
                 }
             }
-            __syncthreads();
+            const bool any_far = __syncthreads_or(far);
             // ---- the predecessor of every cell: neighbours in ascending CellIdx ----
             const int off[6] = {-(int)PL, -(int)PW, -1, 1, (int)PW, (int)PL};
             constexpr uint32_t in_plane[6] = {kInBelow, kInNegY, kInNegX, kInPosX, kInPosY, kInAbove};
@@ -858,7 +864,7 @@ __global__ void __launch_bounds__(kWalkThreads, 2) path_walk_tiled_kernel(PathAr
                 for (uint32_t k = 0; k < kCells; ++k) {
                     const uint32_t q = r0 + k * nw, l = q / WH, yy = q % WH;
                     const uint32_t at = l * PL + (yy + 1) * PW + lane + 1;
-                    const bool have = q < L * WH && word[at] != kMax;
+                    const bool have = q < L * WH && word[at] < kWalkFar;
                     const uint32_t wc = have ? word[at] : 0u;
                     const uint32_t *pr = b.planes + ((uint64_t)l * b.h + (uint32_t)(ty0 + (int)yy)) * wp + (uint32_t)(tx0 + (int)lane);
 #pragma unroll
@@ -866,7 +872,7 @@ __global__ void __launch_bounds__(kWalkThreads, 2) path_walk_tiled_kernel(PathAr
                         p[k][n] = kPackedInf;
                         if (!have || (n == 0 && l == 0) || (n == 5 && l + 1 == L)) continue;
                         const uint32_t wq = word[(int)at + off[n]];
-                        if (wq != kMax && wq > wc) p[k][n] = __ldg(pr + in_plane[n] * NP);
+                        if (wq < kWalkFar && wq > wc) p[k][n] = __ldg(pr + in_plane[n] * NP);
                     }
                 }
 #pragma unroll
@@ -882,6 +888,19 @@ __global__ void __launch_bounds__(kWalkThreads, 2) path_walk_tiled_kernel(PathAr
                     if (dl) delta[at] = (int16_t)dl;
                 }
             }
+            if (any_far) {  // no offset where such a neighbour may be the predecessor as well
+                for (uint32_t i = tid; i < L * WH * W; i += blockDim.x) {  // (the cells this thread wrote)
+                    const uint32_t xx = i % W, q = i / W, l = q / WH, yy = q - l * WH, at = l * PL + (yy + 1) * PW + xx + 1;
+                    const uint32_t wc = word[at];
+                    if (!delta[at]) continue;
+                    const uint32_t *pr = b.planes + ((uint64_t)l * b.h + (uint32_t)(ty0 + (int)yy)) * wp + (uint32_t)(tx0 + (int)xx);
+                    for (int n = 0; n < 6; ++n) {
+                        if ((n == 0 && l == 0) || (n == 5 && l + 1 == L) || word[(int)at + off[n]] != kWalkFar) continue;
+                        const uint32_t p = __ldg(pr + in_plane[n] * NP);
+                        if (p < kPackedInf && (((wc + p) >> HB) >= dist_lim || (wc & hop_mask) == hop_mask)) delta[at] = 0;
+                    }
+                }
+            }
             if (s_nspec) {  // the same for the whole CTA
                 __syncthreads();
                 const uint32_t ns = min(s_nspec, kWalkSpec);
@@ -890,7 +909,7 @@ __global__ void __launch_bounds__(kWalkThreads, 2) path_walk_tiled_kernel(PathAr
                     const int kind = (int)(i % 6);
                     const uint32_t l = at / PL, q = at - l * PL, yy = q / PW, xx = q - yy * PW;
                     const uint32_t wc = word[at];
-                    if (wc == kMax || (kind == 0 && l == 0) || (kind == 5 && l + 1 == L)) continue;
+                    if (wc >= kWalkFar || (kind == 0 && l == 0) || (kind == 5 && l + 1 == L)) continue;
                     int px = tx0 + (int)xx - 1, py = ty0 + (int)yy - 1, pz = (int)l;
                     const uint32_t gx = (uint32_t)px, gy = (uint32_t)py;
                     const int off = kind == 0 ? -(int)PL : kind == 1 ? -(int)PW : kind == 2 ? -1 : kind == 3 ? 1
@@ -901,13 +920,15 @@ __global__ void __launch_bounds__(kWalkThreads, 2) path_walk_tiled_kernel(PathAr
                     const uint32_t st = walk_step_exact(a.boards + f.board, a.fields + blockIdx.x, a.pads,
                                                         ((uint32_t)pz * b.h + (uint32_t)py) * b.w + (uint32_t)px,
                                                         (l * b.h + gy) * b.w + gx, gx, gy, l, kind);
-                    if (st < dist_lim && wq == wc + ((st << HB) | 1u)) atomicMin(&s_code[e], (uint32_t)kind);
+                    if (st < dist_lim && wq == wc + ((st << HB) | 1u)) atomicMin(&s_code[e], (uint32_t)kind + 1u);
+                    if (wq == kWalkFar && st != kMax && (dsum(st, wc >> HB) >= dist_lim || (wc & hop_mask) == hop_mask))
+                        atomicMin(&s_code[e], 0u);  // it may be the predecessor: no offset (no kind is below it)
                 }
                 __syncthreads();
                 for (uint32_t e = tid; e < ns; e += blockDim.x) {
                     const uint32_t c = s_code[e];
-                    delta[s_spec[e]] = (int16_t)(c == 0 ? -(int)PL : c == 1 ? -(int)PW : c == 2 ? -1 : c == 3 ? 1
-                                               : c == 4 ? (int)PW : c == 5 ? (int)PL : 0);
+                    delta[s_spec[e]] = (int16_t)(c == 1 ? -(int)PL : c == 2 ? -(int)PW : c == 3 ? -1 : c == 4 ? 1
+                                               : c == 5 ? (int)PW : c == 6 ? (int)PL : 0);
                 }
                 // more such cells than the list holds: none of the window's steps is taken from it
                 if (s_nspec > kWalkSpec) {

@@ -51,6 +51,49 @@ def test_tile_edges_and_word_limits(oracle, layers, price):
         engine.close()
 
 
+@pytest.mark.parametrize("layers", [1, 2, 3, 4])
+@pytest.mark.parametrize("price", [1, 40, (1 << 14) - 1, (1 << 16) + 1, 1 << 25])
+def test_axis_gaps_tie(oracle, layers, price):
+    """Boards priced by axis gaps, where many paths cost the same and the canonical
+    one hangs on every tie, up to prices of which a word holds only a few steps:
+    windows around 32 x 16 tiles, with and without own pads."""
+    rng = np.random.default_rng(77 * layers + price % 991)
+    w, h = 72, 37
+    dims = Dims(w, h, layers)
+    cost = np.ones(len(dims), np.uint32)
+    cost[rng.random(len(dims)) < 0.12] = COST_MAX
+    cost[rng.random(len(dims)) < 0.2] = 3
+    gx = rng.integers(max(price // 2, 1), price + 1, w - 1).astype(np.uint32)
+    gy = rng.integers(max(price // 2, 1), price + 1, h - 1).astype(np.uint32)
+    free = np.flatnonzero(cost != COST_MAX)
+    cells = np.arange(len(dims))
+    nets, wins = [], []
+    for x0 in range(4):
+        for ww, wh in ((31, 15), (32, 16), (33, 17), (64, 32), (65, 33), (1, 36), (68, 1), (40, 23), (34, 24)):
+            y0 = int(rng.integers(0, h - wh + 1))
+            box = (cells % w >= x0) & (cells % w < x0 + ww) & (cells // w % h >= y0) & (cells // w % h < y0 + wh)
+            inside = free[box[free]]
+            if len(inside) < 2:
+                continue
+            src, dst = (int(v) for v in rng.choice(inside, 2))
+            walls = np.flatnonzero(box & (cost == COST_MAX))
+            pads = sorted({src, dst, *(int(c) for c in walls[rng.random(len(walls)) < 0.3])})
+            nets.append(NetEndpoints(f"n{len(nets)}", src, dst, pads if len(nets) % 2 else []))
+            wins.append(IsolatedRouteWindow(x0, y0, x0 + ww - 1, y0 + wh - 1))
+    vias = [int(v) for v in rng.integers(1, 2 * price + 1, layers - 1)]
+    req = IsolatedRouteRequest(Grid(dims, cost), nets, wins, gx, gy, vias)
+    engine = mrcuda.Engine(0)
+    try:
+        exp = oracle.isolated_batch(req, retry_full=False, mode="field")
+        got = engine.route_isolated_batch(req, retry_full=False, keep_fields=True)
+        assert (got.paths, got.search_costs) == exp
+        _assert_fields(oracle, req, got)
+        paths_only = engine.route_isolated_batch(req, retry_full=False)
+        assert (paths_only.paths, paths_only.search_costs) == exp
+    finally:
+        engine.close()
+
+
 def test_a_field_that_leaves_the_packed_range(oracle):
     """Long hop counts and costs: a serpentine whose labels spread past one word
     inside a tile (walls every other row, a gap at alternating ends)."""
