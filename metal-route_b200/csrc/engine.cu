@@ -837,6 +837,7 @@ struct mrc_batch {
     std::vector<DevField> fields;  // ascending lab_off (largest windows first)
     uint64_t total_cells = 0;
     uint32_t total_tiles = 0, max_tiles = 0, tile_h = 32, threads = kRelaxThreads, grid = 1;
+    uint32_t rows = 32;  // rows of a tile: tile_h, or the layer kernel's tall tile
     size_t smem = 0;
     DBuf d_tover;                  // per tile: holds price overrides of its field (has_over batches)
     DBuf d_boards, d_fields, d_pads, d_lists, d_lens, d_heads, d_cells, d_out;
@@ -970,15 +971,34 @@ mrc_status batch_layout(mrc_batch *bt, uint32_t tile_h, uint32_t threads) {
     bt->layer = bt->async_q && !bt->warp && bt->cta_planes && tile_h == kLayerTileH && bt->max_layers <= kLayerMax;
     bt->tile_h = bt->warp ? kWarpTileH : tile_h;
     bt->threads = bt->warp ? warp_relax_threads() : threads;
+    const uint32_t sms = (uint32_t)ctx->sms;
+    bt->rows = bt->tile_h;
+    if (bt->layer && !bt->has_over && !bt->directed_any && bt->max_layers <= kLayerTallMax) {
+        // Tall tiles halve the visits a wavefront makes up and down a window, and a
+        // visit's cost is mostly its wait for the neighbours' labels.  At 1 to 4
+        // layers on boards priced by axis gaps (relax us, 8 rows then 16): 32
+        // layered 128 x 128 fields 163, 115; one net of 160 x 140 30, 20; 128 pad
+        // nets of 300 x 280 258, 194; single-layer 320 x 320, 64 nets 386, 267.
+        // Not with a price per cell: a visit then takes more passes, the more the
+        // taller the tile (random prices of 64 x 64, 64 nets 80, 99; one search of
+        // 800 x 640 323, 438).  And not past kTallTiles tiles an SM, where the
+        // device is full and an activation's own work counts, which a tall tile
+        // spends on rows that the wavefront hasn't reached: 256 nets of 512 x 512,
+        // 43 867 tiles 1425, 1503; 128 of them, 23 416 tiles 886, 882.
+        uint64_t tiles = 0;
+        for (const DevField &f : bt->fields)
+            tiles += (uint64_t)((f.ww + (f.x0 & 3u) + 31) / 32) * ((f.wh + kLayerTileH - 1) / kLayerTileH);
+        if (tiles <= (uint64_t)kTallTiles * sms) bt->rows = kLayerTallH;
+    }
     bt->smem =
-        bt->warp ? 0 : bt->layer ? layer_smem_bytes(bt->max_layers)
+        bt->warp ? 0 : bt->layer ? layer_smem_bytes(bt->max_layers, bt->rows)
                                  : relax_smem_bytes(bt->max_layers, tile_h, bt->directed_any);
     uint64_t toff = 0;
     uint32_t max_tiles = 1;
     for (DevField &f : bt->fields) {
         f.xa = bt->layer ? f.x0 & 3u : 0u;  // a tile's first column is a multiple of 4 (16 bytes, the TMA rule)
         const uint32_t tw = bt->warp ? warp_tile_w(bt->boards[f.board]->view.layers) : 32u;
-        const uint64_t tiles = (uint64_t)((f.ww + f.xa + tw - 1) / tw) * ((f.wh + bt->tile_h - 1) / bt->tile_h);
+        const uint64_t tiles = (uint64_t)((f.ww + f.xa + tw - 1) / tw) * ((f.wh + bt->rows - 1) / bt->rows);
         f.tile_off = (uint32_t)std::min<uint64_t>(toff, 0xFFFFFFFFull);
         toff += tiles;
         max_tiles = (uint32_t)std::max<uint64_t>(max_tiles, tiles);
@@ -993,7 +1013,7 @@ mrc_status batch_layout(mrc_batch *bt, uint32_t tile_h, uint32_t threads) {
     if (bt->warp) {
         MRC_CUDA(warp_relax_occupancy(&per_sm), "relax occupancy");
     } else if (bt->layer) {
-        MRC_CUDA(layer_configure(bt->max_layers, bt->smem, bt->has_over, bt->goal, &per_sm), "configure relax kernel");
+        MRC_CUDA(layer_configure(bt->max_layers, bt->rows, bt->smem, bt->has_over, bt->goal, &per_sm), "configure relax kernel");
     } else {
         MRC_CUDA(relax_configure(tile_h, threads, bt->smem, bt->async_q, bt->has_over), "configure relax kernel");
         MRC_CUDA(relax_occupancy(tile_h, threads, bt->smem, &per_sm, bt->async_q, bt->has_over), "relax occupancy");
@@ -1026,7 +1046,7 @@ mrc_status batch_layout(mrc_batch *bt, uint32_t tile_h, uint32_t threads) {
         MRC_TRY(upload(ctx, bt->d_pchunks, chunks.data(), chunks.size() * 8, "plane chunk table"));
         if (bt->layer) {
             std::vector<CUtensorMap> maps(bt->devs.size());
-            for (size_t k = 0; k < bt->devs.size(); ++k) MRC_TRY(encode_planes_map(bt->devs[k], tile_h, &maps[k]));
+            for (size_t k = 0; k < bt->devs.size(); ++k) MRC_TRY(encode_planes_map(bt->devs[k], bt->rows, &maps[k]));
             // pool blocks are 256-byte aligned: every 128-byte map is 64-byte aligned
             MRC_TRY(upload(ctx, bt->d_tmaps, maps.data(), maps.size() * sizeof(CUtensorMap), "tensor maps"));
             for (size_t k = 0; k < bt->devs.size(); ++k) bt->devs[k].tmap = bt->d_tmaps.as<CUtensorMap>() + k;
@@ -1189,9 +1209,9 @@ PathArgs path_args(const mrc_batch *bt) {
     pa.lab = bt->lab();
     pa.tvisit = bt->tvisit();
     pa.tover = bt->has_over ? bt->d_tover.as<uint8_t>() : nullptr;
-    pa.tile_h = bt->tile_h;
+    pa.tile_h = bt->rows;
     pa.arena_filled = bt->async_q ? 1u : 0u;
-    pa.hop_bits = layer_hop_bits(bt->max_layers);
+    pa.hop_bits = layer_hop_bits(bt->max_layers, bt->rows);
     pa.walk_smem = bt->layer && !bt->has_over ? (uint32_t)walk_smem_bytes(bt->max_layers) : 0u;
     pa.offsets = bt->d_heads.as<unsigned long long>();
     pa.costs = reinterpret_cast<uint32_t *>(pa.offsets + bt->fields.size() + 1);
@@ -1204,7 +1224,7 @@ PathArgs path_args(const mrc_batch *bt) {
 // Step-price planes of the batch's boards (and the extremes of the prices).
 mrc_status planes_enqueue(mrc_batch *bt, cudaStream_t st, uint32_t *launches) {
     MRC_CUDA(planes_launch(bt->d_boards.as<DevBoard>(), bt->d_pchunks.as<uint64_t>(), (uint32_t)bt->devs.size(),
-                           bt->n_pchunks, (uint32_t)bt->ctx->sms, bt->layer ? layer_hop_bits(bt->max_layers) : 0, st),
+                           bt->n_pchunks, (uint32_t)bt->ctx->sms, bt->layer ? layer_hop_bits(bt->max_layers, bt->rows) : 0, st),
              "launch step-price planes");
     *launches += 1;
     return MRC_OK;
@@ -1229,7 +1249,7 @@ mrc_status batch_enqueue(mrc_batch *bt, cudaStream_t st, bool capturing) {
     ra.tover = nullptr;
     if (bt->has_over && n) {
         MRC_CUDA(cudaMemsetAsync(bt->d_tover.p, 0, (size_t)bt->total_tiles, st), "reset override tile flags");
-        MRC_CUDA(mark_over_tiles_launch(bt->d_fields.as<DevField>(), n, bt->d_boards.as<DevBoard>(), bt->tile_h,
+        MRC_CUDA(mark_over_tiles_launch(bt->d_fields.as<DevField>(), n, bt->d_boards.as<DevBoard>(), bt->rows,
                                         bt->d_tover.as<uint8_t>(), st),
                  "mark override tiles");
         ++launches;
@@ -1243,7 +1263,7 @@ mrc_status batch_enqueue(mrc_batch *bt, cudaStream_t st, bool capturing) {
         ra.tpark = bt->tpark();
     }
     ra.ctl = bt->ctl();
-    ra.tile_h = bt->tile_h;
+    ra.tile_h = bt->rows;
     ra.round_limit = 64u * bt->max_tiles + 4096u;
     ra.activation_limit = 1024ull * bt->total_tiles + 65536ull;  // runaway guard, far above any measured need
     if (n && bt->async_q) MRC_CUDA(cudaMemsetAsync(bt->d_ones.p, 0xFF, bt->ones_bytes, st), "fill label arena");
@@ -2934,7 +2954,7 @@ mrc_status mrc_server_create(mrc_context *ctx, const mrc_server_params *params, 
         s->tile_h = 8;
         s->threads = kRelaxThreads;
         int per_sm = 0;
-        MRC_CUDA(layer_configure(s->p.max_layers, layer_smem_bytes(s->p.max_layers), false, true, &per_sm),
+        MRC_CUDA(layer_configure(s->p.max_layers, kLayerTileH, layer_smem_bytes(s->p.max_layers, kLayerTileH), false, true, &per_sm),
                  "configure relax kernel");
         if ((uint32_t)per_sm * (uint32_t)ctx->sms < s->p.slots) return fail(MRC_ERR_LIMIT, "too many slots");
         s->streams.resize(s->p.slots);

@@ -257,16 +257,21 @@ cudaError_t relax_launch(const RelaxArgs &a, uint32_t grid, uint32_t threads, si
 // source labels and source tiles of a queue form (relax_launch includes it)
 cudaError_t seed_launch(const RelaxArgs &a, cudaStream_t st);
 
-// The layer kernel (layer_relax.cu): the queue form on 32 x 8 tiles with a warp
+// The layer kernel (layer_relax.cu): the queue form on 32 x 8 or 32 x 16 tiles with a warp
 // per layer, labels packed into 32 bits, prices from the boards' packed price
 // planes by TMA; boards of up to kLayerMax layers.  goal: paths and costs only
 // (RelaxArgs::goal).
 constexpr uint32_t kLayerMax = 16;
 constexpr uint32_t kLayerTileH = 8;
-// bits of a packed word that hold hops (the rest, below bit 30, the dist)
-__host__ __device__ inline uint32_t layer_hop_bits(uint32_t max_layers) { return max_layers <= 8 ? 12 : 13; }
-size_t layer_smem_bytes(uint32_t max_layers);
-cudaError_t layer_configure(uint32_t max_layers, size_t smem, bool over, bool goal, int *blocks_per_sm);
+constexpr uint32_t kLayerTallH = 16, kLayerTallMax = 4;  // tall tiles: up to so many layers, no overrides
+constexpr uint32_t kTallTiles = 240;  // tall up to so many 8-row tiles an SM
+// bits of a packed word that hold hops (the rest, below bit 30, the dist): a path
+// through a tile has no more hops than the tile cells
+__host__ __device__ constexpr uint32_t layer_hop_bits(uint32_t max_layers, uint32_t tile_h) {
+    return max_layers * tile_h <= 64 ? 12 : 13;
+}
+size_t layer_smem_bytes(uint32_t max_layers, uint32_t tile_h);
+cudaError_t layer_configure(uint32_t max_layers, uint32_t tile_h, size_t smem, bool over, bool goal, int *blocks_per_sm);
 cudaError_t layer_launch(const RelaxArgs &a, uint32_t grid, size_t smem, cudaStream_t st, bool over, bool goal);
 // tover[f.tile_off + t] = 1 for every tile t of every field that holds one of
 // the field's directed-price overrides (tover zeroed before).

@@ -1,7 +1,8 @@
 // layer_relax.cu — the queue-driven relax kernel with a warp per layer and 32-bit labels.
 //
-// A CTA holds one 32 x 8 tile over all L layers of a field, warp l its layer l:
-// lane x keeps the eight labels of column x in registers.  Inside an activation a
+// A CTA holds one 32 x TH tile over all L layers of a field, warp l its layer l:
+// lane x keeps the TH labels of column x in registers.  TH is 8, or 16 where the
+// batch's longest chains of tiles bound it (batch_layout has the rule).  Inside an activation a
 // label is one word, (dist - least staged dist) << HB | (hops - least staged
 // hops), and a step price is (price << HB) | 1, so the lexicographic min-plus step
 // of (dist, hops) is one add-and-min instruction (__viaddmin_u32) where 64-bit
@@ -10,7 +11,8 @@
 //   columns  each lane runs its column down and up in registers (the halo rows in
 //            two more registers), no data exchanged;
 //   rows     through shared memory (one store and two 16-byte loads a lane): four
-//            lanes a row, eight cells each, joined by a two-step scan; the warp
+//            lanes a row, eight cells each, eight rows at a time, joined by a two-step
+//            scan; the warp
 //            repeats columns and rows until its plane is closed, with no CTA barrier;
 //   stacks   a thread per (y, x) runs the layers up and down; only here the warps
 //            of a tile meet.
@@ -38,7 +40,6 @@
 namespace mrc {
 namespace {
 
-constexpr int TH = kLayerTileH;
 constexpr uint32_t kBig = kPackedInf;   // +inf
 constexpr uint32_t kNarrow = 1u << 29;  // staged labels, final labels and prices lie below
 // Pitch of a row of labels or prices: 16-byte aligned, and the rows' segments and
@@ -47,7 +48,9 @@ constexpr uint32_t kPitch = kPlaneTmaBoxW;
 constexpr uint32_t kSpecCap = 512;      // cells of a tile priced for the net itself
 constexpr int kPlaneIters = 2;          // column and row passes of a plane between two meetings
 
-__host__ __device__ inline size_t layer_st_off(uint32_t L) { return ((size_t)L * TH * kPitch * 4 + 127) & ~(size_t)127; }
+__host__ __device__ inline size_t layer_st_off(uint32_t L, uint32_t TH) {
+    return ((size_t)L * TH * kPitch * 4 + 127) & ~(size_t)127;
+}
 
 struct LayerShared {
     u64 item;
@@ -56,13 +59,13 @@ struct LayerShared {
     uint32_t n_spec, near_pad, wide, dmin, hmin, hmax, ub, thr, more;
     uint32_t push;              // bits: left, right, top, bottom improved
     uint32_t park[4];           // GD: the smallest f that waits to enter each
-    uint32_t hy[TH + 2];        // GD: remaining price along y, rows -1 .. TH
+    uint32_t hy[kLayerTallH + 2];  // GD: remaining price along y, rows -1 .. TH
     uint32_t spec[kSpecCap];
 };
 
 // The 64-bit form of one item, from the start (the hold is taken again, which
 // drops a dirty mark, but the labels are read after it).
-template <bool OV, bool GD>
+template <int TH, bool OV, bool GD>
 __device__ __noinline__ bool wide_item(const RelaxArgs &a, uint32_t fi, uint32_t t, unsigned char *smem_raw,
                                        unsigned long long *cnt) {
     return process_item<TH, true, OV, GD, true>(a, fi, t, 0, smem_raw, cnt);
@@ -85,7 +88,7 @@ __device__ __forceinline__ uint32_t pack_price(uint32_t p, uint32_t *wide) {
 // The stacks of rows y = y0, y0 + step, ...: the layers upward, then downward.  NL is
 // the layer count at compile time, so that all labels and prices of a stack are
 // loaded before any is used.
-template <int NL>
+template <int NL, int TH>
 __device__ __forceinline__ void stack_rows(uint32_t *lab, const uint32_t *st, uint32_t y0, uint32_t step) {
     constexpr uint32_t LS = TH * kPitch, SP = NL * LS;  // words from a layer, from a plane, to the next
 #pragma unroll 1
@@ -108,20 +111,20 @@ __device__ __forceinline__ void stack_rows(uint32_t *lab, const uint32_t *st, ui
     }
 }
 
-template <int LM>
+template <int LM, int TH>
 __device__ __forceinline__ void stack_pass_layers(uint32_t *lab, const uint32_t *st, uint32_t L, uint32_t y0,
                                                   uint32_t step) {
     switch (L) {
-        case 2: return stack_rows<2>(lab, st, y0, step);
-        case 3: return stack_rows<3>(lab, st, y0, step);
-        case 4: return stack_rows<4>(lab, st, y0, step);
+        case 2: return stack_rows<2, TH>(lab, st, y0, step);
+        case 3: return stack_rows<3, TH>(lab, st, y0, step);
+        case 4: return stack_rows<4, TH>(lab, st, y0, step);
     }
     if constexpr (LM > 4) {
         switch (L) {
-            case 5: return stack_rows<5>(lab, st, y0, step);
-            case 6: return stack_rows<6>(lab, st, y0, step);
-            case 7: return stack_rows<7>(lab, st, y0, step);
-            case 8: return stack_rows<8>(lab, st, y0, step);
+            case 5: return stack_rows<5, TH>(lab, st, y0, step);
+            case 6: return stack_rows<6, TH>(lab, st, y0, step);
+            case 7: return stack_rows<7, TH>(lab, st, y0, step);
+            case 8: return stack_rows<8, TH>(lab, st, y0, step);
         }
     }
     if constexpr (LM > 8) {  // 9 .. 16 layers, in shared memory
@@ -138,6 +141,7 @@ __device__ __forceinline__ void stack_pass_layers(uint32_t *lab, const uint32_t 
 
 // Labels of one layer of the tiles beyond `sides` of the tile at (x, y) of a ww x wh
 // window into L2: one 128-byte line a lane, three lines a row of eight.
+template <int TH>
 __device__ __noinline__ void prefetch_neighbours(const u64 *lab, uint32_t sides, uint32_t lane, int x, int y,
                                                  uint32_t ww, uint32_t wh) {
     for (; sides; sides &= sides - 1u) {
@@ -151,13 +155,13 @@ __device__ __noinline__ void prefetch_neighbours(const u64 *lab, uint32_t sides,
 
 // Relaxes one held-to-be item; thread 0 returns whether it was the last one in
 // flight, of the launch or (GD) of its field.
-template <int LM, bool OV, bool GD>
+template <int LM, int TH, bool OV, bool GD>
 __device__ __forceinline__ bool layer_item(const RelaxArgs &a, uint32_t fi, uint32_t t, unsigned char *smem_raw,
                                            LayerShared &sh, uint32_t &phase) {
-    constexpr int HB = LM <= 8 ? 12 : 13;
+    constexpr int HB = (int)layer_hop_bits(LM, TH), RG = TH / 8, NB = 2 + RG;  // row groups, border cells of a lane
     constexpr uint32_t kHopMask = (1u << HB) - 1u;
     const uint32_t tid = threadIdx.x, lane = tid & 31u, wl = tid >> 5;
-    const uint32_t r = lane >> 2, seg = lane & 3u;  // row layout: row and segment of 8 cells
+    const uint32_t r = lane >> 2, seg = lane & 3u;  // row layout: row (of each group of 8) and segment of 8 cells
     const DevField f = a.fields[fi];
     const DevBoard b = a.boards[f.board];
     const uint32_t L = b.layers;
@@ -167,7 +171,7 @@ __device__ __forceinline__ bool layer_item(const RelaxArgs &a, uint32_t fi, uint
     const uint32_t tw = min(kTW, f.ww + f.xa - txi * kTW), th = min((uint32_t)TH, f.wh - tyi * TH);
     const uint32_t xlo = txi == 0 ? f.xa : 0u;
     uint32_t *lab = reinterpret_cast<uint32_t *>(smem_raw);
-    uint32_t *st = reinterpret_cast<uint32_t *>(smem_raw + layer_st_off(L));
+    uint32_t *st = reinterpret_cast<uint32_t *>(smem_raw + layer_st_off(L, TH));
     uint32_t *live = GD ? &a.goal[fi].active : &a.ctl->count[1];
     uint32_t *state = a.tstamp + f.tile_off + t;
     const bool mine = wl < L;                            // this warp has a layer
@@ -220,28 +224,42 @@ __device__ __forceinline__ bool layer_item(const RelaxArgs &a, uint32_t fi, uint
 
     const u64 *glab = a.lab + f.lab_off;
     const int64_t row0 = ((int64_t)wl * f.wh + (ty0 - (int)f.y0)) * (int64_t)f.ww + (tx0 - (int)f.x0);
-    uint32_t pt = kBig, pb = kBig, ps = kBig;  // prices into the neighbour tiles' border cells
+    uint32_t price[NB];                        // prices into the neighbour tiles' border cells
     const bool top = tyi > 0, bottom = tyi + 1 < nty;
-    const bool side = mine && r < th && ((seg == 0 && txi > 0) || (seg == 3 && txi + 1 < ntx));
+    // border cells of a lane: 0 the top and 1 the bottom of its column, 2 + g its end of
+    // row r of group g
+    bool side[RG];
+#pragma unroll
+    for (int g = 0; g < RG; ++g) {
+        side[g] = mine && r + 8u * g < th && ((seg == 0 && txi > 0) || (seg == 3 && txi + 1 < ntx));
+        price[2 + g] = kBig;
+    }
+    price[0] = price[1] = kBig;
     bool last = false;
     for (uint32_t cont = 0;; ++cont) {
         // ---- labels of the column, the halo rows and the halo columns ----------
-        u64 v[TH], vt = kInf, vb = kInf, vs = kInf;
+        u64 v[TH], vh[NB];
 #pragma unroll
         for (int y = 0; y < TH; ++y) {
             v[y] = kInf;
             if (col_in && y < (int)th) v[y] = __ldcg(glab + row0 + (int64_t)y * f.ww + lane);
         }
-        if (col_in && top) vt = __ldcg(glab + row0 - (int64_t)f.ww + lane);
-        if (col_in && bottom) vb = __ldcg(glab + row0 + (int64_t)TH * f.ww + lane);
-        if (side) vs = __ldcg(glab + row0 + (int64_t)r * f.ww + (seg == 0 ? -1 : (int)kTW));
+        vh[0] = col_in && top ? __ldcg(glab + row0 - (int64_t)f.ww + lane) : kInf;
+        vh[1] = col_in && bottom ? __ldcg(glab + row0 + (int64_t)TH * f.ww + lane) : kInf;
+#pragma unroll
+        for (int g = 0; g < RG; ++g)
+            vh[2 + g] = side[g] ? __ldcg(glab + row0 + (int64_t)(r + 8u * g) * f.ww + (seg == 0 ? -1 : (int)kTW)) : kInf;
         if (cont == 0) {
             const uint32_t wp = planes_pitch(b.w);
             const uint64_t NP = (uint64_t)wp * b.h * L;
             const uint32_t *pl = b.planes + ((uint64_t)wl * b.h + (uint32_t)ty0) * wp + (uint32_t)tx0;
-            if (col_in && top) pt = __ldg(pl + kInPosY * NP + lane - wp);
-            if (col_in && bottom) pb = __ldg(pl + kInNegY * NP + lane + (uint64_t)TH * wp);
-            if (side) ps = __ldg(pl + (seg == 0 ? kInPosX : kInNegX) * NP + (uint64_t)r * wp + (seg == 0 ? -1 : (int)kTW));
+            if (col_in && top) price[0] = __ldg(pl + kInPosY * NP + lane - wp);
+            if (col_in && bottom) price[1] = __ldg(pl + kInNegY * NP + lane + (uint64_t)TH * wp);
+#pragma unroll
+            for (int g = 0; g < RG; ++g)
+                if (side[g])
+                    price[2 + g] = __ldg(pl + (seg == 0 ? kInPosX : kInNegX) * NP + (uint64_t)(r + 8u * g) * wp +
+                                         (seg == 0 ? -1 : (int)kTW));
             // cells of this tile whose prices depend on the net: its own pads, its via pads
             for (uint32_t k = tid; k < f.n_pads + f.n_vpads; k += blockDim.x) {
                 const bool q = k >= f.n_pads;
@@ -265,9 +283,8 @@ __device__ __forceinline__ bool layer_item(const RelaxArgs &a, uint32_t fi, uint
             };
 #pragma unroll
             for (int y = 0; y < TH; ++y) see(v[y]);
-            see(vt);
-            see(vb);
-            see(vs);
+#pragma unroll
+            for (int k = 0; k < NB; ++k) see(vh[k]);
             dm = __reduce_min_sync(0xFFFFFFFFu, dm);
             hm = __reduce_min_sync(0xFFFFFFFFu, hm);
             hM = __reduce_max_sync(0xFFFFFFFFu, hM);
@@ -281,10 +298,10 @@ __device__ __forceinline__ bool layer_item(const RelaxArgs &a, uint32_t fi, uint
         const uint32_t dbase = sh.dmin, hbase = sh.hmin;
         // hops of a path through the tile stay below the dist bits, and no dist of
         // the tile can saturate
-        bool bad = dbase != kMax && ((int64_t)(sh.hmax - hbase) + 256 * L + 4 > (int64_t)kHopMask ||
+        bool bad = dbase != kMax && ((int64_t)(sh.hmax - hbase) + kTW * TH * L + 4 > (int64_t)kHopMask ||
                                      dbase > kMax - (kBig >> HB));
         uint32_t ub = kMax;
-        uint32_t w[TH], w0[TH], lim[TH], ht, hb, hs;
+        uint32_t w[TH], w0[TH], lim[TH], there[NB];  // there: staged labels beyond the border
         if constexpr (GD) ub = sh.ub;
         // GD: the word from which on a label at a cell with remaining price h is past
         // the bound `top`: (top - dbase - h + 1) << HB between 0 and kBig
@@ -306,9 +323,13 @@ __device__ __forceinline__ bool layer_item(const RelaxArgs &a, uint32_t fi, uint
         set_limits();
 #pragma unroll
         for (int y = 0; y < TH; ++y) w0[y] = w[y] = pack(v[y], lim[y]);
-        ht = pack(vt, GD ? limit(ub, dsum(hxl, sh.hy[0])) : kBig);
-        hb = pack(vb, GD ? limit(ub, dsum(hxl, sh.hy[TH + 1])) : kBig);
-        hs = pack(vs, GD ? limit(ub, dsum(hxls, sh.hy[r + 1])) : kBig);
+        // GD: remaining price from the cell beyond border cell k
+        auto beyond = [&](int k) -> uint32_t {
+            if (!GD) return 0u;
+            return k == 0 ? dsum(hxl, sh.hy[0]) : k == 1 ? dsum(hxl, sh.hy[TH + 1]) : dsum(hxls, sh.hy[r + 8u * (k - 2) + 1]);
+        };
+#pragma unroll
+        for (int k = 0; k < NB; ++k) there[k] = pack(vh[k], limit(ub, beyond(k)));
         if (cont == 0) {
             // the planes: a bounded wait for the TMA load (a load that never lands
             // sets the status and the launch ends without results)
@@ -322,7 +343,7 @@ __device__ __forceinline__ bool layer_item(const RelaxArgs &a, uint32_t fi, uint
             ++phase;
             if (board_wide) {
                 __syncthreads();  // everybody is past the load and the staged words
-                return wide_item<OV, GD>(a, fi, t, smem_raw, sh.cnt);
+                return wide_item<TH, OV, GD>(a, fi, t, smem_raw, sh.cnt);
             }
             if (mine && (tw < kTW || th < TH || xlo)) {  // no step enters a cell past the window
                 for (uint32_t y = 0; y < TH; ++y) {
@@ -366,13 +387,15 @@ __device__ __forceinline__ bool layer_item(const RelaxArgs &a, uint32_t fi, uint
 
         // ---- relax to local convergence --------------------------------------
         uint32_t *colp = lab + (wl * TH) * kPitch + lane;              // this lane's column, row y at + y * kPitch
-        uint4 *rowp = reinterpret_cast<uint4 *>(lab + (wl * TH + r) * kPitch + seg * 8);
+        uint4 *rowp = reinterpret_cast<uint4 *>(lab + (wl * TH + r) * kPitch + seg * 8);  // group g at + g * 2 * kPitch
         const uint32_t *stc = st + (wl * TH) * kPitch + lane;          // prices of the column, plane p at + p * L * TH * kPitch
         const uint32_t *str = st + (wl * TH + r) * kPitch + seg * 8;   // prices of the row segment
         const uint32_t SP = L * TH * kPitch;
         bool plane = false;  // this warp's plane is open (warp-uniform)
         if (mine) {
-            bool any = (ht & hb & hs) != kBig;
+            bool any = false;
+#pragma unroll
+            for (int k = 0; k < NB; ++k) any |= there[k] != kBig;
 #pragma unroll
             for (int y = 0; y < TH; ++y) {
                 any |= w[y] < lim[y];
@@ -389,11 +412,11 @@ __device__ __forceinline__ bool layer_item(const RelaxArgs &a, uint32_t fi, uint
                     // columns
                     bool ch = false;
                     {
-                        uint32_t u[TH], prev = ht;
+                        uint32_t u[TH], prev = there[0];
 #pragma unroll
                         for (int y = 0; y < TH; ++y)
                             prev = u[y] = __viaddmin_u32(prev, stc[kInNegY * SP + y * kPitch], w[y]);
-                        prev = hb;
+                        prev = there[1];
 #pragma unroll
                         for (int y = TH - 1; y >= 0; --y) {
                             prev = u[y] = __viaddmin_u32(prev, stc[kInPosY * SP + y * kPitch], u[y]);
@@ -412,11 +435,14 @@ __device__ __forceinline__ bool layer_item(const RelaxArgs &a, uint32_t fi, uint
 #pragma unroll
                     for (int y = 0; y < TH; ++y) colp[y * kPitch] = w[y];
                     __syncwarp();
-                    {
+#pragma unroll
+                    for (int g = 0; g < RG; ++g) {
+                        uint4 *rp = rowp + g * 2 * kPitch;
+                        const uint32_t *sg = str + g * 8 * kPitch, hs = there[2 + g];
                         uint32_t u[8], p[8], P[8];
-                        *reinterpret_cast<uint4 *>(u) = rowp[0];
-                        *reinterpret_cast<uint4 *>(u + 4) = rowp[1];
-                        const uint4 *pf = reinterpret_cast<const uint4 *>(str + kInNegX * SP);
+                        *reinterpret_cast<uint4 *>(u) = rp[0];
+                        *reinterpret_cast<uint4 *>(u + 4) = rp[1];
+                        const uint4 *pf = reinterpret_cast<const uint4 *>(sg + kInNegX * SP);
                         *reinterpret_cast<uint4 *>(p) = pf[0];
                         *reinterpret_cast<uint4 *>(p + 4) = pf[1];
                         // forward: the halo column enters the first segment's chain
@@ -442,7 +468,7 @@ __device__ __forceinline__ bool layer_item(const RelaxArgs &a, uint32_t fi, uint
 #pragma unroll
                         for (int i = 0; i < 8; ++i) u[i] = __viaddmin_u32(C, P[i], u[i]);
                         // backward over the forward results
-                        const uint4 *pq = reinterpret_cast<const uint4 *>(str + kInPosX * SP);
+                        const uint4 *pq = reinterpret_cast<const uint4 *>(sg + kInPosX * SP);
                         *reinterpret_cast<uint4 *>(p) = pq[0];
                         *reinterpret_cast<uint4 *>(p + 4) = pq[1];
                         if (seg == 3) u[7] = __viaddmin_u32(hs, p[7], u[7]);
@@ -467,8 +493,8 @@ __device__ __forceinline__ bool layer_item(const RelaxArgs &a, uint32_t fi, uint
                         if (seg == 3) C = kBig;
 #pragma unroll
                         for (int i = 0; i < 8; ++i) u[i] = __viaddmin_u32(C, P[i], u[i]);
-                        rowp[0] = *reinterpret_cast<uint4 *>(u);
-                        rowp[1] = *reinterpret_cast<uint4 *>(u + 4);
+                        rp[0] = *reinterpret_cast<uint4 *>(u);
+                        rp[1] = *reinterpret_cast<uint4 *>(u + 4);
                     }
                     __syncwarp();
                     ch = false;
@@ -509,7 +535,7 @@ __device__ __forceinline__ bool layer_item(const RelaxArgs &a, uint32_t fi, uint
             if (L == 1) continue;
             // the plane's labels are in shared memory, as of the last row pass or the
             // start; a column pass that ended the loop changed nothing
-            stack_pass_layers<LM>(lab + lane, st + lane, L, wl, blockDim.x >> 5);
+            stack_pass_layers<LM, TH>(lab + lane, st + lane, L, wl, blockDim.x >> 5);
             __syncthreads();
             if (mine) {
                 bool ch = false;
@@ -529,7 +555,7 @@ __device__ __forceinline__ bool layer_item(const RelaxArgs &a, uint32_t fi, uint
             for (int y = 0; y < TH; ++y) bad |= w[y] >= kNarrow && w[y] < kBig;
         }
         if (__syncthreads_or(bad || *(volatile uint32_t *)&sh.wide))
-            return wide_item<OV, GD>(a, fi, t, smem_raw, sh.cnt);
+            return wide_item<TH, OV, GD>(a, fi, t, smem_raw, sh.cnt);
         if constexpr (GD) ub = *(volatile uint32_t *)&sh.ub;
 
         // ---- write back the labels that fell -----------------------------------
@@ -540,64 +566,68 @@ __device__ __forceinline__ bool layer_item(const RelaxArgs &a, uint32_t fi, uint
                 if (w[y] < min(w0[y], lim[y]))
                     out[(int64_t)y * f.ww] = ((u64)(dbase + (w[y] >> HB)) << 32) | (hbase + (w[y] & kHopMask));
             // ---- neighbours this tile can improve --------------------------------
-            // Each lane has three border cells: the top and the bottom of its column
-            // and, in the row layout, the first or last of its row.  own: our label
-            // there; price: of the move into the neighbour; there: the neighbour's
-            // staged label.
-            const uint32_t edge = side ? lab[(wl * TH + r) * kPitch + (seg == 0 ? 0u : kTW - 1)] : kBig;
-            uint32_t own[3] = {w[0], w[TH - 1], edge}, price[3] = {pt, pb, ps}, there[3] = {ht, hb, hs};
-            bool better[3], wait[3] = {false, false, false};  // improved; GD: improved, past the threshold
-            uint32_t ex[3] = {kMax, kMax, kMax};               // dist of an exactly priced improvement
+            // own: our label at a border cell; price: of the move into the neighbour
+            // beyond; there: the neighbour's staged label.
+            uint32_t own[NB];
+            bool better[NB], wait[NB];  // improved; GD: improved, past the threshold
+            uint32_t ex[NB];            // dist of an exactly priced improvement
             const uint32_t thr = GD ? sh.thr : kMax;
-            const uint32_t h[3] = {GD ? dsum(hxl, sh.hy[0]) : 0u, GD ? dsum(hxl, sh.hy[TH + 1]) : 0u,
-                                   GD ? dsum(hxls, sh.hy[r + 1]) : 0u};
+            own[0] = w[0];
+            own[1] = w[TH - 1];
 #pragma unroll
-            for (int k = 0; k < 3; ++k) {
+            for (int g = 0; g < RG; ++g)
+                own[2 + g] = side[g] ? lab[(wl * TH + r + 8u * g) * kPitch + (seg == 0 ? 0u : kTW - 1)] : kBig;
+#pragma unroll
+            for (int k = 0; k < NB; ++k) {
                 const uint32_t cand = own[k] + price[k];  // (no price or label: at least kBig, as `there` at most)
                 better[k] = cand < there[k];
+                wait[k] = false;
+                ex[k] = kMax;
                 if constexpr (GD) {
-                    better[k] &= cand < limit(ub, h[k]);
-                    wait[k] = better[k] && cand >= limit(thr, h[k]);
+                    better[k] &= cand < limit(ub, beyond(k));
+                    wait[k] = better[k] && cand >= limit(thr, beyond(k));
                 }
             }
             if (sh.near_pad || (OV && f.n_over)) {  // its own pads, or its own prices, beyond the border
-#pragma unroll 1
-                for (int k = 0; k < 3; ++k) {
-                    const uint32_t o = k == 0 ? w[0] : k == 1 ? w[TH - 1] : edge, p0 = k == 0 ? pt : k == 1 ? pb : ps;
-                    const bool ok = (k == 0 ? col_in && top : k == 1 ? col_in && bottom : side) && o < kBig;
-                    bool exact = p0 == kBig;
+#pragma unroll
+                for (int k = 0; k < NB; ++k) {
+                    const bool ok = (k == 0 ? col_in && top : k == 1 ? col_in && bottom : side[k < 2 ? 0 : k - 2]) && own[k] < kBig;
+                    bool exact = price[k] == kBig;
                     if constexpr (OV) {
                         const uint32_t nb = k == 0 ? t - ntx : k == 1 ? t + ntx : seg == 0 ? t - 1 : t + 1;
                         exact |= ok && f.n_over && a.tover[f.tile_off + nb];
                     }
                     if (!ok || !exact) continue;
                     const uint32_t gx = k < 2 ? (uint32_t)tx0 + lane : seg == 0 ? (uint32_t)tx0 - 1 : (uint32_t)tx0 + kTW;
-                    const uint32_t gy = k == 0 ? (uint32_t)ty0 - 1 : k == 1 ? (uint32_t)ty0 + TH : (uint32_t)ty0 + r;
+                    const uint32_t gy = k == 0 ? (uint32_t)ty0 - 1 : k == 1 ? (uint32_t)ty0 + TH : (uint32_t)ty0 + r + 8u * (k - 2);
                     const uint32_t dir = k == 0 ? kInPosY : k == 1 ? kInNegY : seg == 0 ? kInPosX : kInNegX;
                     const uint32_t p = exact_price(a.boards + f.board, a.fields + fi, a.pads, dir, wl, gy, gx);
-                    const uint32_t q = k == 0 ? ht : k == 1 ? hb : hs;
-                    const u64 c64 = ext2(((u64)(dbase + (o >> HB)) << 32) | (hbase + (o & kHopMask)), p, 1);
-                    const u64 q64 = q >= kBig ? kInf : ((u64)(dbase + (q >> HB)) << 32) | (hbase + (q & kHopMask));
-                    const bool b64 = c64 < q64;
-                    const uint32_t d = (uint32_t)(c64 >> 32), fx = min(dsum(d, k == 0 ? h[0] : k == 1 ? h[1] : h[2]), kCap);
-                    const bool ok64 = b64 && (!GD || fx <= ub), late = GD && ok64 && fx > thr;
-                    if (k == 0) { better[0] = ok64; wait[0] = late; ex[0] = d; }
-                    else if (k == 1) { better[1] = ok64; wait[1] = late; ex[1] = d; }
-                    else { better[2] = ok64; wait[2] = late; ex[2] = d; }
+                    const u64 c64 = ext2(((u64)(dbase + (own[k] >> HB)) << 32) | (hbase + (own[k] & kHopMask)), p, 1);
+                    const u64 q64 = there[k] >= kBig ? kInf : ((u64)(dbase + (there[k] >> HB)) << 32) |
+                                                                  (hbase + (there[k] & kHopMask));
+                    ex[k] = (uint32_t)(c64 >> 32);
+                    const uint32_t fx = min(dsum(ex[k], beyond(k)), kCap);
+                    better[k] = c64 < q64 && (!GD || fx <= ub);
+                    wait[k] = GD && better[k] && fx > thr;
                 }
             }
+            bool side_now = false, any_wait = false;
 #pragma unroll
-            for (int k = 0; k < 3; ++k) better[k] &= !wait[k];
-            uint32_t sides = (__any_sync(0xFFFFFFFFu, better[2] && seg == 0) ? 1u : 0u) |
-                             (__any_sync(0xFFFFFFFFu, better[2] && seg == 3) ? 2u : 0u) |
+            for (int k = 0; k < NB; ++k) {
+                better[k] &= !wait[k];
+                any_wait |= wait[k];
+                if (k >= 2) side_now |= better[k];
+            }
+            uint32_t sides = (__any_sync(0xFFFFFFFFu, side_now && seg == 0) ? 1u : 0u) |
+                             (__any_sync(0xFFFFFFFFu, side_now && seg == 3) ? 2u : 0u) |
                              (__any_sync(0xFFFFFFFFu, better[0]) ? 4u : 0u) | (__any_sync(0xFFFFFFFFu, better[1]) ? 8u : 0u);
             if (lane == 0 && sides) atomicOr(&sh.push, sides);
-            if (GD && __any_sync(0xFFFFFFFFu, wait[0] || wait[1] || wait[2])) {
+            if (GD && __any_sync(0xFFFFFFFFu, any_wait)) {
 #pragma unroll
-                for (int k = 0; k < 3; ++k) {
+                for (int k = 0; k < NB; ++k) {
                     if (!wait[k]) continue;
                     const uint32_t d = ex[k] != kMax ? ex[k] : dbase + ((own[k] + price[k]) >> HB);
-                    atomicMin(&sh.park[k < 2 ? k + 2 : seg == 0 ? 0 : 1], min(dsum(d, h[k]), kCap));
+                    atomicMin(&sh.park[k < 2 ? k + 2 : seg == 0 ? 0 : 1], min(dsum(d, beyond(k)), kCap));
                 }
             }
         }
@@ -665,7 +695,7 @@ __device__ __forceinline__ bool layer_item(const RelaxArgs &a, uint32_t fi, uint
             // registers are short and it costs 2 % (512x512x4 1.44 -> 1.48 ms).
             const uint32_t sides = *(volatile uint32_t *)&sh.push;
             for (uint32_t l = wl == 1 ? 0u : wl; l <= wl && l < L; ++l)
-                prefetch_neighbours(glab + (int64_t)l * f.wh * f.ww, sides, lane, tx0 - (int)f.x0, ty0 - (int)f.y0, f.ww, f.wh);
+                prefetch_neighbours<TH>(glab + (int64_t)l * f.wh * f.ww, sides, lane, tx0 - (int)f.x0, ty0 - (int)f.y0, f.ww, f.wh);
         }
         __syncthreads();
         if (!sh.more) break;
@@ -687,6 +717,7 @@ __device__ __forceinline__ void end_launch(const RelaxArgs &a) {
 // releases); with one, every f up to the target's dist goes.
 // Returns whether it was the launch's last field.
 __device__ __noinline__ bool field_release(const RelaxArgs &a, uint32_t fi) {
+    const uint32_t TH = a.tile_h;
     __shared__ uint32_t s_min;
     const DevField f = a.fields[fi];
     FieldGoal *fg = a.goal + fi;
@@ -755,8 +786,8 @@ __device__ __noinline__ bool field_release(const RelaxArgs &a, uint32_t fi) {
 
 constexpr u64 kReleaseField = kInf - 1;  // in place of an item: this CTA finished the last one in flight
 
-template <int LM, bool OV, bool GD>
-__global__ void __launch_bounds__(LM * 32, LM == 4 ? 5 : LM == 8 ? 3 : 1) relax_layer_kernel(const __grid_constant__ RelaxArgs a) {
+template <int LM, int TH, bool OV, bool GD>
+__global__ void __launch_bounds__(LM * 32, LM == 4 ? (TH == 8 ? 5 : 3) : LM == 8 ? 3 : 1) relax_layer_kernel(const __grid_constant__ RelaxArgs a) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ LayerShared sh;
     uint32_t phase = 0, fi = 0;
@@ -788,7 +819,7 @@ __global__ void __launch_bounds__(LM * 32, LM == 4 ? 5 : LM == 8 ? 3 : 1) relax_
             last = false;
         } else {
             fi = (uint32_t)(item >> 32);
-            last = layer_item<LM, OV, GD>(a, fi, (uint32_t)item, smem_raw, sh, phase);
+            last = layer_item<LM, TH, OV, GD>(a, fi, (uint32_t)item, smem_raw, sh, phase);
         }
         __syncthreads();
     }
@@ -798,27 +829,39 @@ __global__ void __launch_bounds__(LM * 32, LM == 4 ? 5 : LM == 8 ? 3 : 1) relax_
     }
 }
 
-template <int LM>
+template <int LM, int TH>
 const void *layer_fn_lm(bool over, bool goal) {
-    if (over) return goal ? (const void *)relax_layer_kernel<LM, true, true> : (const void *)relax_layer_kernel<LM, true, false>;
-    return goal ? (const void *)relax_layer_kernel<LM, false, true> : (const void *)relax_layer_kernel<LM, false, false>;
+    if constexpr (TH == kLayerTileH) {
+        if (over)
+            return goal ? (const void *)relax_layer_kernel<LM, TH, true, true> : (const void *)relax_layer_kernel<LM, TH, true, false>;
+    } else if (over) {
+        return nullptr;
+    }
+    return goal ? (const void *)relax_layer_kernel<LM, TH, false, true> : (const void *)relax_layer_kernel<LM, TH, false, false>;
 }
 
-const void *layer_fn(uint32_t max_layers, bool over, bool goal) {
-    return max_layers <= 4 ? layer_fn_lm<4>(over, goal) : max_layers <= 8 ? layer_fn_lm<8>(over, goal)
-                                                                          : layer_fn_lm<16>(over, goal);
+const void *layer_fn(uint32_t max_layers, uint32_t tile_h, bool over, bool goal) {
+    if (tile_h == kLayerTallH) return max_layers <= kLayerTallMax ? layer_fn_lm<4, kLayerTallH>(over, goal) : nullptr;
+    return max_layers <= 4   ? layer_fn_lm<4, kLayerTileH>(over, goal)
+           : max_layers <= 8 ? layer_fn_lm<8, kLayerTileH>(over, goal)
+                             : layer_fn_lm<16, kLayerTileH>(over, goal);
 }
 
 }  // namespace
 
-size_t layer_smem_bytes(uint32_t max_layers) {
-    const size_t narrow = layer_st_off(max_layers) + (size_t)6 * max_layers * TH * kPitch * 4;
-    return std::max(narrow, tile_layout(max_layers, TH).total);  // a wide tile is staged in the same block
+size_t layer_smem_bytes(uint32_t max_layers, uint32_t tile_h) {
+    const size_t narrow = layer_st_off(max_layers, tile_h) + (size_t)6 * max_layers * tile_h * kPitch * 4;
+    return std::max(narrow, tile_layout(max_layers, tile_h).total);  // a wide tile is staged in the same block
 }
 
-cudaError_t layer_configure(uint32_t max_layers, size_t smem, bool over, bool goal, int *blocks_per_sm) {
-    const void *fn = layer_fn(max_layers, over, goal);
-    const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+cudaError_t layer_configure(uint32_t max_layers, uint32_t tile_h, size_t smem, bool over, bool goal, int *blocks_per_sm) {
+    const void *fn = layer_fn(max_layers, tile_h, over, goal);
+    if (!fn) return cudaErrorInvalidValue;
+    // the most any layer count of this kernel takes: a batch of more layers may
+    // already be laid out, and is launched after this call
+    const uint32_t most = max_layers <= 4 ? 4u : max_layers <= 8 ? 8u : 16u;
+    const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)layer_smem_bytes(most, tile_h));
     if (e != cudaSuccess) return e;
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, fn, (int)max_layers * 32, smem);
 }
@@ -828,7 +871,7 @@ cudaError_t layer_launch(const RelaxArgs &a, uint32_t grid, size_t smem, cudaStr
     if (e != cudaSuccess) return e;
     RelaxArgs copy = a;
     void *args[] = {&copy};
-    return cudaLaunchKernel(layer_fn(a.max_layers, over, goal), dim3(grid), dim3(a.max_layers * 32), args, smem, st);
+    return cudaLaunchKernel(layer_fn(a.max_layers, a.tile_h, over, goal), dim3(grid), dim3(a.max_layers * 32), args, smem, st);
 }
 
 }  // namespace mrc

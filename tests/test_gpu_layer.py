@@ -116,3 +116,30 @@ def test_a_field_that_leaves_the_packed_range(oracle):
             _assert_fields(oracle, req, got)
     finally:
         engine.close()
+
+
+@pytest.mark.parametrize("nets,copies", [(1, 1), (9, 3), (9, 16)])
+@pytest.mark.parametrize("layers", [1, 4, 5])
+def test_tile_height_rule(oracle, layers, nets, copies):
+    """Both tile heights on the same nets: the batch alone, and so often repeated
+    that it has more tiles than the taller ones are taken for; five layers and
+    prices per cell always run on the lower ones."""
+    rng = np.random.default_rng(31 * layers)
+    dims = Dims(640, 400, layers)
+    cost = np.ones(len(dims), np.uint32)
+    cost[rng.random(len(dims)) < 0.1] = COST_MAX
+    free = np.flatnonzero(cost != COST_MAX)
+    ends = [(int(a), int(b)) for a, b in rng.choice(free, (nets, 2))]
+    full = IsolatedRouteWindow.full(dims)
+    base = [NetEndpoints(f"n{k}", a, b) for k, (a, b) in enumerate(ends)]
+    grid, gx, gy = Grid(dims, cost), np.full(639, 2, np.uint32), rng.integers(1, 9, 399).astype(np.uint32)
+    vias = [5] * (layers - 1)
+    engine = mrcuda.Engine(0)
+    try:
+        paths, costs = oracle.isolated_batch(IsolatedRouteRequest(grid, base, [full] * nets, gx, gy, vias),
+                                             retry_full=False, mode="field")
+        req = IsolatedRouteRequest(grid, base * copies, [full] * (nets * copies), gx, gy, vias)
+        got = engine.route_isolated_batch(req, retry_full=False)
+        assert (got.paths, got.search_costs) == (list(paths) * copies, list(costs) * copies)
+    finally:
+        engine.close()
