@@ -869,7 +869,7 @@ struct mrc_batch {
     bool layer = false;      // this layout runs the layer kernel (packed price planes by TMA)
     std::vector<DevBoard> devs;  // the board table (step-price plane pointers patched in by batch_layout)
     DBuf d_planes, d_pchunks;    // step-price planes of every board, chunk table of their kernel
-    DBuf d_tmaps;                // one TMA tensor map per board over its planes (CTA queue form)
+    DBuf d_tmaps;                // one TMA tensor map per board over its planes (layer kernel)
     uint64_t n_pchunks = 0;
     // goal-directed relax (the layer kernel, when only paths and costs are asked
     // for): state per field; extremes of the prices per board and waiting f per tile elsewhere
@@ -930,7 +930,7 @@ mrc_status encode_fn(EncodeTiledFn *out) {
 }
 
 // The tensor map of one board's price planes: u32 elements, dims {pitch, h,
-// layers, 6}, a box of kPlaneTmaBoxW x tile_h x layers x 6 (one tile's planes).
+// layers, 6}, a box of kPlaneTmaBoxW x (rows of a tile) x layers x 6 (one tile's planes).
 mrc_status encode_planes_map(const DevBoard &d, uint32_t tile_h, CUtensorMap *map) {
     EncodeTiledFn enc = nullptr;
     MRC_TRY(encode_fn(&enc));
@@ -1211,7 +1211,7 @@ PathArgs path_args(const mrc_batch *bt) {
     pa.tover = bt->has_over ? bt->d_tover.as<uint8_t>() : nullptr;
     pa.tile_h = bt->rows;
     pa.arena_filled = bt->async_q ? 1u : 0u;
-    pa.hop_bits = layer_hop_bits(bt->max_layers, bt->rows);
+    pa.hop_bits = kLayerHopBits;
     pa.walk_smem = bt->layer && !bt->has_over ? (uint32_t)walk_smem_bytes(bt->max_layers) : 0u;
     pa.offsets = bt->d_heads.as<unsigned long long>();
     pa.costs = reinterpret_cast<uint32_t *>(pa.offsets + bt->fields.size() + 1);
@@ -1224,7 +1224,7 @@ PathArgs path_args(const mrc_batch *bt) {
 // Step-price planes of the batch's boards (and the extremes of the prices).
 mrc_status planes_enqueue(mrc_batch *bt, cudaStream_t st, uint32_t *launches) {
     MRC_CUDA(planes_launch(bt->d_boards.as<DevBoard>(), bt->d_pchunks.as<uint64_t>(), (uint32_t)bt->devs.size(),
-                           bt->n_pchunks, (uint32_t)bt->ctx->sms, bt->layer ? layer_hop_bits(bt->max_layers, bt->rows) : 0, st),
+                           bt->n_pchunks, (uint32_t)bt->ctx->sms, bt->layer ? kLayerHopBits : 0, st),
              "launch step-price planes");
     *launches += 1;
     return MRC_OK;

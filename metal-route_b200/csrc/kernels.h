@@ -211,8 +211,6 @@ uint32_t warp_relax_threads();
 cudaError_t warp_relax_occupancy(int *blocks_per_sm);
 // seeds, then the persistent warp kernel (label arena +inf-filled, queue tags zeroed, as for the queue form)
 cudaError_t warp_relax_launch(const RelaxArgs &a, uint32_t grid, cudaStream_t st);
-// Step-price planes of every board of a batch (DevBoard::planes, 6 x cells u32
-// each); chunk_start[k] = first chunk of board k (prefix sum of planes_chunks).
 // Columns of the TMA box that brings one tile's price planes to shared memory:
 // the tile's 32 columns plus the slack of rounding its first column down to a
 // multiple of 4 (16 bytes, the TMA rule for the innermost coordinate).
@@ -231,6 +229,8 @@ inline size_t walk_smem_bytes(uint32_t max_layers) {
 // Rows of a price plane are padded to a multiple of 4 cells (16 bytes), so a
 // tensor map over the planes has 16-byte strides.
 __host__ __device__ inline uint32_t planes_pitch(uint32_t w) { return (w + 3u) & ~3u; }
+// Step-price planes of every board of a batch (DevBoard::planes, 6 x cells u32
+// each); chunk_start[k] = first chunk of board k (prefix sum of planes_chunks).
 // hop_bits: 0 = plain prices (the warp schedule), else packed for the layer
 // kernel: (price << hop_bits) | 1, kPackedInf for no step; a board with a finite
 // price that does not fit is marked (BoardGoal::wide).
@@ -265,11 +265,12 @@ constexpr uint32_t kLayerMax = 16;
 constexpr uint32_t kLayerTileH = 8;
 constexpr uint32_t kLayerTallH = 16, kLayerTallMax = 4;  // tall tiles: up to so many layers, no overrides
 constexpr uint32_t kTallTiles = 240;  // tall up to so many 8-row tiles an SM
-// bits of a packed word that hold hops (the rest, below bit 30, the dist): a path
-// through a tile has no more hops than the tile cells
-__host__ __device__ constexpr uint32_t layer_hop_bits(uint32_t max_layers, uint32_t tile_h) {
-    return max_layers * tile_h <= 64 ? 12 : 13;
-}
+// Bits of a packed word that hold hops; the rest, below bit 30, hold the dist.  A
+// tile and its border span 50 to 60 steps and a few detours, so that 10 bits leave
+// room for hops and 2^19 for dists: prices of up to some 10 000 a step stay packed.
+// (12 bits, enough for any path through 2048 cells, left 2^17: 256 nets of 512 x
+// 512 with gaps of 3000 took 7.3 ms.)
+constexpr uint32_t kLayerHopBits = 10;
 size_t layer_smem_bytes(uint32_t max_layers, uint32_t tile_h);
 cudaError_t layer_configure(uint32_t max_layers, uint32_t tile_h, size_t smem, bool over, bool goal, int *blocks_per_sm);
 cudaError_t layer_launch(const RelaxArgs &a, uint32_t grid, size_t smem, cudaStream_t st, bool over, bool goal);

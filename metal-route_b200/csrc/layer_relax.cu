@@ -21,8 +21,12 @@
 //
 // The packing is exact or not used: a tile whose staged labels spread too far, or
 // whose largest final label comes within one price of kBig (the only way a sum
-// could have been clamped), is relaxed on 64-bit labels instead (wide_item), from
-// the labels in HBM, which this kernel has not touched by then.  So is every tile
+// could have been clamped), or with a final label at the last value of the hops, is
+// relaxed on 64-bit labels instead (wide_item), from the labels in HBM, which this
+// kernel has not touched by then.  (Words are sums dist 2^HB + hops, so a word is
+// the lexicographic least label as long as that label's hops fit, whatever other
+// paths carried into the dist; and the first label of a best path that doesn't fit
+// follows one whose hops are the last value.)  So is every tile
 // of a board with a finite price of 2^(29 - HB) or more.
 //
 // Bound by the chain of activations (a queue hop, the label loads, the sweeps, the
@@ -158,7 +162,7 @@ __device__ __noinline__ void prefetch_neighbours(const u64 *lab, uint32_t sides,
 template <int LM, int TH, bool OV, bool GD>
 __device__ __forceinline__ bool layer_item(const RelaxArgs &a, uint32_t fi, uint32_t t, unsigned char *smem_raw,
                                            LayerShared &sh, uint32_t &phase) {
-    constexpr int HB = (int)layer_hop_bits(LM, TH), RG = TH / 8, NB = 2 + RG;  // row groups, border cells of a lane
+    constexpr int HB = (int)kLayerHopBits, RG = TH / 8, NB = 2 + RG;  // row groups, border cells of a lane
     constexpr uint32_t kHopMask = (1u << HB) - 1u;
     const uint32_t tid = threadIdx.x, lane = tid & 31u, wl = tid >> 5;
     const uint32_t r = lane >> 2, seg = lane & 3u;  // row layout: row (of each group of 8) and segment of 8 cells
@@ -296,10 +300,8 @@ __device__ __forceinline__ bool layer_item(const RelaxArgs &a, uint32_t fi, uint
         }
         __syncthreads();
         const uint32_t dbase = sh.dmin, hbase = sh.hmin;
-        // hops of a path through the tile stay below the dist bits, and no dist of
-        // the tile can saturate
-        bool bad = dbase != kMax && ((int64_t)(sh.hmax - hbase) + kTW * TH * L + 4 > (int64_t)kHopMask ||
-                                     dbase > kMax - (kBig >> HB));
+        // staged hops stay below the dist bits, and no dist of the tile can saturate
+        bool bad = dbase != kMax && (sh.hmax - hbase >= kHopMask || dbase > kMax - (kBig >> HB));
         uint32_t ub = kMax;
         uint32_t w[TH], w0[TH], lim[TH], there[NB];  // there: staged labels beyond the border
         if constexpr (GD) ub = sh.ub;
@@ -551,8 +553,13 @@ __device__ __forceinline__ bool layer_item(const RelaxArgs &a, uint32_t fi, uint
 
         // ---- is the packing exact for this tile? -------------------------------
         if (mine) {
+            uint32_t over = kMax, hops = 0;  // least label from kNarrow on (kBig is at kNarrow), most hops
 #pragma unroll
-            for (int y = 0; y < TH; ++y) bad |= w[y] >= kNarrow && w[y] < kBig;
+            for (int y = 0; y < TH; ++y) {
+                over = __viaddmin_u32(w[y], 0u - kNarrow, over);
+                hops = max(hops, w[y] & kHopMask);
+            }
+            bad |= over < kNarrow || hops == kHopMask;
         }
         if (__syncthreads_or(bad || *(volatile uint32_t *)&sh.wide))
             return wide_item<TH, OV, GD>(a, fi, t, smem_raw, sh.cnt);

@@ -94,6 +94,40 @@ def test_axis_gaps_tie(oracle, layers, price):
         engine.close()
 
 
+@pytest.mark.parametrize("layers,w,h", [(1, 200, 40), (2, 40, 32), (4, 64, 32), (8, 64, 16)])
+@pytest.mark.parametrize("price", [1, 3, (1 << 19) - 1, 1 << 19])
+def test_long_ways_inside_a_tile(oracle, layers, w, h, price):
+    """More hops inside a tile and its border than a word holds: a serpentine on
+    every layer, joined by single vias into one way, and equal costs beside it."""
+    cost = np.ones((layers, h, w), np.uint32)
+    cost[:, 1::2, :] = COST_MAX
+    for k, y in enumerate(range(1, h, 2)):
+        cost[:, y, w - 1 if k % 2 == 0 else 0] = 1
+    rng = np.random.default_rng(layers + w)
+    holes = rng.random(cost.shape) < 0.01
+    cost[holes & (cost == COST_MAX)] = 2
+    dims = Dims(w, h, layers)
+    last = (h - 2) * w if (h // 2) % 2 == 0 else (h - 2) * w + w - 1
+    forbidden = np.ones((layers, h * w), np.uint8)
+    for l in range(layers - 1):
+        forbidden[l:l + 2, 0 if l % 2 else last] = 0
+    full = IsolatedRouteWindow.full(dims)
+    far = (layers - 1) * w * h
+    nets = [NetEndpoints("a", 0, far + last), NetEndpoints("b", far, 4), NetEndpoints("c", 2 * w + 1, far + 2 * w + 1)]
+    req = IsolatedRouteRequest(Grid(dims, cost.reshape(-1), None, forbidden.reshape(-1)), nets, [full] * 3,
+                               np.full(w - 1, price, np.uint32), np.full(h - 1, price, np.uint32), [price] * (layers - 1))
+    engine = mrcuda.Engine(0)
+    try:
+        exp = oracle.isolated_batch(req, retry_full=False, mode="field")
+        got = engine.route_isolated_batch(req, retry_full=False, keep_fields=True)
+        assert (got.paths, got.search_costs) == exp
+        _assert_fields(oracle, req, got)
+        paths_only = engine.route_isolated_batch(req, retry_full=False)
+        assert (paths_only.paths, paths_only.search_costs) == exp
+    finally:
+        engine.close()
+
+
 def test_a_field_that_leaves_the_packed_range(oracle):
     """Long hop counts and costs: a serpentine whose labels spread past one word
     inside a tile (walls every other row, a gap at alternating ends)."""
