@@ -1,9 +1,12 @@
 #!/usr/bin/env python3
-"""Benchmark of the batched isolated-route engine (fields + canonical paths).
+"""Benchmark of the batched isolated-route engine (canonical paths and complete fields).
 
 Workload (default): the congestion board — 512x512x4, 256 nets, directed edge
 prices, exact polygon outline, windows by net_window — one "step" routes every
-net of the batch (complete u32 fields over every window + canonical paths).
+net of the batch to its canonical path and cost.  A batch that is asked for
+paths alone searches goal-directed; `complete_fields` in the line is the same
+batch with the complete u32 field of every window kept as well, and the roofline
+is taken from that launch, whose work the window cells count.
 `--workload plain` is the 128x128x2 board with 64 nets and whole-board fields;
 `--workload uneven` is 4096 independent one-net instances of log-normal size
 and 2-8 layers, staged as one multi-board batch.  The launch sequence is
@@ -235,6 +238,40 @@ def run_reference(args):
     return 0
 
 
+def _complete_fields(batch, boards, wl, stream, flush, steps, max_over_ranks, world):
+    """The same nets with every window's complete field kept (device time, L2
+    flushed between launches)."""
+    import torch
+
+    import mrcuda
+
+    kw = {} if len(boards) == 1 else {"net_board": wl.net_board}
+    full = mrcuda.Batch(boards[0] if len(boards) == 1 else boards, wl.nets, wl.windows, retry_full=True,
+                        time_kernels=True, keep_fields=True, **kw)
+    cfg = batch.config()
+    if cfg["schedule"] != 2:
+        full.set_config(cfg["tile_h"], cfg["threads"])
+    full.set_schedule(cfg["schedule"])
+    ms, relax_ms = [], []
+    for k in range(3 + steps):
+        with torch.cuda.stream(stream):
+            flush.zero_()
+        s, e = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        s.record(stream)
+        full.launch(stream.cuda_stream)
+        e.record(stream)
+        stream.synchronize()
+        if k >= 3:
+            ms.append(s.elapsed_time(e))
+            relax_ms.append(full.relax_ms())
+    out = {"ms_per_step": max_over_ranks(statistics.fmean(ms), device="cuda"), "steps": steps,
+           "relax_ms": statistics.fmean(relax_ms)}
+    out["value"] = len(wl.nets) * world / (out["ms_per_step"] / 1000.0)
+    work = full.stats()
+    full.close()
+    return out, work
+
+
 def measure_batch(args, name, eng, rank, world, local, dist, nets=0, steps=None, main=True):
     """One batched workload on the resident engine: autotune, graph capture,
     warm-up, K device-timed steps (L2 flushed between them), the end-to-end
@@ -299,10 +336,11 @@ def measure_batch(args, name, eng, rank, world, local, dist, nets=0, steps=None,
     if dist:
         dist.barrier()
     clk = clocks.stop()
-    work = batch.stats()
     ms = statistics.fmean(step_ms)
     ms_max = max_over_ranks(ms, device="cuda")
     value = len(wl.nets) * world / (ms_max / 1000.0)
+
+    fields, work = _complete_fields(batch, boards, wl, stream, flush, min(steps, 10), max_over_ranks, world)
 
     # end to end through the public call with host buffers: first the caller's
     # ordinary (pageable) arrays, then the same boards in page-locked memory
@@ -331,18 +369,15 @@ def measure_batch(args, name, eng, rank, world, local, dist, nets=0, steps=None,
     # roofline of the dominant kernel (the relax kernel)
     peak, peak_kind = _peaks()
     alg_bytes = wl.algorithmic_bytes() + 4 * path_cells
-    relax_avg = statistics.fmean(relax_ms) if relax_ms and min(relax_ms) > 0 else ms
+    relax_avg = fields["relax_ms"] if fields["relax_ms"] > 0 else fields["ms_per_step"]
     achieved = alg_bytes / (relax_avg / 1000.0) / 1e9
     sched = batch.config()
-    kname = {0: "relax_rounds_kernel", 1: "relax_async_kernel", 2: "relax_warp_kernel",
-             3: "relax_async_kernel"}[sched["schedule"]]
-    # the queue kernel's third template argument: step prices staged from the price planes by TMA
+    queue = f"relax_async_kernel<{sched['tile_h']},{sched['threads']}>"
     kfull = {0: f"relax_rounds_kernel<{sched['tile_h']},{sched['threads']}>",
-             1: f"relax_async_kernel<{sched['tile_h']},{sched['threads']},true>",
-             2: "relax_warp_kernel",
-             3: f"relax_async_kernel<{sched['tile_h']},{sched['threads']},false>"}[sched["schedule"]]
+             1: "relax_layer_kernel" if sched["tile_h"] == 8 else queue,
+             2: "relax_warp_kernel", 3: queue}[sched["schedule"]]
     # DRAM bytes and instruction counts of one launch, from the ncu capture of this kernel and workload
-    prof = _profile_figures(kfull.split("<")[0] + ("_tma" if sched["schedule"] == 1 else ""), name)
+    prof = _profile_figures(kfull.split("<")[0], name)
     acts = max(work["activations"], 1)
     counters = {"tile_activations": work["activations"], "tiles": work["tiles"],
                 "activations_per_tile": work["activations"] / max(work["tiles"], 1),
@@ -365,6 +400,8 @@ def measure_batch(args, name, eng, rank, world, local, dist, nets=0, steps=None,
                 "inputs": "page-locked host arrays", "outputs": "CSR arrays (offsets, cells, costs)",
                 "pageable_value": e2e_pageable,
                 "vs_device_value": e2e_value / value},
+        "complete_fields": fields,
+        "relax_ms": statistics.fmean(relax_ms),
         "gpu_launches": batch.kernel_launches * steps,
         "roofline": dict({"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                           "traffic": None if prof is None else prof.get("dram_bytes_per_launch"),
@@ -383,6 +420,8 @@ def _summary(line):
     """The compact form of a workload's line inside `workloads`."""
     out = {"workload": line["config"]["workload"], "value": line["value"], "unit": line["unit"],
            "ms_per_step": line["ms_per_step"], "e2e": line["e2e"]["value"], "clocks": line.get("clocks")}
+    if "complete_fields" in line:
+        out["complete_fields"] = line["complete_fields"]["value"]
     r = line.get("roofline")
     if r:
         out["roofline"] = {k: r[k] for k in ("kernel", "kernel_ms", "achieved", "frac", "traffic",
@@ -578,7 +617,8 @@ def measure_snapshot(args, eng, local, rounds, warmup, cpu):
         "gpu_launches": None,
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                      "traffic": None, "peak_kind": peak_kind, "kernel": "whole round (relax + price + merge)",
-                     "algorithmic_bytes": int(alg), "bytes_per_cell": wl.bytes_per_cell()},
+                     "algorithmic_bytes": int(alg), "bytes_per_cell": wl.bytes_per_cell(),
+                     "bytes_are": "of complete windows; the rounds' goal-directed search touches a part of them"},
         "clocks": clk,
     }
     if cpu:

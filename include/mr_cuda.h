@@ -124,7 +124,8 @@ void mrc_context_destroy(mrc_context *ctx);
 const char *mrc_last_error(const mrc_context *ctx);
 uint32_t mrc_abi_version(void);
 
-/* Page-locked host memory, mapped into every device's address space.  Board
+/* Page-locked host memory, mapped into every device's address space.  Freed
+ * blocks are kept for reuse up to a process-wide bound.  Board
  * arrays (cost, masks, directed prices) held here are read in place by one
  * gather launch in mrc_route_instances instead of being staged, and reach HBM
  * at full link rate in the single-board calls.  Ordinary (pageable) arrays
@@ -205,7 +206,9 @@ mrc_status mrc_batch_create_multi(mrc_context *ctx, const mrc_board *const *boar
 /* Capture the batch's launch sequence (resets, relax, path kernels) into a CUDA
  * graph; later mrc_batch_launch calls replay it with one cudaGraphLaunch. */
 mrc_status mrc_batch_capture_graph(mrc_context *ctx, mrc_batch *batch);
-/* Enqueue the whole window solve (fields + canonical paths) on `stream`
+/* Enqueue the whole window solve on `stream`: canonical paths and costs, and
+ * with MRC_FLAG_KEEP_FIELDS every window's complete field (without it the
+ * search may leave cells that cannot be on a shortest path unsolved)
  * (a cudaStream_t, NULL = the context's stream) without any host sync. */
 mrc_status mrc_batch_launch(mrc_context *ctx, mrc_batch *batch, void *stream);
 /* Wait for the batch, run the full-board retry if flagged, copy results out. */
@@ -221,9 +224,11 @@ mrc_status mrc_batch_autotune(mrc_context *ctx, mrc_batch *batch, uint32_t *tile
 mrc_status mrc_batch_set_config(mrc_context *ctx, mrc_batch *batch, uint32_t tile_h, uint32_t threads);
 /* The relax schedule: 0 = bulk-synchronous rounds over a shared tile list
  * (cooperative launch, grid barrier between rounds); 1 = one asynchronous
- * work queue (no rounds; a tile held by one CTA at a time), step prices brought
- * to each tile by one TMA load from per-board price planes computed once per
- * launch; 2 = the same queue with one warp per tile (tiles of 4 S x 8 cells
+ * work queue (no rounds; a tile held by one CTA at a time) of tiles with a warp
+ * per layer and labels packed into 32 bits, step prices brought to each tile by
+ * one TMA load from per-board price planes computed once per batch layout
+ * (8-row tiles and at most 16 layers, else schedule 3's kernel; the library
+ * takes 16-row tiles itself where they are faster); 2 = the same queue with one warp per tile (tiles of 4 S x 8 cells
  * over every layer, S = 32 / next_pow2(layers), labels in shared memory;
  * boards of at most 16 layers, else MRC_ERR_LIMIT; a batch whose nets carry
  * negotiation price overrides runs 1 instead); 3 = the queue of 1 with step

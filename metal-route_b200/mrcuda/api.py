@@ -582,7 +582,8 @@ class Batch:
 
     def set_schedule(self, schedule: int) -> None:
         """0 = bulk-synchronous rounds, 1 = asynchronous work queue (a CTA per
-        tile, prices from the TMA-loaded price planes), 2 = the queue with a warp
+        tile, a warp per layer, labels packed into 32 bits, prices from the
+        TMA-loaded price planes), 2 = the queue with a warp
         per tile, 3 = the CTA queue with prices formed per tile."""
         e = self.engine
         e._check(e.lib.mrc_batch_set_schedule(e.ctx, self.handle, int(schedule)))
