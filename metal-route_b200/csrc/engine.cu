@@ -1322,6 +1322,15 @@ struct BatchOut {
     FieldBlock fields;
 };
 
+// Waits for a stream when a function leaves before it did so itself.
+struct DrainOnExit {
+    cudaStream_t st;
+    bool waited = false;
+    ~DrainOnExit() {
+        if (!waited) cudaStreamSynchronize(st);
+    }
+};
+
 // Copy one batch's outputs to the host: status, offsets and costs and as many path
 // cells as such a batch usually has in one go through the page-locked block,
 // fields straight into theirs, and one wait for all of it.
@@ -1333,14 +1342,16 @@ mrc_status batch_collect(mrc_batch *bt, bool keep_fields, BatchOut *out) {
     const uint64_t early = std::min<uint64_t>(bt->total_cells, (uint64_t)n * kCellsPerNet);
     const size_t heads = ((size_t)n + 1) * 8 + (size_t)n * 4, o_cells = (16 + heads + 15) & ~(size_t)15;
     MRC_CUDA(ctx->down.reserve(o_cells + early * 4), "pinned download buffer");
+    const bool fields = keep_fields && bt->total_cells && bt->d_out.p;
+    if (keep_fields && !out->fields.alloc(bt->total_cells)) return fail(MRC_ERR_OUT_OF_MEMORY, "host memory for the fields");
+    DrainOnExit drain{st};  // a call that fails from here on leaves no copy into either block behind
     unsigned char *host = static_cast<unsigned char *>(ctx->down.p);
     MRC_CUDA(cudaMemcpyAsync(host, &bt->ctl()->status, 4, cudaMemcpyDeviceToHost, st), "read status");
     MRC_CUDA(cudaMemcpyAsync(host + 16, bt->d_heads.p, heads, cudaMemcpyDeviceToHost, st), "read offsets and costs");
     if (early) MRC_CUDA(cudaMemcpyAsync(host + o_cells, bt->d_cells.p, early * 4, cudaMemcpyDeviceToHost, st), "read paths");
-    const bool fields = keep_fields && bt->total_cells && bt->d_out.p;
-    if (keep_fields && !out->fields.alloc(bt->total_cells)) return fail(MRC_ERR_OUT_OF_MEMORY, "host memory for the fields");
     if (fields)
         MRC_CUDA(cudaMemcpyAsync(out->fields.data(), bt->d_out.p, bt->total_cells * 4, cudaMemcpyDeviceToHost, st), "read fields");
+    drain.waited = true;
     MRC_CUDA(cudaStreamSynchronize(st), "batch execution");
     uint32_t status = 0;
     std::memcpy(&status, host, 4);

@@ -1,0 +1,67 @@
+"""The host runtime (csrc/engine.cu) on a CUDA runtime made of host memory
+(fake_cuda.cpp): what it does with streams, page-locked memory and failing calls.
+Each test is a child process, so that this one keeps the real library."""
+import os
+import shutil
+import subprocess
+import sys
+
+import pytest
+
+from conftest import ROOT
+
+CUDA = next((d for d in (os.environ.get("CUDA_HOME"), "/usr/local/cuda") if d and os.path.exists(d + "/include/cuda.h")), None)
+pytestmark = pytest.mark.skipif(CUDA is None or shutil.which("g++") is None, reason="needs g++ and the CUDA headers")
+
+PROLOGUE = """
+import ctypes as C, sys
+import numpy as np
+import mrcuda
+from mrcuda.types import *
+L = mrcuda.load_library(sys.argv[1])
+L.fake_fail.argtypes = [C.c_char_p, C.c_int]
+L.fake_pinned_bytes.restype = C.c_uint64
+eng = mrcuda.Engine(0)
+fail = lambda call, nth=1: L.fake_fail(call.encode(), nth)
+def grid(w, h, layers=1):
+    return Grid(Dims(w, h, layers), np.ones(w * h * layers, np.uint32))
+def board(w, h, layers=1, gap=1):
+    return eng.board(grid(w, h, layers), [gap] * (w - 1), [gap] * (h - 1), [1] * (layers - 1))
+def nets(w, h, n=1):
+    return [NetEndpoints(f"n{i}", 0, w * h - 1) for i in range(n)]
+"""
+
+
+@pytest.fixture(scope="session")
+def fake_library(tmp_path_factory):
+    so = str(tmp_path_factory.mktemp("fake") / "libfake.so")
+    csrc = os.path.join(ROOT, "metal-route_b200", "csrc")
+    subprocess.check_call(["g++", "-x", "c++", "-std=c++17", "-O1", "-w", "-fPIC", "-shared", "-D__ldg(p)=(*(p))",
+                           "-I", CUDA + "/include", "-I", os.path.join(ROOT, "include"), "-I", csrc,
+                           os.path.join(csrc, "engine.cu"), os.path.join(ROOT, "tests", "fake_cuda.cpp"),
+                           "-Wl,--wrap=malloc", "-Wl,--no-undefined", "-lpthread", "-o", so])
+    return so
+
+
+@pytest.fixture
+def run(fake_library):
+    def go(body):
+        env = dict(os.environ, PYTHONPATH=os.path.join(ROOT, "metal-route_b200"))
+        p = subprocess.run([sys.executable, "-c", PROLOGUE + body, fake_library], env=env, capture_output=True,
+                           text=True, timeout=120)
+        assert p.returncode == 0, p.stdout + p.stderr
+    return go
+
+
+def test_no_copy_is_in_flight_after_a_failed_finish(run):
+    """Host memory for the fields runs out: the call returns with nothing on its way
+    into the context's download block, which the next call of any stream uses."""
+    run("""
+bt = mrcuda.Batch(board(40, 30), nets(40, 30), keep_fields=True)
+bt.launch()
+fail("cudaHostAlloc", 2); fail("malloc")  # (the first page-locked block is the download block)
+try: bt.finish(); assert False
+except mrcuda.OutOfMemory: pass
+assert L.fake_pending_host_writes() == 0
+bt.finish()
+""")
