@@ -1677,6 +1677,7 @@ mrc_status mrc_distance_fields(mrc_context *ctx, const mrc_grid *grid, const uin
     mrc_batch bt;
     MRC_TRY(batch_build(ctx, {&board}, std::move(nc), std::move(wins), MRC_FLAG_KEEP_FIELDS, &bt));
     MRC_TRY(batch_launch(&bt, ctx->stream));
+    DrainOnExit drain{ctx->stream};  // the caller may free its rows as soon as a failed call returns
     uint32_t status = 0;
     MRC_CUDA(cudaMemcpyAsync(&status, &bt.ctl()->status, 4, cudaMemcpyDeviceToHost, ctx->stream), "read status");
     for (size_t k = 0, e; k < slot.size(); k = e) {
@@ -1685,6 +1686,7 @@ mrc_status mrc_distance_fields(mrc_context *ctx, const mrc_grid *grid, const uin
                                  cudaMemcpyDeviceToHost, ctx->stream),
                  "read fields");
     }
+    drain.waited = true;
     MRC_CUDA(cudaStreamSynchronize(ctx->stream), "distance fields");
     if (status) return status_error(status);
     return MRC_OK;

@@ -65,3 +65,15 @@ except mrcuda.OutOfMemory: pass
 assert L.fake_pending_host_writes() == 0
 bt.finish()
 """)
+
+
+def test_no_copy_is_in_flight_after_failed_distance_fields(run):
+    """A copy fails after others were put on the stream: none of those still writes into
+    the caller's rows, which the caller may free."""
+    run("""
+g = grid(40, 30); g.cost[1] = COST_MAX
+fail("copy to host", 3)  # status, rows before the refused source, rows after it
+try: eng.distance_fields(g, [0, 1, 2]); assert False
+except mrcuda.BackendUnavailable: pass
+assert L.fake_pending_host_writes() == 0
+""")
