@@ -236,6 +236,11 @@ mrc_status mrc_batch_set_config(mrc_context *ctx, mrc_batch *batch, uint32_t til
  * the same labels and paths.  The autotuner tries every one.  These replace
  * the per-round dispatch loop of crates/mr-metal/src/gpu.rs:1630-2039. */
 mrc_status mrc_batch_set_schedule(mrc_context *ctx, mrc_batch *batch, uint32_t schedule);
+/* Guard against a launch that never ends: past this many tile activations the workers
+ * of a queue schedule leave, and the batch fails with MRC_ERR_ITERATION_LIMIT (each
+ * notices after up to 64 activations of its own).  0, the default: 1024 for every tile
+ * of the batch and 65 536 more, far above any need.  Drops a captured graph. */
+mrc_status mrc_batch_set_activation_limit(mrc_context *ctx, mrc_batch *batch, uint64_t limit);
 /* Schedule of batches built on this context while it holds no autotuned
  * configuration for their layer count and price form: 0, 1 (the default), 2
  * or 3 (see mrc_batch_set_schedule); with 2, batches with more than 16 layers

@@ -878,13 +878,11 @@ __device__ __forceinline__ bool process_item(const RelaxArgs &a, uint32_t fi, ui
                 if constexpr (ASYNC) {
                     // the work counters are per CTA (s_cnt), added to the launch's
                     // every kCountBatch activations and when the CTA exits, so this
-                    // thread makes no round trip to L2 here
+                    // thread makes no round trip to L2 here (s_cnt[2]: the CTA leaves
+                    // a failed launch after this item)
                     s_cnt[1] += sweep;
                     if (++s_cnt[0] == kCountBatch) {
-                        if (atomicAdd(&ctl->activations, (unsigned long long)kCountBatch) + kCountBatch >
-                            a.activation_limit)
-                            atomicOr(&ctl->status, kStatusActivationLimit);
-                        atomicAdd(&ctl->sweeps, s_cnt[1]);
+                        if (!count_flush(a, s_cnt[0], s_cnt[1])) s_cnt[2] = 1;
                         s_cnt[0] = s_cnt[1] = 0;
                     }
                 } else {

@@ -856,6 +856,7 @@ struct mrc_batch {
     u64 *lab() const { return d_ones.as<u64>(); }
     uint32_t *tpark() const { return reinterpret_cast<uint32_t *>(d_ones.as<unsigned char>() + o_tpark); }
     uint32_t launches = 0;
+    uint64_t activation_limit = 0;  // 0: by the number of tiles
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     cudaGraphExec_t graph = nullptr;  // captured launch sequence (mrc_batch_capture_graph)
@@ -1265,7 +1266,8 @@ mrc_status batch_enqueue(mrc_batch *bt, cudaStream_t st, bool capturing) {
     ra.ctl = bt->ctl();
     ra.tile_h = bt->rows;
     ra.round_limit = 64u * bt->max_tiles + 4096u;
-    ra.activation_limit = 1024ull * bt->total_tiles + 65536ull;  // runaway guard, far above any measured need
+    // runaway guard, far above any measured need
+    ra.activation_limit = bt->activation_limit ? bt->activation_limit : 1024ull * bt->total_tiles + 65536ull;
     if (n && bt->async_q) MRC_CUDA(cudaMemsetAsync(bt->d_ones.p, 0xFF, bt->ones_bytes, st), "fill label arena");
     if (n) {
         const unsigned rec = capturing ? cudaEventRecordExternal : cudaEventRecordDefault;
@@ -1962,6 +1964,17 @@ mrc_status mrc_batch_set_schedule(mrc_context *ctx, mrc_batch *batch, uint32_t s
     batch->cta_planes = schedule != 3;
     // leaving the warp schedule: the default CTA tile (8 rows, 256 threads)
     return batch_layout(batch, was_warp ? 8u : batch->tile_h, was_warp ? 256u : batch->threads);
+}
+
+mrc_status mrc_batch_set_activation_limit(mrc_context *ctx, mrc_batch *batch, uint64_t limit) {
+    if (!ctx || !batch) return fail(MRC_ERR_INVALID_ARGUMENT, "NULL argument");
+    Lock lock(ctx, 0);
+    batch->activation_limit = limit;
+    if (batch->graph) {  // a captured graph bakes in the old limit
+        cudaGraphExecDestroy(batch->graph);
+        batch->graph = nullptr;
+    }
+    return MRC_OK;
 }
 
 mrc_status mrc_context_set_schedule(mrc_context *ctx, uint32_t schedule) {

@@ -59,7 +59,7 @@ __host__ __device__ inline size_t layer_st_off(uint32_t L, uint32_t TH) {
 struct LayerShared {
     u64 item;
     uint64_t mbar;  // completion of the price-plane TMA loads
-    unsigned long long cnt[2];  // activations and sweeps not yet added to the launch's
+    unsigned long long cnt[3];  // activations and sweeps not yet added to the launch's; the CTA leaves
     uint32_t n_spec, near_pad, wide, dmin, hmin, hmax, ub, thr, more;
     uint32_t push;              // bits: left, right, top, bottom improved
     uint32_t park[4];           // GD: the smallest f that waits to enter each
@@ -333,18 +333,21 @@ __device__ __forceinline__ bool layer_item(const RelaxArgs &a, uint32_t fi, uint
 #pragma unroll
         for (int k = 0; k < NB; ++k) there[k] = pack(vh[k], limit(ub, beyond(k)));
         if (cont == 0) {
-            // the planes: a bounded wait for the TMA load (a load that never lands
-            // sets the status and the launch ends without results)
+            // the planes: a bounded wait for the TMA load.  A load that never lands sets
+            // the status, and the CTA leaves before the write-back
             for (uint32_t spins = 0; !mbar_try_wait(&sh.mbar, phase & 1u); ++spins) {
                 if (spins == kTmaSpinLimit) {
                     if (tid == 0) atomicOr(&a.ctl->status, kStatusQueueOverflow);
                 } else if (spins > 2 * kTmaSpinLimit) {
+                    *(volatile unsigned long long *)&sh.cnt[2] = 1;
+                    bad = true;
                     break;
                 }
             }
             ++phase;
             if (board_wide) {
-                __syncthreads();  // everybody is past the load and the staged words
+                if (__syncthreads_or(bad && *(volatile unsigned long long *)&sh.cnt[2])) return false;
+                // everybody is past the load and the staged words
                 return wide_item<TH, OV, GD>(a, fi, t, smem_raw, sh.cnt);
             }
             if (mine && (tw < kTW || th < TH || xlo)) {  // no step enters a cell past the window
@@ -561,8 +564,10 @@ __device__ __forceinline__ bool layer_item(const RelaxArgs &a, uint32_t fi, uint
             }
             bad |= over < kNarrow || hops == kHopMask;
         }
-        if (__syncthreads_or(bad || *(volatile uint32_t *)&sh.wide))
+        if (__syncthreads_or(bad || *(volatile uint32_t *)&sh.wide)) {
+            if (*(volatile unsigned long long *)&sh.cnt[2]) return false;  // without its prices
             return wide_item<TH, OV, GD>(a, fi, t, smem_raw, sh.cnt);
+        }
         if constexpr (GD) ub = *(volatile uint32_t *)&sh.ub;
 
         // ---- write back the labels that fell -----------------------------------
@@ -685,9 +690,7 @@ __device__ __forceinline__ bool layer_item(const RelaxArgs &a, uint32_t fi, uint
                 sh.hmax = 0;
                 sh.cnt[1] += sweep;
                 if (++sh.cnt[0] == kCountBatch) {
-                    if (atomicAdd(&a.ctl->activations, (unsigned long long)kCountBatch) + kCountBatch > a.activation_limit)
-                        atomicOr(&a.ctl->status, kStatusActivationLimit);
-                    atomicAdd(&a.ctl->sweeps, sh.cnt[1]);
+                    if (!count_flush(a, sh.cnt[0], sh.cnt[1])) sh.cnt[2] = 1;
                     sh.cnt[0] = sh.cnt[1] = 0;
                 }
             }
@@ -722,7 +725,7 @@ __device__ __forceinline__ void end_launch(const RelaxArgs &a) {
 // Without a target label the threshold grows (twice the distance above the
 // bound, at least to the smallest f that waits; everything after kGoalPhases
 // releases); with one, every f up to the target's dist goes.
-// Returns whether it was the launch's last field.
+// Returns whether the launch is over: it was the last field, or the launch has failed.
 __device__ __noinline__ bool field_release(const RelaxArgs &a, uint32_t fi) {
     const uint32_t TH = a.tile_h;
     __shared__ uint32_t s_min;
@@ -733,7 +736,7 @@ __device__ __noinline__ bool field_release(const RelaxArgs &a, uint32_t fi) {
     for (;;) {
         __threadfence();
         if (threadIdx.x == 0) s_min = kMax;
-        __syncthreads();
+        if (__syncthreads_or(threadIdx.x == 0 && launch_failed(a))) return true;  // its tiles may never be released
         const uint32_t ub = *(volatile const uint32_t *)&fg->ub;
         uint32_t m = kMax;
         for (uint32_t i = threadIdx.x; i < ntiles; i += 4 * blockDim.x) {
@@ -800,14 +803,14 @@ __global__ void __launch_bounds__(LM * 32, LM == 4 ? (TH == 8 ? 5 : 3) : LM == 8
     uint32_t phase = 0, fi = 0;
     bool last = false;
     if (threadIdx.x == 0) {
-        sh.cnt[0] = sh.cnt[1] = 0;
+        sh.cnt[0] = sh.cnt[1] = sh.cnt[2] = 0;
         mbar_init(&sh.mbar, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
     for (;;) {
         if (threadIdx.x == 0) {
-            sh.item = last ? kReleaseField : async_pop<64>(a);
+            sh.item = sh.cnt[2] ? kInf : last ? kReleaseField : async_pop<64>(a);
             sh.n_spec = sh.near_pad = sh.wide = 0;
             sh.dmin = sh.hmin = kMax;
             sh.hmax = 0;

@@ -92,6 +92,22 @@ __device__ __forceinline__ void async_release(const RelaxArgs &a, uint32_t fi, u
     }
 }
 
+// Whether the launch has failed: a limit was passed, or a wait ran out.
+__device__ __forceinline__ bool launch_failed(const RelaxArgs &a) {
+    return *(volatile const uint32_t *)&a.ctl->status != 0u;
+}
+
+// Adds a worker's activations and sweeps to the launch's.  False: the launch has
+// failed, by too many activations or otherwise, and the worker leaves it.  A
+// queue that never runs dry keeps its workers from waiting, and so from reading the
+// status word in async_pop; they read it here, every kCountBatch activations.
+__device__ __forceinline__ bool count_flush(const RelaxArgs &a, unsigned long long acts, unsigned long long sweeps) {
+    if (atomicAdd(&a.ctl->activations, acts) + acts > a.activation_limit)
+        atomicOr(&a.ctl->status, kStatusActivationLimit);
+    atomicAdd(&a.ctl->sweeps, sweeps);
+    return !launch_failed(a);
+}
+
 // Next item for the calling worker (one thread) as field << 32 | tile, or kInf when
 // no work is left.  The wait is bounded: kQueueSpinLimit polls, then
 // kStatusBarrier and an exit.  Each waiter polls its own slot; the shared words
@@ -113,7 +129,7 @@ __device__ __forceinline__ u64 async_pop(const RelaxArgs &a) {
         }
         if (spins % kCheck == kCheck - 1u) {
             if (*(volatile const uint32_t *)&c->count[1] == 0u) return kInf;  // nothing queued or running
-            if (*(volatile const uint32_t *)&c->status) return kInf;
+            if (launch_failed(a)) return kInf;
         }
         if (spins > kQueueSpinLimit) {
             atomicOr(&c->status, kStatusBarrier);

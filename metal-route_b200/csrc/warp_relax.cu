@@ -534,15 +534,15 @@ __device__ __forceinline__ uint32_t neighbour_price(const WTile &t, int dir, uin
 // Work counters a warp accumulates and adds to the control block in batches.
 struct WarpStats {
     uint32_t acts = 0, passes = 0, rows = 0;
+    bool leave = false;  // the launch has failed
 };
 
 __device__ __forceinline__ void flush_stats(const RelaxArgs &a, WarpStats &w) {
     if (!w.acts) return;
-    if (atomicAdd(&a.ctl->activations, (unsigned long long)w.acts) + w.acts > a.activation_limit)
-        atomicOr(&a.ctl->status, kStatusActivationLimit);
-    atomicAdd(&a.ctl->sweeps, (unsigned long long)w.passes);
+    const bool leave = !count_flush(a, w.acts, w.passes);
     atomicAdd(&a.ctl->rows, (unsigned long long)w.rows);
     w = WarpStats{};
+    w.leave = leave;
 }
 
 __device__ void warp_item(const RelaxArgs &a, uint32_t fi, uint32_t tile, WarpSmem &sm, uint32_t lane,
@@ -818,7 +818,7 @@ __global__ void __launch_bounds__(NW * 32, 4) relax_warp_kernel(RelaxArgs a) {
     WarpStats ws;
     for (;;) {
         u64 item = 0;
-        if (lane == 0) item = async_pop(a);
+        if (lane == 0) item = ws.leave ? kInf : async_pop(a);
         item = __shfl_sync(kFull, item, 0);
         if (item == kInf) break;
         warp_item(a, (uint32_t)(item >> 32), (uint32_t)item, sm, lane, ws);

@@ -183,6 +183,7 @@ def load_library(path: str = _LIB_PATH) -> C.CDLL:
                                              C.POINTER(C.c_float)]),
             "mrc_batch_destroy": (None, [vp]),
             "mrc_batch_set_schedule": (C.c_int, [vp, vp, C.c_uint32]),
+            "mrc_batch_set_activation_limit": (C.c_int, [vp, vp, C.c_uint64]),
             "mrc_context_set_schedule": (C.c_int, [vp, C.c_uint32]),
             "mrc_batch_config": (C.c_int, [vp, C.POINTER(C.c_uint32), C.POINTER(C.c_uint32),
                                            C.POINTER(C.c_uint32)]),
@@ -587,6 +588,12 @@ class Batch:
         per tile, 3 = the CTA queue with prices formed per tile."""
         e = self.engine
         e._check(e.lib.mrc_batch_set_schedule(e.ctx, self.handle, int(schedule)))
+
+    def set_activation_limit(self, limit: int) -> None:
+        """Tile activations after which a launch gives up with IterationLimit (0: the
+        library's own guard, far above any need)."""
+        e = self.engine
+        e._check(e.lib.mrc_batch_set_activation_limit(e.ctx, self.handle, int(limit)))
 
     def config(self) -> dict:
         th, nt, sc = C.c_uint32(), C.c_uint32(), C.c_uint32()
