@@ -203,7 +203,7 @@ class HostPool {
         return *pool;
     }
     // `result`: a block for results, refused (null) when too large to keep or
-    // when kLent bytes are already out, so that results a caller hoards are pageable
+    // when kLent bytes of results are already out, so that results a caller hoards are pageable
     void *alloc(size_t bytes, bool result) {
         const size_t want = Pool::size_class(bytes);
         {
@@ -212,7 +212,7 @@ class HostPool {
             auto it = free_.lower_bound(want);
             if (it != free_.end() && it->first <= 2 * want + (1u << 20)) {
                 void *p = it->second;
-                lend(p, it->first);
+                lend(p, it->first, result);
                 kept_ -= it->first;
                 free_.erase(it);
                 return p;
@@ -224,7 +224,7 @@ class HostPool {
             return nullptr;
         }
         std::lock_guard<std::mutex> lk(mu_);
-        lend(p, want);
+        lend(p, want, result);
         return p;
     }
     void release(void *p) {
@@ -233,9 +233,9 @@ class HostPool {
             std::lock_guard<std::mutex> lk(mu_);
             auto it = used_.find(p);
             if (it == used_.end()) return;
-            const size_t bytes = it->second;
+            const size_t bytes = it->second.bytes;
+            if (it->second.result) lent_ -= bytes;
             used_.erase(it);
-            lent_ -= bytes;
             if (users_ && bytes <= kBlock && kept_ + bytes <= kKept) {
                 free_.emplace(bytes, p);
                 kept_ += bytes;
@@ -260,14 +260,18 @@ class HostPool {
     }
 
    private:
-    void lend(void *p, size_t bytes) {
-        used_[p] = bytes;
-        lent_ += bytes;
+    struct Lent {
+        size_t bytes;
+        bool result;
+    };
+    void lend(void *p, size_t bytes, bool result) {
+        used_[p] = {bytes, result};
+        if (result) lent_ += bytes;
     }
     std::mutex mu_;
     std::multimap<size_t, void *> free_;
-    std::unordered_map<void *, size_t> used_;
-    size_t kept_ = 0, lent_ = 0;
+    std::unordered_map<void *, Lent> used_;
+    size_t kept_ = 0, lent_ = 0;  // bytes of free_; of results in used_
     uint32_t users_ = 0;
 };
 

@@ -77,3 +77,16 @@ try: eng.distance_fields(g, [0, 1, 2]); assert False
 except mrcuda.BackendUnavailable: pass
 assert L.fake_pending_host_writes() == 0
 """)
+
+
+def test_page_locked_boards_leave_results_page_locked(run):
+    """Only results count toward what results may hold page-locked: a program with many
+    page-locked boards still gets its fields page-locked."""
+    run("""
+held = [eng.pinned_empty((16 << 20,), np.uint32) for _ in range(9)]  # 576 MB of boards
+bt = mrcuda.Batch(board(400, 300), nets(400, 300, 8), keep_fields=True)
+bt.launch(); first = bt.finish()  # (also takes the download block)
+before = L.fake_pinned_bytes()
+bt.launch(); second = bt.finish()
+assert L.fake_pinned_bytes() - before >= second.fields[0].nbytes * 8
+""")
