@@ -221,7 +221,11 @@ class HostPool {
         void *p = nullptr;
         if (cudaHostAlloc(&p, want, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
             (void)cudaGetLastError();
-            return nullptr;
+            // once more without the blocks kept for reuse
+            if (!trim() || cudaHostAlloc(&p, want, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+                (void)cudaGetLastError();
+                return nullptr;
+            }
         }
         std::lock_guard<std::mutex> lk(mu_);
         lend(p, want, result);
@@ -249,17 +253,25 @@ class HostPool {
         ++users_;
     }
     void detach() {
-        std::multimap<size_t, void *> gone;
         {
             std::lock_guard<std::mutex> lk(mu_);
             if (--users_) return;
+        }
+        trim();
+    }
+
+   private:
+    // Frees the blocks kept for reuse; whether there were any.
+    bool trim() {
+        std::multimap<size_t, void *> gone;
+        {
+            std::lock_guard<std::mutex> lk(mu_);
             gone.swap(free_);
             kept_ = 0;
         }
         for (auto &kv : gone) cudaFreeHost(kv.second);
+        return !gone.empty();
     }
-
-   private:
     struct Lent {
         size_t bytes;
         bool result;

@@ -90,3 +90,13 @@ before = L.fake_pinned_bytes()
 bt.launch(); second = bt.finish()
 assert L.fake_pinned_bytes() - before >= second.fields[0].nbytes * 8
 """)
+
+
+def test_a_failed_page_locked_allocation_is_tried_again_without_the_kept_blocks(run):
+    run("""
+kept = eng.pinned_empty((4 << 20,), np.uint32); del kept
+before = L.fake_pinned_bytes()
+fail("cudaHostAlloc")
+big = eng.pinned_empty((16 << 20,), np.uint32)  # larger than any kept block
+assert L.fake_pinned_bytes() == before - (16 << 20) + (64 << 20)
+""")
