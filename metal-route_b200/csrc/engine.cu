@@ -166,7 +166,9 @@ struct TraceScope {
 struct HostStage {
     void *p = nullptr;
     size_t bytes = 0;
+    size_t least;                // bytes of the first block
     cudaEvent_t done = nullptr;  // the last copy out of the stage
+    explicit HostStage(size_t first) : least(first) {}
     ~HostStage() {
         if (p) cudaFreeHost(p);
         if (done) cudaEventDestroy(done);
@@ -182,9 +184,12 @@ struct HostStage {
         if (p) cudaFreeHost(p);
         p = nullptr;
         bytes = 0;
-        const size_t want = std::max(n + n / 4, (size_t)64 << 20);
+        const size_t want = std::max(n + n / 4, least);
         e = cudaHostAlloc(&p, want, cudaHostAllocMapped);
-        if (e != cudaSuccess) return e;
+        if (e != cudaSuccess) {
+            (void)cudaGetLastError();
+            return e;
+        }
         bytes = want;
         return cudaSuccess;
     }
@@ -326,8 +331,8 @@ struct mrc_context {
     cudaStream_t stream = nullptr;
     std::mutex mu;
     Pool pool;
-    HostStage stage;
-    HostStage down;  // results on their way to the caller
+    HostStage stage{64u << 20};  // boards
+    HostStage down{1u << 20};    // results on their way to the caller
     int sms = 148;
     size_t smem_optin = 0;
     // autotuned relax configuration per (layers, directed): tile height, CTA
@@ -1356,8 +1361,8 @@ mrc_status batch_collect(mrc_batch *bt, bool keep_fields, BatchOut *out) {
     mrc_context *ctx = bt->ctx;
     cudaStream_t st = bt->stream;
     const uint32_t n = (uint32_t)bt->fields.size();
-    constexpr size_t kCellsPerNet = 256;  // path cells copied before their number is known
-    const uint64_t early = std::min<uint64_t>(bt->total_cells, (uint64_t)n * kCellsPerNet);
+    // path cells copied before their number is known: 256 a net, at most 16 MB
+    const uint64_t early = std::min<uint64_t>({bt->total_cells, (uint64_t)n * 256, 4u << 20});
     const size_t heads = ((size_t)n + 1) * 8 + (size_t)n * 4, o_cells = (16 + heads + 15) & ~(size_t)15;
     MRC_CUDA(ctx->down.reserve(o_cells + early * 4), "pinned download buffer");
     const bool fields = keep_fields && bt->total_cells && bt->d_out.p;

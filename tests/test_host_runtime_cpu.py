@@ -100,3 +100,16 @@ fail("cudaHostAlloc")
 big = eng.pinned_empty((16 << 20,), np.uint32)  # larger than any kept block
 assert L.fake_pinned_bytes() == before - (16 << 20) + (64 << 20)
 """)
+
+
+def test_downloads_lock_no_more_pages_than_they_need(run):
+    """A small call locks about what it brings back; a call of very many nets no more
+    than a bound."""
+    run("""
+bt = mrcuda.Batch(board(20, 20), nets(20, 20))
+bt.launch(); bt.finish()
+assert L.fake_pinned_bytes() <= 2 << 20
+many = mrcuda.Batch(board(20, 20), nets(20, 20, 70000))
+many.launch(); many.finish()
+assert L.fake_pinned_bytes() <= 24 << 20
+""")
