@@ -216,7 +216,8 @@ mrc_status mrc_batch_finish(mrc_context *ctx, mrc_batch *batch, mrc_result **out
 /* Autotuner: time every relax configuration (tile height 8/16/32/64 cells,
  * 128 or 256 threads per CTA, and with them the CTAs per SM) on this batch,
  * keep the fastest for the batch, and cache it in the context for later batches
- * with the same layer count and price form.  Outputs may be NULL. */
+ * with the same layer count, price form and MRC_FLAG_KEEP_FIELDS.  Outputs may
+ * be NULL. */
 mrc_status mrc_batch_autotune(mrc_context *ctx, mrc_batch *batch, uint32_t *tile_h, uint32_t *threads,
                               float *best_ms);
 /* Force a relax configuration on a batch: tile height in {8, 16, 32, 64} cells
@@ -242,7 +243,7 @@ mrc_status mrc_batch_set_schedule(mrc_context *ctx, mrc_batch *batch, uint32_t s
  * of the batch and 65 536 more, far above any need.  Drops a captured graph. */
 mrc_status mrc_batch_set_activation_limit(mrc_context *ctx, mrc_batch *batch, uint64_t limit);
 /* Schedule of batches built on this context while it holds no autotuned
- * configuration for their layer count and price form: 0, 1 (the default), 2
+ * configuration for such batches (mrc_batch_autotune): 0, 1 (the default), 2
  * or 3 (see mrc_batch_set_schedule); with 2, batches with more than 16 layers
  * run 1. */
 mrc_status mrc_context_set_schedule(mrc_context *ctx, uint32_t schedule);

@@ -335,7 +335,7 @@ struct mrc_context {
     HostStage down{1u << 20};    // results on their way to the caller
     int sms = 148;
     size_t smem_optin = 0;
-    // autotuned relax configuration per (layers, directed): tile height, CTA
+    // autotuned relax configuration per tune_key: tile height, CTA
     // width, schedule (0 = bulk-synchronous rounds, 1 = asynchronous queue)
     std::map<uint32_t, std::array<uint32_t, 3>> tuned;
     uint32_t default_schedule = 1;  // for batches without a tuned configuration
@@ -928,7 +928,11 @@ mrc_status choose_tile(mrc_context *ctx, uint32_t layers, bool directed, uint32_
     return fail(MRC_ERR_LIMIT, "too many layers for one shared-memory tile");
 }
 
-uint32_t tune_key(uint32_t layers, bool directed) { return layers * 2u + (directed ? 1u : 0u); }
+// Batches that an autotuned configuration holds for: paths alone and complete fields are
+// different searches (goal-directed or not).
+uint32_t tune_key(uint32_t layers, bool directed, uint32_t flags) {
+    return layers * 4u + (directed ? 2u : 0u) + (flags & MRC_FLAG_KEEP_FIELDS ? 1u : 0u);
+}
 
 // cuTensorMapEncodeTiled, looked up once through the runtime's driver entry
 // point (the library links only the CUDA runtime).
@@ -1142,7 +1146,7 @@ mrc_status batch_build(mrc_context *ctx, std::vector<const mrc_board *> boards, 
     for (const NetCopy &nc : bt->nets) bt->has_over = bt->has_over || nc.n_over;
     uint32_t tile_h = 0, threads = kRelaxThreads;
     size_t smem = 0;
-    auto tuned = ctx->tuned.find(tune_key(bt->max_layers, bt->directed_any));
+    auto tuned = ctx->tuned.find(tune_key(bt->max_layers, bt->directed_any, flags));
     if (bt->force_tile_h) {
         tile_h = bt->force_tile_h;
         threads = bt->force_threads ? bt->force_threads : kRelaxThreads;
@@ -1951,7 +1955,7 @@ mrc_status mrc_batch_autotune(mrc_context *ctx, mrc_batch *batch, uint32_t *tile
     batch->warp = best_sched == 2;
     batch->cta_planes = best_sched != 3;
     MRC_TRY(batch_layout(batch, best_th, best_nt));
-    ctx->tuned[tune_key(layers, batch->directed_any)] = {best_th, best_nt, best_sched};
+    ctx->tuned[tune_key(layers, batch->directed_any, batch->flags)] = {best_th, best_nt, best_sched};
     if (tile_h) *tile_h = best_th;
     if (threads) *threads = best_nt;
     if (best_ms) *best_ms = best;

@@ -113,3 +113,17 @@ many = mrcuda.Batch(board(20, 20), nets(20, 20, 70000))
 many.launch(); many.finish()
 assert L.fake_pinned_bytes() <= 24 << 20
 """)
+
+
+def test_autotuned_fields_leave_path_batches_alone(run):
+    """Complete fields and paths alone are different searches: what an autotuner finds for
+    one says nothing about the other.  (The timings here make it take its last candidate.)"""
+    run("""
+b = board(128, 128, 2)
+mk = lambda keep: mrcuda.Batch(b, nets(128, 128), keep_fields=keep)
+default = mk(False).config()
+tuned = mk(True).autotune()
+assert tuned["schedule"] != default["schedule"]
+assert mk(False).config() == default
+assert mk(True).config() == {k: tuned[k] for k in default}
+""")
