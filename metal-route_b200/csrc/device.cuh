@@ -71,7 +71,7 @@ struct BoardGoal {
     uint32_t inv_min_cost;      // ~(smallest enter weight)
     u64 sum_dir, n_dir;         // of the directed prices from -x: their mean sets the first threshold
     u64 sum_cost, n_cost;
-    uint32_t wide;              // packed planes: a finite price did not fit (planes_kernel)
+    uint32_t wide;              // packed planes: a finite price did not fit a packed word (planes_kernel)
     uint32_t pad_;
 };
 

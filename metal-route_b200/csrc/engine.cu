@@ -1237,7 +1237,6 @@ PathArgs path_args(const mrc_batch *bt) {
     pa.tover = bt->has_over ? bt->d_tover.as<uint8_t>() : nullptr;
     pa.tile_h = bt->rows;
     pa.arena_filled = bt->async_q ? 1u : 0u;
-    pa.hop_bits = kLayerHopBits;
     pa.walk_smem = bt->layer && !bt->has_over ? (uint32_t)walk_smem_bytes(bt->max_layers) : 0u;
     pa.offsets = bt->d_heads.as<unsigned long long>();
     pa.costs = reinterpret_cast<uint32_t *>(pa.offsets + bt->fields.size() + 1);
@@ -1250,7 +1249,7 @@ PathArgs path_args(const mrc_batch *bt) {
 // Step-price planes of the batch's boards (and the extremes of the prices).
 mrc_status planes_enqueue(mrc_batch *bt, cudaStream_t st, uint32_t *launches) {
     MRC_CUDA(planes_launch(bt->d_boards.as<DevBoard>(), bt->d_pchunks.as<uint64_t>(), (uint32_t)bt->devs.size(),
-                           bt->n_pchunks, (uint32_t)bt->ctx->sms, bt->layer ? kLayerHopBits : 0, st),
+                           bt->n_pchunks, (uint32_t)bt->ctx->sms, bt->layer, st),
              "launch step-price planes");
     *launches += 1;
     return MRC_OK;

@@ -54,9 +54,8 @@ struct PathArgs {
     const uint32_t *tvisit;
     const uint8_t *tover;            // nullable: as RelaxArgs::tover
     uint32_t tile_h;
-    uint32_t hop_bits;               // of the packed price planes (tile-staged walk)
     uint32_t arena_filled;           // 1: the label arena was +inf-filled (queue schedule), tvisit not needed
-    uint32_t walk_smem;              // > 0: the tile-staged walk (packed planes, no overrides), its smem
+    uint32_t walk_smem;              // > 0: the tile-staged walk (the layer kernel's planes, no overrides), its smem
     uint32_t *costs;                 // [n] by output slot
     uint32_t *lens;                  // [n] by output slot
     unsigned long long *offsets;     // [n+1] by output slot
@@ -215,13 +214,13 @@ cudaError_t warp_relax_launch(const RelaxArgs &a, uint32_t grid, cudaStream_t st
 // the tile's 32 columns plus the slack of rounding its first column down to a
 // multiple of 4 (16 bytes, the TMA rule for the innermost coordinate).
 constexpr uint32_t kPlaneTmaBoxW = 36;
-// Tile-staged path walk: windows of 32 x walk_rows cells over all layers, a label
+// Tile-staged path walk: windows of 32 x walk_rows cells over all layers, a 64-bit label
 // word and a predecessor offset per cell (ring included).
 __host__ __device__ inline uint32_t walk_rows(uint32_t layers) { return layers == 1 ? 64 : layers == 2 ? 32 : 16; }
 inline size_t walk_smem_bytes(uint32_t max_layers) {
     size_t most = 0;
     for (uint32_t l = 1; l <= max_layers; ++l) {
-        const size_t s = (size_t)l * (walk_rows(l) + 2) * 34 * 6;
+        const size_t s = (size_t)l * (walk_rows(l) + 2) * 34 * 10;
         most = s > most ? s : most;
     }
     return most;
@@ -231,13 +230,13 @@ inline size_t walk_smem_bytes(uint32_t max_layers) {
 __host__ __device__ inline uint32_t planes_pitch(uint32_t w) { return (w + 3u) & ~3u; }
 // Step-price planes of every board of a batch (DevBoard::planes, 6 x cells u32
 // each); chunk_start[k] = first chunk of board k (prefix sum of planes_chunks).
-// hop_bits: 0 = plain prices (the warp schedule), else packed for the layer
-// kernel: (price << hop_bits) | 1, kPackedInf for no step; a board with a finite
-// price that does not fit is marked (BoardGoal::wide).
+// packed: the layer kernel's words (plane_word), kPackedInf for no step; a board with a
+// finite price that does not fit a packed word is marked (BoardGoal::wide).  Else plain
+// prices (the warp schedule).
 constexpr uint32_t kPackedInf = 1u << 30;
 uint64_t planes_chunks(uint32_t w, uint32_t h, uint32_t layers);
 cudaError_t planes_launch(const DevBoard *boards, const uint64_t *chunk_start, uint32_t n_boards, uint64_t n_chunks,
-                          uint32_t sms, uint32_t hop_bits, cudaStream_t st);
+                          uint32_t sms, bool packed, cudaStream_t st);
 
 // Shared memory of one tile of 32 x tile_h cells over `layers` (tile_h in {8, 16, 32, 64}) with 64-bit labels
 // and prices formed per tile.

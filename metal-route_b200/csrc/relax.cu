@@ -706,21 +706,19 @@ cudaError_t relax_launch(const RelaxArgs &a, uint32_t grid, uint32_t threads, si
     return cudaLaunchKernelExC(&cfg, fn, args);
 }
 
-// Tile-staged walk, for batches whose boards carry packed price planes (the layer
-// kernel) and whose nets carry no price overrides.  One CTA per field.  The CTA
-// stages the labels of a window of 32 x walk_rows(L) cells over all layers, with a
-// one-cell ring, relative to the current cell (D, H): word = (D - dist) << HB |
-// (H - hops), so q is a predecessor of c by a step with packed price p exactly
-// when word(q) == word(c) + p.  All threads then look for the canonical (lowest
-// CellIdx) predecessor of every cell of the window, reading a price only where a
-// neighbour's label is lower, and keep it as the offset to that neighbour in
-// shared memory; the walk itself is one thread following offsets, a shared-memory
-// load a step, until it leaves the window.  Cells priced for the net itself (own
-// pads, via pads) are looked up with exact prices, and a step that no word
-// describes (too large a price, a board of wide prices) is taken from HBM.  A cell
-// that a neighbour further back than a word holds could precede gets no offset: of
-// two predecessors the one of lower CellIdx may be the one that has no word, and
-// the next window, which starts at the cell, has words for both.
+// Tile-staged walk, for batches of the layer kernel whose nets carry no price
+// overrides.  One CTA per field.  The CTA stages the labels of a window of 32 x
+// walk_rows(L) cells over all layers, with a one-cell ring, relative to the current
+// cell (D, H): word = (D - dist) << kLayerHopBits | (H - hops), so q is a predecessor of c
+// by a step of price word p exactly when word(q) == word(c) + p.  All threads then look
+// for the canonical (lowest CellIdx) predecessor of every cell of the window, reading a
+// price only where a neighbour's label is lower, and keep it as the offset to that
+// neighbour in shared memory; the walk itself is one thread following offsets, a
+// shared-memory load a step, until it leaves the window.  A window with a cell that may
+// be on the path and is further back than a word holds (large prices) is staged once
+// more, and the rest of the path after it, in words of 64 bits.  Cells priced for the
+// net itself (own pads, via pads) are looked up with exact prices; a step from more of
+// them than the list holds is taken from HBM.
 //
 // Bound by a window's two round trips to HBM (labels, prices), some 3 us, and the
 // number of windows; a step inside one costs about 50 cycles.  Testing the six
@@ -754,7 +752,39 @@ constexpr int kWalkThreads = 512;
 constexpr uint32_t kWalkSteps = 512;     // steps recorded per window
 constexpr uint32_t kWalkUnroll = 8;      // steps taken between two looks at whether the walk goes on
 constexpr uint32_t kWalkSpec = 256;      // cells of a window priced for the net itself
-constexpr uint32_t kWalkFar = kMax - 1;  // word of a cell that may be on the path, further back than a word holds
+
+// Words of a window's labels.  Of a cell that is not on the path: kNone, from which, and to
+// which, no step leads.
+struct WalkWord {  // 32 bits; only for windows all of whose cells are in range
+    using type = uint32_t;
+    static constexpr uint32_t kNone = kMax, kHops = (1u << kLayerHopBits) - 1u;
+    static __device__ __forceinline__ bool in(uint32_t dist, uint32_t hops) {
+        return dist < (1u << (29 - kLayerHopBits)) && hops <= kHops;
+    }
+    static __device__ __forceinline__ type make(uint32_t dist, uint32_t hops) { return (dist << kLayerHopBits) | hops; }
+    static __device__ __forceinline__ type none() { return kNone; }
+    static __device__ __forceinline__ uint32_t dist(type w) { return w >> kLayerHopBits; }
+    static __device__ __forceinline__ uint32_t hops(type w) { return w & kHops; }
+    static __device__ __forceinline__ bool is(type w) { return w != kNone; }
+    // may q precede c, by a step of some price
+    static __device__ __forceinline__ bool asks(type c, type q) { return q != kNone && q > c; }
+    // does it, by a step of price word p (one that does costs less than a plain price)
+    static __device__ __forceinline__ bool by(type c, type q, uint32_t p) { return q == c + p && p < kPackedInf; }
+};
+struct WalkWide {  // 64 bits
+    using type = uint2;  // hops, dist
+    static __device__ __forceinline__ bool in(uint32_t, uint32_t) { return true; }
+    static __device__ __forceinline__ type make(uint32_t dist, uint32_t hops) { return make_uint2(hops, dist); }
+    static __device__ __forceinline__ type none() { return make_uint2(kMax, 0u); }
+    static __device__ __forceinline__ uint32_t dist(type w) { return w.y; }
+    static __device__ __forceinline__ uint32_t hops(type w) { return w.x; }
+    static __device__ __forceinline__ bool is(type w) { return w.x != kMax; }
+    static __device__ __forceinline__ bool asks(type c, type q) { return q.x == c.x + 1u && q.y >= c.y; }
+    static __device__ __forceinline__ bool by(type c, type q, uint32_t p) {
+        const uint32_t want = q.y - c.y;
+        return p == (want < (1u << (29 - kLayerHopBits)) ? (want << kLayerHopBits) | 1u : want | kPricePlain);
+    }
+};
 
 __global__ void __launch_bounds__(kWalkThreads, 2) path_walk_tiled_kernel(PathArgs a) {
     extern __shared__ __align__(16) unsigned char wsm[];
@@ -766,15 +796,12 @@ __global__ void __launch_bounds__(kWalkThreads, 2) path_walk_tiled_kernel(PathAr
     if (len == 0) return;  // the same for the whole CTA
     const DevBoard b = a.boards[f.board];
     const uint32_t L = b.layers, WH = walk_rows(L), W = kTW, PW = W + 2, PL = (WH + 2) * PW;  // ring included
-    const uint32_t HB = a.hop_bits, hop_mask = (1u << HB) - 1u, dist_lim = 1u << (29 - HB);
     const uint32_t plane = b.w * b.h, tid = threadIdx.x, lane = tid & 31;
-    uint32_t *word = reinterpret_cast<uint32_t *>(wsm);
-    int16_t *delta = reinterpret_cast<int16_t *>(word + L * PL);
     const int wx0 = (int)f.x0, wy0 = (int)f.y0, wx1 = (int)(f.x0 + f.ww), wy1 = (int)(f.y0 + f.wh);
     const u64 *lab = a.lab + f.lab_off;
     const uint32_t wp = planes_pitch(b.w);
     const uint64_t NP = (uint64_t)wp * b.h * L;
-    const bool wide = b.goal->wide != 0;
+    bool wide = b.goal->wide != 0;  // windows in 64-bit words
     uint32_t *out = a.cells + a.offsets[f.out];
     const uint32_t src_xy = f.src % plane;
     const int sx = (int)(src_xy % b.w), sy = (int)(src_xy / b.w);  // the walk heads for the source
@@ -795,10 +822,15 @@ __global__ void __launch_bounds__(kWalkThreads, 2) path_walk_tiled_kernel(PathAr
     int dx = walk_dir(cx, sx), dy = walk_dir(cy, sy);
     while (pos) {
         const int tx0 = walk_origin(cx, dx, (int)W), ty0 = walk_origin(cy, dy, (int)WH);
-        const uint32_t D = (uint32_t)(need >> 32), H = (uint32_t)need;
-        __syncthreads();  // every thread is past the previous window
-        if (!wide) {
-            bool far = false;  // a word kWalkFar was set
+        // Stages the window, looks up its predecessors and walks as far as it goes; false:
+        // a cell is out of the words' range.
+        auto window = [&](auto words) -> bool {
+            using Q = decltype(words);
+            const uint32_t D = (uint32_t)(need >> 32), H = (uint32_t)need;
+            auto *word = reinterpret_cast<typename Q::type *>(wsm);
+            int16_t *delta = reinterpret_cast<int16_t *>(word + L * PL);
+            bool far = false;
+            __syncthreads();  // every thread is past the previous window
             // ---- labels of the window and its ring: a warp per row, several rows in flight
             // word of the cell in column xx, row yy (ring included) of layer l, from its label
             auto put = [&](uint32_t i, u64 v, int gx, int gy, int l) {
@@ -806,8 +838,9 @@ __global__ void __launch_bounds__(kWalkThreads, 2) path_walk_tiled_kernel(PathAr
                 // at least their distance in cells
                 const uint32_t d = (uint32_t)(v >> 32), h = (uint32_t)v;
                 const uint32_t away = (uint32_t)(abs(gx - cx) + abs(gy - cy) + abs(l - cl));
-                const bool can = d <= D && h <= H && H - h >= away, in = D - d < dist_lim && H - h <= hop_mask;
-                word[i] = !can ? kMax : in ? ((D - d) << HB) | (H - h) : kWalkFar;
+                const bool can = d <= D && h <= H && H - h >= away;
+                const bool in = Q::in(D - d, H - h);
+                word[i] = can && in ? Q::make(D - d, H - h) : Q::none();
                 far |= can && !in;
                 delta[i] = 0;
             };
@@ -853,26 +886,27 @@ __global__ void __launch_bounds__(kWalkThreads, 2) path_walk_tiled_kernel(PathAr
                     s_code[i] = 7;
                 }
             }
-            const bool any_far = __syncthreads_or(far);
+            if (__syncthreads_or(far)) {
+                if (tid == 0) s_nspec = 0;
+                return false;
+            }
             // ---- the predecessor of every cell: neighbours in ascending CellIdx ----
             const int off[6] = {-(int)PL, -(int)PW, -1, 1, (int)PW, (int)PL};
             constexpr uint32_t in_plane[6] = {kInBelow, kInNegY, kInNegX, kInPosX, kInPosY, kInAbove};
             constexpr uint32_t kCells = 4;  // cells of one thread whose prices are in flight together
             for (uint32_t r0 = wid; r0 < L * WH; r0 += kCells * nw) {
-                uint32_t p[kCells][6];
+                uint32_t p[kCells][6], most = 0;
 #pragma unroll
                 for (uint32_t k = 0; k < kCells; ++k) {
                     const uint32_t q = r0 + k * nw, l = q / WH, yy = q % WH;
                     const uint32_t at = l * PL + (yy + 1) * PW + lane + 1;
-                    const bool have = q < L * WH && word[at] < kWalkFar;
-                    const uint32_t wc = have ? word[at] : 0u;
+                    const auto wc = q < L * WH ? word[at] : Q::none();
                     const uint32_t *pr = b.planes + ((uint64_t)l * b.h + (uint32_t)(ty0 + (int)yy)) * wp + (uint32_t)(tx0 + (int)lane);
 #pragma unroll
                     for (int n = 0; n < 6; ++n) {
                         p[k][n] = kPackedInf;
-                        if (!have || (n == 0 && l == 0) || (n == 5 && l + 1 == L)) continue;
-                        const uint32_t wq = word[(int)at + off[n]];
-                        if (wq < kWalkFar && wq > wc) p[k][n] = __ldg(pr + in_plane[n] * NP);
+                        if (!Q::is(wc) || (n == 0 && l == 0) || (n == 5 && l + 1 == L)) continue;
+                        if (Q::asks(wc, word[(int)at + off[n]])) p[k][n] = __ldg(pr + in_plane[n] * NP);
                     }
                 }
 #pragma unroll
@@ -880,25 +914,38 @@ __global__ void __launch_bounds__(kWalkThreads, 2) path_walk_tiled_kernel(PathAr
                     const uint32_t q = r0 + k * nw, l = q / WH, yy = q % WH;
                     const uint32_t at = l * PL + (yy + 1) * PW + lane + 1;
                     if (q >= L * WH) continue;
-                    const uint32_t wc = word[at];
+                    const auto wc = word[at];
                     int dl = 0;
 #pragma unroll
-                    for (int n = 5; n >= 0; --n)  // a price was read only where the neighbour has a word
-                        if (p[k][n] < kPackedInf && word[(int)at + off[n]] == wc + p[k][n]) dl = off[n];
+                    for (int n = 5; n >= 0; --n) {
+                        if (p[k][n] == kPackedInf) continue;  // (a price was read only where one is asked for)
+                        if (Q::by(wc, word[(int)at + off[n]], p[k][n])) dl = off[n];
+                        most = max(most, p[k][n]);
+                    }
                     if (dl) delta[at] = (int16_t)dl;
                 }
-            }
-            if (any_far) {  // no offset where such a neighbour may be the predecessor as well
-                for (uint32_t i = tid; i < L * WH * W; i += blockDim.x) {  // (the cells this thread wrote)
-                    const uint32_t xx = i % W, q = i / W, l = q / WH, yy = q - l * WH, at = l * PL + (yy + 1) * PW + xx + 1;
-                    const uint32_t wc = word[at];
-                    if (!delta[at]) continue;
-                    const uint32_t *pr = b.planes + ((uint64_t)l * b.h + (uint32_t)(ty0 + (int)yy)) * wp + (uint32_t)(tx0 + (int)xx);
-                    for (int n = 0; n < 6; ++n) {
-                        if ((n == 0 && l == 0) || (n == 5 && l + 1 == L) || word[(int)at + off[n]] != kWalkFar) continue;
-                        const uint32_t p = __ldg(pr + in_plane[n] * NP);
-                        if (p < kPackedInf && (((wc + p) >> HB) >= dist_lim || (wc & hop_mask) == hop_mask)) delta[at] = 0;
+                if (sizeof(typename Q::type) == 4 || most != kPriceLook) continue;
+                // prices that no word holds: formed from the board's words
+#pragma unroll 1
+                for (uint32_t k = 0; k < kCells; ++k) {
+                    const uint32_t q = r0 + k * nw, l = q / WH, yy = q % WH;
+                    const uint32_t at = l * PL + (yy + 1) * PW + lane + 1;
+                    if (q >= L * WH) continue;
+                    const auto wc = word[at];
+                    int dl = 0;
+#pragma unroll 1
+                    for (int n = 5; n >= 0; --n) {
+                        const int o = n == 0 ? -(int)PL : n == 1 ? -(int)PW : n == 2 ? -1 : n == 3 ? 1 : n == 4 ? (int)PW : (int)PL;
+                        if (!Q::is(wc) || (n == 0 && l == 0) || (n == 5 && l + 1 == L) || !Q::asks(wc, word[(int)at + o])) continue;
+                        int px = tx0 + (int)lane, py = ty0 + (int)yy, pz = (int)l;
+                        const uint32_t gx = (uint32_t)px, gy = (uint32_t)py;
+                        walk_offset(n, px, py, pz);
+                        if (walk_step_exact(a.boards + f.board, a.fields + blockIdx.x, a.pads,
+                                            ((uint32_t)pz * b.h + (uint32_t)py) * b.w + (uint32_t)px,
+                                            (l * b.h + gy) * b.w + gx, gx, gy, l, n) == Q::dist(word[(int)at + o]) - Q::dist(wc))
+                            dl = o;
                     }
+                    delta[at] = (int16_t)dl;
                 }
             }
             if (s_nspec) {  // the same for the whole CTA
@@ -908,21 +955,19 @@ __global__ void __launch_bounds__(kWalkThreads, 2) path_walk_tiled_kernel(PathAr
                     const uint32_t e = i / 6, at = s_spec[e];
                     const int kind = (int)(i % 6);
                     const uint32_t l = at / PL, q = at - l * PL, yy = q / PW, xx = q - yy * PW;
-                    const uint32_t wc = word[at];
-                    if (wc >= kWalkFar || (kind == 0 && l == 0) || (kind == 5 && l + 1 == L)) continue;
+                    const auto wc = word[at];
+                    if (!Q::is(wc) || (kind == 0 && l == 0) || (kind == 5 && l + 1 == L)) continue;
                     int px = tx0 + (int)xx - 1, py = ty0 + (int)yy - 1, pz = (int)l;
                     const uint32_t gx = (uint32_t)px, gy = (uint32_t)py;
                     const int off = kind == 0 ? -(int)PL : kind == 1 ? -(int)PW : kind == 2 ? -1 : kind == 3 ? 1
                                   : kind == 4 ? (int)PW : (int)PL;
-                    const uint32_t wq = word[(int)at + off];
-                    if (wq == kMax) continue;
+                    const auto wq = word[(int)at + off];
+                    if (!Q::asks(wc, wq) || Q::hops(wq) != Q::hops(wc) + 1u) continue;
                     walk_offset(kind, px, py, pz);
                     const uint32_t st = walk_step_exact(a.boards + f.board, a.fields + blockIdx.x, a.pads,
                                                         ((uint32_t)pz * b.h + (uint32_t)py) * b.w + (uint32_t)px,
                                                         (l * b.h + gy) * b.w + gx, gx, gy, l, kind);
-                    if (st < dist_lim && wq == wc + ((st << HB) | 1u)) atomicMin(&s_code[e], (uint32_t)kind + 1u);
-                    if (wq == kWalkFar && st != kMax && (dsum(st, wc >> HB) >= dist_lim || (wc & hop_mask) == hop_mask))
-                        atomicMin(&s_code[e], 0u);  // it may be the predecessor: no offset (no kind is below it)
+                    if (st == Q::dist(wq) - Q::dist(wc)) atomicMin(&s_code[e], (uint32_t)kind + 1u);
                 }
                 __syncthreads();
                 for (uint32_t e = tid; e < ns; e += blockDim.x) {
@@ -959,20 +1004,25 @@ __global__ void __launch_bounds__(kWalkThreads, 2) path_walk_tiled_kernel(PathAr
                 s_nspec = 0;  // for the next window
             }
             __syncthreads();
-        }
-        const uint32_t n = s_n;
-        if (n) {
-            for (uint32_t k = tid; k < n; k += blockDim.x) {
-                const uint32_t at = s_path[k], l = at / PL, q = at - l * PL, yy = q / PW, xx = q - yy * PW;
-                out[pos - 1 - k] = (l * b.h + (uint32_t)(ty0 + (int)yy - 1)) * b.w + (uint32_t)(tx0 + (int)xx - 1);
+            const uint32_t n = s_n;
+            if (n) {
+                for (uint32_t k = tid; k < n; k += blockDim.x) {
+                    const uint32_t at = s_path[k], l = at / PL, q = at - l * PL, yy = q / PW, xx = q - yy * PW;
+                    out[pos - 1 - k] = (l * b.h + (uint32_t)(ty0 + (int)yy - 1)) * b.w + (uint32_t)(tx0 + (int)xx - 1);
+                }
+                const uint32_t at = s_path[n - 1], l = at / PL, q = at - l * PL, yy = q / PW, xx = q - yy * PW;
+                const auto w = word[at];
+                cx = tx0 + (int)xx - 1;
+                cy = ty0 + (int)yy - 1;
+                cl = (int)l;
+                need = ((u64)(D - Q::dist(w)) << 32) | (H - Q::hops(w));
+                pos -= n;
             }
-            const uint32_t at = s_path[n - 1], l = at / PL, q = at - l * PL, yy = q / PW, xx = q - yy * PW, w = word[at];
-            cx = tx0 + (int)xx - 1;
-            cy = ty0 + (int)yy - 1;
-            cl = (int)l;
-            need = ((u64)(D - (w >> HB)) << 32) | (H - (w & hop_mask));
-            pos -= n;
-        } else {
+            return true;
+        };
+        if (!wide) wide = !window(WalkWord{});
+        if (wide) window(WalkWide{});
+        if (s_n == 0) {
             // one step from HBM with exact prices
             if (tid < 32) {
                 bool ok = false;

@@ -29,6 +29,16 @@ __device__ __forceinline__ uint32_t dsum(uint32_t a, uint32_t b) {
     return s < a ? kMax : s;
 }
 
+// The word of a step price in the layer kernel's planes, exact for every price below
+// 2^31 - 1: price << kLayerHopBits | 1 where that stays below 2^29 (a packed word),
+// else the price itself with the top bit set; kPackedInf for no step, kPriceLook for a
+// price to be formed from the board's words.
+constexpr uint32_t kPriceLook = 0xFFFFFFFFu, kPricePlain = 1u << 31;
+__device__ __forceinline__ uint32_t plane_word(uint32_t p) {
+    if (p < (1u << (29 - kLayerHopBits))) return (p << kLayerHopBits) | 1u;
+    return p == kMax ? kPackedInf : p < kPriceLook - kPricePlain ? kPricePlain | p : kPriceLook;
+}
+
 __device__ __forceinline__ u64 umin64(u64 a, u64 b) { return a < b ? a : b; }
 
 // Work queue of the queue forms.  count[0] = tickets handed to pushers (tail),

@@ -70,7 +70,7 @@ __device__ __forceinline__ uint32_t flags4(const uint8_t *p, bool aligned, uint3
 // 256 uneven boards (363 MB of planes, 303 -> 244 us) three blocks an SM of 80
 // registers measured best (two of 126: 271 us).
 __global__ void __launch_bounds__(256, 3) planes_kernel(const DevBoard *boards, const uint64_t *chunk_start,
-                                                     uint32_t n_boards, uint64_t n_chunks, uint32_t hop_bits) {
+                                                     uint32_t n_boards, uint64_t n_chunks, bool packed) {
     __shared__ uint32_t s_u[8][4];
     __shared__ u64 s_s[8][2];
     const uint64_t ch0 = n_chunks * blockIdx.x / gridDim.x, ch1 = n_chunks * (blockIdx.x + 1) / gridDim.x;
@@ -191,17 +191,11 @@ __global__ void __launch_bounds__(256, 3) planes_kernel(const DevBoard *boards, 
             const uint64_t o = (uint64_t)row * wp + x0;
 #pragma unroll
             for (int p = 0; p < 6; ++p) {
-                if (hop_bits) {  // the layer kernel's words
+                if (packed) {  // the layer kernel's words
 #pragma unroll
                     for (uint32_t k = 0; k < 4; ++k) {
-                        uint32_t v = s[p][k];
-                        if (v < (1u << (29 - hop_bits))) {
-                            v = (v << hop_bits) | 1u;
-                        } else {
-                            if (v != kMax) b.goal->wide = 1;
-                            v = kPackedInf;
-                        }
-                        s[p][k] = v;
+                        s[p][k] = plane_word(s[p][k]);
+                        if (s[p][k] >= kPricePlain) b.goal->wide = 1;
                     }
                 }
                 *reinterpret_cast<uint4 *>(out + (uint64_t)p * NP + o) = make_uint4(s[p][0], s[p][1], s[p][2], s[p][3]);
@@ -854,10 +848,10 @@ uint64_t planes_chunks(uint32_t w, uint32_t h, uint32_t layers) {
 }
 
 cudaError_t planes_launch(const DevBoard *boards, const uint64_t *chunk_start, uint32_t n_boards, uint64_t n_chunks,
-                          uint32_t sms, uint32_t hop_bits, cudaStream_t st) {
+                          uint32_t sms, bool packed, cudaStream_t st) {
     if (!n_boards || !n_chunks) return cudaSuccess;
     const uint64_t blocks = std::min<uint64_t>(n_chunks, (uint64_t)sms * 8);
-    planes_kernel<<<(uint32_t)blocks, 256, 0, st>>>(boards, chunk_start, n_boards, n_chunks, hop_bits);
+    planes_kernel<<<(uint32_t)blocks, 256, 0, st>>>(boards, chunk_start, n_boards, n_chunks, packed);
     return cudaGetLastError();
 }
 

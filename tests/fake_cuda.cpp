@@ -181,7 +181,7 @@ uint32_t warp_relax_threads() { return 128; }
 cudaError_t warp_relax_occupancy(int *n) { return *n = 1, cudaSuccess; }
 cudaError_t warp_relax_launch(const RelaxArgs &, uint32_t, cudaStream_t) { return cudaSuccess; }
 uint64_t planes_chunks(uint32_t, uint32_t, uint32_t) { return 1; }
-cudaError_t planes_launch(const DevBoard *, const uint64_t *, uint32_t, uint64_t, uint32_t, uint32_t, cudaStream_t) {
+cudaError_t planes_launch(const DevBoard *, const uint64_t *, uint32_t, uint64_t, uint32_t, bool, cudaStream_t) {
     return cudaSuccess;
 }
 size_t relax_smem_bytes(uint32_t layers, uint32_t tile_h, bool) { return (size_t)layers * tile_h * 1088; }
