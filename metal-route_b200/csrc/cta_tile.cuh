@@ -878,12 +878,12 @@ __device__ __forceinline__ bool process_item(const RelaxArgs &a, uint32_t fi, ui
                 if constexpr (ASYNC) {
                     // the work counters are per CTA (s_cnt), added to the launch's
                     // every kCountBatch activations and when the CTA exits, so this
-                    // thread makes no round trip to L2 here (s_cnt[2]: the CTA leaves
-                    // a failed launch after this item)
+                    // thread makes no round trip to L2 here (kLeaveLaunch: the CTA
+                    // leaves a failed launch after this item)
                     s_cnt[1] += sweep;
                     if (++s_cnt[0] == kCountBatch) {
-                        if (!count_flush(a, s_cnt[0], s_cnt[1])) s_cnt[2] = 1;
-                        s_cnt[0] = s_cnt[1] = 0;
+                        s_cnt[0] = count_flush(a, s_cnt[0], s_cnt[1]) ? 0 : kLeaveLaunch;
+                        s_cnt[1] = 0;
                     }
                 } else {
                     if (!s_vis[0]) atomicExch(a.tvisit + f.tile_off + t, 1u);

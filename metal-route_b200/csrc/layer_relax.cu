@@ -59,7 +59,7 @@ __host__ __device__ inline size_t layer_st_off(uint32_t L, uint32_t TH) {
 struct LayerShared {
     u64 item;
     uint64_t mbar;  // completion of the price-plane TMA loads
-    unsigned long long cnt[3];  // activations and sweeps not yet added to the launch's; the CTA leaves
+    unsigned long long cnt[2];  // activations and sweeps not yet added to the launch's
     uint32_t n_spec, near_pad, wide, dmin, hmin, hmax, ub, thr, more;
     uint32_t push;              // bits: left, right, top, bottom improved
     uint32_t park[4];           // GD: the smallest f that waits to enter each
@@ -339,14 +339,14 @@ __device__ __forceinline__ bool layer_item(const RelaxArgs &a, uint32_t fi, uint
                 if (spins == kTmaSpinLimit) {
                     if (tid == 0) atomicOr(&a.ctl->status, kStatusQueueOverflow);
                 } else if (spins > 2 * kTmaSpinLimit) {
-                    *(volatile unsigned long long *)&sh.cnt[2] = 1;
+                    *(volatile unsigned long long *)&sh.cnt[0] = kLeaveLaunch;
                     bad = true;
                     break;
                 }
             }
             ++phase;
             if (board_wide) {
-                if (__syncthreads_or(bad && *(volatile unsigned long long *)&sh.cnt[2])) return false;
+                if (__syncthreads_or(bad && *(volatile unsigned long long *)&sh.cnt[0] == kLeaveLaunch)) return false;
                 // everybody is past the load and the staged words
                 return wide_item<TH, OV, GD>(a, fi, t, smem_raw, sh.cnt);
             }
@@ -565,7 +565,7 @@ __device__ __forceinline__ bool layer_item(const RelaxArgs &a, uint32_t fi, uint
             bad |= over < kNarrow || hops == kHopMask;
         }
         if (__syncthreads_or(bad || *(volatile uint32_t *)&sh.wide)) {
-            if (*(volatile unsigned long long *)&sh.cnt[2]) return false;  // without its prices
+            if (*(volatile unsigned long long *)&sh.cnt[0] == kLeaveLaunch) return false;  // without its prices
             return wide_item<TH, OV, GD>(a, fi, t, smem_raw, sh.cnt);
         }
         if constexpr (GD) ub = *(volatile uint32_t *)&sh.ub;
@@ -690,8 +690,8 @@ __device__ __forceinline__ bool layer_item(const RelaxArgs &a, uint32_t fi, uint
                 sh.hmax = 0;
                 sh.cnt[1] += sweep;
                 if (++sh.cnt[0] == kCountBatch) {
-                    if (!count_flush(a, sh.cnt[0], sh.cnt[1])) sh.cnt[2] = 1;
-                    sh.cnt[0] = sh.cnt[1] = 0;
+                    sh.cnt[0] = count_flush(a, sh.cnt[0], sh.cnt[1]) ? 0 : kLeaveLaunch;
+                    sh.cnt[1] = 0;
                 }
             }
             __syncwarp();
@@ -803,14 +803,14 @@ __global__ void __launch_bounds__(LM * 32, LM == 4 ? (TH == 8 ? 5 : 3) : LM == 8
     uint32_t phase = 0, fi = 0;
     bool last = false;
     if (threadIdx.x == 0) {
-        sh.cnt[0] = sh.cnt[1] = sh.cnt[2] = 0;
+        sh.cnt[0] = sh.cnt[1] = 0;
         mbar_init(&sh.mbar, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
     for (;;) {
         if (threadIdx.x == 0) {
-            sh.item = sh.cnt[2] ? kInf : last ? kReleaseField : async_pop<64>(a);
+            sh.item = sh.cnt[0] == kLeaveLaunch ? kInf : last ? kReleaseField : async_pop<64>(a);
             sh.n_spec = sh.near_pad = sh.wide = 0;
             sh.dmin = sh.hmin = kMax;
             sh.hmax = 0;
@@ -834,7 +834,7 @@ __global__ void __launch_bounds__(LM * 32, LM == 4 ? (TH == 8 ? 5 : 3) : LM == 8
         __syncthreads();
     }
     if (threadIdx.x == 0) {
-        if (sh.cnt[0]) atomicAdd(&a.ctl->activations, sh.cnt[0]);
+        if (sh.cnt[0] && sh.cnt[0] != kLeaveLaunch) atomicAdd(&a.ctl->activations, sh.cnt[0]);
         if (sh.cnt[1]) atomicAdd(&a.ctl->sweeps, sh.cnt[1]);
     }
 }

@@ -129,18 +129,18 @@ template <int TH, int NT, bool OV>
 __global__ void __launch_bounds__(NT, 65536 / (NT * 64)) relax_async_kernel(RelaxArgs a) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ u64 s_item;
-    __shared__ unsigned long long s_cnt[3];  // activations and sweeps not yet added to the launch's; leave
-    if (threadIdx.x == 0) s_cnt[0] = s_cnt[1] = s_cnt[2] = 0;
+    __shared__ unsigned long long s_cnt[2];  // activations and sweeps not yet added to the launch's
+    if (threadIdx.x == 0) s_cnt[0] = s_cnt[1] = 0;
     __syncthreads();
     for (;;) {
-        if (threadIdx.x == 0) s_item = s_cnt[2] ? kInf : async_pop(a);
+        if (threadIdx.x == 0) s_item = s_cnt[0] == kLeaveLaunch ? kInf : async_pop(a);
         __syncthreads();
         const u64 item = s_item;
         if (item == kInf) break;
         process_item<TH, true, OV, false>(a, (uint32_t)(item >> 32), (uint32_t)item, 0, smem_raw, s_cnt);
     }
     if (threadIdx.x == 0) {
-        if (s_cnt[0]) atomicAdd(&a.ctl->activations, s_cnt[0]);
+        if (s_cnt[0] && s_cnt[0] != kLeaveLaunch) atomicAdd(&a.ctl->activations, s_cnt[0]);
         if (s_cnt[1]) atomicAdd(&a.ctl->sweeps, s_cnt[1]);
     }
 }

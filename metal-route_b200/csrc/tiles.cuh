@@ -107,6 +107,9 @@ __device__ __forceinline__ bool launch_failed(const RelaxArgs &a) {
     return *(volatile const uint32_t *)&a.ctl->status != 0u;
 }
 
+// A CTA's count of activations not yet added to the launch's, once it is to leave.
+constexpr unsigned long long kLeaveLaunch = ~0ull;
+
 // Adds a worker's activations and sweeps to the launch's.  False: the launch has
 // failed, by too many activations or otherwise, and the worker leaves it.  A
 // queue that never runs dry keeps its workers from waiting, and so from reading the
