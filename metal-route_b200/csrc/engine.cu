@@ -492,6 +492,7 @@ struct mrc_board {
     std::vector<uint8_t> board;    // host copy of the board mask (may be empty)
     std::vector<uint8_t> viaf;     // host copy of the static via mask (may be empty)
     bool directed = false;
+    uint64_t spread = 0;           // of the labels of a tile, estimated (label_spread)
     DBuf d_cost, d_flags, d_edges, d_dir;
     DevBoard dev{};
 };
@@ -549,6 +550,31 @@ void view_edges(const uint32_t *base, uint32_t w, uint32_t h, uint32_t layers, D
     dev->x_sum = base + o.x_sum;
     dev->y_sum = base + o.y_sum;
     dev->via_sum = base + o.via_sum;
+}
+
+// About how far the labels of a tile and its border lie apart: 52 steps (a 32 x 16 tile
+// from corner to corner, border included) between the cheapest and the mean price,
+// and a via.  Gap prices and vias as they are, weights and directed prices from up to
+// `samples` cells of each.
+uint64_t label_spread(const GridView &g, const mrc_edges &e, uint64_t samples) {
+    auto middle = [](const uint32_t *v, uint64_t n, uint64_t most) -> uint64_t {  // of the least and the mean
+        uint64_t sum = 0, k = 0, least = kMax;
+        const uint64_t step = std::max<uint64_t>(n / std::max<uint64_t>(most, 1), 1) | 1;  // (odd: all slots of directed prices)
+        for (uint64_t i = 0; i < n; i += step) {
+            if (v[i] == kMax) continue;
+            sum += v[i];
+            least = std::min<uint64_t>(least, v[i]);
+            ++k;
+        }
+        return k ? (sum / k + least) / 2 : 0;
+    };
+    uint64_t gap, via = 0;
+    if (e.directed_in_costs) gap = middle(e.directed_in_costs, g.n * 4, samples);
+    else gap = std::max(middle(e.x_edge_costs, e.n_x_edge_costs, ~0ull), middle(e.y_edge_costs, e.n_y_edge_costs, ~0ull));
+    for (uint32_t k = 0; k < e.n_via_edge_costs; ++k)
+        if (e.via_allowed[k]) via = std::max<uint64_t>(via, e.via_edge_costs[k]);
+    const uint64_t weight = middle(g.cost, g.n, samples);
+    return std::min<uint64_t>(std::max<uint64_t>(weight, 1), kMax) * std::min<uint64_t>(52 * gap + via, 1ull << 31);
 }
 
 // The device-readable address of page-locked, mapped host memory; null for
@@ -618,6 +644,7 @@ mrc_status board_build(mrc_context *ctx, const mrc_grid *grid, const mrc_edges *
             MRC_CUDA(cudaStreamSynchronize(ctx->stream), "combine masks");
         }
     }
+    b->spread = label_spread(g, *edges, 256);
     std::vector<uint32_t> words(EdgeWords(g.w, g.h, g.layers).total, 0);
     fill_edges(*edges, g.w, g.h, g.layers, words.data(), &b->dev);
     MRC_TRY(upload(ctx, b->d_edges, words.data(), words.size() * 4, "upload edge prices"));
@@ -749,6 +776,7 @@ mrc_status board_pack_build(mrc_context *ctx, const mrc_isolated_request *inst, 
             return fail(MRC_ERR_INVALID_ARGUMENT, "instance " + std::to_string(k) + ": edge price pointer is NULL");
         b->ctx = ctx;
         b->directed = e.directed_in_costs != nullptr;
+        b->spread = label_spread(g, e, std::max(4u, 512u / n));
         Off &o = offs[k];
         o.cost = take(g.n * 4);
         o.flags = (g.board || g.via_forbidden) ? take(g.n) : SIZE_MAX;
@@ -864,10 +892,10 @@ struct mrc_batch {
     DBuf d_boards, d_fields, d_pads, d_lists, d_lens, d_heads, d_cells, d_out;
     // What a launch starts from, in two blocks so that a reset is two memsets:
     // zeros (control block, tile stamps, then the queue's ticket tags or the
-    // rounds form's visited words) and ones (the label arena, waiting f per tile;
+    // rounds form's visited words, then the layer kernel's misfits per field) and ones (the label arena, waiting f per tile;
     // the rounds form needs no reset of its labels)
     DBuf d_zero, d_ones;
-    size_t zero_bytes = 0, ones_bytes = 0, o_tstamp = 0, o_tail = 0, o_tpark = 0;
+    size_t zero_bytes = 0, ones_bytes = 0, o_tstamp = 0, o_tail = 0, o_misfits = 0, o_tpark = 0;
     Ctl *ctl() const { return d_zero.as<Ctl>(); }
     uint32_t *tstamp() const { return reinterpret_cast<uint32_t *>(d_zero.as<unsigned char>() + o_tstamp); }
     u64 *tags() const { return async_q ? reinterpret_cast<u64 *>(d_zero.as<unsigned char>() + o_tail) : nullptr; }
@@ -889,6 +917,7 @@ struct mrc_batch {
     bool warp = false;     // the warp-per-tile schedule (implies the queue and a +inf-filled arena)
     bool cta_planes = true;  // schedule 1: the layer kernel (where it applies: `layer`), else the CTA queue form
     bool layer = false;      // this layout runs the layer kernel (packed price planes by TMA)
+    bool both = false;       // labels of some board may not fit 32 bits within a tile
     std::vector<DevBoard> devs;  // the board table (step-price plane pointers patched in by batch_layout)
     DBuf d_planes, d_pchunks;    // step-price planes of every board, chunk table of their kernel
     DBuf d_tmaps;                // one TMA tensor map per board over its planes (layer kernel)
@@ -1039,7 +1068,7 @@ mrc_status batch_layout(mrc_batch *bt, uint32_t tile_h, uint32_t threads) {
     if (bt->warp) {
         MRC_CUDA(warp_relax_occupancy(&per_sm), "relax occupancy");
     } else if (bt->layer) {
-        MRC_CUDA(layer_configure(bt->max_layers, bt->rows, bt->smem, bt->has_over, bt->goal, &per_sm), "configure relax kernel");
+        MRC_CUDA(layer_configure(bt->max_layers, bt->rows, bt->smem, bt->has_over, bt->goal, bt->both, &per_sm), "configure relax kernel");
     } else {
         MRC_CUDA(relax_configure(tile_h, threads, bt->smem, bt->async_q, bt->has_over), "configure relax kernel");
         MRC_CUDA(relax_occupancy(tile_h, threads, bt->smem, &per_sm, bt->async_q, bt->has_over), "relax occupancy");
@@ -1089,12 +1118,20 @@ mrc_status batch_layout(mrc_batch *bt, uint32_t tile_h, uint32_t threads) {
         bt->d_tmaps.reset();
         bt->n_pchunks = 0;
     }
-    {  // the board table, and behind it the zeroed heads of the price bounds
-        const size_t nb = bt->devs.size(), o_heads = (nb * sizeof(DevBoard) + 255) & ~(size_t)255;
-        std::vector<unsigned char> table(o_heads + (bt->layer ? nb * sizeof(BoardGoal) : 0), 0);
+    {  // the board table, and behind it the zeroed heads of the price bounds and marks of large prices
+        const size_t nb = bt->devs.size(), o_heads = (nb * sizeof(DevBoard) + 255) & ~(size_t)255,
+                     o_dear = o_heads + nb * sizeof(BoardGoal);
+        size_t dear = 0;
+        for (const DevBoard &d : bt->devs) dear += (size_t)dear_pitch(d.w) * ((d.h + 7) / 8);
+        std::vector<unsigned char> table(bt->layer ? o_dear + dear : o_heads, 0);
         MRC_TRY(bt->d_boards.get(ctx, std::max<size_t>(table.size(), 4), "board table"));
         BoardGoal *heads = reinterpret_cast<BoardGoal *>(bt->d_boards.as<unsigned char>() + o_heads);
-        for (size_t k = 0; k < nb; ++k) bt->devs[k].goal = bt->layer ? heads + k : nullptr;
+        uint8_t *marks = bt->d_boards.as<uint8_t>() + o_dear;
+        for (size_t k = 0; k < nb; ++k) {
+            bt->devs[k].goal = bt->layer ? heads + k : nullptr;
+            bt->devs[k].dear = bt->layer ? marks : nullptr;
+            marks += (size_t)dear_pitch(bt->devs[k].w) * ((bt->devs[k].h + 7) / 8);
+        }
         if (nb) std::memcpy(table.data(), bt->devs.data(), nb * sizeof(DevBoard));
         MRC_CUDA(cudaMemcpyAsync(bt->d_boards.p, table.data(), table.size(), cudaMemcpyHostToDevice, ctx->stream),
                  "upload board table");
@@ -1115,7 +1152,8 @@ mrc_status batch_layout(mrc_batch *bt, uint32_t tile_h, uint32_t threads) {
     auto up256 = [](size_t v) { return (v + 255) & ~(size_t)255; };
     bt->o_tstamp = up256(sizeof(Ctl));
     bt->o_tail = up256(bt->o_tstamp + (size_t)bt->total_tiles * 4);
-    bt->zero_bytes = bt->o_tail + (bt->async_q ? (size_t)bt->list_cap * 8 : (size_t)bt->total_tiles * 4);
+    bt->o_misfits = up256(bt->o_tail + (bt->async_q ? (size_t)bt->list_cap * 8 : (size_t)bt->total_tiles * 4));
+    bt->zero_bytes = bt->o_misfits + (bt->layer ? bt->fields.size() * 4 : 0);
     MRC_TRY(bt->d_zero.get(ctx, bt->zero_bytes, "tile state"));
     bt->o_tpark = up256(std::max<uint64_t>(bt->total_cells, 1) * 8);
     bt->ones_bytes = bt->o_tpark + (bt->goal ? (size_t)bt->total_tiles * 4 : 0);
@@ -1142,6 +1180,8 @@ mrc_status batch_build(mrc_context *ctx, std::vector<const mrc_board *> boards, 
         bt->directed_any = bt->directed_any || b->directed;
     }
     const uint32_t n = (uint32_t)bt->nets.size();
+    bt->both = false;
+    for (const mrc_board *b : bt->boards) bt->both = bt->both || b->spread >= kWideSpread;
     bt->has_over = false;
     for (const NetCopy &nc : bt->nets) bt->has_over = bt->has_over || nc.n_over;
     uint32_t tile_h = 0, threads = kRelaxThreads;
@@ -1283,6 +1323,7 @@ mrc_status batch_enqueue(mrc_batch *bt, cudaStream_t st, bool capturing) {
     ra.lists = bt->d_lists.as<u64>();
     ra.tags = bt->tags();
     ra.list_cap = bt->list_cap;
+    if (bt->layer) ra.misfits = reinterpret_cast<int *>(bt->d_zero.as<unsigned char>() + bt->o_misfits);
     if (bt->goal) {
         ra.goal = bt->d_fgoal.as<FieldGoal>();
         ra.tpark = bt->tpark();
@@ -1306,7 +1347,7 @@ mrc_status batch_enqueue(mrc_batch *bt, cudaStream_t st, bool capturing) {
             MRC_CUDA(warp_relax_launch(ra, bt->grid, st), "launch relax kernel");
             launches += 2;  // seeds, relax
         } else {
-            MRC_CUDA(bt->layer ? layer_launch(ra, bt->grid, bt->smem, st, bt->has_over, bt->goal)
+            MRC_CUDA(bt->layer ? layer_launch(ra, bt->grid, bt->smem, st, bt->has_over, bt->goal, bt->both)
                                : relax_launch(ra, bt->grid, bt->threads, bt->smem, st, bt->async_q, bt->has_over),
                      "launch relax kernel");
             launches += bt->async_q ? 2 : 1;  // (+ the seed kernel)
@@ -2375,6 +2416,7 @@ mrc_status mrc_negotiation_route(mrc_context *ctx, mrc_negotiation *ng, mrc_roun
     sa.weight = ng->params.present_weight;
     sa.halo_weight = ng->halo_weight;
     MRC_CUDA(snapshot_launch(sa, s), "price snapshot");
+    ng->snap->spread = ng->base->spread + 4ull * st->pfac * ng->params.present_weight;  // and a few used slots
     if (n_dirty) {
         std::vector<NetCopy> nets;
         std::vector<mrc_window> wins;
@@ -3004,7 +3046,7 @@ mrc_status mrc_server_create(mrc_context *ctx, const mrc_server_params *params, 
         s->tile_h = 8;
         s->threads = kRelaxThreads;
         int per_sm = 0;
-        MRC_CUDA(layer_configure(s->p.max_layers, kLayerTileH, layer_smem_bytes(s->p.max_layers, kLayerTileH), false, true, &per_sm),
+        MRC_CUDA(layer_configure(s->p.max_layers, kLayerTileH, layer_smem_bytes(s->p.max_layers, kLayerTileH), false, true, false, &per_sm),
                  "configure relax kernel");
         if ((uint32_t)per_sm * (uint32_t)ctx->sms < s->p.slots) return fail(MRC_ERR_LIMIT, "too many slots");
         s->streams.resize(s->p.slots);

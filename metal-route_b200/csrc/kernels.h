@@ -40,6 +40,7 @@ struct RelaxArgs {
     Ctl *ctl;                   // zeroed before launch
     FieldGoal *goal;            // goal-directed launches: per field (written by the seed kernel)
     uint32_t *tpark;            // goal-directed: per tile, the smallest f waiting to enter it (0xFF filled)
+    int *misfits;               // layer kernel: per field, tiles that 32-bit words did not hold, less those they did (zeroed)
     uint32_t tile_h;            // 32, 16 or 8
     uint32_t round_limit;       // guard on the number of rounds
     unsigned long long activation_limit;  // guard on tile activations (asynchronous form)
@@ -259,7 +260,10 @@ cudaError_t seed_launch(const RelaxArgs &a, cudaStream_t st);
 // The layer kernel (layer_relax.cu): the queue form on 32 x 8 or 32 x 16 tiles with a warp
 // per layer, labels packed into 32 bits, prices from the boards' packed price
 // planes by TMA; boards of up to kLayerMax layers.  goal: paths and costs only
-// (RelaxArgs::goal).
+// (RelaxArgs::goal).  both: for boards whose labels may not fit 32 bits within a tile
+// (kWideSpread); such tiles are relaxed in 64-bit words then.  It takes 4 to 6 % longer on boards
+// whose labels fit (256 nets of 512 x 512: 1416, 1498 us), so the others run the kernel
+// without, which has tiles that don't fit relaxed on prices formed per tile.
 constexpr uint32_t kLayerMax = 16;
 constexpr uint32_t kLayerTileH = 8;
 constexpr uint32_t kLayerTallH = 16, kLayerTallMax = 4;  // tall tiles: up to so many layers, no overrides
@@ -270,9 +274,10 @@ constexpr uint32_t kTallTiles = 240;  // tall up to so many 8-row tiles an SM
 // (12 bits, enough for any path through 2048 cells, left 2^17: 256 nets of 512 x
 // 512 with gaps of 3000 took 7.3 ms.)
 constexpr uint32_t kLayerHopBits = 10;
+constexpr uint64_t kWideSpread = 1u << (29 - kLayerHopBits);  // estimated spread from which 64-bit words stand by
 size_t layer_smem_bytes(uint32_t max_layers, uint32_t tile_h);
-cudaError_t layer_configure(uint32_t max_layers, uint32_t tile_h, size_t smem, bool over, bool goal, int *blocks_per_sm);
-cudaError_t layer_launch(const RelaxArgs &a, uint32_t grid, size_t smem, cudaStream_t st, bool over, bool goal);
+cudaError_t layer_configure(uint32_t max_layers, uint32_t tile_h, size_t smem, bool over, bool goal, bool both, int *blocks_per_sm);
+cudaError_t layer_launch(const RelaxArgs &a, uint32_t grid, size_t smem, cudaStream_t st, bool over, bool goal, bool both);
 // tover[f.tile_off + t] = 1 for every tile t of every field that holds one of
 // the field's directed-price overrides (tover zeroed before).
 cudaError_t mark_over_tiles_launch(const DevField *fields, uint32_t n_fields, const DevBoard *boards, uint32_t tile_h,

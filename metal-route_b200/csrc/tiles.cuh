@@ -38,6 +38,12 @@ __device__ __forceinline__ uint32_t plane_word(uint32_t p) {
     if (p < (1u << (29 - kLayerHopBits))) return (p << kLayerHopBits) | 1u;
     return p == kMax ? kPackedInf : p < kPriceLook - kPricePlain ? kPricePlain | p : kPriceLook;
 }
+// The price of a word; `look` forms one that no word holds.
+template <class Look>
+__device__ __forceinline__ uint32_t plane_price(uint32_t word, Look look) {
+    if (word < kPackedInf) return word >> kLayerHopBits;
+    return word == kPackedInf ? kMax : word == kPriceLook ? look() : word & (kPricePlain - 1u);
+}
 
 __device__ __forceinline__ u64 umin64(u64 a, u64 b) { return a < b ? a : b; }
 

@@ -195,7 +195,10 @@ __global__ void __launch_bounds__(256, 3) planes_kernel(const DevBoard *boards, 
 #pragma unroll
                     for (uint32_t k = 0; k < 4; ++k) {
                         s[p][k] = plane_word(s[p][k]);
-                        if (s[p][k] >= kPricePlain) b.goal->wide = 1;
+                        if (s[p][k] >= kPricePlain) {
+                            b.goal->wide = 1;
+                            b.dear[(y / 8) * dear_pitch(b.w) + x0 / 32] = 1;
+                        }
                     }
                 }
                 *reinterpret_cast<uint4 *>(out + (uint64_t)p * NP + o) = make_uint4(s[p][0], s[p][1], s[p][2], s[p][3]);

@@ -189,8 +189,8 @@ cudaError_t relax_configure(uint32_t, uint32_t, size_t, bool, bool) { return cud
 cudaError_t relax_occupancy(uint32_t, uint32_t, size_t, int *n, bool, bool) { return *n = 1, cudaSuccess; }
 cudaError_t relax_launch(const RelaxArgs &, uint32_t, uint32_t, size_t, cudaStream_t, bool, bool) { return cudaSuccess; }
 size_t layer_smem_bytes(uint32_t layers, uint32_t tile_h) { return (size_t)layers * tile_h * 1024; }
-cudaError_t layer_configure(uint32_t, uint32_t, size_t, bool, bool, int *n) { return *n = 1, cudaSuccess; }
-cudaError_t layer_launch(const RelaxArgs &, uint32_t, size_t, cudaStream_t, bool, bool) { return cudaSuccess; }
+cudaError_t layer_configure(uint32_t, uint32_t, size_t, bool, bool, bool, int *n) { return *n = 1, cudaSuccess; }
+cudaError_t layer_launch(const RelaxArgs &, uint32_t, size_t, cudaStream_t, bool, bool, bool) { return cudaSuccess; }
 cudaError_t mark_over_tiles_launch(const DevField *, uint32_t, const DevBoard *, uint32_t, uint8_t *, cudaStream_t) {
     return cudaSuccess;
 }

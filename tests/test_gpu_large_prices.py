@@ -31,7 +31,7 @@ def _check(eng, oracle, grid, x, y, vias, nets, wins, directed=None):
 
 # both sides of what packed price words hold, of what plain ones hold, and of the largest
 @pytest.mark.parametrize("price", [2**19 - 1, 2**19, 2**24 + 1, 2**29 - 1, 2**29, 2**31 - 2, 2**31 - 1, 2**31, 2**32 - 2])
-@pytest.mark.parametrize("layers", [1, 3, 6])
+@pytest.mark.parametrize("layers", [1, 3, 6, 12])
 def test_price_limits(eng, oracle, price, layers):
     """Uniform gaps (ties everywhere), one dear line, and dear cells on a cheap board."""
     rng = np.random.default_rng(price % 1000 + layers)
@@ -75,6 +75,42 @@ def test_directed_price_limits(eng, oracle, price):
            d.reshape(-1))
 
 
+def test_boards_of_small_and_large_prices_in_one_batch(eng, oracle):
+    """A launch over both, replayed as a graph, with and without fields."""
+    boards = [W.plain_board(seed=3, w=70, h=50, n_nets=6), W.plain_board(seed=4, w=90, h=40, n_nets=6)]
+    reqs = []
+    for wl, gap in zip(boards, (3, 70_000)):
+        d = wl.grid.dims
+        reqs.append(IsolatedRouteRequest(wl.grid, wl.nets, wl.windows, np.full(d.w - 1, gap, np.uint32),
+                                         np.full(d.h - 1, gap + 1, np.uint32), [2 * gap]))
+    held = [eng.board(r.grid, r.x_edge_costs, r.y_edge_costs, r.via_edge_costs) for r in reqs]
+    want = [oracle.isolated_batch(r, retry_full=False, mode="field") for r in reqs]
+    for keep in (False, True):
+        bt = mrcuda.Batch(held, [n for r in reqs for n in r.nets], [w for r in reqs for w in r.windows], retry_full=False,
+                          keep_fields=keep, net_board=[k for k, r in enumerate(reqs) for _ in r.nets])
+        bt.capture_graph()
+        for _ in range(3):
+            bt.launch()
+            got = bt.finish()
+            assert got.paths == want[0][0] + want[1][0] and got.search_costs == want[0][1] + want[1][1]
+        bt.close()
+    for b in held:
+        b.close()
+
+
+@pytest.mark.parametrize("factor,weight", [(4000, 16), (1, 1 << 18)])
+def test_negotiation_with_large_prices(eng, oracle, factor, weight):
+    """Price overrides (a clearance) on a board of large prices, and large penalties on a
+    board of small ones."""
+    from test_gpu_negotiation import _run_both
+
+    wl = W.snapshot_board(w=96, h=80, layers=3, n_nets=24, median=40)
+    directed = np.where(wl.directed == COST_MAX, COST_MAX, wl.directed.astype(np.uint64) * factor).astype(np.uint32)
+    req = IsolatedRouteRequest(wl.grid, wl.nets, wl.windows, wl.x, wl.y, [v * factor for v in wl.vias], directed)
+    _run_both(eng, oracle, req, rounds=3, weight=weight, clearance=1)
+    _run_both(eng, oracle, req, rounds=3, weight=weight)
+
+
 def _times(eng, factor):
     """Least device times (relax, walk) in ms of a board with its prices times `factor`."""
     import torch
@@ -106,3 +142,32 @@ def test_walk_time_does_not_depend_on_the_prices(eng, factor):
     _, small = _times(eng, 1)
     _, large = _times(eng, factor)
     assert large < 2 * small, (small, large)
+
+
+@pytest.mark.parametrize("factor", [1000, 2500, 20000])
+def test_relax_time_hardly_depends_on_the_prices(eng, factor):
+    """Tiles whose labels don't fit 32-bit words take more work, on 64-bit ones, but no
+    attempt on 32 bits each time."""
+    small, _ = _times(eng, 1)
+    large, _ = _times(eng, factor)
+    assert large < 3.2 * small, (small, large)  # what a relax on 64-bit labels throughout took
+
+
+def test_a_dear_corner_costs_the_rest_of_the_board_nothing(eng):
+    """A few cells of a large price: the tiles without them stay on 32-bit words."""
+    wl = W.plain_board(seed=1)
+    cost = wl.grid.cost.copy()
+    cost[:3] = 10**6
+    times = []
+    for c in (wl.grid.cost, cost):
+        b = eng.board(Grid(wl.grid.dims, c, wl.grid.board_constraint, wl.grid.via_forbidden), wl.x, wl.y, wl.vias)
+        bt = mrcuda.Batch(b, wl.nets, wl.windows, time_kernels=True)
+        ms = []
+        for _ in range(8):
+            bt.launch()
+            bt.finish()
+            ms.append(bt.relax_ms())
+        times.append(min(ms[2:]))
+        bt.close()
+        b.close()
+    assert times[1] < 1.5 * times[0], times
