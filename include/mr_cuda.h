@@ -228,7 +228,7 @@ mrc_status mrc_batch_set_config(mrc_context *ctx, mrc_batch *batch, uint32_t til
  * work queue (no rounds; a tile held by one CTA at a time) of tiles with a warp
  * per layer and labels packed into 32 bits, step prices brought to each tile by
  * one TMA load from per-board price planes computed once per batch layout
- * (8-row tiles and at most 16 layers, else schedule 3's kernel; the library
+ * (tile height 8, else schedule 3's kernel; the library
  * takes 16-row tiles itself where they are faster); 2 = the same queue with one warp per tile (tiles of 4 S x 8 cells
  * over every layer, S = 32 / next_pow2(layers), labels in shared memory;
  * boards of at most 16 layers, else MRC_ERR_LIMIT; a batch whose nets carry

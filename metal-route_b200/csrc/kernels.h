@@ -264,7 +264,11 @@ cudaError_t seed_launch(const RelaxArgs &a, cudaStream_t st);
 // (kWideSpread); such tiles are relaxed in 64-bit words then.  It takes 4 to 6 % longer on boards
 // whose labels fit (256 nets of 512 x 512: 1416, 1498 us), so the others run the kernel
 // without, which has tiles that don't fit relaxed on prices formed per tile.
-constexpr uint32_t kLayerMax = 16;
+// With 24 layers a tile's prices and labels take 218 KB of shared memory, and 25 don't
+// fit; 768 threads still have 80 registers each.  (160 x 160 boards of 20 layers, 64 nets,
+// paths, relax us: the 64-bit queue form 2980 with price planes, 3090 with prices formed
+// per tile; this kernel 505.)
+constexpr uint32_t kLayerMax = 24;
 constexpr uint32_t kLayerTileH = 8;
 constexpr uint32_t kLayerTallH = 16, kLayerTallMax = 4;  // tall tiles: up to so many layers, no overrides
 constexpr uint32_t kTallTiles = 240;  // tall up to so many 8-row tiles an SM

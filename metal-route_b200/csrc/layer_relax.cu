@@ -969,8 +969,9 @@ template <bool BOTH>
 const void *layer_fn_words(uint32_t max_layers, uint32_t tile_h, bool over, bool goal) {
     if (tile_h == kLayerTallH) return max_layers <= kLayerTallMax ? layer_fn_lm<4, kLayerTallH, BOTH>(over, goal) : nullptr;
     return max_layers <= 4   ? layer_fn_lm<4, kLayerTileH, BOTH>(over, goal)
-           : max_layers <= 8 ? layer_fn_lm<8, kLayerTileH, BOTH>(over, goal)
-                             : layer_fn_lm<16, kLayerTileH, BOTH>(over, goal);
+           : max_layers <= 8  ? layer_fn_lm<8, kLayerTileH, BOTH>(over, goal)
+           : max_layers <= 16 ? layer_fn_lm<16, kLayerTileH, BOTH>(over, goal)
+                              : layer_fn_lm<kLayerMax, kLayerTileH, BOTH>(over, goal);
 }
 
 const void *layer_fn(uint32_t max_layers, uint32_t tile_h, bool over, bool goal, bool both) {
@@ -989,7 +990,7 @@ cudaError_t layer_configure(uint32_t max_layers, uint32_t tile_h, size_t smem, b
     if (!fn) return cudaErrorInvalidValue;
     // the most any layer count of this kernel takes: a batch of more layers may
     // already be laid out, and is launched after this call
-    const uint32_t most = max_layers <= 4 ? 4u : max_layers <= 8 ? 8u : 16u;
+    const uint32_t most = max_layers <= 4 ? 4u : max_layers <= 8 ? 8u : max_layers <= 16 ? 16u : kLayerMax;
     const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                (int)layer_smem_bytes(most, tile_h));
     if (e != cudaSuccess) return e;
