@@ -221,15 +221,15 @@ mrc_status mrc_batch_finish(mrc_context *ctx, mrc_batch *batch, mrc_result **out
 mrc_status mrc_batch_autotune(mrc_context *ctx, mrc_batch *batch, uint32_t *tile_h, uint32_t *threads,
                               float *best_ms);
 /* Force a relax configuration on a batch: tile height in {8, 16, 32, 64} cells
- * and 128 or 256 threads per CTA.  MRC_ERR_LIMIT when the tile does not fit. */
+ * and 128 or 256 threads per CTA (schedules 0 and 3; schedules 1 and 2 have tiles
+ * of their own).  MRC_ERR_LIMIT when the tile does not fit. */
 mrc_status mrc_batch_set_config(mrc_context *ctx, mrc_batch *batch, uint32_t tile_h, uint32_t threads);
 /* The relax schedule: 0 = bulk-synchronous rounds over a shared tile list
  * (cooperative launch, grid barrier between rounds); 1 = one asynchronous
  * work queue (no rounds; a tile held by one CTA at a time) of tiles with a warp
- * per layer and labels packed into 32 bits, step prices brought to each tile by
- * one TMA load from per-board price planes computed once per batch layout
- * (tile height 8, else schedule 3's kernel; the library
- * takes 16-row tiles itself where they are faster); 2 = the same queue with one warp per tile (tiles of 4 S x 8 cells
+ * per layer and packed labels, 8 or 16 rows as the library finds faster, step
+ * prices brought to each tile by one TMA load from per-board price planes computed
+ * once per batch layout; 2 = the same queue with one warp per tile (tiles of 4 S x 8 cells
  * over every layer, S = 32 / next_pow2(layers), labels in shared memory;
  * boards of at most 16 layers, else MRC_ERR_LIMIT; a batch whose nets carry
  * negotiation price overrides runs 1 instead); 3 = the queue of 1 with step

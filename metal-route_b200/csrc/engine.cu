@@ -1021,13 +1021,15 @@ mrc_status batch_layout(mrc_batch *bt, uint32_t tile_h, uint32_t threads) {
         threads = kOverThreads;
     }
     if (bt->warp) bt->async_q = true;
-    // schedule 1 with another tile height than the layer kernel's, or with more
-    // layers than it takes, runs the CTA queue form with prices formed per tile
-    bt->layer = bt->async_q && !bt->warp && bt->cta_planes && tile_h == kLayerTileH && bt->max_layers <= kLayerMax;
+    // Schedule 1 is the layer kernel, which has tiles of its own: the tile height and CTA
+    // width asked for are those of schedules 0 and 3.  (It was faster than their kernels
+    // on every height: 64 nets of 128 x 128 x 2, complete fields, relax us at 8, 16, 32
+    // and 64 rows 297, 242, 250 and 332; 122 for the layer kernel.)
+    bt->layer = bt->async_q && !bt->warp && bt->cta_planes && bt->max_layers <= kLayerMax;
     bt->tile_h = bt->warp ? kWarpTileH : tile_h;
     bt->threads = bt->warp ? warp_relax_threads() : threads;
     const uint32_t sms = (uint32_t)ctx->sms;
-    bt->rows = bt->tile_h;
+    bt->rows = bt->layer ? kLayerTileH : bt->tile_h;
     if (bt->layer && !bt->has_over && !bt->directed_any && bt->max_layers <= kLayerTallMax) {
         // Tall tiles halve the visits a wavefront makes up and down a window, and a
         // visit's cost is mostly its wait for the neighbours' labels.  At 1 to 4
