@@ -172,9 +172,12 @@ __global__ void async_seed_kernel(RelaxArgs a) {
                 // of the bound.  A path through random prices avoids the dear ones: its
                 // mean step lies about a third of the way from the cheapest to the mean
                 // price (congestion board: path cost 1.38 x the bound where mean /
-                // cheapest is 2.3; negotiation board 1.01 x at 1.1).  Relax time of the
-                // congestion board with a share of 0, 0.17, 0.35 and 0.6 of that
-                // distance: 4.9, 4.9, 4.5, 4.9 ms.  With a zero bound nothing waits.
+                // cheapest is 2.3; negotiation board 1.01 x at 1.1).  Relax us with a share
+                // of 0, 0.17, 0.25, 0.35, 0.45 and 0.6 of that distance: two congestion
+                // boards 1906, 1617, 1420, 1449, 1449, 1520 and 2047, 1690, 1540, 1503,
+                // 1537, 1575; negotiation boards of 1280 x 1153 x 6 and 640 x 500 x 4 1487,
+                // 1520, 1571, 1530, 1545, 1578 and 761, 666, 676, 662, 670, 668; 512 uneven
+                // instances 750 at each.  With a zero bound nothing waits.
                 float spread = 1.0f;  // mean over cheapest price
                 if (bg.n_cost && ~bg.inv_min_cost) spread *= (float)bg.sum_cost / (float)bg.n_cost / (float)~bg.inv_min_cost;
                 if (b.directed && bg.n_dir && each) spread *= (float)bg.sum_dir / (float)bg.n_dir / (float)each;
@@ -924,28 +927,30 @@ __global__ void __launch_bounds__(kWalkThreads, 2) path_walk_tiled_kernel(PathAr
                     }
                     if (dl) delta[at] = (int16_t)dl;
                 }
-                if (sizeof(typename Q::type) == 4 || most != kPriceLook) continue;
-                // prices that no word holds: formed from the board's words
+                if constexpr (sizeof(typename Q::type) == 8) {
+                    if (most != kPriceLook) continue;
+                    // prices that no word holds: formed from the board's words
 #pragma unroll 1
-                for (uint32_t k = 0; k < kCells; ++k) {
-                    const uint32_t q = r0 + k * nw, l = q / WH, yy = q % WH;
-                    const uint32_t at = l * PL + (yy + 1) * PW + lane + 1;
-                    if (q >= L * WH) continue;
-                    const auto wc = word[at];
-                    int dl = 0;
+                    for (uint32_t k = 0; k < kCells; ++k) {
+                        const uint32_t q = r0 + k * nw, l = q / WH, yy = q % WH;
+                        const uint32_t at = l * PL + (yy + 1) * PW + lane + 1;
+                        if (q >= L * WH) continue;
+                        const auto wc = word[at];
+                        int dl = 0;
 #pragma unroll 1
-                    for (int n = 5; n >= 0; --n) {
-                        const int o = n == 0 ? -(int)PL : n == 1 ? -(int)PW : n == 2 ? -1 : n == 3 ? 1 : n == 4 ? (int)PW : (int)PL;
-                        if (!Q::is(wc) || (n == 0 && l == 0) || (n == 5 && l + 1 == L) || !Q::asks(wc, word[(int)at + o])) continue;
-                        int px = tx0 + (int)lane, py = ty0 + (int)yy, pz = (int)l;
-                        const uint32_t gx = (uint32_t)px, gy = (uint32_t)py;
-                        walk_offset(n, px, py, pz);
-                        if (walk_step_exact(a.boards + f.board, a.fields + blockIdx.x, a.pads,
-                                            ((uint32_t)pz * b.h + (uint32_t)py) * b.w + (uint32_t)px,
-                                            (l * b.h + gy) * b.w + gx, gx, gy, l, n) == Q::dist(word[(int)at + o]) - Q::dist(wc))
-                            dl = o;
+                        for (int n = 5; n >= 0; --n) {
+                            const int o = n == 0 ? -(int)PL : n == 1 ? -(int)PW : n == 2 ? -1 : n == 3 ? 1 : n == 4 ? (int)PW : (int)PL;
+                            if (!Q::is(wc) || (n == 0 && l == 0) || (n == 5 && l + 1 == L) || !Q::asks(wc, word[(int)at + o])) continue;
+                            int px = tx0 + (int)lane, py = ty0 + (int)yy, pz = (int)l;
+                            const uint32_t gx = (uint32_t)px, gy = (uint32_t)py;
+                            walk_offset(n, px, py, pz);
+                            if (walk_step_exact(a.boards + f.board, a.fields + blockIdx.x, a.pads,
+                                                ((uint32_t)pz * b.h + (uint32_t)py) * b.w + (uint32_t)px,
+                                                (l * b.h + gy) * b.w + gx, gx, gy, l, n) == Q::dist(word[(int)at + o]) - Q::dist(wc))
+                                dl = o;
+                        }
+                        delta[at] = (int16_t)dl;
                     }
-                    delta[at] = (int16_t)dl;
                 }
             }
             if (s_nspec) {  // the same for the whole CTA

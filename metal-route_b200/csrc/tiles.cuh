@@ -53,7 +53,13 @@ __device__ __forceinline__ u64 umin64(u64 a, u64 b) { return a < b ? a : b; }
 // the ring: one 64-bit word per slot, lap << 56 | field << 28 | tile, so an item is
 // published and taken with one store and one load (zeroed before launch; laps count
 // 1..255).  A tile is queued at most once at a time (its tstamp word is the queued
-// flag), so list_cap >= total tiles never overflows.
+// flag), so at most list_cap items are queued at once.  Nothing keeps a slot for a worker that
+// holds its ticket and has not read it yet, though, while other tiles go round the ring: that
+// is a margin, not a handshake.  A ring has kMinRing slots at least, more than three
+// times the workers of any launch (2368 warps of the warp schedule), so a worker would
+// have to miss three items of every other worker, microseconds each, between two polls,
+// which lie at most 128 ns apart; an item lost that way would end the launch with
+// kStatusBarrier.
 constexpr uint32_t kQueueSpinLimit = 1u << 25;  // polls of one wait (seconds with the backoff below)
 constexpr u64 kSlotItem = (1ull << 56) - 1;     // the item bits of a slot word; all ones: the launch is over
 
