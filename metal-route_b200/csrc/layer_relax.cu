@@ -244,7 +244,9 @@ __device__ __forceinline__ uint32_t layer_item(const RelaxArgs &a, uint32_t fi, 
             lim0 = __ldcg(reinterpret_cast<const uint2 *>(a.goal + fi));
         }
     }
-    if (!WIDE && wl == 0 && __ldg(&b.goal->wide)) {  // is a price in or around this tile too large?
+    // is a price in or around this tile too large?  (the last warp looks: the first one
+    // has the hold to wait for)
+    if (!WIDE && wl + 1u == (blockDim.x >> 5) && __ldg(&b.goal->wide)) {
         const uint32_t bx = (uint32_t)max(tx0 - 1, 0) / 32u + lane % 3u, by = (uint32_t)max(ty0 - 1, 0) / 8u + lane / 3u;
         if (bx <= ((uint32_t)tx0 + kTW) / 32u && by <= ((uint32_t)ty0 + TH) / 8u && bx * 32u < b.w && by * 8u < b.h &&
             __ldg(b.dear + by * dear_pitch(b.w) + bx))
