@@ -189,19 +189,27 @@ __global__ void __launch_bounds__(256, 3) planes_kernel(const DevBoard *boards, 
                 }
             }
             const uint64_t o = (uint64_t)row * wp + x0;
+            bool dear = false;
 #pragma unroll
             for (int p = 0; p < 6; ++p) {
                 if (packed) {  // the layer kernel's words
 #pragma unroll
                     for (uint32_t k = 0; k < 4; ++k) {
-                        s[p][k] = plane_word(s[p][k]);
-                        if (s[p][k] >= kPricePlain) {
-                            b.goal->wide = 1;
-                            b.dear[(y / 8) * dear_pitch(b.w) + x0 / 32] = 1;
+                        uint32_t v = s[p][k];
+                        if (v < (1u << (29 - kLayerHopBits))) {
+                            v = (v << kLayerHopBits) | 1u;
+                        } else {
+                            if (v != kMax) dear = true;
+                            v = v == kMax ? kPackedInf : plane_word(v);
                         }
+                        s[p][k] = v;
                     }
                 }
                 *reinterpret_cast<uint4 *>(out + (uint64_t)p * NP + o) = make_uint4(s[p][0], s[p][1], s[p][2], s[p][3]);
+            }
+            if (dear) {
+                b.goal->wide = 1;
+                b.dear[(y / 8) * dear_pitch(b.w) + x0 / 32] = 1;
             }
         }
         if (b.goal) {  // the same for the whole block
