@@ -57,7 +57,7 @@ struct DevBoard {
     const uint32_t *over_cells;
     const uint4 *over_price;
     BoardGoal *goal;            // nullable: extremes of the prices (zeroed before planes_kernel)
-    // with `goal`: per 32 x 8 cells, 1 = a price into one of them, on some layer, does not
+    // with `goal`: per 8 x 8 cells, 1 = a price into one of them, on some layer, does not
     // fit a packed word (zeroed before planes_kernel); rows of dear_pitch
     uint8_t *dear;
     // prefix sums of the gap and via prices (saturating at kCap), the smallest gap
@@ -78,7 +78,7 @@ struct BoardGoal {
     uint32_t pad_;
 };
 
-__host__ __device__ inline uint32_t dear_pitch(uint32_t w) { return (w + 31u) / 32u; }
+__host__ __device__ inline uint32_t dear_pitch(uint32_t w) { return (w + 7u) / 8u; }
 
 // Search state of one field of a goal-directed launch.  A label at cell c with
 // f = dist + bound(c) above `ub` cannot lie on a cheapest path and is not

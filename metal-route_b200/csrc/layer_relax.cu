@@ -77,7 +77,8 @@ struct Words<u64> {
 constexpr uint32_t kPitch = kPlaneTmaBoxW;  // of a row of prices
 constexpr uint32_t kSpecCap = 512;      // cells of a tile priced for the net itself
 // A field's tiles go straight to 64-bit words from this count of misfits on; one counts
-// as much as kMisfitWeight of those that fit.
+// as much as kMisfitWeight of those that fit.  (8, 16 or 32: no difference on boards of
+// large prices, nor with a dear corner.)
 constexpr int kMisfitWeight = 4, kMisfits = 32;
 constexpr int kPlaneIters = 2;          // column and row passes of a plane between two meetings
 
@@ -247,8 +248,9 @@ __device__ __forceinline__ uint32_t layer_item(const RelaxArgs &a, uint32_t fi, 
     // is a price in or around this tile too large?  (the last warp looks: the first one
     // has the hold to wait for)
     if (!WIDE && wl + 1u == (blockDim.x >> 5) && __ldg(&b.goal->wide)) {
-        const uint32_t bx = (uint32_t)max(tx0 - 1, 0) / 32u + lane % 3u, by = (uint32_t)max(ty0 - 1, 0) / 8u + lane / 3u;
-        if (bx <= ((uint32_t)tx0 + kTW) / 32u && by <= ((uint32_t)ty0 + TH) / 8u && bx * 32u < b.w && by * 8u < b.h &&
+        // a lane per 8 x 8 cells: the tile and its ring touch 6 x 4 at most
+        const uint32_t bx = (uint32_t)max(tx0 - 1, 0) / 8u + lane % 6u, by = (uint32_t)max(ty0 - 1, 0) / 8u + lane / 6u;
+        if (bx <= ((uint32_t)tx0 + kTW) / 8u && by <= ((uint32_t)ty0 + TH) / 8u && bx * 8u < b.w && by * 8u < b.h &&
             __ldg(b.dear + by * dear_pitch(b.w) + bx))
             *(volatile uint32_t *)&sh.wide = 1;
     }

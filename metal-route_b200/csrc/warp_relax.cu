@@ -209,7 +209,7 @@ __global__ void __launch_bounds__(256, 3) planes_kernel(const DevBoard *boards, 
             }
             if (dear) {
                 b.goal->wide = 1;
-                b.dear[(y / 8) * dear_pitch(b.w) + x0 / 32] = 1;
+                b.dear[(y / 8) * dear_pitch(b.w) + x0 / 8] = 1;
             }
         }
         if (b.goal) {  // the same for the whole block
