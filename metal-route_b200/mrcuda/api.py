@@ -577,15 +577,16 @@ class Batch:
         return int(self.engine.lib.mrc_batch_kernel_launches(self.handle))
 
     def set_config(self, tile_h: int, threads: int) -> None:
-        """Force the relax kernel's tile height and CTA width for this batch."""
+        """Force the tile height and CTA width of schedules 0 and 3 for this batch (1 and 2
+        have tiles of their own)."""
         e = self.engine
         e._check(e.lib.mrc_batch_set_config(e.ctx, self.handle, int(tile_h), int(threads)))
 
     def set_schedule(self, schedule: int) -> None:
         """0 = bulk-synchronous rounds, 1 = asynchronous work queue (a CTA per
-        tile, a warp per layer, labels packed into 32 bits, prices from the
-        TMA-loaded price planes), 2 = the queue with a warp
-        per tile, 3 = the CTA queue with prices formed per tile."""
+        tile, a warp per layer, packed labels, prices from the TMA-loaded price
+        planes), 2 = the queue with a warp per tile, 3 = the CTA queue with prices
+        formed per tile."""
         e = self.engine
         e._check(e.lib.mrc_batch_set_schedule(e.ctx, self.handle, int(schedule)))
 
